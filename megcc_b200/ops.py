@@ -16,11 +16,13 @@ ALGO = {"auto": 0, "direct": 1, "umma": 2, "patch": 3}
 
 
 def _stream():
-    return C.c_void_p(torch.cuda.current_stream().cuda_stream)
+    """The current CUDA stream of the current device, as an address. (torch.cuda.current_stream
+    wraps the same two look-ups in a Stream object, 3 us of every operator call against 0.15.)"""
+    return torch._C._cuda_getCurrentRawStream(torch._C._cuda_getDevice())
 
 
 def _ptr(t):
-    return None if t is None else C.c_void_p(t.data_ptr())
+    return None if t is None else t.data_ptr()
 
 
 def conv_param(n, ic, ih, iw, oc, kh, kw, stride, pad, groups, act, s_src, s_flt, s_dst,
@@ -54,7 +56,7 @@ def conv_bias_qs8_nhwc(p, src, flt_packed, bias, dst=None, flt_scales=None, algo
                        src_is_nchw=False):
     oh, ow = out_hw(p)
     if dst is None:
-        dst = torch.empty((p.n, oh, ow, p.oc), dtype=torch.int8, device=src.device)
+        dst = src.new_empty((p.n, oh, ow, p.oc))
     check(lib().mb200_conv_bias_qs8_nhwc(
         C.byref(p), _ptr(src), int(src_is_nchw), _ptr(flt_packed), _ptr(bias), _ptr(flt_scales),
         _ptr(dst), ALGO[algo], _stream()))
@@ -66,7 +68,7 @@ def conv_bias_qs8_nhwc_fused(p, src, flt_packed, bias, z, mode, z_scale, out_sca
     tensor z of the output's NHWC shape, in one kernel."""
     from ._lib import ConvFuse
     oh, ow = out_hw(p)
-    dst = torch.empty((p.n, oh, ow, p.oc), dtype=torch.int8, device=src.device)
+    dst = src.new_empty((p.n, oh, ow, p.oc))
     fuse = ConvFuse(z.data_ptr(), QELEM[mode], z_scale, out_scale)
     check(lib().mb200_conv_bias_qs8_nhwc_fused(
         C.byref(p), _ptr(src), 0, _ptr(flt_packed), _ptr(bias), None, C.byref(fuse), _ptr(dst),
@@ -85,9 +87,9 @@ def conv_acc_qs8_nhwc(p, src, flt_packed, bias):
 def conv_bias_qs8_nchw(p, src, flt_oihw, bias, flt_scales=None, algo="auto"):
     """ConvBias in the reference's own layouts (NCHW activations, OIHW filter)."""
     oh, ow = out_hw(p)
-    dst = torch.empty((p.n, p.oc, oh, ow), dtype=torch.int8, device=src.device)
+    dst = src.new_empty((p.n, p.oc, oh, ow))
     nbytes = lib().mb200_conv_bias_qs8_nchw_workspace(C.byref(p))
-    ws = torch.empty(nbytes + 256, dtype=torch.int8, device=src.device)
+    ws = src.new_empty(nbytes + 256)
     off = (-ws.data_ptr()) % 256
     check(lib().mb200_conv_bias_qs8_nchw(
         C.byref(p), _ptr(src), _ptr(flt_oihw), _ptr(bias), _ptr(flt_scales), _ptr(dst),
@@ -114,7 +116,7 @@ def matmul_s8_s32(a, b_packed):
 def matmul_s8_qs8(a, b_packed, acc_scale, dst_scale):
     m, k = a.shape
     n = b_packed.shape[0]
-    c = torch.empty((m, n), dtype=torch.int8, device=a.device)
+    c = a.new_empty((m, n))
     check(lib().mb200_matmul_s8_qs8(m, n, k, _ptr(a), _ptr(b_packed), _ptr(c), acc_scale,
                                     dst_scale, _stream()))
     return c
@@ -197,7 +199,9 @@ def conv_f32_param(n, ic, ih, iw, oc, kh, kw, stride, pad, groups=1, act="IDENTI
 
 
 def _scratch(nbytes, device):
-    """256-byte aligned device scratch of at least nbytes (None when nbytes == 0)."""
+    """256-byte aligned device scratch of at least nbytes (None when nbytes == 0), for kernels
+    of the current stream: torch hands freed memory out again in that stream's order only, so
+    the scratch may be dropped as soon as they are launched."""
     if nbytes == 0:
         return None, None
     buf = torch.empty(nbytes + 256, dtype=torch.int8, device=device)
@@ -221,8 +225,7 @@ def conv_bias_f32_nhwc(p, src, flt_packed, bias=None, z=None, dst=None, dst_pitc
     keep, ws = _scratch(nbytes, src.device)
     check(lib().mb200_conv_bias_f32_nhwc(
         C.byref(p), _ptr(src), _ptr(flt_packed), _ptr(bias), _ptr(z), _ptr(dst), dst_pitch,
-        None if ws is None else C.c_void_p(ws), nbytes, ALGO[algo], _stream()))
-    torch.cuda.current_stream().synchronize()  # the scratch must outlive the kernels
+        ws, nbytes, ALGO[algo], _stream()))
     return dst
 
 
@@ -233,12 +236,10 @@ def matmul_f32(a, b):
     packed = torch.empty(lib().mb200_matmul_f32_packed_b_bytes(k, n) // 4, dtype=torch.float32,
                          device=a.device)
     check(lib().mb200_matmul_f32_pack_b(k, n, _ptr(b), _ptr(packed), _stream()))
-    c = torch.empty((m, n), dtype=torch.float32, device=a.device)
+    c = a.new_empty((m, n))
     nbytes = lib().mb200_matmul_f32_workspace_bytes(m, k)
     keep, ws = _scratch(nbytes, a.device)
-    check(lib().mb200_matmul_f32(m, n, k, _ptr(a), _ptr(packed), _ptr(c),
-                                 None if ws is None else C.c_void_p(ws), nbytes, _stream()))
-    torch.cuda.current_stream().synchronize()
+    check(lib().mb200_matmul_f32(m, n, k, _ptr(a), _ptr(packed), _ptr(c), ws, nbytes, _stream()))
     return c
 
 
@@ -324,7 +325,7 @@ def conv_bias_qs8_s2d(p, src, flt_packed, bias, flt_scales=None, src_is_nchw=Tru
     """First-layer ConvBias (few input channels) through the space-to-depth form; flt_packed
     from mb200_conv_s2d_pack_filter or pack_filter_nchw44."""
     oh, ow = out_hw(p)
-    dst = torch.empty((p.n, oh, ow, p.oc), dtype=torch.int8, device=src.device)
+    dst = src.new_empty((p.n, oh, ow, p.oc))
     nbytes = lib().mb200_conv_s2d_workspace_bytes(C.byref(p))
     keep, ws = _scratch(nbytes, src.device)
     check(lib().mb200_conv_bias_qs8_s2d(
