@@ -30,15 +30,29 @@
 //   * filter: split once at load time (the Init step) into two K-major planes
 //     [2][OC][KH][KW][IC];
 //   * activation: fetched as it is by TMA (im2col, or tiled for a 1x1 filter) and split ON
-//     CHIP: four converter warps turn each arrived fp32 tile into its hi plane in place and
-//     its lo plane in the neighbouring slot of the stage. The split is elementwise and the
-//     TMA swizzle is a function of the shared-memory address, so both planes keep the layout
-//     the MMA descriptors expect; no pre-pass over global memory, no scratch tensor, and the
-//     input is read once instead of five times (read, two plane writes, two plane reads);
+//     CHIP: converter warps read each arrived fp32 tile, one pixel row per thread, and write its
+//     hi and lo planes into TENSOR MEMORY, from where the MMAs take their A operand. What
+//     bounds a tf32 contraction here is the SM's shared-memory port (128 bytes a clock): with
+//     both operands in shared memory a 128 x 128 x 32 step moves 192 KB through it (TMA
+//     writes, the converter's reads and its two plane writes, A and B reads of twelve MMAs),
+//     1536 clocks against 768 of tensor time. With A in tensor memory 112 KB are left;
+//   * accumulators. 128-column tiles: two main sets (segments alternate) and one correction
+//     set per tile. The corrections are 2^-11 of the main sum, so one chain over the whole
+//     tile is accurate enough, and the first correction MMA of a tile is issued behind the
+//     tile's first main MMAs so that the wait for the previous tile's corrections to be
+//     read is covered. 64 and 32 columns: main and correction columns lie side by side and
+//     one MMA over the filter's two planes (2 BN columns) computes hi * [hi | lo] of both, so a
+//     K step costs two instructions instead of three;
+//   * a filter that fits shared memory beside a ring of A tiles stays resident (one tile
+//     column, small K): the ring then carries activations only;
+//   * few tiles (a small batch): the K loop is split over the CTAs of a cluster (2, 4 or 8), each
+//     leaves its fp32 partial tile in its shared memory and finishes an equal share of the
+//     rows, summing the partials over distributed shared memory in rank order (the result
+//     does not depend on timing);
 //   * structure of the kernel as in conv_umma.cu: persistent CTAs, warp 0 TMA producer, warp 1
 //     MMA issuer and TMEM owner, warps 2..9 epilogue (tcgen05.ld -> + bias -> activation ->
-//     optional residual add -> 16-byte NHWC stores), warps 10..13 converters, two accumulator
-//     buffers, bounded waits.
+//     optional residual add -> NHWC stores), warps 10..13 or 10..17 converters (one or two groups
+//     of four), bounded waits.
 //
 // Replaces, for the fp32 configurations, the reference's im2col + 4x12 SIMD GEMM
 // (compiler/lib/KernelGen/GeneralIntrinsic/ConvKernel/Fp32Im2col.cpp:122-217,
@@ -49,6 +63,8 @@
 // 1e-4 relative / 1e-5 absolute, not bit for bit.
 #include <stdio.h>
 #include <stdlib.h>
+
+#include <type_traits>
 
 #include "f32_internal.h"
 #include "pdl.h"
@@ -62,7 +78,7 @@ using namespace umma;
 namespace {
 
 constexpr int kBM = 128;
-constexpr int kMaxStages = 6;
+constexpr int kMaxStages = 8;
 
 // kind::tf32 instruction descriptor: fp32 accumulate, tf32 A and B, both K-major
 __host__ __device__ constexpr uint32_t umma_idesc_tf32(int m, int n) {
@@ -70,24 +86,28 @@ __host__ __device__ constexpr uint32_t umma_idesc_tf32(int m, int n) {
            ((uint32_t)(m >> 4) << 24);
 }
 
-template <bool ACCUMULATE>
-__device__ __forceinline__ void umma_tf32_c(
-        uint32_t tmem_d, uint64_t adesc, uint64_t bdesc, uint32_t idesc) {
+// A operand (fp32 bits, 10 mantissa bits used) in tensor memory, B in shared memory (descriptor as
+// its two words); issued by the lane whose `leader` is non-zero
+__device__ __forceinline__ void umma_tf32_ta(
+        uint32_t leader, uint32_t tmem_d, uint32_t tmem_a, uint32_t b_lo, uint32_t b_hi,
+        uint32_t idesc, uint32_t accumulate) {
     asm volatile(
-            "{\n\t.reg .pred p;\n\t"
-            "setp.ne.b32 p, %4, 0;\n\t"
-            "tcgen05.mma.cta_group::1.kind::tf32 [%0], %1, %2, %3, p;\n\t}" ::"r"(tmem_d),
-            "l"(adesc), "l"(bdesc), "r"(idesc), "n"(ACCUMULATE ? 1 : 0)
+            "{\n\t.reg .pred p, q;\n\t.reg .b64 d;\n\t"
+            "mov.b64 d, {%2, %3};\n\t"
+            "setp.ne.b32 p, %5, 0;\n\tsetp.ne.b32 q, %6, 0;\n\t"
+            "@q tcgen05.mma.cta_group::1.kind::tf32 [%0], [%1], d, %4, p;\n\t}" ::"r"(tmem_d),
+            "r"(tmem_a), "r"(b_lo), "r"(b_hi), "r"(idesc), "r"(accumulate), "r"(leader)
             : "memory");
 }
 
-__device__ __forceinline__ void umma_tf32(
-        uint32_t tmem_d, uint64_t adesc, uint64_t bdesc, uint32_t idesc, uint32_t accumulate) {
+// 16 columns of this warp's 32 TMEM lanes <- registers (complete after tcgen05.wait::st)
+__device__ __forceinline__ void tmem_st16(uint32_t taddr, const uint32_t (&v)[16]) {
     asm volatile(
-            "{\n\t.reg .pred p;\n\t"
-            "setp.ne.b32 p, %4, 0;\n\t"
-            "tcgen05.mma.cta_group::1.kind::tf32 [%0], %1, %2, %3, p;\n\t}" ::"r"(tmem_d),
-            "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate)
+            "tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], "
+            "{%1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, %16};" ::"r"(taddr),
+            "r"(v[0]), "r"(v[1]), "r"(v[2]), "r"(v[3]), "r"(v[4]), "r"(v[5]), "r"(v[6]), "r"(v[7]),
+            "r"(v[8]), "r"(v[9]), "r"(v[10]), "r"(v[11]), "r"(v[12]), "r"(v[13]), "r"(v[14]),
+            "r"(v[15])
             : "memory");
 }
 
@@ -104,7 +124,9 @@ __host__ __device__ inline float round_tf32(float v) {
 // ------------------------------------------------------------------------------------------
 // filter packing (load time)
 // ------------------------------------------------------------------------------------------
-// OIHW fp32 -> two K-major planes [2][OC][KH][KW][ICp] (hi, lo), ICp >= IC zero-filled
+// OIHW fp32 -> two K-major planes [2][OC][KH][KW][ICp] (hi, lo), ICp >= IC zero-filled. The lo
+// plane holds the exact remainder (12 significant bits, the tensor core reads 11), so that
+// hi + lo gives the weight back to the CUDA-core kernel.
 __global__ void __launch_bounds__(256) pack_filter_f32_kernel(
         const float* __restrict__ src, float* __restrict__ dst, int oc, int ic, int icp, int kh,
         int kw) {
@@ -122,7 +144,33 @@ __global__ void __launch_bounds__(256) pack_filter_f32_kernel(
             v = src[(((size_t)o * ic + c) * kh + fy) * kw + fx];
         const float h = round_tf32(v);
         dst[i] = h;
-        dst[plane + i] = round_tf32(__fsub_rn(v, h));
+        dst[plane + i] = __fsub_rn(v, h);
+    }
+}
+
+// [K][N] fp32 (the second operand of a matrix product) -> the same two planes [2][N][Kp] in one
+// pass: a 32 x 32 tile through shared memory, rows of 128 bytes read and written. Bound by HBM:
+// 12 bytes per element.
+__global__ void __launch_bounds__(256) pack_matrix_f32_kernel(
+        const float* __restrict__ src, float* __restrict__ dst, int k, int n, int kp) {
+    __shared__ float tile[32][33];
+    const int n0 = blockIdx.x * 32, k0 = blockIdx.y * 32;
+    const size_t plane = (size_t)n * kp;
+#pragma unroll
+    for (int j = threadIdx.y; j < 32; j += 8) {
+        const int r = k0 + j, c = n0 + threadIdx.x;
+        tile[j][threadIdx.x] = r < k && c < n ? __ldg(src + (size_t)r * n + c) : 0.f;
+    }
+    __syncthreads();
+#pragma unroll
+    for (int j = threadIdx.y; j < 32; j += 8) {
+        const int c = n0 + j, r = k0 + threadIdx.x;
+        if (c < n && r < kp) {
+            const float v = tile[threadIdx.x][j];
+            const float h = round_tf32(v);
+            dst[(size_t)c * kp + r] = h;
+            dst[plane + (size_t)c * kp + r] = __fsub_rn(v, h);
+        }
     }
 }
 
@@ -138,60 +186,97 @@ struct F32Epilogue {
     long long dst_pitch;  // floats between consecutive pixels of dst (>= oc)
 };
 
-__device__ __forceinline__ float act_f32(int act, float x) {
+template <int ACT>
+__device__ __forceinline__ float act_f32(float x) {
+    if (ACT == MB200_F32_RELU)
+        return x > 0.f ? x : 0.f;
+    if (ACT == MB200_F32_SIGMOID)
+        return __fdividef(1.f, 1.f + __expf(-x));
+    if (ACT == MB200_F32_SILU)
+        return __fdividef(x, 1.f + __expf(-x));
+    if (ACT == MB200_F32_H_SWISH) {
+        float t = x + 3.f;
+        t = t > 0.f ? t : 0.f;
+        t = t > 6.f ? 6.f : t;
+        return x * t * (1.f / 6.f);
+    }
+    return x;
+}
+
+// Calls f with the activation as a compile-time constant. The choice is made once per tile and
+// warp: made per element (a run-time switch inside the unrolled loops) it serialised the
+// elements, 250 clocks each, and the epilogue was the kernel's longest chain.
+template <class F>
+__device__ __forceinline__ void with_act(int act, F&& f) {
     switch (act) {
-        case MB200_F32_RELU:
-            return x > 0.f ? x : 0.f;
-        case MB200_F32_SIGMOID:
-            return __fdividef(1.f, 1.f + __expf(-x));
-        case MB200_F32_SILU:
-            return __fdividef(x, 1.f + __expf(-x));
-        case MB200_F32_H_SWISH: {
-            float t = x + 3.f;
-            t = t > 0.f ? t : 0.f;
-            t = t > 6.f ? 6.f : t;
-            return x * t * (1.f / 6.f);
-        }
-        default:
-            return x;
+        case MB200_F32_RELU: f(std::integral_constant<int, MB200_F32_RELU>()); break;
+        case MB200_F32_SIGMOID: f(std::integral_constant<int, MB200_F32_SIGMOID>()); break;
+        case MB200_F32_SILU: f(std::integral_constant<int, MB200_F32_SILU>()); break;
+        case MB200_F32_H_SWISH: f(std::integral_constant<int, MB200_F32_H_SWISH>()); break;
+        default: f(std::integral_constant<int, MB200_F32_IDENTITY>()); break;
     }
 }
 
-// 32 consecutive channels (from ch0) of pixel `m`
-__device__ __forceinline__ void store_f32_chunk(
-        const float (&v)[32], const F32Epilogue& e, size_t m, int ch0) {
+// NC consecutive channels (from ch0) of pixel `m`
+template <int NC, int ACT>
+__device__ __forceinline__ void store_f32_chunk_t(
+        const float (&v)[NC], const F32Epilogue& e, size_t m, int ch0) {
     float* out = e.dst + m * e.dst_pitch + ch0;
     const float* zin = e.z ? e.z + m * e.z_pitch + ch0 : nullptr;
-    const bool vec = ch0 + 32 <= e.oc && (((uintptr_t)out | (uintptr_t)zin) & 15) == 0 &&
+    const bool vec = ch0 + NC <= e.oc && (((uintptr_t)out | (uintptr_t)zin) & 15) == 0 &&
                      (!e.bias || ((uintptr_t)(e.bias + ch0) & 15) == 0);
     if (vec) {
+        // a thread's channels are whole 32-byte sectors when the pixel starts on one: 256-bit
+        // stores, so that no sector is written in two halves
+        const bool sector = ((uintptr_t)out & 31) == 0;
 #pragma unroll
-        for (int j = 0; j < 8; ++j) {
-            float4 b = make_float4(0.f, 0.f, 0.f, 0.f);
-            if (e.bias)
-                b = __ldg(reinterpret_cast<const float4*>(e.bias + ch0) + j);
-            float4 r;
-            r.x = act_f32(e.act, v[4 * j + 0] + b.x);
-            r.y = act_f32(e.act, v[4 * j + 1] + b.y);
-            r.z = act_f32(e.act, v[4 * j + 2] + b.z);
-            r.w = act_f32(e.act, v[4 * j + 3] + b.w);
-            if (zin) {
-                const float4 zz = __ldg(reinterpret_cast<const float4*>(zin) + j);
-                r.x += zz.x; r.y += zz.y; r.z += zz.z; r.w += zz.w;
+        for (int j = 0; j < NC / 8; ++j) {
+            float r[8];
+#pragma unroll
+            for (int h = 0; h < 2; ++h) {
+                float4 b = make_float4(0.f, 0.f, 0.f, 0.f);
+                if (e.bias)
+                    b = __ldg(reinterpret_cast<const float4*>(e.bias + ch0) + 2 * j + h);
+                r[4 * h + 0] = act_f32<ACT>(v[8 * j + 4 * h + 0] + b.x);
+                r[4 * h + 1] = act_f32<ACT>(v[8 * j + 4 * h + 1] + b.y);
+                r[4 * h + 2] = act_f32<ACT>(v[8 * j + 4 * h + 2] + b.z);
+                r[4 * h + 3] = act_f32<ACT>(v[8 * j + 4 * h + 3] + b.w);
+                if (zin) {
+                    const float4 zz = *(reinterpret_cast<const float4*>(zin) + 2 * j + h);
+                    r[4 * h + 0] += zz.x;
+                    r[4 * h + 1] += zz.y;
+                    r[4 * h + 2] += zz.z;
+                    r[4 * h + 3] += zz.w;
+                }
             }
-            reinterpret_cast<float4*>(out)[j] = r;
+            if (sector) {
+                asm volatile("st.global.v8.f32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"l"(
+                                     out + 8 * j),
+                             "f"(r[0]), "f"(r[1]), "f"(r[2]), "f"(r[3]), "f"(r[4]), "f"(r[5]),
+                             "f"(r[6]), "f"(r[7])
+                             : "memory");
+            } else {
+                reinterpret_cast<float4*>(out)[2 * j] = make_float4(r[0], r[1], r[2], r[3]);
+                reinterpret_cast<float4*>(out)[2 * j + 1] = make_float4(r[4], r[5], r[6], r[7]);
+            }
         }
     } else {
 #pragma unroll
-        for (int i = 0; i < 32; ++i) {
+        for (int i = 0; i < NC; ++i) {
             if (ch0 + i < e.oc) {
-                float r = act_f32(e.act, v[i] + (e.bias ? e.bias[ch0 + i] : 0.f));
+                float r = act_f32<ACT>(v[i] + (e.bias ? e.bias[ch0 + i] : 0.f));
                 if (zin)
                     r += zin[i];
                 out[i] = r;
             }
         }
     }
+}
+
+template <int NC>
+__device__ __forceinline__ void store_f32_chunk(
+        const float (&v)[NC], const F32Epilogue& e, size_t m, int ch0) {
+    with_act(e.act, [&](auto a) { store_f32_chunk_t<NC, decltype(a)::value>(v, e, m, ch0); });
 }
 
 // ------------------------------------------------------------------------------------------
@@ -202,77 +287,118 @@ struct F32ConvParams {
     int cblocks;  // row-sized channel blocks per tap
     int taps_w;
     int k_iters;
-    int seg_iters;  // pipeline steps per accumulation segment
     int sh, sw, base_h, base_w;
     int m_tiles, n_tiles;
     int a_tiled;      // 1x1, stride 1, no padding: A is the plain matrix [pixels][channels]
     int b_lo_offset;  // rows from the hi plane to the lo plane of the filter
+    int stages;       // depth of the shared-memory ring
+    int b_resident;   // 1: the whole filter sits in front of the ring, stages hold A only
+    int splits;       // CTAs of a cluster that share a tile's K loop (1: none)
     F32Epilogue ep;
     int* status;
     long long wait_cycles;
 };
 
 template <int BN, int ROWB>
-struct F32Smem {
-    static constexpr int kStages = ROWB == 128 ? (BN == 128 ? 3 : 4) : 6;
+struct F32Cfg {
+    static constexpr int kChans = ROWB / 4;  // floats per row = TMEM columns of an A plane
+    static constexpr bool kWide = BN == 128;
+    static constexpr int kAccCols = kWide ? 3 * BN : 4 * BN;
+    static constexpr int kTRaw = (512 - kAccCols) / (2 * kChans);
+    static constexpr int kTStages = kTRaw > 4 ? 4 : kTRaw;  // A stages in tensor memory
+    static_assert(kTStages == 2 || kTStages == 4, "a whole number of turns of the converter groups");
+    static constexpr int kSegIters = 256 / ROWB;  // stages per segment: eight K = 8 steps
     static constexpr int kABytes = kBM * ROWB;
-    static constexpr int kBBytes = BN * ROWB;
-    static constexpr int kStageBytes = 2 * kABytes + 2 * kBBytes;
-    static constexpr int kTiles = kStages * kStageBytes;
-    static constexpr int kBarOff = kTiles;
-    static constexpr int kTotal = kBarOff + (3 * kMaxStages + 5) * 8 + 16;
-    static constexpr int kDynamic = kTotal + 1024;
+    static constexpr int kBBytes = 2 * BN * ROWB;  // both planes of a filter tile
+    static constexpr int kBarBytes = 1024;         // barriers, in front of the tiles
+    static constexpr int kPartPitch = BN + 4;      // floats per row of a split part's tile
 };
 
-// Eight epilogue warps (two 32-column chunks each for BN = 128). Sixteen, one chunk each,
-// halve a warp's chain of dependent TMEM loads per hand-over, but measured no faster on the
-// ConvBias layers and 10 % slower on the 4096^3 MatrixMul.
-__host__ __device__ constexpr int f32_epilogue_warps(int bn) { return bn >= 64 ? 8 : 8; }
-constexpr int kF32ConvertWarps = 4;
-__host__ __device__ constexpr int f32_threads(int bn) { return 64 + 32 * f32_epilogue_warps(bn) + 32 * kF32ConvertWarps; }
+// Eight epilogue warps, and one converter group of four warps for 128 columns (its epilogue holds
+// 64 sums per thread: with 14 warps in the block a thread may have 128 registers), two groups
+// that take turns for the narrower tiles, whose steps are shorter.
+constexpr int kF32EpilogueWarps = 8;
+__host__ __device__ constexpr int f32_groups(int bn) { return bn == 128 ? 1 : 2; }
+__host__ __device__ constexpr int f32_threads(int bn) {
+    return 64 + 32 * kF32EpilogueWarps + 128 * f32_groups(bn);
+}
 
-// v = hi + lo with both halves exact tf32 values (which way a tie rounds does not matter:
-// v - hi is exact, and lo is its nearest tf32)
-__device__ __forceinline__ void split_tf32(float v, float& hi, float& lo) {
-    uint32_t h, l;
-    asm("cvt.rna.tf32.f32 %0, %1;" : "=r"(h) : "f"(v));
-    hi = __uint_as_float(h);
-    asm("cvt.rna.tf32.f32 %0, %1;" : "=r"(l) : "f"(__fsub_rn(v, hi)));
-    lo = __uint_as_float(l);
+// v = hi + lo: hi is v rounded to a tf32 value (ties away from zero), v - hi is exact and has
+// at most 12 significant bits, of which the tensor core reads 11. Integer rounding: the
+// conversion instruction runs at a fifth of the rate.
+__device__ __forceinline__ void split_tf32(uint32_t v, uint32_t& hi, uint32_t& lo) {
+    hi = (v + 0x1000u) & 0xFFFFE000u;
+    lo = __float_as_uint(__fsub_rn(__uint_as_float(v), __uint_as_float(hi)));
+}
+
+__device__ __forceinline__ uint32_t f32_cluster_rank() {
+    uint32_t r;
+    asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
+    return r;
+}
+__device__ __forceinline__ void f32_cluster_sync() {
+    asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+    asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
 
 template <int BN, int ROWB>
 __global__ void __launch_bounds__(f32_threads(BN), 1) conv_f32_umma_kernel(
         const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b,
         const F32ConvParams p) {
-    using L = F32Smem<BN, ROWB>;
-    constexpr int kSt = L::kStages;
-    constexpr int kChans = ROWB / 4;  // floats per row
-    constexpr int kF32EpilogueWarps = f32_epilogue_warps(BN);
+    using C = F32Cfg<BN, ROWB>;
+    constexpr int kChans = C::kChans;
+    constexpr int kT = C::kTStages;
+    constexpr int kTmemA = C::kAccCols;  // first column of the A stages
     extern __shared__ uint8_t smem_raw[];
     uint8_t* smem = (uint8_t*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
-    uint64_t* full_bar = (uint64_t*)(smem + L::kBarOff);
-    uint64_t* empty_bar = full_bar + kMaxStages;
-    uint64_t* conv_bar = empty_bar + kMaxStages;  // the stage's A tile is split: MMAs may read it
-    uint64_t* acc_full = conv_bar + kMaxStages;  // [2]
-    uint64_t* acc_empty = acc_full + 2;           // [2]
-    uint64_t* drain_bar = acc_empty + 2;
+    uint64_t* full_bar = (uint64_t*)smem;             // [kMaxStages] TMA -> converters, MMA
+    uint64_t* empty_bar = full_bar + kMaxStages;      // [kMaxStages]
+    uint64_t* t_full = empty_bar + kMaxStages;        // [kT] converters -> MMA
+    uint64_t* t_empty = t_full + 4;                   // [kT]
+    uint64_t* acc_full = t_empty + 4;                 // [2]
+    uint64_t* acc_empty = acc_full + 2;               // [2]
+    uint64_t* corr_empty = acc_empty + 2;
+    uint64_t* b_full = corr_empty + 1;
+    uint64_t* drain_bar = b_full + 1;
     uint32_t* tmem_slot = (uint32_t*)(drain_bar + 1);
     volatile int* abort_flag = (volatile int*)(tmem_slot + 1);
+    uint8_t* tiles = smem + C::kBarBytes;
+    uint8_t* tiles_b = tiles;  // resident filter (if any), then the ring
+    uint8_t* ring = tiles + (p.b_resident ? p.k_iters * C::kBBytes : 0);
+    const int stage_bytes = C::kABytes + (p.b_resident ? 0 : C::kBBytes);
 
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int warp = uniform_warp_index(), lane = threadIdx.x & 31;
     const int total_tiles = p.m_tiles * p.n_tiles;
+    // Work of this CTA. Split: one tile per cluster, a K range per CTA; else whole tiles, one
+    // every gridDim.x.
+    const int rank = p.splits > 1 ? (int)f32_cluster_rank() : 0;
+    const int first_tile = (int)blockIdx.x / p.splits;
+    const int tile_step = p.splits > 1 ? total_tiles : (int)gridDim.x;
+    const int my_tiles =
+            first_tile < total_tiles ? (total_tiles - 1 - first_tile) / tile_step + 1 : 0;
+    int kb = 0, ke = p.k_iters;
+    if (p.splits > 1) {
+        kb = (int)((long long)p.k_iters * rank / p.splits);
+        ke = (int)((long long)p.k_iters * (rank + 1) / p.splits);
+    }
 
     if (threadIdx.x == 0) {
         for (int s = 0; s < kMaxStages; ++s) {
             mbar_init(&full_bar[s], 1);
-            mbar_init(&empty_bar[s], 1);
-            mbar_init(&conv_bar[s], 32 * kF32ConvertWarps);
+            // with a resident filter a stage is free once its converters have read it
+            // (128 arrivals), otherwise once one of them has seen that the MMAs over it retired
+            mbar_init(&empty_bar[s], p.b_resident ? 128 : 1);
+        }
+        for (int t = 0; t < kT; ++t) {
+            mbar_init(&t_full[t], 128);
+            mbar_init(&t_empty[t], 1);
         }
         for (int b = 0; b < 2; ++b) {
             mbar_init(&acc_full[b], 1);
             mbar_init(&acc_empty[b], 32 * kF32EpilogueWarps);
         }
+        mbar_init(corr_empty, 32 * kF32EpilogueWarps);
+        mbar_init(b_full, 1);
         mbar_init(drain_bar, 1);
         *abort_flag = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -281,7 +407,7 @@ __global__ void __launch_bounds__(f32_threads(BN), 1) conv_f32_umma_kernel(
         asm volatile(
                 "tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(
                         smem_u32(tmem_slot)),
-                "r"(4 * BN)
+                "r"(512)
                 : "memory");
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
     }
@@ -291,13 +417,29 @@ __global__ void __launch_bounds__(f32_threads(BN), 1) conv_f32_umma_kernel(
     const uint32_t tmem_base = *tmem_slot;
     pdl_start();  // set-up done: from here on the kernel touches global memory
 
+    auto give_up = [&](int code) {
+        if (!*abort_flag) {
+            *abort_flag = 1;
+            atomicExch(p.status, code);
+        }
+    };
+
     if (warp == 0) {
         // ---------------- TMA producer ----------------
         if (lane == 0) {
+            if (p.b_resident) {
+                mbar_expect_tx(b_full, (uint32_t)(p.k_iters * C::kBBytes));
+                for (int it = 0; it < p.k_iters; ++it) {
+                    uint8_t* b = tiles_b + it * C::kBBytes;
+                    tma_load_2d(b, &map_b, b_full, it * kChans, 0);
+                    tma_load_2d(b + C::kBBytes / 2, &map_b, b_full, it * kChans, p.b_lo_offset);
+                }
+            }
+            const uint32_t tx = (uint32_t)stage_bytes;
             int s = 0;
             uint32_t phase = 0;
             bool ok = true;
-            for (int tile = blockIdx.x; tile < total_tiles && ok; tile += gridDim.x) {
+            for (int tile = first_tile; tile < total_tiles && ok; tile += tile_step) {
                 const int tile_n = tile % p.n_tiles, tile_m = tile / p.n_tiles;
                 const int m0 = tile_m * kBM, n0 = tile_n * BN;
                 const int img = m0 / (p.oh * p.ow);
@@ -305,28 +447,31 @@ __global__ void __launch_bounds__(f32_threads(BN), 1) conv_f32_umma_kernel(
                 const int oy = rem / p.ow, ox = rem - oy * p.ow;
                 const int base_w = ox * p.sw + p.base_w, base_h = oy * p.sh + p.base_h;
                 int cb = 0, fx = 0, fy = 0;
-                for (int it = 0; it < p.k_iters; ++it) {
+                if (kb != 0) {  // a later part of a split tile starts inside the filter
+                    const int tap = kb / p.cblocks;
+                    cb = kb - tap * p.cblocks;
+                    fy = tap / p.taps_w;
+                    fx = tap - fy * p.taps_w;
+                }
+                for (int it = kb; it < ke; ++it) {
                     if (!mbar_wait(&empty_bar[s], phase ^ 1u, abort_flag, p.wait_cycles)) {
-                        if (!*abort_flag) {
-                            *abort_flag = 1;
-                            atomicExch(p.status, ERR_PRODUCER_WAIT);
-                        }
+                        give_up(ERR_PRODUCER_WAIT);
                         ok = false;
                         break;
                     }
-                    // the fp32 A tile lands in the hi slot; the lo slot is filled on chip
-                    mbar_expect_tx(&full_bar[s], (uint32_t)(L::kABytes + 2 * L::kBBytes));
-                    uint8_t* a_hi = smem + s * L::kStageBytes;
-                    uint8_t* a_lo = a_hi + L::kABytes;
-                    uint8_t* b_hi = a_lo + L::kABytes;
-                    uint8_t* b_lo = b_hi + L::kBBytes;
+                    mbar_expect_tx(&full_bar[s], tx);
+                    uint8_t* a = ring + s * stage_bytes;
                     if (p.a_tiled)
-                        tma_load_2d(a_hi, &map_a, &full_bar[s], cb * kChans, m0);
+                        tma_load_2d(a, &map_a, &full_bar[s], cb * kChans, m0);
                     else
-                        tma_load_im2col_4d(a_hi, &map_a, &full_bar[s], cb * kChans, base_w, base_h,
+                        tma_load_im2col_4d(a, &map_a, &full_bar[s], cb * kChans, base_w, base_h,
                                            img, (uint16_t)fx, (uint16_t)fy);
-                    tma_load_2d(b_hi, &map_b, &full_bar[s], it * kChans, n0);
-                    tma_load_2d(b_lo, &map_b, &full_bar[s], it * kChans, n0 + p.b_lo_offset);
+                    if (!p.b_resident) {
+                        uint8_t* b = a + C::kABytes;
+                        tma_load_2d(b, &map_b, &full_bar[s], it * kChans, n0);
+                        tma_load_2d(b + C::kBBytes / 2, &map_b, &full_bar[s], it * kChans,
+                                    n0 + p.b_lo_offset);
+                    }
                     if (++cb == p.cblocks) {
                         cb = 0;
                         if (++fx == p.taps_w) {
@@ -334,7 +479,7 @@ __global__ void __launch_bounds__(f32_threads(BN), 1) conv_f32_umma_kernel(
                             ++fy;
                         }
                     }
-                    if (++s == kSt) {
+                    if (++s == p.stages) {
                         s = 0;
                         phase ^= 1u;
                     }
@@ -342,113 +487,179 @@ __global__ void __launch_bounds__(f32_threads(BN), 1) conv_f32_umma_kernel(
             }
         }
     } else if (warp == 1) {
-        // ---------------- MMA issuer ----------------
-        if (lane == 0) {
-            constexpr uint32_t idesc = umma_idesc_tf32(kBM, BN);
-            // swizzled K-major tiles: 8-row groups 8 * ROWB bytes apart
-            constexpr uint32_t kLayout = ROWB == 128 ? 2u : 4u;
-            constexpr uint32_t kSbo = 8 * ROWB;
-            int local = 0, s = 0;  // `local` counts accumulation segments
-            uint32_t phase = 0;
-            bool ok = true;
-            for (int tile = blockIdx.x; tile < total_tiles && ok; tile += gridDim.x) {
-                for (int k0 = 0; k0 < p.k_iters && ok; k0 += p.seg_iters, ++local) {
-                    const int k1 = min(k0 + p.seg_iters, p.k_iters);
-                    const int buf = local & 1;
-                    const uint32_t acc_phase = (uint32_t)(local >> 1) & 1u;
-                    if (!mbar_wait(&acc_empty[buf], acc_phase ^ 1u, abort_flag, p.wait_cycles)) {
-                        if (!*abort_flag) {
-                            *abort_flag = 1;
-                            atomicExch(p.status, ERR_MMA_ACC_WAIT);
-                        }
-                        ok = false;
-                        break;
-                    }
-                    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-                    // main sum (hi * hi) and correction sum (lo * hi + hi * lo) of this set
-                    const uint32_t tmem_d = tmem_base + (uint32_t)(buf * 2 * BN);
-                    const uint32_t tmem_c = tmem_d + (uint32_t)BN;
-                    for (int it = k0; it < k1; ++it) {
-                        if (!mbar_wait(&conv_bar[s], phase, abort_flag, p.wait_cycles)) {
-                            if (!*abort_flag) {
-                                *abort_flag = 1;
-                                atomicExch(p.status, ERR_MMA_WAIT);
-                            }
-                            ok = false;
-                            break;
-                        }
-                        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-                        const uint32_t a_addr = smem_u32(smem + s * L::kStageBytes);
-                        const uint64_t a_hi = umma_smem_desc(a_addr, 16, kSbo, kLayout);
-                        const uint64_t a_lo =
-                                umma_smem_desc(a_addr + L::kABytes, 16, kSbo, kLayout);
-                        const uint64_t b_hi =
-                                umma_smem_desc(a_addr + 2 * L::kABytes, 16, kSbo, kLayout);
-                        const uint64_t b_lo = umma_smem_desc(
-                                a_addr + 2 * L::kABytes + L::kBBytes, 16, kSbo, kLayout);
-                        // a K step of 8 floats is 32 bytes inside the swizzled row: +2 in the
-                        // descriptor's 16-byte address units
-                        const uint32_t acc = it != k0 ? 1u : 0u;
-                        umma_tf32(tmem_c, a_lo, b_hi, idesc, acc);
-                        umma_tf32_c<true>(tmem_c, a_hi, b_lo, idesc);
-                        umma_tf32(tmem_d, a_hi, b_hi, idesc, acc);
-#pragma unroll
-                        for (int k = 1; k < ROWB / 32; ++k) {
-                            umma_tf32_c<true>(tmem_c, a_lo + 2 * k, b_hi + 2 * k, idesc);
-                            umma_tf32_c<true>(tmem_c, a_hi + 2 * k, b_lo + 2 * k, idesc);
-                            umma_tf32_c<true>(tmem_d, a_hi + 2 * k, b_hi + 2 * k, idesc);
-                        }
-                        umma_commit(&empty_bar[s]);
-                        if (++s == kSt) {
-                            s = 0;
-                            phase ^= 1u;
-                        }
-                    }
-                    if (ok)
-                        umma_commit(&acc_full[buf]);
-                }
-            }
-        }
-    } else if (warp >= 2 + kF32EpilogueWarps) {
-        // ---------------- converters: fp32 A tile -> hi (in place) and lo planes ----------------
-        const int ct = (int)threadIdx.x - (64 + 32 * kF32EpilogueWarps);
-        constexpr int kVecs = L::kABytes / 16;
-        constexpr int kPerThread = kVecs / (32 * kF32ConvertWarps);
-        static_assert(kVecs % (32 * kF32ConvertWarps) == 0, "whole vectors per converter thread");
-        int s = 0;
-        uint32_t phase = 0;
-        bool ok = true;
-        for (int tile = blockIdx.x; tile < total_tiles && ok; tile += gridDim.x) {
-            for (int it = 0; it < p.k_iters; ++it) {
-                ok = mbar_wait(&full_bar[s], phase, abort_flag, p.wait_cycles);
-                if (!ok && !*abort_flag) {
-                    *abort_flag = 1;
-                    atomicExch(p.status, ERR_PRODUCER_WAIT);
-                }
-                ok = __all_sync(0xffffffffu, ok);
+        // ---------------- MMA issuer (the whole warp waits, one lane issues) ----------------
+        // The tensor pipe holds only a few MMAs beyond the one it executes, so every instruction
+        // of this loop that is not an MMA shows as idle tensor time (a lone warp takes four to
+        // six clocks for each). Hence: one segment per trip with its steps unrolled, descriptor
+        // words and TMEM columns as running sums, one wait and one commit per step. The wait
+        // for the converters covers the filter tile of the step too: they have waited for the
+        // stage's TMA barrier before they arrived.
+        const uint32_t leader = elect_one() ? 1u : 0u;
+        constexpr uint32_t idesc = umma_idesc_tf32(kBM, BN);
+        constexpr uint32_t idesc2 = umma_idesc_tf32(kBM, C::kWide ? BN : 2 * BN);
+        // swizzled K-major tiles: 8-row groups 8 * ROWB bytes apart
+        constexpr uint64_t kDesc = ((uint64_t)1 << 16) | ((uint64_t)(8 * ROWB / 16) << 32) |
+                                   ((uint64_t)1 << 46) | ((uint64_t)(ROWB == 128 ? 2 : 4) << 61);
+        constexpr uint32_t kDescHi = (uint32_t)(kDesc >> 32);
+        constexpr int kSteps = ROWB / 32;          // K = 8 steps per stage
+        constexpr int kSeg = C::kSegIters;         // stages per segment
+        constexpr uint32_t kPlane = C::kBBytes / 2 / 16;
+        const uint32_t t_full_a = smem_u32(t_full), t_empty_a = smem_u32(t_empty);
+        const uint32_t acc_full_a = smem_u32(acc_full), acc_empty_a = smem_u32(acc_empty);
+        const int k_len = ke - kb;
+        // where the filter tiles lie: the ring's slots, or the resident filter's steps
+        const int slots = p.b_resident ? k_len : p.stages;
+        const uint32_t slot_step = (uint32_t)(p.b_resident ? C::kBBytes : stage_bytes) >> 4;
+        const uint32_t b_first =
+                (((p.b_resident ? smem_u32(tiles_b) : smem_u32(ring) + C::kABytes) & 0x3FFFFu) >> 4) |
+                (uint32_t)kDesc;
+        uint32_t b_lo = b_first;
+        int slot = 0, t = 0;
+        uint32_t t_parity = 0, tile_parity = 0, buf = 0, acc_parity = 1;
+        bool ok = !p.b_resident || mbar_wait(b_full, 0, abort_flag, p.wait_cycles);
+        for (int tile = 0; tile < my_tiles && ok; ++tile) {
+            for (int left = k_len; left > 0; left -= kSeg) {
+                ok = mbar_wait_u32(acc_empty_a + 8 * buf, acc_parity, abort_flag, p.wait_cycles);
                 if (!ok)
                     break;
-                float4* hi = reinterpret_cast<float4*>(smem + s * L::kStageBytes);
-                float4* lo = hi + kVecs;
+                const uint32_t tmem_d = tmem_base + buf * (C::kWide ? BN : 2 * BN);
+                const uint32_t tmem_c = C::kWide ? tmem_base + 2 * BN : tmem_d + (uint32_t)BN;
 #pragma unroll
-                for (int j = 0; j < kPerThread; ++j) {
-                    const int idx = ct + j * 32 * kF32ConvertWarps;
-                    const float4 v = hi[idx];
-                    float4 h, l;
-                    split_tf32(v.x, h.x, l.x);
-                    split_tf32(v.y, h.y, l.y);
-                    split_tf32(v.z, h.z, l.z);
-                    split_tf32(v.w, h.w, l.w);
-                    hi[idx] = h;
-                    lo[idx] = l;
+                for (int j = 0; j < kSeg; ++j) {
+                    if (j == 0 || j < left) {
+                        ok = mbar_wait_u32(t_full_a + 8 * t, t_parity, abort_flag, p.wait_cycles);
+                        if (!ok)
+                            break;
+                        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+                        const uint32_t a_hi = tmem_base + kTmemA + (uint32_t)(t * 2 * kChans);
+                        const uint32_t a_lo = a_hi + kChans;
+                        // a K step of 8 floats: 8 columns of A, 32 bytes inside B's swizzled row
+                        // (+2 in the descriptor's 16-byte address units)
+                        if constexpr (C::kWide) {
+#pragma unroll
+                            for (int k = 0; k < kSteps; ++k)
+                                umma_tf32_ta(leader, tmem_d, a_hi + 8 * k, b_lo + 2 * k, kDescHi,
+                                             idesc, (j | k) != 0);
+                            if (j == 0 && left == k_len) {
+                                // the previous tile's corrections must have been read
+                                ok = mbar_wait(corr_empty, tile_parity ^ 1u, abort_flag,
+                                               p.wait_cycles);
+                                if (!ok)
+                                    break;
+                                asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+                            }
+#pragma unroll
+                            for (int k = 0; k < kSteps; ++k) {
+                                umma_tf32_ta(leader, tmem_c, a_lo + 8 * k, b_lo + 2 * k, kDescHi,
+                                             idesc, (j | k) != 0 ? 1u : (left != k_len ? 1u : 0u));
+                                umma_tf32_ta(leader, tmem_c, a_hi + 8 * k, b_lo + kPlane + 2 * k,
+                                             kDescHi, idesc, 1);
+                            }
+                        } else {
+                            // [main | correction] += hi * [hi | lo], correction += lo * hi
+#pragma unroll
+                            for (int k = 0; k < kSteps; ++k) {
+                                umma_tf32_ta(leader, tmem_d, a_hi + 8 * k, b_lo + 2 * k, kDescHi,
+                                             idesc2, (j | k) != 0);
+                                umma_tf32_ta(leader, tmem_c, a_lo + 8 * k, b_lo + 2 * k, kDescHi,
+                                             idesc, 1);
+                            }
+                        }
+                        umma_commit_if(leader, t_empty_a + 8 * t);
+                        b_lo += slot_step;
+                        if (++slot == slots) {
+                            slot = 0;
+                            b_lo = b_first;
+                        }
+                        if (++t == kT) {
+                            t = 0;
+                            t_parity ^= 1u;
+                        }
+                    }
                 }
-                // generic-proxy writes, read next by the tensor core through the async proxy
-                asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-                mbar_arrive(&conv_bar[s]);
-                if (++s == kSt) {
-                    s = 0;
-                    phase ^= 1u;
+                if (!ok)
+                    break;
+                umma_commit_if(leader, acc_full_a + 8 * buf);
+                buf ^= 1u;
+                acc_parity ^= buf ^ 1u;  // flips each time set 0 comes round again
+            }
+            tile_parity ^= 1u;
+        }
+        if (!ok)
+            give_up(ERR_MMA_WAIT);
+        __syncwarp();
+    } else if (warp >= 2 + kF32EpilogueWarps) {
+        // ---------------- converters: fp32 A tile -> hi and lo planes in tensor memory ----------------
+        constexpr int kGroups = f32_groups(BN);
+        const int group = (warp - 2 - kF32EpilogueWarps) >> 2;  // takes every kGroups-th stage
+        const int q = warp & 3;
+        const int row = q * 32 + lane;
+        // 16-byte unit u of row r sits at unit u ^ swz of its row
+        const int swz = ROWB == 128 ? (row & 7) : ((row >> 1) & 3);
+        const int total_iters = my_tiles * (ke - kb);
+        int s = group, t = group;
+        uint32_t phase = 0, t_phase = 0;
+        // ring slot of the step whose MMAs the next t_empty wait is for (g - kT)
+        int s_done = group;
+        for (int g = group; g < total_iters; g += kGroups) {
+            bool ok = mbar_wait(&full_bar[s], phase, abort_flag, p.wait_cycles);
+            ok = __all_sync(0xffffffffu, ok);
+            if (!ok) {
+                give_up(ERR_PRODUCER_WAIT);
+                break;
+            }
+            const uint4* src = reinterpret_cast<const uint4*>(ring + s * stage_bytes + row * ROWB);
+            uint4 v[ROWB / 16];
+#pragma unroll
+            for (int u = 0; u < ROWB / 16; ++u)
+                v[u] = src[u ^ swz];
+            ok = mbar_wait(&t_empty[t], t_phase ^ 1u, abort_flag, p.wait_cycles);
+            ok = __all_sync(0xffffffffu, ok);
+            if (!ok) {
+                give_up(ERR_PRODUCER_WAIT);
+                break;
+            }
+            if (!p.b_resident && g >= kT) {
+                // the MMAs of step g - kT have retired: its ring slot goes back to the producer
+                // (on the MMA warp's behalf, whose time is the dearest here)
+                if (threadIdx.x % 128 == 64)
+                    mbar_arrive(&empty_bar[s_done]);
+                s_done += kGroups;
+                if (s_done >= p.stages)
+                    s_done -= p.stages;
+            }
+            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+            const uint32_t ta = tmem_base + ((uint32_t)(q * 32) << 16) + kTmemA +
+                                (uint32_t)(t * 2 * kChans);
+#pragma unroll
+            for (int h = 0; h < kChans / 16; ++h) {
+                uint32_t hi[16], lo[16];
+#pragma unroll
+                for (int j = 0; j < 4; ++j) {
+                    split_tf32(v[4 * h + j].x, hi[4 * j + 0], lo[4 * j + 0]);
+                    split_tf32(v[4 * h + j].y, hi[4 * j + 1], lo[4 * j + 1]);
+                    split_tf32(v[4 * h + j].z, hi[4 * j + 2], lo[4 * j + 2]);
+                    split_tf32(v[4 * h + j].w, hi[4 * j + 3], lo[4 * j + 3]);
                 }
+                tmem_st16(ta + 16 * h, hi);
+                tmem_st16(ta + kChans + 16 * h, lo);
+            }
+            asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
+            asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+            mbar_arrive(&t_full[t]);
+            // The raw tile goes back only now, when its values have been used: a load still on its
+            // way to a register is not ordered before the TMA's next write of the slot.
+            if (p.b_resident)
+                mbar_arrive(&empty_bar[s]);
+            s += kGroups;
+            if (s >= p.stages) {
+                s -= p.stages;
+                phase ^= 1u;
+            }
+            t += kGroups;
+            if (t >= kT) {
+                t -= kT;
+                t_phase ^= 1u;
             }
         }
     } else {
@@ -456,63 +667,135 @@ __global__ void __launch_bounds__(f32_threads(BN), 1) conv_f32_umma_kernel(
         const int q = warp & 3;
         const int row = q * 32 + lane;
         const int half = (warp - 2) >> 2;
-        constexpr int kChunksPerWarp = (BN / 32) / (kF32EpilogueWarps / 4);
-        static_assert(kChunksPerWarp >= 1, "every epilogue warp must own a chunk");
+        constexpr int kCols = BN / 2;        // columns of this warp
+        constexpr int kChunks = kCols / 16;  // ... in 16-column loads
         int local = 0;
         bool ok = true;
-        for (int tile = blockIdx.x; tile < total_tiles && ok; tile += gridDim.x) {
+        for (int tile = first_tile; tile < total_tiles && ok; tile += tile_step) {
             const int tile_n = tile % p.n_tiles, tile_m = tile / p.n_tiles;
             const int m = tile_m * kBM + row, n0 = tile_n * BN;
             // running fp32 sums of this thread's accumulators over the tile's segments
-            float sum[kChunksPerWarp][32];
-            for (int k0 = 0; k0 < p.k_iters && ok; k0 += p.seg_iters, ++local) {
+            float sum[kCols];
+#pragma unroll
+            for (int j = 0; j < kCols; ++j)
+                sum[j] = 0.f;
+            // Adds this warp's columns from `ta` on. (Each load is waited for in the statement that
+            // issues it: with a load in flight across other code, a register that it has yet to
+            // write must never be spilled, and with this many sums nothing guarantees that.)
+            auto add_columns = [&](uint32_t ta) {
+#pragma unroll
+                for (int c = 0; c < kChunks; ++c) {
+                    uint32_t v[16];
+                    tmem_ld16(ta + 16 * c, v);
+#pragma unroll
+                    for (int j = 0; j < 16; ++j)
+                        sum[16 * c + j] = __fadd_rn(sum[16 * c + j], __uint_as_float(v[j]));
+                }
+            };
+            const uint32_t lane_base =
+                    tmem_base + ((uint32_t)(q * 32) << 16) + (uint32_t)(half * kCols);
+            for (int k0 = kb; k0 < ke && ok; k0 += C::kSegIters, ++local) {
                 const int buf = local & 1;
                 const uint32_t acc_phase = (uint32_t)(local >> 1) & 1u;
                 ok = mbar_wait(&acc_full[buf], acc_phase, abort_flag, p.wait_cycles);
-                if (!ok && !*abort_flag) {
-                    *abort_flag = 1;
-                    atomicExch(p.status, ERR_EPILOGUE_WAIT);
-                }
                 ok = __all_sync(0xffffffffu, ok);
-                if (!ok)
+                if (!ok) {
+                    give_up(ERR_EPILOGUE_WAIT);
                     break;
-                asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-                const uint32_t taddr =
-                        tmem_base + ((uint32_t)(q * 32) << 16) + (uint32_t)(buf * 2 * BN);
-#pragma unroll
-                for (int cc = 0; cc < kChunksPerWarp; ++cc) {
-                    const uint32_t col = (uint32_t)((half * kChunksPerWarp + cc) * 32);
-                    uint32_t v[32];
-                    tmem_ld32(taddr + col, v);  // main sum
-                    if (k0 == 0) {
-#pragma unroll
-                        for (int j = 0; j < 32; ++j)
-                            sum[cc][j] = __uint_as_float(v[j]);
-                    } else {
-#pragma unroll
-                        for (int j = 0; j < 32; ++j)
-                            sum[cc][j] = __fadd_rn(sum[cc][j], __uint_as_float(v[j]));
-                    }
-                    tmem_ld32(taddr + (uint32_t)BN + col, v);  // correction sum
-                    if (cc + 1 == kChunksPerWarp) {
-                        // this thread's accumulators are in registers: hand the set back
-                        asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-                        mbar_arrive(&acc_empty[buf]);
-                    }
-#pragma unroll
-                    for (int j = 0; j < 32; ++j)
-                        sum[cc][j] = __fadd_rn(sum[cc][j], __uint_as_float(v[j]));
                 }
+                asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+                if constexpr (C::kWide) {
+                    if (k0 + C::kSegIters >= ke) {
+                        // last segment: every correction MMA of the tile has retired as well
+                        add_columns(lane_base + 2 * BN);
+                        asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+                        mbar_arrive(corr_empty);
+                    }
+                    add_columns(lane_base + (uint32_t)(buf * BN));
+                } else {
+                    add_columns(lane_base + (uint32_t)(buf * 2 * BN));
+                    add_columns(lane_base + (uint32_t)(buf * 2 * BN + BN));
+                }
+                // this thread's accumulators are in registers: hand the set back
+                asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+                mbar_arrive(&acc_empty[buf]);
             }
             if (!ok)
                 break;
+            if (p.splits > 1) {
+                // (every load of the ring has been consumed and every MMA has retired: the
+                // partial tile takes the ring's place)
+                float* part = reinterpret_cast<float*>(tiles) + row * C::kPartPitch + half * kCols;
 #pragma unroll
-            for (int cc = 0; cc < kChunksPerWarp; ++cc) {
-                const int ch0 = n0 + (half * kChunksPerWarp + cc) * 32;
-                if (m < p.m_total && ch0 < p.oc)
-                    store_f32_chunk(sum[cc], p.ep, (size_t)m, ch0);
+                for (int j = 0; j < kCols / 4; ++j)
+                    reinterpret_cast<float4*>(part)[j] = make_float4(
+                            sum[4 * j], sum[4 * j + 1], sum[4 * j + 2], sum[4 * j + 3]);
+            } else if (m < p.m_total && n0 + half * kCols < p.oc) {
+                store_f32_chunk<kCols>(sum, p.ep, (size_t)m, n0 + half * kCols);
             }
         }
+    }
+
+    if (p.splits > 1) {
+        // every CTA of the cluster comes here, whatever became of its waits
+        __syncwarp();
+        f32_cluster_sync();  // the partial tiles are in place
+        const int et = (int)threadIdx.x - 64;
+        if (et >= 0 && et < 32 * kF32EpilogueWarps && !*abort_flag) {
+            const int rows = kBM / p.splits;
+            const int tile_n = first_tile % p.n_tiles, tile_m = first_tile / p.n_tiles;
+            const uint32_t part = smem_u32(tiles);
+            for (int u = et; u < rows * (BN / 4); u += 32 * kF32EpilogueWarps) {
+                const int r = rank * rows + u / (BN / 4), c = (u % (BN / 4)) * 4;
+                const int m = tile_m * kBM + r, ch = tile_n * BN + c;
+                if (m >= p.m_total || ch >= p.oc)
+                    continue;
+                float v[4] = {0.f, 0.f, 0.f, 0.f};
+                for (int i = 0; i < p.splits; ++i) {
+                    uint32_t addr;
+                    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;"
+                                 : "=r"(addr)
+                                 : "r"(part + (uint32_t)((r * C::kPartPitch + c) * 4)), "r"(i));
+                    float x[4];
+                    asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];"
+                                 : "=f"(x[0]), "=f"(x[1]), "=f"(x[2]), "=f"(x[3])
+                                 : "r"(addr)
+                                 : "memory");
+#pragma unroll
+                    for (int j = 0; j < 4; ++j)
+                        v[j] = __fadd_rn(v[j], x[j]);
+                }
+                float* out = p.ep.dst + (size_t)m * p.ep.dst_pitch + ch;
+                const float* zin = p.ep.z ? p.ep.z + (size_t)m * p.ep.z_pitch + ch : nullptr;
+                const int left = min(4, p.oc - ch);
+#pragma unroll
+                for (int j = 0; j < 4; ++j)
+                    if (j < left) {
+                        v[j] += p.ep.bias ? p.ep.bias[ch + j] : 0.f;
+                    }
+                with_act(p.ep.act, [&](auto a) {
+#pragma unroll
+                    for (int j = 0; j < 4; ++j)
+                        v[j] = act_f32<decltype(a)::value>(v[j]);
+                });
+                if (zin) {
+#pragma unroll
+                    for (int j = 0; j < 4; ++j)
+                        if (j < left)
+                            v[j] += zin[j];
+                }
+                if (left == 4 && ((uintptr_t)out & 15) == 0) {
+                    *reinterpret_cast<float4*>(out) = make_float4(v[0], v[1], v[2], v[3]);
+                } else {
+#pragma unroll
+                    for (int j = 0; j < 4; ++j)
+                        if (j < left)
+                            out[j] = v[j];
+                }
+            }
+        }
+        __syncwarp();
+        f32_cluster_sync();  // nobody leaves while its partial tile may still be read
     }
 
     // ---------------- teardown ----------------
@@ -535,7 +818,7 @@ __global__ void __launch_bounds__(f32_threads(BN), 1) conv_f32_umma_kernel(
     }
     if (warp == 1) {
         asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base),
-                     "r"(4 * BN)
+                     "r"(512)
                      : "memory");
     }
 }
@@ -545,9 +828,10 @@ __global__ void __launch_bounds__(f32_threads(BN), 1) conv_f32_umma_kernel(
 // ------------------------------------------------------------------------------------------
 __global__ void __launch_bounds__(256) conv_f32_direct_kernel(
         ConvF32Args a, const float* __restrict__ src, const float* __restrict__ flt,
-        const float* __restrict__ bias, const float* __restrict__ z, float* __restrict__ dst) {
+        const float* __restrict__ flt_lo, int flt_ic, const float* __restrict__ bias,
+        const float* z, float* dst) {
     pdl_start();
-    // flt: the unsplit K-major filter [OC][KH][KW][ICpg]
+    // flt: the K-major filter [OC][KH][KW][flt_ic], or its hi plane with the lo plane beside it
     const size_t total = (size_t)a.m * a.oc;
     const int icpg = a.ic / a.groups, ocpg = a.oc / a.groups;
     for (size_t idx = blockIdx.x * (size_t)blockDim.x + threadIdx.x; idx < total;
@@ -559,7 +843,7 @@ __global__ void __launch_bounds__(256) conv_f32_direct_kernel(
         const int oy = (int)(t % a.oh);
         const int n = (int)(t / a.oh);
         const int g = o / ocpg;
-        const float* w = flt + (size_t)o * a.kh * a.kw * icpg;
+        const size_t w0 = (size_t)o * a.kh * a.kw * flt_ic;
         float acc = 0.f;
         for (int fy = 0; fy < a.kh; ++fy) {
             const int iy = oy * a.sh + fy - a.ph;
@@ -571,12 +855,19 @@ __global__ void __launch_bounds__(256) conv_f32_direct_kernel(
                     continue;
                 const float* s = src + (((size_t)n * a.ih + iy) * a.iw + ix) * a.src_pitch +
                                  g * icpg;
-                const float* wk = w + (size_t)(fy * a.kw + fx) * icpg;
-                for (int c = 0; c < icpg; ++c)
-                    acc = fmaf(s[c], wk[c], acc);
+                const float* wk = flt + w0 + (size_t)(fy * a.kw + fx) * flt_ic;
+                if (flt_lo) {
+                    const float* wl = flt_lo + (wk - flt);
+                    for (int c = 0; c < icpg; ++c)
+                        acc = fmaf(s[c], __fadd_rn(wk[c], wl[c]), acc);
+                } else {
+                    for (int c = 0; c < icpg; ++c)
+                        acc = fmaf(s[c], wk[c], acc);
+                }
             }
         }
-        float r = act_f32(a.act, acc + (bias ? bias[o] : 0.f));
+        float r = acc + (bias ? bias[o] : 0.f);
+        with_act(a.act, [&](auto k) { r = act_f32<decltype(k)::value>(r); });
         if (z)
             r += z[m * a.z_pitch + o];
         dst[m * a.dst_pitch + o] = r;
@@ -607,27 +898,64 @@ int grid_1d(size_t work, int block) {
     return g < 1 ? 1 : (int)g;
 }
 
+// The shared memory a CTA may ask for, less the alignment slack and the barriers.
+constexpr int kF32TileBudget = 227 * 1024 - 1024 - 1024;
+
 template <int BN, int ROWB>
 int launch_f32_kernel(
-        const CUtensorMap& ma, const CUtensorMap& mb, const F32ConvParams& p, cudaStream_t st) {
-    using L = F32Smem<BN, ROWB>;
-    if (cudaFuncSetAttribute(conv_f32_umma_kernel<BN, ROWB>,
-                             cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             L::kDynamic) != cudaSuccess)
+        const CUtensorMap& ma, const CUtensorMap& mb, F32ConvParams& p, cudaStream_t st) {
+    using C = F32Cfg<BN, ROWB>;
+    constexpr int kDynamic = kF32TileBudget + 2048;
+    static KernelReady ready;
+    if (!ready.smem(conv_f32_umma_kernel<BN, ROWB>, kDynamic))
         return check_launch("conv_f32_umma smem attribute");
-    constexpr int kF32Threads = f32_threads(BN);
-    const int per_sm = resident_ctas_per_sm(conv_f32_umma_kernel<BN, ROWB>, kF32Threads,
-                                            L::kDynamic, 4 * BN);
+    // The filter stays resident where one tile column covers the channels and at least five
+    // A stages fit behind it (a TMA round trip is four to five stages of conversion).
+    const long long b_all = (long long)p.k_iters * C::kBBytes;
+    p.b_resident = p.splits == 1 && p.n_tiles == 1 && p.m_tiles > sm_count() &&
+                   b_all + 5 * C::kABytes <= kF32TileBudget;
+    const int stage = C::kABytes + (p.b_resident ? 0 : C::kBBytes);
+    int stages = (int)((kF32TileBudget - (p.b_resident ? b_all : 0)) / stage);
+    p.stages = stages > kMaxStages ? kMaxStages : stages;
     const int total = p.m_tiles * p.n_tiles;
-    int grid = sm_count() * per_sm;
-    if (grid > total)
-        grid = total;
+    int grid = total * p.splits;
+    if (p.splits == 1 && grid > sm_count())
+        grid = sm_count();
     if (tuning().debug)
-        fprintf(stderr, "conv_f32_umma<%d,%d>: per_sm %d grid %d tiles %d k_iters %d smem %d\n", BN,
-                ROWB, per_sm, grid, total, p.k_iters, L::kDynamic);
-    launch_pdl(conv_f32_umma_kernel<BN, ROWB>, dim3(grid), dim3(kF32Threads), (size_t)L::kDynamic, st,
-               ma, mb, p);
+        fprintf(stderr, "conv_f32_umma<%d,%d>: grid %d tiles %d k_iters %d stages %d resident %d "
+                "splits %d\n", BN, ROWB, grid, total, p.k_iters, p.stages, p.b_resident, p.splits);
+    launch_pdl_cluster(conv_f32_umma_kernel<BN, ROWB>, dim3(grid), dim3(f32_threads(BN)),
+                       (size_t)kDynamic, p.splits, st, ma, mb, p);
     return check_launch("conv_f32_umma");
+}
+
+// Tile width and K split for a problem of `m_tiles` x `oc` with `k_iters` steps of `rowb` bytes:
+// the pair with the shortest estimated time of its busiest SM. Clocks per step and tile: 12
+// MMAs of 64 clocks for 128 columns, half that for 64, and for 32 what the handshakes of a step
+// cost. A split adds the
+// exchange of the partial tiles; it is taken only where the clusters all run at once.
+void choose_f32_tile(int m_tiles, int oc, int k_iters, int rowb, int* bn, int* splits) {
+    const int sms = sm_count();
+    long long best = -1;
+    for (int b = 128; b >= 32; b /= 2) {
+        if (b > 32 && oc <= b / 2)
+            continue;
+        const int step = (b == 128 ? 800 : b == 64 ? 460 : 380) * rowb / 128;
+        const int tile_end = b == 128 ? 1500 : b == 64 ? 900 : 600;  // sums, activation, stores
+        const long long tiles = (long long)m_tiles * ((oc + b - 1) / b);
+        for (int s = 1; s <= 8; s *= 2) {
+            if (s > 1 && (tiles * s > sms / 8 * 8 || k_iters / s < 2))
+                break;
+            const long long waves = (tiles * s + sms - 1) / sms;
+            const long long clocks =
+                    waves * ((long long)((k_iters + s - 1) / s) * step + tile_end) + (s > 1 ? 2500 : 0);
+            if (best < 0 || clocks < best) {
+                best = clocks;
+                *bn = b;
+                *splits = s;
+            }
+        }
+    }
 }
 
 bool plain_matrix(const ConvF32Args& a) {
@@ -645,26 +973,39 @@ size_t conv_f32_split_filter_floats(const ConvF32Args& a) {
     return 2 * (size_t)a.oc * a.kh * a.kw * conv_f32_padded_ic(a.ic);
 }
 
-// Tensor-core path: dense, channel count a whole number of TMA rows (16, or a multiple of 32
-// floats), the source a contiguous NHWC tensor of at least 128 KiB, 16-byte aligned operands.
+// Channel counts the tensor-core kernel takes: rows the TMA can address (16-byte multiples).
+// A last, partial row of 32 channels is filled with zeros by the load; the im2col form asks
+// for whole rows of a tensor at least that wide.
+bool conv_f32_split_eligible(const ConvF32Args& a) {
+    if (a.groups != 1 || a.ic % 4 != 0)
+        return false;
+    return plain_matrix(a) || a.ic == 16 || a.ic >= 32;
+}
+
+// Images of `src` the activation's im2col map describes (see descriptor_images in internal.h)
+static int f32_descriptor_images(const ConvF32Args& a, const float* src) {
+    constexpr size_t kMinMapBytes = 131072;
+    const size_t image = (size_t)a.ih * a.iw * a.src_pitch * 4;
+    if ((size_t)a.n * image >= kMinMapBytes)
+        return a.n;
+    const size_t images = (kMinMapBytes + image - 1) / image;
+    return readable_through(src, images * image) ? (int)images : 0;
+}
+
+// Tensor-core path: dense, an eligible channel count, 16-byte aligned operands and pitches,
+// and, with a spatial filter, 128 KiB of readable memory behind `src` for the TMA map.
 bool conv_f32_umma_supported(const ConvF32Args& a, const float* src, const float* dst) {
-    if (a.groups != 1)
-        return false;
-    if (!(a.ic == 16 || a.ic % 32 == 0))
-        return false;
-    if (a.src_pitch != a.ic)
+    if (!conv_f32_split_eligible(a))
         return false;
     if (a.kh * a.kw > 49 || a.ph > 64 || a.pw > 64 || a.sh > 8 || a.sw > 8)
-        return false;
-    if ((size_t)a.n * a.ih * a.iw * a.ic * 4 < 131072)
         return false;
     if ((size_t)a.n * a.ih * a.iw >= (1ull << 31) || (size_t)a.m >= (1ull << 31))
         return false;
     if (((uintptr_t)src | (uintptr_t)dst) & 15)
         return false;
-    if ((a.dst_pitch & 3) || (a.z_pitch & 3))
+    if (a.src_pitch & 3)
         return false;
-    return true;
+    return plain_matrix(a) || f32_descriptor_images(a, src) != 0;
 }
 
 size_t conv_f32_workspace_bytes(const ConvF32Args& a) {
@@ -690,11 +1031,24 @@ int launch_conv_f32_pack_filter_plain(
     return check_launch("pack_filter_f32_plain");
 }
 
+int launch_matmul_f32_pack_split(
+        int k, int n, const float* b, float* out, cudaStream_t st) {
+    const int kp = conv_f32_padded_ic(k);
+    dim3 grid((n + 31) / 32, (kp + 31) / 32), block(32, 8);
+    if (grid.y > 65535)
+        return set_error(ST_OUT_OF_RANGE, "matmul: k = %d exceeds the grid limit", k);
+    pack_matrix_f32_kernel<<<grid, block, 0, st>>>(b, out, k, n, kp);
+    return check_launch("pack_matrix_f32");
+}
+
 int launch_conv_f32_direct(
-        const ConvF32Args& a, const float* src, const float* flt_plain, const float* bias,
+        const ConvF32Args& a, const float* src, const float* flt_packed, const float* bias,
         const float* z, float* dst, cudaStream_t st) {
+    const bool split = conv_f32_split_eligible(a);
+    const int icp = split ? conv_f32_padded_ic(a.ic) : a.ic / a.groups;
+    const float* lo = split ? flt_packed + (size_t)a.oc * a.kh * a.kw * icp : nullptr;
     launch_pdl(conv_f32_direct_kernel, dim3(grid_1d((size_t)a.m * a.oc, 256)), dim3(256), 0, st, a,
-               src, flt_plain, bias, z, dst);
+               src, flt_packed, lo, icp, bias, z, dst);
     return check_launch("conv_f32_direct");
 }
 
@@ -708,17 +1062,28 @@ int launch_conv_f32_umma(
     if ((uintptr_t)flt_split & 15)
         return set_error(ST_INVALID_LAYOUT, "the filter must be 16-byte aligned");
 
-    const int rowb = a.ic == 16 ? 64 : 128;
+    const int rowb = a.ic <= 16 ? 64 : 128;
     const int chans = rowb / 4;
+    const int icp = conv_f32_padded_ic(a.ic);
     const CUtensorMapSwizzle swz =
             rowb == 128 ? CU_TENSOR_MAP_SWIZZLE_128B : CU_TENSOR_MAP_SWIZZLE_64B;
-    const int bn = a.oc <= 64 ? 64 : 128;
     const int taps = a.kh * a.kw;
     const bool a_tiled = plain_matrix(a);
+    F32ConvParams p;
+    p.m_tiles = (a.m + kBM - 1) / kBM;
+    p.cblocks = icp / chans;
+    p.k_iters = taps * p.cblocks;
+    int bn = 128;
+    choose_f32_tile(p.m_tiles, a.oc, p.k_iters, rowb, &bn, &p.splits);
+    if (tuning().f32_bn == 32 || tuning().f32_bn == 64 || tuning().f32_bn == 128)
+        bn = tuning().f32_bn;
+    if (tuning().f32_split == 1 || tuning().f32_split == 2 || tuning().f32_split == 4 ||
+        tuning().f32_split == 8)
+        p.splits = p.k_iters >= tuning().f32_split ? tuning().f32_split : 1;
     CUtensorMap map_a, map_b;
     if (a_tiled) {
         cuuint64_t dims[2] = {(cuuint64_t)a.ic, (cuuint64_t)a.m};
-        cuuint64_t strides[1] = {(cuuint64_t)a.ic * 4};
+        cuuint64_t strides[1] = {(cuuint64_t)a.src_pitch * 4};
         cuuint32_t box[2] = {(cuuint32_t)chans, (cuuint32_t)kBM};
         cuuint32_t estr[2] = {1, 1};
         CUresult r = api.tiled(&map_a, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 2, (void*)src, dims, strides,
@@ -728,10 +1093,13 @@ int launch_conv_f32_umma(
         if (r != CUDA_SUCCESS)
             return set_error(ST_RUNTIME, "cuTensorMapEncodeTiled(f32 activation) failed: %d", (int)r);
     } else {
+        const int images = f32_descriptor_images(a, src);
+        if (images == 0)
+            return set_error(ST_INVALID_LAYOUT, "activation below 128 KiB outside a registered range");
         cuuint64_t dims[4] = {(cuuint64_t)a.ic, (cuuint64_t)a.iw, (cuuint64_t)a.ih,
-                              (cuuint64_t)a.n};
-        cuuint64_t strides[3] = {(cuuint64_t)a.ic * 4, (cuuint64_t)a.iw * a.ic * 4,
-                                 (cuuint64_t)a.ih * a.iw * a.ic * 4};
+                              (cuuint64_t)images};
+        cuuint64_t strides[3] = {(cuuint64_t)a.src_pitch * 4, (cuuint64_t)a.iw * a.src_pitch * 4,
+                                 (cuuint64_t)a.ih * a.iw * a.src_pitch * 4};
         int lower[2] = {-a.pw, -a.ph};
         int upper[2] = {(a.ow - 1) * a.sw - a.pw - (a.iw - 1), (a.oh - 1) * a.sh - a.ph - (a.ih - 1)};
         cuuint32_t estr[4] = {1, (cuuint32_t)a.sw, (cuuint32_t)a.sh, 1};
@@ -743,7 +1111,7 @@ int launch_conv_f32_umma(
             return set_error(ST_RUNTIME, "cuTensorMapEncodeIm2col(f32) failed: %d", (int)r);
     }
     {
-        const cuuint64_t k_total = (cuuint64_t)taps * a.ic;
+        const cuuint64_t k_total = (cuuint64_t)taps * icp;
         cuuint64_t dims[2] = {k_total, (cuuint64_t)2 * a.oc};
         cuuint64_t strides[1] = {k_total * 4};
         cuuint32_t box[2] = {(cuuint32_t)chans, (cuuint32_t)bn};
@@ -755,21 +1123,15 @@ int launch_conv_f32_umma(
         if (r != CUDA_SUCCESS)
             return set_error(ST_RUNTIME, "cuTensorMapEncodeTiled(f32 filter) failed: %d", (int)r);
     }
-    F32ConvParams p;
     p.m_total = a.m;
     p.oc = a.oc;
     p.oh = a.oh;
     p.ow = a.ow;
-    p.cblocks = a.ic / chans;
     p.taps_w = a.kw;
-    p.k_iters = taps * p.cblocks;
-    // eight K = 8 steps per TMEM accumulation chain
-    p.seg_iters = 8 / (rowb / 32);
     p.sh = a.sh;
     p.sw = a.sw;
     p.base_h = -a.ph;
     p.base_w = -a.pw;
-    p.m_tiles = (a.m + kBM - 1) / kBM;
     p.n_tiles = (a.oc + bn - 1) / bn;
     p.a_tiled = a_tiled ? 1 : 0;
     p.b_lo_offset = a.oc;
@@ -785,10 +1147,12 @@ int launch_conv_f32_umma(
         return ST_MALLOC;
     p.wait_cycles = kWaitCycles;
     if (rowb == 128)
-        return bn == 64 ? launch_f32_kernel<64, 128>(map_a, map_b, p, st)
-                        : launch_f32_kernel<128, 128>(map_a, map_b, p, st);
-    return bn == 64 ? launch_f32_kernel<64, 64>(map_a, map_b, p, st)
-                    : launch_f32_kernel<128, 64>(map_a, map_b, p, st);
+        return bn == 32   ? launch_f32_kernel<32, 128>(map_a, map_b, p, st)
+               : bn == 64 ? launch_f32_kernel<64, 128>(map_a, map_b, p, st)
+                          : launch_f32_kernel<128, 128>(map_a, map_b, p, st);
+    return bn == 32   ? launch_f32_kernel<32, 64>(map_a, map_b, p, st)
+           : bn == 64 ? launch_f32_kernel<64, 64>(map_a, map_b, p, st)
+                      : launch_f32_kernel<128, 64>(map_a, map_b, p, st);
 }
 
 }  // namespace mb200

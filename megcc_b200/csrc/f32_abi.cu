@@ -51,11 +51,6 @@ int make_f32_args(const mb200_conv_f32_param* p, long long dst_pitch, ConvF32Arg
     return ST_SUCCESS;
 }
 
-// does the packed filter of this shape carry the tf32 planes?
-bool split_eligible(const ConvF32Args& a) {
-    return a.groups == 1 && (a.ic == 16 || a.ic % 32 == 0);
-}
-
 size_t plain_filter_bytes(const ConvF32Args& a) {
     return up256((size_t)a.oc * (a.ic / a.groups) * a.kh * a.kw * sizeof(float));
 }
@@ -68,10 +63,8 @@ size_t mb200_conv_f32_packed_filter_bytes(const mb200_conv_f32_param* p) {
     ConvF32Args a{};
     if (make_f32_args(p, 0, &a))
         return 0;
-    size_t bytes = plain_filter_bytes(a);
-    if (split_eligible(a))
-        bytes += up256(conv_f32_split_filter_floats(a) * sizeof(float));
-    return bytes;
+    return conv_f32_split_eligible(a) ? up256(conv_f32_split_filter_floats(a) * sizeof(float))
+                                      : plain_filter_bytes(a);
 }
 
 int mb200_conv_f32_pack_filter(
@@ -85,19 +78,15 @@ int mb200_conv_f32_pack_filter(
     if (((uintptr_t)flt_oihw & 3) || ((uintptr_t)flt_packed & 15))
         return set_error(ST_INVALID_LAYOUT, "filter must be 4-byte, packed filter 16-byte aligned");
     cudaStream_t st = (cudaStream_t)stream;
-    if ((rc = launch_conv_f32_pack_filter_plain(a, flt_oihw, flt_packed, st)))
-        return rc;
-    if (split_eligible(a))
-        rc = launch_conv_f32_pack_filter_split(
-                a, flt_oihw, (float*)((uint8_t*)flt_packed + plain_filter_bytes(a)), st);
-    return rc;
+    return conv_f32_split_eligible(a) ? launch_conv_f32_pack_filter_split(a, flt_oihw, flt_packed, st)
+                                      : launch_conv_f32_pack_filter_plain(a, flt_oihw, flt_packed, st);
 }
 
 size_t mb200_conv_f32_workspace_bytes(const mb200_conv_f32_param* p) {
     ConvF32Args a{};
     if (make_f32_args(p, 0, &a))
         return 0;
-    return split_eligible(a) ? up256(conv_f32_workspace_bytes(a)) : 0;
+    return conv_f32_split_eligible(a) ? up256(conv_f32_workspace_bytes(a)) : 0;
 }
 
 int mb200_conv_bias_f32_nhwc(
@@ -114,18 +103,17 @@ int mb200_conv_bias_f32_nhwc(
          (uintptr_t)z) & 3)
         return set_error(ST_INVALID_LAYOUT, "fp32 operands must be 4-byte aligned");
     cudaStream_t st = (cudaStream_t)stream;
-    const bool umma_ok = split_eligible(a) && conv_f32_umma_supported(a, src, dst) &&
+    const bool umma_ok = conv_f32_umma_supported(a, src, dst) &&
                          workspace_bytes >= conv_f32_workspace_bytes(a) &&
                          (((uintptr_t)workspace | (uintptr_t)flt_packed | (uintptr_t)bias |
                            (uintptr_t)z) & 15) == 0;
     if (algo == MB200_ALGO_UMMA && !umma_ok)
         return set_error(ST_NO_IMPLEMENT,
-                         "tensor-core fp32 ConvBias needs a dense filter, ic == 16 or ic %% 32 == 0, "
-                         "16-byte aligned operands and >= 128 KiB of input");
+                         "tensor-core fp32 ConvBias needs a dense filter, ic %% 4 == 0 (with a spatial "
+                         "filter ic == 16 or ic >= 32), 16-byte aligned operands and, with a spatial "
+                         "filter, >= 128 KiB of readable memory from the input on");
     if (algo == MB200_ALGO_UMMA || (algo == MB200_ALGO_AUTO && umma_ok))
-        return launch_conv_f32_umma(
-                a, src, (const float*)((const uint8_t*)flt_packed + plain_filter_bytes(a)), bias, z,
-                dst, workspace, st);
+        return launch_conv_f32_umma(a, src, flt_packed, bias, z, dst, workspace, st);
     if (algo != MB200_ALGO_AUTO && algo != MB200_ALGO_DIRECT)
         return set_error(ST_OUT_OF_RANGE, "unknown algo %d", algo);
     return launch_conv_f32_direct(a, src, flt_packed, bias, z, dst, st);
@@ -151,8 +139,7 @@ size_t mb200_matmul_f32_packed_b_bytes(int k, int n) {
     mb200_conv_f32_param p;
     if (matmul_f32_param(1, n, k, &p))
         return 0;
-    // [N][K] transposed copy first (the conv's OIHW filter), then what the conv packs from it
-    return up256((size_t)k * n * sizeof(float)) + mb200_conv_f32_packed_filter_bytes(&p);
+    return mb200_conv_f32_packed_filter_bytes(&p);
 }
 
 int mb200_matmul_f32_pack_b(int k, int n, const float* b, float* b_packed, void* stream) {
@@ -162,12 +149,15 @@ int mb200_matmul_f32_pack_b(int k, int n, const float* b, float* b_packed, void*
         return rc;
     if (!b || !b_packed)
         return set_error(ST_NULL_PTR, "matmul operand pointer is NULL");
+    if (((uintptr_t)b & 3) || ((uintptr_t)b_packed & 15))
+        return set_error(ST_INVALID_LAYOUT, "B must be 4-byte, the packed B 16-byte aligned");
     cudaStream_t st = (cudaStream_t)stream;
-    // [K][N] row-major -> [N][K] = the OIHW filter of a 1x1 conv
-    if ((rc = launch_transpose_f32(b, b_packed, 1, k, n, st)))
+    ConvF32Args a{};
+    if ((rc = make_f32_args(&p, 0, &a)))
         return rc;
-    return mb200_conv_f32_pack_filter(
-            &p, b_packed, (float*)((uint8_t*)b_packed + up256((size_t)k * n * sizeof(float))), st);
+    // [K][N] row-major -> [N][K], the K-major filter of a 1x1 conv (or its two planes)
+    return conv_f32_split_eligible(a) ? launch_matmul_f32_pack_split(k, n, b, b_packed, st)
+                                      : launch_transpose_f32(b, b_packed, 1, k, n, st);
 }
 
 size_t mb200_matmul_f32_workspace_bytes(int m, int k) {
@@ -186,9 +176,7 @@ int mb200_matmul_f32(
         return rc;
     if (!a || !b_packed || !c)
         return set_error(ST_NULL_PTR, "matmul operand pointer is NULL");
-    const float* packed =
-            (const float*)((const uint8_t*)b_packed + up256((size_t)k * n * sizeof(float)));
-    return mb200_conv_bias_f32_nhwc(&p, a, packed, nullptr, nullptr, c, 0, workspace,
+    return mb200_conv_bias_f32_nhwc(&p, a, b_packed, nullptr, nullptr, c, 0, workspace,
                                     workspace_bytes, MB200_ALGO_AUTO, stream);
 }
 

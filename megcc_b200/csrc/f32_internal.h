@@ -22,6 +22,8 @@ struct ConvF32Args {
 };
 
 int conv_f32_padded_ic(int ic);
+// does the packed filter of this shape consist of the two tf32 planes (else: plain K-major)?
+bool conv_f32_split_eligible(const ConvF32Args& a);
 size_t conv_f32_split_filter_floats(const ConvF32Args& a);
 bool conv_f32_umma_supported(const ConvF32Args& a, const float* src, const float* dst);
 size_t conv_f32_workspace_bytes(const ConvF32Args& a);
@@ -29,8 +31,10 @@ int launch_conv_f32_pack_filter_split(
         const ConvF32Args& a, const float* flt_oihw, float* out, cudaStream_t st);
 int launch_conv_f32_pack_filter_plain(
         const ConvF32Args& a, const float* flt_oihw, float* out, cudaStream_t st);
+// [K][N] -> the planes of the 1x1 filter [N][K]
+int launch_matmul_f32_pack_split(int k, int n, const float* b, float* out, cudaStream_t st);
 int launch_conv_f32_direct(
-        const ConvF32Args& a, const float* src, const float* flt_plain, const float* bias,
+        const ConvF32Args& a, const float* src, const float* flt_packed, const float* bias,
         const float* z, float* dst, cudaStream_t st);
 int launch_conv_f32_umma(
         const ConvF32Args& a, const float* src, const float* flt_split, const float* bias,

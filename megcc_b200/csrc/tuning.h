@@ -14,6 +14,8 @@ struct Tuning {
     int patch_alone = 0;    // MB200_PATCH_ALONE    1 = patch kernel even with one CTA per SM
     int patch_plain = 0;    // MB200_PATCH_PLAIN    1 = 16-channel planes for 64-channel layers
     int overlap_loads = 1;  // MB200_OVERLAP_LOADS  0 = one 32-column TMEM load per chunk in the halo-patch epilogue
+    int f32_bn = 0;         // MB200_F32_BN         0 = by shape, 32 | 64 | 128 = that fp32 tile width
+    int f32_split = 0;      // MB200_F32_SPLIT      0 = by shape, 1 | 2 | 4 | 8 = CTAs per tile's K loop
     int dw_tensor = 1;      // MB200_DW_TENSOR      0 = depthwise 3x3/1 on the CUDA cores only
     int dw_out = 0;         // MB200_DW_OUT         2 | 4 = outputs per thread of the depthwise kernel
     int dw_one_output = 0;  // MB200_DW_ONE_OUTPUT  1 = one output per thread

@@ -6,6 +6,8 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include <atomic>
+
 #ifndef MB200_TRY_WAIT_HINT_NS
 #define MB200_TRY_WAIT_HINT_NS 2000
 #endif
@@ -27,6 +29,25 @@ enum : int {
 
 __device__ __forceinline__ uint32_t smem_u32(const void* p) {
     return (uint32_t)__cvta_generic_to_shared(p);
+}
+
+// The warp index as a value the compiler knows to be the same in all lanes, and one lane chosen
+// by the hardware. A role that runs as a whole warp and only issues under `if (leader)` keeps
+// its descriptors and addresses in uniform registers, where tcgen05.mma takes them from; in a
+// `lane == 0` branch every operand is moved there first, instruction by instruction (measured
+// alone, tf32 with A in tensor memory: 128 x 32 x 8 in 16 clocks against 45, 128 x 64 in 32
+// against 45).
+__device__ __forceinline__ int uniform_warp_index() {
+    return __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0);
+}
+__device__ __forceinline__ bool elect_one() {
+    uint32_t r;
+    asm volatile(
+            "{\n\t.reg .pred p;\n\t"
+            "elect.sync _|p, 0xffffffff;\n\t"
+            "selp.u32 %0, 1, 0, p;\n\t}"
+            : "=r"(r));
+    return r != 0;
 }
 
 __device__ __forceinline__ void mbar_init(uint64_t* bar, int count) {
@@ -84,6 +105,47 @@ __device__ __forceinline__ bool mbar_wait(
                 return false;
         }
     }
+}
+
+// The same on a shared-memory address: no generic pointer is converted per call.
+__device__ __forceinline__ bool mbar_try_wait_u32(uint32_t bar, uint32_t parity) {
+    uint32_t ok;
+    asm volatile(
+            "{\n\t.reg .pred p;\n\t"
+            "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2, %3;\n\t"
+            "selp.u32 %0, 1, 0, p;\n\t}"
+            : "=r"(ok)
+            : "r"(bar), "r"(parity), "r"((uint32_t)MB200_TRY_WAIT_HINT_NS)
+            : "memory");
+    return ok != 0;
+}
+
+// One try in line (a loop that is seldom late spends its instructions there), the bounded wait
+// behind it out of line.
+static __device__ __noinline__ bool mbar_wait_slow(
+        uint32_t bar, uint32_t parity, volatile int* abort_flag, long long limit) {
+    const long long t0 = clock64();
+    unsigned ns = 20;
+#pragma unroll 1
+    for (int spin = 0;; ++spin) {
+        if (mbar_try_wait_u32(bar, parity))
+            return true;
+        if (spin >= 8) {
+            __nanosleep(ns);
+            if (ns < MB200_WAIT_SLEEP_CAP)
+                ns *= 2;
+        }
+        if ((spin & 63) == 63) {
+            if (*abort_flag)
+                return false;
+            if (clock64() - t0 > limit)
+                return false;
+        }
+    }
+}
+__device__ __forceinline__ bool mbar_wait_u32(
+        uint32_t bar, uint32_t parity, volatile int* abort_flag, long long limit = kWaitCycles) {
+    return mbar_try_wait_u32(bar, parity) || mbar_wait_slow(bar, parity, abort_flag, limit);
 }
 
 __device__ __forceinline__ void tma_load_2d(
@@ -183,6 +245,16 @@ __device__ __forceinline__ void umma_commit(uint64_t* bar) {
             : "memory");
 }
 
+// tcgen05.commit by the lane whose `leader` is non-zero (no branch around it)
+__device__ __forceinline__ void umma_commit_if(uint32_t leader, uint32_t bar) {
+    asm volatile(
+            "{\n\t.reg .pred q;\n\tsetp.ne.b32 q, %1, 0;\n\t"
+            "@q tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n\t}" ::"r"(
+                    bar),
+            "r"(leader)
+            : "memory");
+}
+
 __device__ __forceinline__ void tmem_ld32(uint32_t taddr, uint32_t (&v)[32]) {
     asm volatile(
             "tcgen05.ld.sync.aligned.32x32b.x32.b32 "
@@ -200,6 +272,19 @@ __device__ __forceinline__ void tmem_ld32(uint32_t taddr, uint32_t (&v)[32]) {
     asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 }
 
+
+// 16 columns, load and wait in one statement
+__device__ __forceinline__ void tmem_ld16(uint32_t taddr, uint32_t (&v)[16]) {
+    asm volatile(
+            "tcgen05.ld.sync.aligned.32x32b.x16.b32 "
+            "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];\n\t"
+            "tcgen05.wait::ld.sync.aligned;"
+            : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]),
+              "=r"(v[7]), "=r"(v[8]), "=r"(v[9]), "=r"(v[10]), "=r"(v[11]), "=r"(v[12]),
+              "=r"(v[13]), "=r"(v[14]), "=r"(v[15])
+            : "r"(taddr)
+            : "memory");
+}
 
 // 16 columns, WITHOUT waiting: the registers may be read only after tmem_ld_wait16(v)
 __device__ __forceinline__ void tmem_ld16_nowait(uint32_t taddr, uint32_t (&v)[16]) {
@@ -281,6 +366,27 @@ inline int sm_count() {
     }
     return sms[dev];
 }
+
+// Remembers, per device, that a kernel was allowed `bytes` of dynamic shared memory: the
+// attribute call costs a launch about a microsecond and never changes. One static object per
+// kernel instantiation; concurrent first calls both set the same value.
+struct KernelReady {
+    std::atomic<int> bytes_set[64] = {};
+    template <class Kernel>
+    bool smem(Kernel kernel, int bytes) {
+        int dev = 0;
+        if (cudaGetDevice(&dev) != cudaSuccess)
+            return false;
+        if (dev >= 0 && dev < 64 && bytes_set[dev].load(std::memory_order_relaxed) >= bytes)
+            return true;
+        if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes) !=
+            cudaSuccess)
+            return false;
+        if (dev >= 0 && dev < 64)
+            bytes_set[dev].store(bytes, std::memory_order_relaxed);
+        return true;
+    }
+};
 
 // CTAs of `threads` threads that one SM holds at once, from the kernel's register count,
 // its dynamic shared memory and its TMEM columns. (The runtime's occupancy query answers 1

@@ -125,6 +125,52 @@ def test_matmul_f32_matches_oracle(ops, oracle, shape):
     assert ops.device_status() == 0
 
 
+# tile widths, K splits over a cluster, the resident filter (more than 148 row tiles in one tile
+# column), partial channel rows and channel tails of the tensor-core kernel
+TILE_CASES = [
+    # n, ic, oc, h, w, k, stride, bn, split
+    (1, 64, 128, 23, 17, 3, 1, 128, 8), (1, 64, 128, 23, 17, 3, 2, 64, 4),
+    (2, 36, 72, 14, 19, 3, 1, 32, 2), (1, 100, 33, 31, 9, 1, 1, 64, 4),
+    (1, 16, 32, 139, 141, 3, 1, 32, 1), (1, 16, 40, 139, 141, 3, 2, 64, 1),
+    (1, 32, 20, 139, 141, 3, 1, 32, 1), (3, 68, 128, 81, 80, 1, 1, 128, 1),
+    (1, 20, 5, 7, 7, 1, 1, 32, 1), (1, 512, 130, 5, 5, 1, 1, 0, 0), (1, 128, 64, 9, 9, 3, 1, 0, 0),
+]
+
+
+@pytest.mark.parametrize("case", TILE_CASES, ids=["-".join(map(str, c)) for c in TILE_CASES])
+def test_conv_f32_tile_forms_match_oracle(ops, oracle, case):
+    n, ic, oc, h, w, k, stride, bn, split = case
+    r = cases.rng_for("f32_tiles_" + "_".join(map(str, case)))
+    src = r.standard_normal((n, ic, h, w)).astype(np.float32)
+    flt = (r.standard_normal((oc, ic, k, k)) / np.sqrt(ic * k * k)).astype(np.float32)
+    bias, z = (r.standard_normal(s).astype(np.float32) for s in ((oc,), (n, oc, -(-h // stride), -(-w // stride))))
+    p = ops.conv_f32_param(n, ic, h, w, oc, k, k, stride, k // 2, 1, "SILU")
+    room = torch.zeros(1 << 17, dtype=torch.float32, device="cuda")  # readable behind a small input
+    x = room[:src.size].view(n, h, w, ic) if src.size < (1 << 16) else torch.empty(
+        (n, h, w, ic), device="cuda")
+    x.copy_(dev(src.transpose(0, 2, 3, 1)))
+    from megcc_b200._lib import check, lib
+    check(lib().mb200_register_readable_range(room.data_ptr(), room.numel() * 4))
+    old = [(name, ops.set_option(name, v)) for name, v in (("f32_bn", bn), ("f32_split", split))]
+    try:
+        got = [ops.conv_bias_f32_nhwc(p, x, ops.pack_filter_f32(p, dev(flt)), dev(bias),
+                                      z=dev(z.transpose(0, 2, 3, 1)), algo="umma") for _ in range(3)]
+    finally:
+        for name, v in old:
+            ops.set_option(name, v)
+        torch.cuda.synchronize()
+        lib().mb200_unregister_readable_range(room.data_ptr())
+    assert all(torch.equal(got[0], g) for g in got)  # the sums do not depend on timing
+    close(to_nchw(got[0]), oracle.conv_bias_f32(src, flt, bias, stride, k // 2, "SILU", z=z))
+    assert ops.device_status() == 0
+
+
+@pytest.mark.parametrize("shape", [(1000, 1000, 1000), (129, 65, 4100), (77, 31, 999)],
+                         ids=["k1000", "k4100_split", "k999_odd"])
+def test_matmul_f32_partial_rows_match_oracle(ops, oracle, shape):
+    test_matmul_f32_matches_oracle(ops, oracle, shape)
+
+
 @pytest.mark.parametrize("mode", ["RELU", "SIGMOID", "SILU", "H_SWISH", "EXP", "ADD", "SUB",
                                   "MUL", "MAX", "FUSE_ADD_RELU"])
 def test_elemwise_f32_matches_oracle(ops, oracle, mode):
