@@ -118,13 +118,14 @@ struct PatchWalker {
     }
 };
 
-// One tile's MMAs. The issuing thread runs alone in its warp and every instruction of its
-// loop costs it several cycles, so the hot filter shapes get their own instantiation
-// (KH > 0) where every operand offset is a compile-time constant: two adds per MMA. Looking
-// the offsets up in a shared-memory table measured slower than the MMAs themselves.
+// One tile's MMAs. The whole warp runs this (one lane issues): operand words then live in uniform
+// registers. Every instruction between two MMAs shows as idle tensor time, so the hot filter
+// shapes get their own instantiation (KH > 0) where every operand offset is a compile-time
+// constant. `a0` / `b0` are the low words of the operands' descriptors, `a_hi` / `b_hi` the rest.
 template <int BN, int KH, int KW, int CHUNKS>
 __device__ __forceinline__ void issue_tile_mmas(
-        const PatchParams& p, uint64_t a0, uint64_t b0, uint32_t tmem_d) {
+        const PatchParams& p, uint32_t leader, uint32_t a0, uint32_t a_hi, uint32_t b0,
+        uint32_t b_hi, uint32_t tmem_d) {
     constexpr uint32_t idesc = umma_idesc_s8(128, BN);
     // all offsets in descriptor address units (16 bytes = one pixel of one chunk plane)
     if constexpr (KH > 0) {
@@ -136,13 +137,9 @@ __device__ __forceinline__ void issue_tile_mmas(
 #pragma unroll
             for (int fy = 0; fy < KH; ++fy) {
 #pragma unroll
-                for (int fx = 0; fx < KW; fx += 2) {
-                    const uint64_t ad = a0 + (fy * ppw + fx), bd = b0 + (uint32_t)((fy * KW + fx) * BN);
-                    if ((fy | fx) == 0)
-                        umma_s8_c<false>(tmem_d, ad, bd, idesc);
-                    else
-                        umma_s8_c<true>(tmem_d, ad, bd, idesc);
-                }
+                for (int fx = 0; fx < KW; fx += 2)
+                    umma_s8(leader, tmem_d, a0 + (fy * ppw + fx), a_hi,
+                            b0 + (uint32_t)((fy * KW + fx) * BN), b_hi, idesc, (fy | fx) != 0);
             }
         } else {
 #pragma unroll
@@ -150,38 +147,33 @@ __device__ __forceinline__ void issue_tile_mmas(
 #pragma unroll
                 for (int fx = 0; fx < KW; ++fx) {
 #pragma unroll
-                    for (int j = 0; j < CHUNKS / 2; ++j) {
+                    for (int j = 0; j < CHUNKS / 2; ++j)
                         // chunks 2j, 2j+1 are the two 16-byte K halves of this step
-                        const uint64_t ad = a0 + (fy * ppw + fx + 2 * j * plane16);
-                        const uint64_t bd = b0 + (uint32_t)(((fy * KW + fx) * CHUNKS + 2 * j) * BN);
-                        if ((fy | fx | j) == 0)
-                            umma_s8_c<false>(tmem_d, ad, bd, idesc);
-                        else
-                            umma_s8_c<true>(tmem_d, ad, bd, idesc);
-                    }
+                        umma_s8(leader, tmem_d, a0 + (fy * ppw + fx + 2 * j * plane16), a_hi,
+                                b0 + (uint32_t)(((fy * KW + fx) * CHUNKS + 2 * j) * BN), b_hi, idesc,
+                                (fy | fx | j) != 0);
                 }
             }
         }
     } else {
         const uint32_t plane16 = (uint32_t)p.plane_stride >> 4;
-        uint32_t acc = 0;
-        uint64_t b_desc = b0;
+        uint32_t acc = 0, b_desc = b0;
         if (p.mma_per_tap > 0) {
             for (int fy = 0; fy < p.kh; ++fy) {
-                uint64_t a_tap = a0 + (uint32_t)(fy * p.ppw);
+                uint32_t a_tap = a0 + (uint32_t)(fy * p.ppw);
                 for (int fx = 0; fx < p.kw; ++fx, ++a_tap) {
-                    uint64_t a_desc = a_tap;
+                    uint32_t a_desc = a_tap;
                     for (int j = 0; j < p.mma_per_tap; ++j, a_desc += 2 * plane16, b_desc += 2 * BN) {
-                        umma_s8(tmem_d, a_desc, b_desc, idesc, acc);
+                        umma_s8(leader, tmem_d, a_desc, a_hi, b_desc, b_hi, idesc, acc);
                         acc = 1;
                     }
                 }
             }
         } else {
             for (int fy = 0; fy < p.kh; ++fy) {
-                uint64_t a_desc = a0 + (uint32_t)(fy * p.ppw);
+                uint32_t a_desc = a0 + (uint32_t)(fy * p.ppw);
                 for (int fx = 0; fx < p.kw; fx += 2, a_desc += 2, b_desc += 2 * BN) {
-                    umma_s8(tmem_d, a_desc, b_desc, idesc, acc);
+                    umma_s8(leader, tmem_d, a_desc, a_hi, b_desc, b_hi, idesc, acc);
                     acc = 1;
                 }
             }
@@ -195,10 +187,11 @@ __device__ __forceinline__ void issue_tile_mmas(
 // row: 720 rows per tile against 288 here. A patch row is padded to 16 columns so that the
 // 8-row groups of a tap lie a multiple of the swizzle pattern (512 bytes) apart; the
 // swizzle is a function of the shared-memory address, so a tap's shifted start needs
-// nothing else. `a0` / `b0` are 64-byte-swizzle descriptors of the stage / filter base.
+// nothing else. `a0` / `b0`: 64-byte-swizzle descriptors of the stage / filter base.
 constexpr int kRowCols = 16;
 template <int BN, int KH, int KW>
-__device__ __forceinline__ void issue_tile_mmas_rows64(uint64_t a0, uint64_t b0, uint32_t tmem_d) {
+__device__ __forceinline__ void issue_tile_mmas_rows64(
+        uint32_t leader, uint32_t a0, uint32_t a_hi, uint32_t b0, uint32_t b_hi, uint32_t tmem_d) {
     constexpr uint32_t idesc = umma_idesc_s8(128, BN);
     constexpr uint32_t pix16 = 64 / 16;  // one pixel in descriptor address units
 #pragma unroll
@@ -206,14 +199,10 @@ __device__ __forceinline__ void issue_tile_mmas_rows64(uint64_t a0, uint64_t b0,
 #pragma unroll
         for (int fx = 0; fx < KW; ++fx) {
 #pragma unroll
-            for (int k = 0; k < 2; ++k) {  // two K steps of 32 bytes inside the 64-byte row
-                const uint64_t ad = a0 + (uint32_t)((fy * kRowCols + fx) * pix16 + 2 * k);
-                const uint64_t bd = b0 + (uint32_t)((fy * KW + fx) * BN * pix16 + 2 * k);
-                if ((fy | fx | k) == 0)
-                    umma_s8_c<false>(tmem_d, ad, bd, idesc);
-                else
-                    umma_s8_c<true>(tmem_d, ad, bd, idesc);
-            }
+            for (int k = 0; k < 2; ++k)  // two K steps of 32 bytes inside the 64-byte row
+                umma_s8(leader, tmem_d, a0 + (uint32_t)((fy * kRowCols + fx) * pix16 + 2 * k), a_hi,
+                        b0 + (uint32_t)((fy * KW + fx) * BN * pix16 + 2 * k), b_hi, idesc,
+                        (fy | fx | k) != 0);
         }
     }
 }
@@ -244,7 +233,7 @@ __global__ void __launch_bounds__(64 + 32 * EW, EW == 16 ? 1 : 2) conv_patch_ker
     // XORed with the pixel's column so that neither the row-wise writes nor the window reads
     // collide on banks
     uint8_t* pool_buf = (uint8_t*)(((uintptr_t)(abort_flag + 1) + 127) & ~(uintptr_t)127);
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int warp = uniform_warp_index(), lane = threadIdx.x & 31;
     // each CTA owns one slice of output channels and walks the patches with a fixed stride
     const int tile_n = blockIdx.x % p.n_tiles;
     const int m_first = blockIdx.x / p.n_tiles;
@@ -374,54 +363,48 @@ __global__ void __launch_bounds__(64 + 32 * EW, EW == 16 ? 1 : 2) conv_patch_ker
             }
         }
     } else if (warp == 1) {
-        // ---------------- MMA issuer ----------------
-        if (lane == 0) {
-            bool ok = mbar_wait(b_full, 0, abort_flag);
-            if (!ok && !*abort_flag) {
-                *abort_flag = 1;
-                atomicExch(p.status, ERR_MMA_WAIT);
-            }
-            const uint32_t sbo_a = (uint32_t)p.ppw * 16;  // the next patch row
-            const uint64_t b0 = ROWS ? umma_smem_desc(smem_u32(smem_b), 16, 512, 4)
-                                     : umma_smem_desc(smem_u32(smem_b), BN * 16, 128, 0);
-            int local = 0, s = 0;
-            uint32_t phase = 0;
-            for (int mt = m_first; mt < p.m_tiles && ok; mt += m_step, ++local) {
-                const int buf = local & 1;
-                const uint32_t acc_phase = (uint32_t)(local >> 1) & 1u;
-                if (!mbar_wait(&acc_empty[buf], acc_phase ^ 1u, abort_flag)) {
-                    if (!*abort_flag) {
-                        *abort_flag = 1;
-                        atomicExch(p.status, ERR_MMA_ACC_WAIT);
-                    }
-                    break;
-                }
-                if (!mbar_wait(&a_full[s], phase, abort_flag)) {
-                    if (!*abort_flag) {
-                        *abort_flag = 1;
-                        atomicExch(p.status, ERR_MMA_WAIT);
-                    }
-                    break;
-                }
-                asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-                const uint32_t a_addr = smem_u32(smem_a + s * p.a_stage_bytes);
-                const uint32_t tmem_d = tmem_base + (uint32_t)(buf * BN);
-                if constexpr (ROWS != 0) {
-                    // 8-row groups (patch rows) are 16 pixels x 64 bytes apart
-                    const uint64_t a0 = umma_smem_desc(a_addr, 16, kRowCols * 64, 4);
-                    issue_tile_mmas_rows64<BN, KH, KW>(a0, b0, tmem_d);
-                } else {
-                    const uint64_t a0 = umma_smem_desc(a_addr, (uint32_t)p.a_lbo, sbo_a, 0);
-                    issue_tile_mmas<BN, KH, KW, CHUNKS>(p, a0, b0, tmem_d);
-                }
-                umma_commit(&a_empty[s]);
-                umma_commit(&acc_full[buf]);
-                if (++s == p.stages) {
-                    s = 0;
-                    phase ^= 1u;
-                }
+        // ---------------- MMA issuer (the whole warp waits, one lane issues) ----------------
+        const uint32_t leader = elect_one() ? 1u : 0u;
+        bool ok = mbar_wait(b_full, 0, abort_flag);
+        const uint32_t sbo_a = (uint32_t)p.ppw * 16;  // the next patch row
+        const uint64_t b0 = ROWS ? umma_smem_desc(smem_u32(smem_b), 16, 512, 4)
+                                 : umma_smem_desc(smem_u32(smem_b), BN * 16, 128, 0);
+        // rows form: 8-row groups (patch rows) are 16 pixels x 64 bytes apart
+        const uint64_t a0 = ROWS ? umma_smem_desc(smem_u32(smem_a), 16, kRowCols * 64, 4)
+                                 : umma_smem_desc(smem_u32(smem_a), (uint32_t)p.a_lbo, sbo_a, 0);
+        const uint32_t a_hi = (uint32_t)(a0 >> 32), b_hi = (uint32_t)(b0 >> 32);
+        const uint32_t a_first = (uint32_t)a0, a_step = (uint32_t)p.a_stage_bytes >> 4;
+        const uint32_t a_full_a = smem_u32(a_full), a_empty_a = smem_u32(a_empty);
+        const uint32_t acc_full_a = smem_u32(acc_full), acc_empty_a = smem_u32(acc_empty);
+        uint32_t phase = 0, buf = 0, acc_parity = 1, a_lo = a_first;
+        int s = 0;
+        for (int mt = m_first; mt < p.m_tiles && ok; mt += m_step) {
+            ok = mbar_wait_u32(acc_empty_a + 8 * buf, acc_parity, abort_flag) &&
+                 mbar_wait_u32(a_full_a + 8 * s, phase, abort_flag);
+            if (!ok)
+                break;
+            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+            const uint32_t tmem_d = tmem_base + buf * BN;
+            if constexpr (ROWS != 0)
+                issue_tile_mmas_rows64<BN, KH, KW>(leader, a_lo, a_hi, (uint32_t)b0, b_hi, tmem_d);
+            else
+                issue_tile_mmas<BN, KH, KW, CHUNKS>(p, leader, a_lo, a_hi, (uint32_t)b0, b_hi, tmem_d);
+            umma_commit_if(leader, a_empty_a + 8 * s);
+            umma_commit_if(leader, acc_full_a + 8 * buf);
+            buf ^= 1u;
+            acc_parity ^= buf ^ 1u;  // flips each time buffer 0 comes round again
+            a_lo += a_step;
+            if (++s == p.stages) {
+                s = 0;
+                phase ^= 1u;
+                a_lo = a_first;
             }
         }
+        if (!ok && !*abort_flag) {
+            *abort_flag = 1;
+            atomicExch(p.status, ERR_MMA_WAIT);
+        }
+        __syncwarp();
     } else {
         // ---------------- epilogue ----------------
         pdl_wait();  // before the first read of z and the first store over memory in use

@@ -152,7 +152,7 @@ __global__ void __launch_bounds__(Shape<BN>::kThreads, Shape<BN>::kMinCtas) conv
     volatile int* abort_flag = (volatile int*)(tmem_slot + 1);
     volatile int* last_flag = (volatile int*)(tmem_slot + 2);
 
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int warp = uniform_warp_index(), lane = threadIdx.x & 31;
     const int total_tiles = SPLITK ? p.total_items : p.m_tiles * p.n_tiles;
 
     if (threadIdx.x == 0) {
@@ -265,73 +265,74 @@ __global__ void __launch_bounds__(Shape<BN>::kThreads, Shape<BN>::kMinCtas) conv
             }
         }
     } else if (warp == 1) {
-        // ---------------- MMA issuer ----------------
-        if (lane == 0) {
-            constexpr uint32_t idesc = umma_idesc_s8(kBM, BN);
-            int local = 0, s = 0;
-            uint32_t phase = 0;
-            bool ok = true;
-            for (int item = blockIdx.x; item < total_tiles && ok; item += gridDim.x, ++local) {
-                const WorkItem w = decode_item<SPLITK>(p, item);
-                const int buf = local & 1;
-                const uint32_t acc_phase = (uint32_t)(local >> 1) & 1u;
-                // the epilogue must have drained this accumulator buffer
-                if (!mbar_wait(&acc_empty[buf], acc_phase ^ 1u, abort_flag, p.wait_cycles)) {
+        // ---------------- MMA issuer (the whole warp waits, one lane issues) ----------------
+        // Instructions between two MMAs show as idle tensor time: descriptor words are running
+        // sums, every lane takes the loop so that they stay in uniform registers.
+        const uint32_t leader = elect_one() ? 1u : 0u;
+        constexpr uint32_t idesc = umma_idesc_s8(kBM, BN);
+        // one descriptor per operand and stage; a K step only moves the address field (16-byte
+        // units): +32 bytes inside the swizzled row, or two 16-byte tap blocks in the plain
+        // layout. 128-byte swizzle: 8-row groups 1024 bytes apart; 64-byte: 512.
+        const uint64_t a0 = GEOM == GEOM_WIDE128 ? umma_smem_desc(smem_u32(tiles_a), 16, 1024, 2)
+                            : GEOM == GEOM_WIDE  ? umma_smem_desc(smem_u32(tiles_a), 16, 512, 4)
+                                                 : umma_smem_desc(smem_u32(tiles_a), kBM * 16, 128, 0);
+        const uint64_t b0 = GEOM == GEOM_WIDE128 ? umma_smem_desc(smem_u32(tiles_b), 16, 1024, 2)
+                            : GEOM == GEOM_WIDE  ? umma_smem_desc(smem_u32(tiles_b), 16, 512, 4)
+                                                 : umma_smem_desc(smem_u32(tiles_b), BN * 16, 128, 0);
+        constexpr uint32_t a_k = GEOM == GEOM_TAP16 ? 2 * (kBM * 16) / 16 : 32 / 16;
+        constexpr uint32_t b_k = GEOM == GEOM_TAP16 ? 2 * (BN * 16) / 16 : 32 / 16;
+        const uint32_t a_hi = (uint32_t)(a0 >> 32), b_hi = (uint32_t)(b0 >> 32);
+        const uint32_t full_a = smem_u32(full_bar), empty_a = smem_u32(empty_bar);
+        const uint32_t acc_full_a = smem_u32(acc_full), acc_empty_a = smem_u32(acc_empty);
+        uint32_t a_lo = (uint32_t)a0, b_lo = (uint32_t)b0;
+        uint32_t phase = 0, buf = 0, acc_parity = 1;
+        int s = 0;
+        bool ok = true;
+        for (int item = blockIdx.x; item < total_tiles && ok; item += gridDim.x) {
+            const WorkItem w = decode_item<SPLITK>(p, item);
+            // the epilogue must have drained this accumulator buffer
+            ok = mbar_wait_u32(acc_empty_a + 8 * buf, acc_parity, abort_flag, p.wait_cycles);
+            if (!ok) {
+                if (!*abort_flag) {
+                    *abort_flag = 1;
+                    atomicExch(p.status, ERR_MMA_ACC_WAIT);
+                }
+                break;
+            }
+            const uint32_t tmem_d = tmem_base + buf * BN;
+            uint32_t acc = 0;
+            for (int it = w.k0; it < w.k1; ++it) {
+                ok = mbar_wait_u32(full_a + 8 * s, phase, abort_flag, p.wait_cycles);
+                if (!ok) {
                     if (!*abort_flag) {
                         *abort_flag = 1;
-                        atomicExch(p.status, ERR_MMA_ACC_WAIT);
+                        atomicExch(p.status, ERR_MMA_WAIT);
                     }
-                    ok = false;
                     break;
                 }
                 asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-                const uint32_t tmem_d = tmem_base + (uint32_t)(buf * BN);
-                for (int it = w.k0; it < w.k1; ++it) {
-                    if (!mbar_wait(&full_bar[s], phase, abort_flag, p.wait_cycles)) {
-                        if (!*abort_flag) {
-                            *abort_flag = 1;
-                            atomicExch(p.status, ERR_MMA_WAIT);
-                        }
-                        ok = false;
-                        break;
-                    }
-                    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-                    const uint32_t a_addr = smem_u32(tiles_a + s * L::kABytes);
-                    const uint32_t b_addr = smem_u32(tiles_b + s * L::kBBytes);
-                    // one descriptor per operand and stage; a K step only moves the address
-                    // field (16-byte units): +32 bytes inside the swizzled row, or two 16-byte
-                    // tap blocks in the plain layout
-                    uint64_t adesc, bdesc;
-                    uint32_t a_step, b_step;
-                    if (GEOM == GEOM_WIDE128) {
-                        // 128-byte swizzle: 8-row groups 1024 bytes apart
-                        adesc = umma_smem_desc(a_addr, 16, 1024, 2);
-                        bdesc = umma_smem_desc(b_addr, 16, 1024, 2);
-                        a_step = b_step = 32 / 16;
-                    } else if (GEOM == GEOM_WIDE) {
-                        adesc = umma_smem_desc(a_addr, 16, 512, 4);
-                        bdesc = umma_smem_desc(b_addr, 16, 512, 4);
-                        a_step = b_step = 32 / 16;
-                    } else {
-                        adesc = umma_smem_desc(a_addr, kBM * 16, 128, 0);
-                        bdesc = umma_smem_desc(b_addr, BN * 16, 128, 0);
-                        a_step = 2 * (kBM * 16) / 16;
-                        b_step = 2 * (BN * 16) / 16;
-                    }
-                    umma_s8(tmem_d, adesc, bdesc, idesc, it != w.k0 ? 1u : 0u);
+                umma_s8(leader, tmem_d, a_lo, a_hi, b_lo, b_hi, idesc, acc);
 #pragma unroll
-                    for (int k = 1; k < kBKc / kUmmaK; ++k)
-                        umma_s8_c<true>(tmem_d, adesc + k * a_step, bdesc + k * b_step, idesc);
-                    umma_commit(&empty_bar[s]);  // frees the stage once these MMAs retire
-                    if (++s == kSt) {
-                        s = 0;
-                        phase ^= 1u;
-                    }
+                for (int k = 1; k < kBKc / kUmmaK; ++k)
+                    umma_s8(leader, tmem_d, a_lo + k * a_k, a_hi, b_lo + k * b_k, b_hi, idesc, 1);
+                umma_commit_if(leader, empty_a + 8 * s);  // frees the stage once these retire
+                acc = 1;
+                a_lo += L::kABytes / 16;
+                b_lo += L::kBBytes / 16;
+                if (++s == kSt) {
+                    s = 0;
+                    phase ^= 1u;
+                    a_lo = (uint32_t)a0;
+                    b_lo = (uint32_t)b0;
                 }
-                if (ok)
-                    umma_commit(&acc_full[buf]);
             }
+            if (!ok)
+                break;
+            umma_commit_if(leader, acc_full_a + 8 * buf);
+            buf ^= 1u;
+            acc_parity ^= buf ^ 1u;  // flips each time buffer 0 comes round again
         }
+        __syncwarp();
     } else {
         // ---------------- epilogue: warps 2..9, TMEM lanes 32*(warp%4).. ----------------
         const int q = warp & 3;

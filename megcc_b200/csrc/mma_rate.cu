@@ -63,7 +63,8 @@ __global__ void __launch_bounds__(128, 1) mma_rate_kernel(int iters, int* status
                         "l"(a0 + step), "l"(b0 + step), "r"(idesc), "r"(i ? 1u : 0u)
                         : "memory");
             else
-                umma_s8(tmem, a0 + step, b0 + step, idesc, i ? 1u : 0u);
+                umma_s8(1u, tmem, (uint32_t)(a0 + step), (uint32_t)(a0 >> 32), (uint32_t)(b0 + step),
+                        (uint32_t)(b0 >> 32), idesc, i ? 1u : 0u);
         }
         umma_commit(&bar);
         if (!mbar_wait(&bar, 0, &abort_flag))

@@ -216,25 +216,18 @@ __host__ __device__ constexpr uint32_t umma_idesc_s8(int m, int n) {
            ((uint32_t)(m >> 4) << 24);
 }
 
+// Issued by the lane whose `leader` is non-zero, without a branch. Descriptors come as their low
+// words (address field and leading-dimension offset, the part that moves from step to step)
+// and constant high words.
 __device__ __forceinline__ void umma_s8(
-        uint32_t tmem_d, uint64_t adesc, uint64_t bdesc, uint32_t idesc, uint32_t accumulate) {
+        uint32_t leader, uint32_t tmem_d, uint32_t a_lo, uint32_t a_hi, uint32_t b_lo, uint32_t b_hi,
+        uint32_t idesc, uint32_t accumulate) {
     asm volatile(
-            "{\n\t.reg .pred p;\n\t"
-            "setp.ne.b32 p, %4, 0;\n\t"
-            "tcgen05.mma.cta_group::1.kind::i8 [%0], %1, %2, %3, p;\n\t}" ::"r"(tmem_d),
-            "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate)
-            : "memory");
-}
-
-// The same with the accumulate flag known at compile time: no register, no compare.
-template <bool ACCUMULATE>
-__device__ __forceinline__ void umma_s8_c(
-        uint32_t tmem_d, uint64_t adesc, uint64_t bdesc, uint32_t idesc) {
-    asm volatile(
-            "{\n\t.reg .pred p;\n\t"
-            "setp.ne.b32 p, %4, 0;\n\t"
-            "tcgen05.mma.cta_group::1.kind::i8 [%0], %1, %2, %3, p;\n\t}" ::"r"(tmem_d),
-            "l"(adesc), "l"(bdesc), "r"(idesc), "n"(ACCUMULATE ? 1 : 0)
+            "{\n\t.reg .pred p, q;\n\t.reg .b64 a, b;\n\t"
+            "mov.b64 a, {%1, %2};\n\tmov.b64 b, {%3, %4};\n\t"
+            "setp.ne.b32 p, %6, 0;\n\tsetp.ne.b32 q, %7, 0;\n\t"
+            "@q tcgen05.mma.cta_group::1.kind::i8 [%0], a, b, %5, p;\n\t}" ::"r"(tmem_d),
+            "r"(a_lo), "r"(a_hi), "r"(b_lo), "r"(b_hi), "r"(idesc), "r"(accumulate), "r"(leader)
             : "memory");
 }
 
