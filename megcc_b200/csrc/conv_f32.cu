@@ -402,6 +402,9 @@ __global__ void __launch_bounds__(f32_threads(BN), 1) conv_f32_umma_kernel(
         mbar_init(drain_bar, 1);
         *abort_flag = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    } else if (threadIdx.x == 32 * 2) {
+        tma_prefetch_map(&map_a);
+        tma_prefetch_map(&map_b);
     }
     if (warp == 1) {
         asm volatile(
@@ -415,7 +418,7 @@ __global__ void __launch_bounds__(f32_threads(BN), 1) conv_f32_umma_kernel(
     __syncthreads();
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     const uint32_t tmem_base = *tmem_slot;
-    pdl_start();  // set-up done: from here on the kernel touches global memory
+    pdl_release();
 
     auto give_up = [&](int code) {
         if (!*abort_flag) {
@@ -427,6 +430,19 @@ __global__ void __launch_bounds__(f32_threads(BN), 1) conv_f32_umma_kernel(
     if (warp == 0) {
         // ---------------- TMA producer ----------------
         if (lane == 0) {
+            // where the first tile starts is worked out before the wait for the previous kernel
+            int tile_n = first_tile % p.n_tiles, tile_m = first_tile / p.n_tiles;
+            int img = tile_m * kBM / (p.oh * p.ow);
+            int rem = tile_m * kBM - img * (p.oh * p.ow);
+            int oy = rem / p.ow, ox = rem - oy * p.ow;
+            int cb = 0, fx = 0, fy = 0;
+            if (kb != 0) {  // a later part of a split tile starts inside the filter
+                const int tap = kb / p.cblocks;
+                cb = kb - tap * p.cblocks;
+                fy = tap / p.taps_w;
+                fx = tap - fy * p.taps_w;
+            }
+            pdl_wait();  // from here on the kernel touches global memory
             if (p.b_resident) {
                 mbar_expect_tx(b_full, (uint32_t)(p.k_iters * C::kBBytes));
                 for (int it = 0; it < p.k_iters; ++it) {
@@ -440,19 +456,17 @@ __global__ void __launch_bounds__(f32_threads(BN), 1) conv_f32_umma_kernel(
             uint32_t phase = 0;
             bool ok = true;
             for (int tile = first_tile; tile < total_tiles && ok; tile += tile_step) {
-                const int tile_n = tile % p.n_tiles, tile_m = tile / p.n_tiles;
-                const int m0 = tile_m * kBM, n0 = tile_n * BN;
-                const int img = m0 / (p.oh * p.ow);
-                const int rem = m0 - img * (p.oh * p.ow);
-                const int oy = rem / p.ow, ox = rem - oy * p.ow;
-                const int base_w = ox * p.sw + p.base_w, base_h = oy * p.sh + p.base_h;
-                int cb = 0, fx = 0, fy = 0;
-                if (kb != 0) {  // a later part of a split tile starts inside the filter
-                    const int tap = kb / p.cblocks;
-                    cb = kb - tap * p.cblocks;
-                    fy = tap / p.taps_w;
-                    fx = tap - fy * p.taps_w;
+                if (tile != first_tile) {
+                    tile_n = tile % p.n_tiles;
+                    tile_m = tile / p.n_tiles;
+                    img = tile_m * kBM / (p.oh * p.ow);
+                    rem = tile_m * kBM - img * (p.oh * p.ow);
+                    oy = rem / p.ow;
+                    ox = rem - oy * p.ow;
+                    cb = fx = fy = 0;
                 }
+                const int m0 = tile_m * kBM, n0 = tile_n * BN;
+                const int base_w = ox * p.sw + p.base_w, base_h = oy * p.sh + p.base_h;
                 for (int it = kb; it < ke; ++it) {
                     if (!mbar_wait(&empty_bar[s], phase ^ 1u, abort_flag, p.wait_cycles)) {
                         give_up(ERR_PRODUCER_WAIT);
@@ -671,6 +685,7 @@ __global__ void __launch_bounds__(f32_threads(BN), 1) conv_f32_umma_kernel(
         constexpr int kChunks = kCols / 16;  // ... in 16-column loads
         int local = 0;
         bool ok = true;
+        pdl_wait();  // before the first read of z and the first store
         for (int tile = first_tile; tile < total_tiles && ok; tile += tile_step) {
             const int tile_n = tile % p.n_tiles, tile_m = tile / p.n_tiles;
             const int m = tile_m * kBM + row, n0 = tile_n * BN;
@@ -750,20 +765,29 @@ __global__ void __launch_bounds__(f32_threads(BN), 1) conv_f32_umma_kernel(
                 const int m = tile_m * kBM + r, ch = tile_n * BN + c;
                 if (m >= p.m_total || ch >= p.oc)
                     continue;
-                float v[4] = {0.f, 0.f, 0.f, 0.f};
-                for (int i = 0; i < p.splits; ++i) {
-                    uint32_t addr;
-                    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;"
-                                 : "=r"(addr)
-                                 : "r"(part + (uint32_t)((r * C::kPartPitch + c) * 4)), "r"(i));
-                    float x[4];
-                    asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];"
-                                 : "=f"(x[0]), "=f"(x[1]), "=f"(x[2]), "=f"(x[3])
-                                 : "r"(addr)
-                                 : "memory");
+                // all parts' loads are in flight together (a remote load takes some 250 clocks)
+                float x[8][4];
 #pragma unroll
-                    for (int j = 0; j < 4; ++j)
-                        v[j] = __fadd_rn(v[j], x[j]);
+                for (int i = 0; i < 8; ++i) {
+                    if (i < p.splits) {
+                        uint32_t addr;
+                        asm volatile("mapa.shared::cluster.u32 %0, %1, %2;"
+                                     : "=r"(addr)
+                                     : "r"(part + (uint32_t)((r * C::kPartPitch + c) * 4)), "r"(i));
+                        asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];"
+                                     : "=f"(x[i][0]), "=f"(x[i][1]), "=f"(x[i][2]), "=f"(x[i][3])
+                                     : "r"(addr)
+                                     : "memory");
+                    }
+                }
+                float v[4] = {x[0][0], x[0][1], x[0][2], x[0][3]};
+#pragma unroll
+                for (int i = 1; i < 8; ++i) {
+                    if (i < p.splits) {
+#pragma unroll
+                        for (int j = 0; j < 4; ++j)
+                            v[j] = __fadd_rn(v[j], x[i][j]);
+                    }
                 }
                 float* out = p.ep.dst + (size_t)m * p.ep.dst_pitch + ch;
                 const float* zin = p.ep.z ? p.ep.z + (size_t)m * p.ep.z_pitch + ch : nullptr;
@@ -902,12 +926,26 @@ int grid_1d(size_t work, int block) {
 constexpr int kF32TileBudget = 227 * 1024 - 1024 - 1024;
 
 template <int BN, int ROWB>
+bool f32_kernel_ready() {
+    static KernelReady ready;
+    return ready.smem(conv_f32_umma_kernel<BN, ROWB>, kF32TileBudget + 2048);
+}
+
+template <int BN, int ROWB>
+int f32_clusters(int size) {
+    static ClusterCapacity capacity;
+    if (!f32_kernel_ready<BN, ROWB>())
+        return 0;
+    return capacity.clusters(conv_f32_umma_kernel<BN, ROWB>, size, f32_threads(BN),
+                             kF32TileBudget + 2048);
+}
+
+template <int BN, int ROWB>
 int launch_f32_kernel(
         const CUtensorMap& ma, const CUtensorMap& mb, F32ConvParams& p, cudaStream_t st) {
     using C = F32Cfg<BN, ROWB>;
     constexpr int kDynamic = kF32TileBudget + 2048;
-    static KernelReady ready;
-    if (!ready.smem(conv_f32_umma_kernel<BN, ROWB>, kDynamic))
+    if (!f32_kernel_ready<BN, ROWB>())
         return check_launch("conv_f32_umma smem attribute");
     // The filter stays resident where one tile column covers the channels and at least five
     // A stages fit behind it (a TMA round trip is four to five stages of conversion).
@@ -929,6 +967,16 @@ int launch_f32_kernel(
     return check_launch("conv_f32_umma");
 }
 
+int f32_cluster_capacity(int bn, int rowb, int size) {
+    if (rowb == 128)
+        return bn == 32   ? f32_clusters<32, 128>(size)
+               : bn == 64 ? f32_clusters<64, 128>(size)
+                          : f32_clusters<128, 128>(size);
+    return bn == 32   ? f32_clusters<32, 64>(size)
+           : bn == 64 ? f32_clusters<64, 64>(size)
+                      : f32_clusters<128, 64>(size);
+}
+
 // Tile width and K split for a problem of `m_tiles` x `oc` with `k_iters` steps of `rowb` bytes:
 // the pair with the shortest estimated time of its busiest SM. Clocks per step and tile: 12
 // MMAs of 64 clocks for 128 columns, half that for 64, and for 32 what the handshakes of a step
@@ -940,13 +988,13 @@ void choose_f32_tile(int m_tiles, int oc, int k_iters, int rowb, int* bn, int* s
     for (int b = 128; b >= 32; b /= 2) {
         if (b > 32 && oc <= b / 2)
             continue;
-        const int step = (b == 128 ? 800 : b == 64 ? 460 : 380) * rowb / 128;
-        const int tile_end = b == 128 ? 1500 : b == 64 ? 900 : 600;  // sums, activation, stores
+        const int step = (b == 128 ? 850 : b == 64 ? 500 : 420) * rowb / 128;
+        const int tile_end = b == 128 ? 2500 : b == 64 ? 1500 : 1000;  // sums, activation, stores
         const long long tiles = (long long)m_tiles * ((oc + b - 1) / b);
         for (int s = 1; s <= 8; s *= 2) {
-            if (s > 1 && (tiles * s > sms / 8 * 8 || k_iters / s < 2))
+            if (s > 1 && (k_iters / s < 2 || tiles > sms / s || tiles > f32_cluster_capacity(b, rowb, s)))
                 break;
-            const long long waves = (tiles * s + sms - 1) / sms;
+            const long long waves = s > 1 ? 1 : (tiles + sms - 1) / sms;
             const long long clocks =
                     waves * ((long long)((k_iters + s - 1) / s) * step + tile_end) + (s > 1 ? 2500 : 0);
             if (best < 0 || clocks < best) {

@@ -148,6 +148,11 @@ __device__ __forceinline__ bool mbar_wait_u32(
     return mbar_try_wait_u32(bar, parity) || mbar_wait_slow(bar, parity, abort_flag, limit);
 }
 
+// brings a tensor map (a kernel parameter) into the descriptor cache ahead of its first use
+__device__ __forceinline__ void tma_prefetch_map(const CUtensorMap* map) {
+    asm volatile("prefetch.tensormap [%0];" ::"l"((uint64_t)map) : "memory");
+}
+
 __device__ __forceinline__ void tma_load_2d(
         void* smem, const CUtensorMap* map, uint64_t* bar, int c0, int c1) {
     asm volatile(
@@ -378,6 +383,38 @@ struct KernelReady {
         if (dev >= 0 && dev < 64)
             bytes_set[dev].store(bytes, std::memory_order_relaxed);
         return true;
+    }
+};
+
+// Clusters of `size` CTAs (one per SM) that the GPU holds at once: whole clusters live inside a
+// GPC, so for eight it is less than sm_count() / 8. Asked once per kernel, size and device.
+struct ClusterCapacity {
+    std::atomic<int> known[64][4] = {};
+    template <class Kernel>
+    int clusters(Kernel kernel, int size, int threads, int dynamic_smem) {
+        const int k = size == 2 ? 1 : size == 4 ? 2 : size == 8 ? 3 : 0;
+        int dev = 0;
+        if (k == 0 || cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64)
+            return 0;
+        int n = known[dev][k].load(std::memory_order_relaxed);
+        if (n == 0) {
+            cudaLaunchConfig_t cfg = {};
+            cfg.gridDim = dim3((unsigned)(sm_count() / size * size));
+            cfg.blockDim = dim3((unsigned)threads);
+            cfg.dynamicSmemBytes = (size_t)dynamic_smem;
+            cudaLaunchAttribute attr;
+            attr.id = cudaLaunchAttributeClusterDimension;
+            attr.val.clusterDim.x = (unsigned)size;
+            attr.val.clusterDim.y = attr.val.clusterDim.z = 1;
+            cfg.attrs = &attr;
+            cfg.numAttrs = 1;
+            if (cudaOccupancyMaxActiveClusters(&n, kernel, &cfg) != cudaSuccess || n <= 0) {
+                cudaGetLastError();
+                n = sm_count() / size * 3 / 4;
+            }
+            known[dev][k].store(n, std::memory_order_relaxed);
+        }
+        return n;
     }
 };
 
