@@ -16,6 +16,8 @@ NVCC_FLAGS = [
     "-gencode", "arch=compute_100a,code=sm_100a", "-lineinfo", "-Wno-deprecated-gpu-targets", "-O3", "-std=c++17",
     "-fmad=false", "-Xcompiler", "-fPIC", "-Xcompiler", "-fvisibility=hidden",
     "-Xcompiler", "-Wall", "-Xptxas", "-v",
+    # the kernels of a file on several cores: the tensor-core files hold dozens of instantiations
+    "-split-compile", "4",
 ]
 
 

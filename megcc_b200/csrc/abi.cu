@@ -96,7 +96,8 @@ const TuningField kTuningFields[] = {
         {"patch_ctas", "MB200_PATCH_CTAS", &Tuning::patch_ctas, false},
         {"patch_alone", "MB200_PATCH_ALONE", &Tuning::patch_alone, false},
         {"patch_plain", "MB200_PATCH_PLAIN", &Tuning::patch_plain, false},
-        {"overlap_loads", "MB200_OVERLAP_LOADS", &Tuning::overlap_loads, false},
+        {"epilogue_forms", "MB200_EPILOGUE_FORMS", &Tuning::epilogue_forms, false},
+        {"conv_csplit", "MB200_CONV_CSPLIT", &Tuning::conv_csplit, false},
         {"f32_bn", "MB200_F32_BN", &Tuning::f32_bn, false},
         {"f32_split", "MB200_F32_SPLIT", &Tuning::f32_split, false},
         {"dw_tensor", "MB200_DW_TENSOR", &Tuning::dw_tensor, false},

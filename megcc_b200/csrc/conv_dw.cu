@@ -19,6 +19,7 @@
 #include <stdlib.h>
 
 #include "internal.h"
+#include "pdl.h"
 #include "tuning.h"
 
 namespace mb200 {
@@ -56,6 +57,7 @@ __global__ void __launch_bounds__(256) conv_dw_kernel(
     extern __shared__ uint4 w_smem[];  // [kTapWords][4 quads][c16] vectors of 4 channels
     const ConvArgs& a = p.a;
     constexpr int kTaps = KH * KW;
+    pdl_start();
     for (int c = threadIdx.x; c < a.ic; c += blockDim.x) {
         uint32_t w[kTapWords] = {0, 0, 0};
         for (int t = 0; t < kTaps; ++t)
@@ -182,6 +184,7 @@ __global__ void __launch_bounds__(128, OUT == 4 ? 4 : 6) conv_dw3x3_row_kernel(
     extern __shared__ uint4 w_smem[];  // [3 dx][4 quads][c16] vectors of 4 channel words
     const ConvArgs& a = p.a;
     constexpr int kOut = OUT, kCols = (kOut - 1) * S + 3;
+    pdl_start();
     for (int c = threadIdx.x; c < a.ic; c += blockDim.x) {
         const int cvv = c >> 4, q = (c >> 2) & 3, i = c & 3;
 #pragma unroll
@@ -350,16 +353,16 @@ int launch_conv_dw(
             cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) !=
                     cudaSuccess)
             return check_launch("conv_dw smem attribute");
-        kernel<<<(int)blocks, 128, smem, st>>>(p, (const uint4*)src, flt, bias, flt_scales,
-                                               (uint4*)dst);
+        launch_pdl(kernel, dim3((unsigned)blocks), dim3(128), (size_t)smem, st, p, (const uint4*)src,
+                   flt, bias, flt_scales, (uint4*)dst);
         return check_launch("conv_dw_row");
     }
     if (smem > 48 * 1024 &&
         cudaFuncSetAttribute(conv_dw_kernel<3, 3>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                              smem) != cudaSuccess)
         return check_launch("conv_dw smem attribute");
-    conv_dw_kernel<3, 3><<<(int)grid, 256, smem, st>>>(
-            p, (const uint4*)src, flt, bias, flt_scales, (uint4*)dst);
+    launch_pdl(conv_dw_kernel<3, 3>, dim3((unsigned)grid), dim3(256), (size_t)smem, st, p,
+               (const uint4*)src, flt, bias, flt_scales, (uint4*)dst);
     return check_launch("conv_dw");
 }
 

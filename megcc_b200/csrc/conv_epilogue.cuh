@@ -137,6 +137,30 @@ __device__ __forceinline__ void requant_pair(
     asm("cvt.rzi.sat.s8.f32 %0, %1;" : "=r"(q1) : "f"(y1));
 }
 
+// The same with one filter scale per value (one per output channel)
+template <int ACT>
+__device__ __forceinline__ void requant_pair_chain(
+        int acc0, int acc1, uint64_t s_flt, const EpilogueParams& e, int& q0, int& q1) {
+    const uint64_t f = f2_pack(__int2float_rn(acc0), __int2float_rn(acc1));
+    const uint64_t t = f2_mul(f2_mul(f, f2_pack(e.s_src, e.s_src)), s_flt);
+    const uint64_t inv = f2_pack(e.inv_dst, e.inv_dst);
+    const uint64_t qa = f2_mul(t, inv);
+    const uint64_t rem = f2_fma(qa, f2_pack(-e.s_dst, -e.s_dst), t);
+    const uint64_t x = f2_fma(rem, inv, qa);
+    uint64_t y;
+    if (ACT == ACT_RELU) {
+        y = f2_add(x, f2_pack(0.49999997f, 0.49999997f));
+    } else {
+        float x0, x1;
+        f2_unpack(x, x0, x1);
+        y = f2_add(x, f2_pack(copysignf(0.49999997f, x0), copysignf(0.49999997f, x1)));
+    }
+    float y0, y1;
+    f2_unpack(y, y0, y1);
+    asm("cvt.rzi.sat.s8.f32 %0, %1;" : "=r"(q0) : "f"(y0));
+    asm("cvt.rzi.sat.s8.f32 %0, %1;" : "=r"(q1) : "f"(y1));
+}
+
 // The verified form (EpilogueParams::fast_mul / fast_add) on two accumulators: ONE fused
 // multiply-add, trunc(fma((float)acc, c, +-d)), saturated. It is written as an explicit fma because
 // the assembler contracts a packed multiply followed by a packed add into one anyway (seen on
@@ -397,74 +421,148 @@ __device__ __forceinline__ uint32_t epilogue_word(
     return umma::pack4_prmt(r0, r1, r2, r3);
 }
 
-// run-time dispatch on (activation, per-channel scales, bounded, fused step); uniform across
-// the CTA. `off` is the element offset of the pixel's first channel of this chunk in the
-// output tensor (and in z, which has the same shape).
-// ---- one 32-column chunk with its TMEM load split in two ----
-// The epilogue warps are bound by the latency of their own chain (wait, tcgen05.ld,
-// requantisation, store), so the chunk's accumulators are fetched as two 16-column loads and
-// the second is in flight while the first half is requantised (halo-patch kernel, batch 256,
-// same box: first layer 134 -> 117 us with its space-to-depth pass, 64 -> 64 layers 44 -> 40 us).
-// Written for the two commonest epilogues only, each with everything fixed at compile time:
-// RELU and QFUSE_ADD_RELU in the verified one-FMA form; everything else takes
-// epilogue_store(). How this is compiled decides whether it pays: twelve instantiations (every
-// verified form and activation) made the compiler spill the accumulators in the tile loop
-// (first layer 142 us), one instantiation per fused-step mode with the operation count and
-// the activation as run-time values was slower than no overlap at all (149 against 141 us),
-// and as functions of their own (__noinline__) the variants crash ptxas 12.9.
-//
-// Can the chunk at channel ch0 take this path? (Uniform over the warp.)
-__device__ __forceinline__ bool epilogue_chunk_overlappable(
-        const EpilogueParams& e, const int8_t* dst, int ch0) {
-    if (e.fast_ops != 1 || e.acc_out || e.flt_scales || (e.oc % 32) != 0 || ch0 + 32 > e.oc)
-        return false;
-    if (((uintptr_t)dst & 31) != 0)
-        return false;
-    // the two commonest epilogues only: RELU without a fused step, QFUSE_ADD_RELU
-    if (!(e.z_mode == 0 && e.act == ACT_RELU) && e.z_mode != 2)
-        return false;
-    if (e.z_mode != 0 && (e.z_fast_a == 0.f || ((uintptr_t)e.z & 31) != 0))
-        return false;
-    return true;
+// Four consecutive channels (from ch0, a multiple of 4) of one output pixel, every epilogue: the
+// reference's float operations in their order. For the CTAs of a split tile, where a thread
+// finishes a few channels only and code that stays small matters more than operations saved.
+__device__ __forceinline__ void epilogue_quad(
+        const int (&acc)[4], const EpilogueParams& e, int8_t* dst, size_t off, int ch0) {
+    int r[4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        const bool in = ch0 + i < e.oc;
+        const int a = acc[i] + (in && e.bias ? e.bias[ch0 + i] : 0);
+        if (e.acc_out) {
+            if (in)
+                e.acc_out[off + i] = a;
+            continue;
+        }
+        const float s = in && e.flt_scales ? e.flt_scales[ch0 + i] : e.s_flt;
+        const float t = __fmul_rn(__fmul_rn(__int2float_rn(a), e.s_src), s);
+        r[i] = round_clamp_s8(apply_act(e.act, div_rn_by_const(t, e.s_dst, e.inv_dst)));
+        if (e.z_mode != 0 && in) {
+            const int zv = (int)e.z[off + i];
+            r[i] = e.z_mode == 1 ? fuse_z<1>(r[i], zv, e) : fuse_z<2>(r[i], zv, e);
+        }
+    }
+    if (e.acc_out)
+        return;
+    if ((e.oc & 3) == 0 && ((uintptr_t)dst & 3) == 0) {
+        *reinterpret_cast<uint32_t*>(dst + off) = umma::pack4_prmt(r[0], r[1], r[2], r[3]);
+    } else {
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+            if (ch0 + i < e.oc)
+                dst[off + i] = (int8_t)r[i];
+    }
 }
 
-// ZMODE 0: ConvBias with RELU; 2: QFUSE_ADD_RELU behind an IDENTITY ConvBias. `release_bar`
-// (or null): the accumulator buffer's "drained" barrier, on which the thread arrives once all
-// its accumulators are in registers. Every lane of the warp must call (the loads are
-// warp-wide); `valid` guards the reads of z and the store.
-template <int ZMODE>
-__device__ __forceinline__ void epilogue_chunk_overlapped_t(
-        uint32_t taddr, const EpilogueParams& e, int8_t* out, const int8_t* zin, int ch0,
-        bool valid, uint64_t* release_bar) {
+// ---- epilogues fixed at compile time ----
+// The kernels' hot loops are compiled once per form below and carry that epilogue only. With all
+// 33 run-time variants in one kernel (FORM_ANY, which stays for everything the forms leave out)
+// its register budget of 96 is a matter of luck: 20 bytes spilled in the tile loop cost a first
+// layer 25 %.
+//   FMA    per-tensor scales in the verified one-FMA form
+//   CHAIN  the reference's operations, two values per instruction: one scale per output channel
+//          (or per-tensor scales that have no one-FMA form)
+// each with RELU, without activation, or with a QFUSE_ADD_RELU step in its verified short form.
+enum EpilogueForm : int {
+    FORM_ANY = -1,
+    FORM_FMA_RELU = 0,
+    FORM_FMA_NONE = 1,
+    FORM_FMA_ADD_RELU = 2,
+    FORM_CHAIN_RELU = 3,
+    FORM_CHAIN_NONE = 4,
+    FORM_CHAIN_ADD_RELU = 5,
+};
+
+// host: the form a launch may use
+inline int epilogue_form(const EpilogueParams& e, const int8_t* dst) {
+    if (e.acc_out || (e.oc & 31) || ((uintptr_t)dst & 31) || e.act == ACT_H_SWISH)
+        return FORM_ANY;
+    int mode = e.act == ACT_RELU ? 0 : 1;
+    if (e.z_mode != 0) {
+        if (e.z_mode != 2 || e.z_fast_a == 0.f || ((uintptr_t)e.z & 31))
+            return FORM_ANY;
+        mode = 2;
+    }
+    if (e.fast_ops == 1 && !e.flt_scales)
+        return FORM_FMA_RELU + mode;
+    return e.flt_scales || e.bounded ? FORM_CHAIN_RELU + mode : FORM_ANY;
+}
+
+// Per-channel scales are on the device only: can any of the layer's results leave the range in
+// which one saturating conversion rounds and clamps (see EpilogueParams::bounded)? Every lane
+// of the warp calls.
+__device__ __forceinline__ bool chain_unbounded(const EpilogueParams& e) {
+    if (!e.flt_scales)
+        return false;
+    float most = 0.f;
+    for (int i = threadIdx.x & 31; i < e.oc; i += 32)
+        most = fmaxf(most, fabsf(e.flt_scales[i]));
+#pragma unroll
+    for (int d = 16; d > 0; d /= 2)
+        most = fmaxf(most, __shfl_xor_sync(0xffffffffu, most, d));
+    // (2^30 with room for the rounding of this estimate; NaN counts as out of range)
+    return !(fabsf(e.s_src) * most * fabsf(e.inv_dst) < 0.49f);
+}
+
+// One 32-column chunk: registers <- TMEM, requantisation, one 32-byte store. The chunk's
+// accumulators come as two 16-column loads of which the second is in flight while the first
+// half is requantised: the warps are bound by the latency of this chain. `release_bar` (or null):
+// the accumulator buffer's "drained" barrier, on which the thread arrives once all its
+// accumulators are in registers. Every lane of the warp must call (the loads are warp-wide);
+// `valid` guards the reads of z and the store.
+template <int FORM>
+__device__ __forceinline__ void epilogue_form_chunk(
+        uint32_t taddr, const EpilogueParams& e, int8_t* dst, size_t off, int ch0, bool valid,
+        bool unbounded, uint64_t* release_bar) {
+    constexpr bool kChain = FORM >= FORM_CHAIN_RELU;
+    constexpr int kMode = FORM % 3;
+    constexpr int kAct = kMode == 0 ? ACT_RELU : ACT_IDENTITY;
     uint32_t lo[16], hi[16], packed[8], zw[8];
     umma::tmem_ld16_nowait(taddr, lo);
-    if (ZMODE != 0 && valid)
+    if (kMode == 2 && valid)
         asm volatile("ld.global.nc.v8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
                      : "=r"(zw[0]), "=r"(zw[1]), "=r"(zw[2]), "=r"(zw[3]), "=r"(zw[4]),
                        "=r"(zw[5]), "=r"(zw[6]), "=r"(zw[7])
-                     : "l"(zin));
+                     : "l"(e.z + off));
     const int4* bias4 = reinterpret_cast<const int4*>(e.bias ? e.bias + ch0 : kZeroBias);
-    constexpr bool relu = ZMODE == 0;
     umma::tmem_ld_wait16(lo);
     umma::tmem_ld16_nowait(taddr + 16u, hi);
     auto half = [&](const uint32_t (&v)[16], int base) {
 #pragma unroll
         for (int j = 0; j < 4; ++j) {
             const int4 b = __ldg(bias4 + base + j);
+            const int a0 = (int)v[4 * j] + b.x, a1 = (int)v[4 * j + 1] + b.y,
+                      a2 = (int)v[4 * j + 2] + b.z, a3 = (int)v[4 * j + 3] + b.w;
             int r0, r1, r2, r3;
-            constexpr int kAct = ZMODE == 0 ? ACT_RELU : ACT_IDENTITY;
-            requant_pair_fast<kAct, 1>((int)v[4 * j] + b.x, (int)v[4 * j + 1] + b.y, e, r0, r1);
-            requant_pair_fast<kAct, 1>((int)v[4 * j + 2] + b.z, (int)v[4 * j + 3] + b.w, e, r2, r3);
-            if (ZMODE != 0) {
+            if constexpr (!kChain) {
+                requant_pair_fast<kAct, 1>(a0, a1, e, r0, r1);
+                requant_pair_fast<kAct, 1>(a2, a3, e, r2, r3);
+            } else {
+                float4 s = make_float4(e.s_flt, e.s_flt, e.s_flt, e.s_flt);
+                if (e.flt_scales)
+                    s = __ldg(reinterpret_cast<const float4*>(e.flt_scales + ch0) + base + j);
+                if (unbounded) {
+                    r0 = requant_one<kAct, false>(a0, e.s_src, s.x, e.s_dst, e.inv_dst);
+                    r1 = requant_one<kAct, false>(a1, e.s_src, s.y, e.s_dst, e.inv_dst);
+                    r2 = requant_one<kAct, false>(a2, e.s_src, s.z, e.s_dst, e.inv_dst);
+                    r3 = requant_one<kAct, false>(a3, e.s_src, s.w, e.s_dst, e.inv_dst);
+                } else {
+                    requant_pair_chain<kAct>(a0, a1, f2_pack(s.x, s.y), e, r0, r1);
+                    requant_pair_chain<kAct>(a2, a3, f2_pack(s.z, s.w), e, r2, r3);
+                }
+            }
+            if (kMode == 2) {
                 const uint32_t z = zw[base + j];
-                r0 = fuse_z_fast<ZMODE>(r0, (int)(int8_t)(z), e.z_fast_a, e.z_fast_b);
-                r1 = fuse_z_fast<ZMODE>(r1, (int)(int8_t)(z >> 8), e.z_fast_a, e.z_fast_b);
-                r2 = fuse_z_fast<ZMODE>(r2, (int)(int8_t)(z >> 16), e.z_fast_a, e.z_fast_b);
-                r3 = fuse_z_fast<ZMODE>(r3, (int)(int8_t)(z >> 24), e.z_fast_a, e.z_fast_b);
+                r0 = fuse_z_fast<2>(r0, (int)(int8_t)(z), e.z_fast_a, e.z_fast_b);
+                r1 = fuse_z_fast<2>(r1, (int)(int8_t)(z >> 8), e.z_fast_a, e.z_fast_b);
+                r2 = fuse_z_fast<2>(r2, (int)(int8_t)(z >> 16), e.z_fast_a, e.z_fast_b);
+                r3 = fuse_z_fast<2>(r3, (int)(int8_t)(z >> 24), e.z_fast_a, e.z_fast_b);
             }
             const uint32_t pk = umma::pack4_prmt(r0, r1, r2, r3);
             // RELU of the ConvBias, or of the fused sum, on packed bytes
-            packed[base + j] = (relu || ZMODE == 2) ? relu_s8x4(pk) : pk;
+            packed[base + j] = kMode == 1 ? pk : relu_s8x4(pk);
         }
     };
     half(lo, 0);
@@ -476,24 +574,15 @@ __device__ __forceinline__ void epilogue_chunk_overlapped_t(
     }
     half(hi, 4);
     if (valid)
-        asm volatile("st.global.v8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"l"(out),
+        asm volatile("st.global.v8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"l"(dst + off),
                      "r"(packed[0]), "r"(packed[1]), "r"(packed[2]), "r"(packed[3]),
                      "r"(packed[4]), "r"(packed[5]), "r"(packed[6]), "r"(packed[7])
                      : "memory");
 }
 
-// `taddr`: the chunk's first TMEM column for this thread's lane; `off`: element offset of the
-// pixel's channel ch0 in dst (and z). The caller has checked epilogue_chunk_overlappable().
-__device__ __forceinline__ void epilogue_chunk_overlapped(
-        uint32_t taddr, const EpilogueParams& e, int8_t* dst, size_t off, int ch0, bool valid,
-        uint64_t* release_bar) {
-    int8_t* out = dst + off;
-    if (e.z_mode == 0)
-        epilogue_chunk_overlapped_t<0>(taddr, e, out, nullptr, ch0, valid, release_bar);
-    else
-        epilogue_chunk_overlapped_t<2>(taddr, e, out, e.z + off, ch0, valid, release_bar);
-}
-
+// run-time dispatch on (activation, per-channel scales, bounded, fused step); uniform across
+// the CTA. `off` is the element offset of the pixel's first channel of this chunk in the
+// output tensor (and in z, which has the same shape).
 template <int NV>
 __device__ __forceinline__ void epilogue_store(
         const uint32_t (&v)[NV], const EpilogueParams& e, int8_t* dst, size_t off, int ch0) {

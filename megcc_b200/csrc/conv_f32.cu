@@ -331,16 +331,6 @@ __device__ __forceinline__ void split_tf32(uint32_t v, uint32_t& hi, uint32_t& l
     lo = __float_as_uint(__fsub_rn(__uint_as_float(v), __uint_as_float(hi)));
 }
 
-__device__ __forceinline__ uint32_t f32_cluster_rank() {
-    uint32_t r;
-    asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
-    return r;
-}
-__device__ __forceinline__ void f32_cluster_sync() {
-    asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
-    asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
-}
-
 template <int BN, int ROWB>
 __global__ void __launch_bounds__(f32_threads(BN), 1) conv_f32_umma_kernel(
         const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b,
@@ -371,7 +361,7 @@ __global__ void __launch_bounds__(f32_threads(BN), 1) conv_f32_umma_kernel(
     const int total_tiles = p.m_tiles * p.n_tiles;
     // Work of this CTA. Split: one tile per cluster, a K range per CTA; else whole tiles, one
     // every gridDim.x.
-    const int rank = p.splits > 1 ? (int)f32_cluster_rank() : 0;
+    const int rank = p.splits > 1 ? (int)cluster_rank() : 0;
     const int first_tile = (int)blockIdx.x / p.splits;
     const int tile_step = p.splits > 1 ? total_tiles : (int)gridDim.x;
     const int my_tiles =
@@ -754,7 +744,7 @@ __global__ void __launch_bounds__(f32_threads(BN), 1) conv_f32_umma_kernel(
     if (p.splits > 1) {
         // every CTA of the cluster comes here, whatever became of its waits
         __syncwarp();
-        f32_cluster_sync();  // the partial tiles are in place
+        cluster_barrier();  // the partial tiles are in place
         const int et = (int)threadIdx.x - 64;
         if (et >= 0 && et < 32 * kF32EpilogueWarps && !*abort_flag) {
             const int rows = kBM / p.splits;
@@ -766,27 +756,21 @@ __global__ void __launch_bounds__(f32_threads(BN), 1) conv_f32_umma_kernel(
                 if (m >= p.m_total || ch >= p.oc)
                     continue;
                 // all parts' loads are in flight together (a remote load takes some 250 clocks)
-                float x[8][4];
+                const uint32_t at = part + (uint32_t)((r * C::kPartPitch + c) * 4);
+                uint4 x[8];
 #pragma unroll
-                for (int i = 0; i < 8; ++i) {
-                    if (i < p.splits) {
-                        uint32_t addr;
-                        asm volatile("mapa.shared::cluster.u32 %0, %1, %2;"
-                                     : "=r"(addr)
-                                     : "r"(part + (uint32_t)((r * C::kPartPitch + c) * 4)), "r"(i));
-                        asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];"
-                                     : "=f"(x[i][0]), "=f"(x[i][1]), "=f"(x[i][2]), "=f"(x[i][3])
-                                     : "r"(addr)
-                                     : "memory");
-                    }
-                }
-                float v[4] = {x[0][0], x[0][1], x[0][2], x[0][3]};
+                for (int i = 0; i < 8; ++i)
+                    if (i < p.splits)
+                        x[i] = ld_cluster_v4(at, i);
+                float v[4] = {__uint_as_float(x[0].x), __uint_as_float(x[0].y),
+                              __uint_as_float(x[0].z), __uint_as_float(x[0].w)};
 #pragma unroll
                 for (int i = 1; i < 8; ++i) {
                     if (i < p.splits) {
-#pragma unroll
-                        for (int j = 0; j < 4; ++j)
-                            v[j] = __fadd_rn(v[j], x[i][j]);
+                        v[0] = __fadd_rn(v[0], __uint_as_float(x[i].x));
+                        v[1] = __fadd_rn(v[1], __uint_as_float(x[i].y));
+                        v[2] = __fadd_rn(v[2], __uint_as_float(x[i].z));
+                        v[3] = __fadd_rn(v[3], __uint_as_float(x[i].w));
                     }
                 }
                 float* out = p.ep.dst + (size_t)m * p.ep.dst_pitch + ch;
@@ -819,7 +803,7 @@ __global__ void __launch_bounds__(f32_threads(BN), 1) conv_f32_umma_kernel(
             }
         }
         __syncwarp();
-        f32_cluster_sync();  // nobody leaves while its partial tile may still be read
+        cluster_barrier();  // nobody leaves while its partial tile may still be read
     }
 
     // ---------------- teardown ----------------

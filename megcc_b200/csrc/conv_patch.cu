@@ -64,6 +64,7 @@ struct PatchParams {
     int kh, kw, ph, pw;
     int pph, ppw;    // input patch extent: kTH + kh - 1, kTW + kw - 1
     int tiles_y, tiles_x, m_tiles, n_tiles;
+    int s_img, s_ty, s_tx;  // a CTA's step from patch to patch (gridDim.x / n_tiles patches)
     int stages;
     int a_stage_bytes, a_tx_bytes, b_bytes;
     int plane_stride;  // one chunk plane: pph x ppw pixels of 16 bytes
@@ -73,7 +74,6 @@ struct PatchParams {
     int a_lbo;        // distance between the two 16-byte K halves of one A operand
     // Depthwise form (64-channel rows kernel only): the raw filter [C][3][3]. Each CTA then
     // convolves input channels n0 .. n0+63 with the block-diagonal operand it builds itself.
-    int overlap;  // 1: chunks of the verified short forms load their accumulators in two halves
     const int8_t* dw_flt;
     // 1: the depthwise tensor has 32 channels and is seen as pixel PAIRS of 64 bytes
     // ([N][H][W/2][2][32]); column 32 h + c of a row is channel c of the pair's pixel h
@@ -83,38 +83,30 @@ struct PatchParams {
     int* status;
 };
 
-// Position of a CTA's current patch (image, patch row, patch column) and the step to its
-// next one, kept as three counters with carries: one division at the start, none per tile.
-// (With 64 output channels an epilogue warp does one 32-column chunk per tile, so whatever
-// the tile decode costs is paid per chunk.)
+// Position of a CTA's current patch (image, patch row, patch column); the step to its next one
+// comes with the parameters (the grid is known to the launcher), so the walk is three counters
+// with carries: one division at the start, none per tile, and no registers for the steps.
 struct PatchWalker {
     int img, ty, tx;
-    int s_img, s_ty, s_tx;
-    int tiles_y, tiles_x;
-    __device__ __forceinline__ PatchWalker(int first, int step, int ty_n, int tx_n)
-            : tiles_y(ty_n), tiles_x(tx_n) {
-        const int per_image = ty_n * tx_n;
+    __device__ __forceinline__ PatchWalker(int first, const PatchParams& p) {
+        const int per_image = p.tiles_y * p.tiles_x;
         img = first / per_image;
         int r = first - img * per_image;
-        ty = r / tx_n;
-        tx = r - ty * tx_n;
-        s_img = step / per_image;
-        r = step - s_img * per_image;
-        s_ty = r / tx_n;
-        s_tx = r - s_ty * tx_n;
+        ty = r / p.tiles_x;
+        tx = r - ty * p.tiles_x;
     }
-    __device__ __forceinline__ void next() {
-        tx += s_tx;
-        if (tx >= tiles_x) {
-            tx -= tiles_x;
+    __device__ __forceinline__ void next(const PatchParams& p) {
+        tx += p.s_tx;
+        if (tx >= p.tiles_x) {
+            tx -= p.tiles_x;
             ++ty;
         }
-        ty += s_ty;
-        if (ty >= tiles_y) {
-            ty -= tiles_y;
+        ty += p.s_ty;
+        if (ty >= p.tiles_y) {
+            ty -= p.tiles_y;
             ++img;
         }
-        img += s_img;
+        img += p.s_img;
     }
 };
 
@@ -207,7 +199,7 @@ __device__ __forceinline__ void issue_tile_mmas_rows64(
     }
 }
 
-template <int BN, int KH, int KW, int CHUNKS, int EW, int ROWS = 0, int POOL = 0>
+template <int BN, int KH, int KW, int CHUNKS, int EW, int ROWS = 0, int POOL = 0, int FORM = FORM_ANY>
 __global__ void __launch_bounds__(64 + 32 * EW, EW == 16 ? 1 : 2) conv_patch_kernel(
         const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b,
         const PatchParams p) {
@@ -254,6 +246,9 @@ __global__ void __launch_bounds__(64 + 32 * EW, EW == 16 ? 1 : 2) conv_patch_ker
         mbar_init(drain_bar, 1);
         *abort_flag = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    } else if (threadIdx.x == 32 * 2) {
+        tma_prefetch_map(&map_a);
+        tma_prefetch_map(&map_b);
     }
     if constexpr (ROWS != 0) {
         if (p.dw_flt) {
@@ -330,8 +325,8 @@ __global__ void __launch_bounds__(64 + 32 * EW, EW == 16 ? 1 : 2) conv_patch_ker
             pdl_wait();  // activations: only once the previous kernel has completed
             int s = 0;
             uint32_t phase = 0;
-            PatchWalker at(m_first, m_step, p.tiles_y, p.tiles_x);
-            for (int mt = m_first; mt < p.m_tiles; mt += m_step, at.next()) {
+            PatchWalker at(m_first, p);
+            for (int mt = m_first; mt < p.m_tiles; mt += m_step, at.next(p)) {
                 if (!mbar_wait(&a_empty[s], phase ^ 1u, abort_flag)) {
                     if (!*abort_flag) {
                         *abort_flag = 1;
@@ -425,9 +420,9 @@ __global__ void __launch_bounds__(64 + 32 * EW, EW == 16 ? 1 : 2) conv_patch_ker
             if (p.ep.flt_scales)
                 pool_scales = __ldg(reinterpret_cast<const float4*>(p.ep.flt_scales + pool_ch));
         }
-        const bool overlap_ok = POOL == 0 && p.overlap && epilogue_chunk_overlappable(p.ep, p.dst, 0);
-        PatchWalker at(m_first, m_step, p.tiles_y, p.tiles_x);
-        for (int mt = m_first; mt < p.m_tiles && ok; mt += m_step, ++local, at.next()) {
+        const bool unbounded = FORM >= FORM_CHAIN_RELU && chain_unbounded(p.ep);
+        PatchWalker at(m_first, p);
+        for (int mt = m_first; mt < p.m_tiles && ok; mt += m_step, ++local, at.next(p)) {
             const int buf = local & 1;
             const uint32_t acc_phase = (uint32_t)(local >> 1) & 1u;
             ok = mbar_wait(&acc_full[buf], acc_phase, abort_flag);
@@ -532,7 +527,7 @@ __global__ void __launch_bounds__(64 + 32 * EW, EW == 16 ? 1 : 2) conv_patch_ker
                 // pipelines: ask for the bytes this thread will want one tile from now, so
                 // that they wait in L2 instead of DRAM when the chunk below loads them.
                 PatchWalker nx = at;
-                nx.next();
+                nx.next(p);
                 const int ny = nx.ty * kTH + py, nxx = nx.tx * kTW + px;
                 if (mt + m_step < p.m_tiles && ny < p.oh && nxx < p.ow) {
                     const uint32_t npix = ((uint32_t)nx.img * p.oh + ny) * p.ow + nxx;
@@ -549,27 +544,31 @@ __global__ void __launch_bounds__(64 + 32 * EW, EW == 16 ? 1 : 2) conv_patch_ker
             // one 32-column chunk: registers <- TMEM, buffer released after the warp's last
             // load, requantisation, store
             auto do_chunk = [&](int c, bool last) {
-                if (overlap_ok && n0 + c * 32 + 32 <= p.oc) {
-                    // a verified short form: the chunk's second 16 columns are fetched while
-                    // the first are requantised
+                if constexpr (FORM != FORM_ANY) {
+                    // (the channel count is a multiple of 32: a chunk exists as a whole or not;
+                    // pixel pairs: bias and channel scales are those of channel column % 32)
                     const int ch0 = n0 + c * 32;
-                    epilogue_chunk_overlapped(
-                            taddr + (uint32_t)(c * 32), p.ep, p.dst, px_off + ch0,
-                            (ROWS != 0 && p.dw_pairs) ? (ch0 & 31) : ch0, valid,
-                            last ? &acc_empty[buf] : nullptr);
-                    return;
+                    uint64_t* release = last ? &acc_empty[buf] : nullptr;
+                    if (ch0 < p.oc)
+                        epilogue_form_chunk<FORM>(
+                                taddr + (uint32_t)(c * 32), p.ep, p.dst, px_off + ch0,
+                                (ROWS != 0 && p.dw_pairs) ? (ch0 & 31) : ch0, valid, unbounded,
+                                release);
+                    else if (release)
+                        mbar_arrive(release);
+                } else {
+                    uint32_t v[32];
+                    tmem_ld32(taddr + (uint32_t)(c * 32), v);
+                    if (last) {
+                        asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+                        mbar_arrive(&acc_empty[buf]);
+                    }
+                    const int ch0 = n0 + c * 32;
+                    if (valid && ch0 < p.oc)
+                        // (pixel pairs: bias and channel scales are those of channel column % 32)
+                        epilogue_store<32>(v, p.ep, p.dst, px_off + ch0,
+                                           (ROWS != 0 && p.dw_pairs) ? (ch0 & 31) : ch0);
                 }
-                uint32_t v[32];
-                tmem_ld32(taddr + (uint32_t)(c * 32), v);
-                if (last) {
-                    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-                    mbar_arrive(&acc_empty[buf]);
-                }
-                const int ch0 = n0 + c * 32;
-                if (valid && ch0 < p.oc)
-                    // (pixel pairs: bias and channel scales are those of channel column % 32)
-                    epilogue_store<32>(v, p.ep, p.dst, px_off + ch0,
-                                       (ROWS != 0 && p.dw_pairs) ? (ch0 & 31) : ch0);
             };
             if constexpr (kChunksPerWarp == 1) {
                 // Written as a strided loop of (at run time) one trip: with the chunk's code
@@ -673,31 +672,58 @@ PatchPlan plan_patch(const ConvArgs& a) {
     return pl;
 }
 
-template <int BN, int KH, int KW, int CHUNKS, int EW, int ROWS = 0, int POOL = 0>
-int launch_patch(
-        const CUtensorMap& ma, const CUtensorMap& mb, const PatchParams& p, int smem, int grid,
+template <int BN, int KH, int KW, int CHUNKS, int EW, int ROWS = 0, int POOL = 0, int FORM = FORM_ANY>
+int launch_patch_form(
+        const CUtensorMap& ma, const CUtensorMap& mb, PatchParams& p, int smem, int grid,
         cudaStream_t st) {
     constexpr int kThreads = 64 + 32 * EW;
-    if (cudaFuncSetAttribute(
-                conv_patch_kernel<BN, KH, KW, CHUNKS, EW, ROWS, POOL>,
-                cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess)
+    static KernelReady ready;
+    if (!ready.smem(conv_patch_kernel<BN, KH, KW, CHUNKS, EW, ROWS, POOL, FORM>, smem))
         return check_launch("conv_patch smem attribute");
     // never more CTAs than are resident at once: a persistent CTA that starts late would
     // leave its share of the patches to the end
-    const int per_sm = resident_ctas_per_sm(conv_patch_kernel<BN, KH, KW, CHUNKS, EW, ROWS, POOL>,
-                                            kThreads, smem, 2 * BN);
+    static ResidentCtas resident;
+    const int per_sm = resident.per_sm(conv_patch_kernel<BN, KH, KW, CHUNKS, EW, ROWS, POOL, FORM>,
+                                       kThreads, smem, 2 * BN);
     {
         int cap = sm_count() * per_sm / p.n_tiles * p.n_tiles;
         if (cap >= p.n_tiles && grid > cap)
             grid = cap;
     }
+    {
+        const int step = grid / p.n_tiles, per_image = p.tiles_y * p.tiles_x;
+        p.s_img = step / per_image;
+        p.s_ty = step % per_image / p.tiles_x;
+        p.s_tx = step % per_image % p.tiles_x;
+    }
     if (tuning().debug)
-        fprintf(stderr, "conv_patch<%d,%d,%d,%d,%d,%d,%d>: per_sm %d grid %d m_tiles %d n_tiles %d "
-                "smem %d stages %d b_single_load %d\n", BN, KH, KW, CHUNKS, EW, ROWS, POOL, per_sm,
+        fprintf(stderr, "conv_patch<%d,%d,%d,%d,%d,%d,%d,%d>: per_sm %d grid %d m_tiles %d n_tiles %d "
+                "smem %d stages %d b_single_load %d\n", BN, KH, KW, CHUNKS, EW, ROWS, POOL, FORM, per_sm,
                 grid, p.m_tiles, p.n_tiles, smem, p.stages, p.b_single_load);
-    launch_pdl(conv_patch_kernel<BN, KH, KW, CHUNKS, EW, ROWS, POOL>, dim3(grid), dim3(kThreads),
+    launch_pdl(conv_patch_kernel<BN, KH, KW, CHUNKS, EW, ROWS, POOL, FORM>, dim3(grid), dim3(kThreads),
                (size_t)smem, st, ma, mb, p);
     return check_launch("conv_patch");
+}
+
+// the instantiation with the launch's epilogue
+template <int BN, int KH, int KW, int CHUNKS, int EW, int ROWS = 0>
+int launch_patch(
+        const CUtensorMap& ma, const CUtensorMap& mb, PatchParams& p, int smem, int grid,
+        cudaStream_t st) {
+#define MB200_PATCH_FORM(F)                                                                    \
+    case F:                                                                                    \
+        return launch_patch_form<BN, KH, KW, CHUNKS, EW, ROWS, 0, F>(ma, mb, p, smem, grid, st);
+    switch (tuning().epilogue_forms ? epilogue_form(p.ep, p.dst) : FORM_ANY) {
+        MB200_PATCH_FORM(FORM_FMA_RELU)
+        MB200_PATCH_FORM(FORM_FMA_NONE)
+        MB200_PATCH_FORM(FORM_FMA_ADD_RELU)
+        MB200_PATCH_FORM(FORM_CHAIN_RELU)
+        MB200_PATCH_FORM(FORM_CHAIN_NONE)
+        MB200_PATCH_FORM(FORM_CHAIN_ADD_RELU)
+        default:
+            return launch_patch_form<BN, KH, KW, CHUNKS, EW, ROWS>(ma, mb, p, smem, grid, st);
+    }
+#undef MB200_PATCH_FORM
 }
 
 }  // namespace
@@ -898,7 +924,7 @@ int launch_conv_patch(
     p.ep.z_scale = a.z_scale;
     p.ep.z_div = 1.0f / a.z_out_scale;  // the reference's scale_div = 1.f / scale_dst
     p.ep.z_fast_a = p.ep.z_fast_b = 0.f;
-    if (p.ep.z_mode != 0 && p.ep.fast_ops != 0)
+    if (p.ep.z_mode != 0)
         residual_fast_constants(a.s_dst, a.z_scale, a.z_out_scale, p.ep.z_mode, &p.ep.z_fast_a,
                                 &p.ep.z_fast_b);
     if (tuning().debug)
@@ -907,7 +933,6 @@ int launch_conv_patch(
                 p.ep.z_fast_a,
                 p.ep.z_fast_b);
     p.ep.acc_out = a.acc_out;
-    p.overlap = tuning().overlap_loads;
     p.dw_flt = a.dw64 ? flt : nullptr;
     p.dw_pairs = a.dw64 == 2 ? 1 : 0;
     p.dst = dst;
@@ -925,22 +950,22 @@ int launch_conv_patch(
     int rc;
     const bool alone = pl.ctas_per_sm == 1;  // one CTA per SM: sixteen epilogue warps
     if (a.pool && a.kh == 4 && a.kw == 4 && a.ic == 16)
-        rc = launch_patch<64, 4, 4, 1, 8, 0, 1>(map_a, map_b, p, pl.smem_bytes, grid, st);
+        rc = launch_patch_form<64, 4, 4, 1, 8, 0, 1>(map_a, map_b, p, pl.smem_bytes, grid, st);
     else if (a.pool)
-        rc = launch_patch<64, 0, 0, 0, 8, 0, 1>(map_a, map_b, p, pl.smem_bytes, grid, st);
+        rc = launch_patch_form<64, 0, 0, 0, 8, 0, 1>(map_a, map_b, p, pl.smem_bytes, grid, st);
     else if (pl.rows64)
         rc = launch_patch<64, 3, 3, 4, 8, 1>(map_a, map_b, p, pl.smem_bytes, grid, st);
     else if (pl.bn == 64 && a.kh == 3 && a.kw == 3 && a.ic == 64 && !alone)
-        rc = launch_patch<64, 3, 3, 4, 8>(map_a, map_b, p, pl.smem_bytes, grid, st);
+        rc = launch_patch_form<64, 3, 3, 4, 8>(map_a, map_b, p, pl.smem_bytes, grid, st);
     else if (pl.bn == 64 && a.kh == 4 && a.kw == 4 && a.ic == 16 && !alone)
         rc = launch_patch<64, 4, 4, 1, 8>(map_a, map_b, p, pl.smem_bytes, grid, st);
     else if (pl.bn == 128 && a.kh == 3 && a.kw == 3 && a.ic == 128 && alone)
-        rc = launch_patch<128, 3, 3, 8, 16>(map_a, map_b, p, pl.smem_bytes, grid, st);
+        rc = launch_patch_form<128, 3, 3, 8, 16>(map_a, map_b, p, pl.smem_bytes, grid, st);
     else if (pl.bn == 64)
         // two 32-column chunks per lane quarter: eight epilogue warps at most
         rc = launch_patch<64, 0, 0, 0, 8>(map_a, map_b, p, pl.smem_bytes, grid, st);
     else
-        rc = alone ? launch_patch<128, 0, 0, 0, 16>(map_a, map_b, p, pl.smem_bytes, grid, st)
+        rc = alone ? launch_patch_form<128, 0, 0, 0, 16>(map_a, map_b, p, pl.smem_bytes, grid, st)
                    : launch_patch<128, 0, 0, 0, 8>(map_a, map_b, p, pl.smem_bytes, grid, st);
     return rc;
 }

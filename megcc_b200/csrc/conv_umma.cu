@@ -88,7 +88,8 @@ struct UmmaConvParams {
     // split-K (SPLITK kernels only): work items below `full_tiles` are whole tiles, the
     // tiles after them are cut into `split` parts of `k_per_part` pipeline steps each
     int full_tiles, split, k_per_part, total_items;
-    int overlap;          // 1: chunks of the verified short forms load their accumulators in two halves
+    // K split over a cluster (whole kernels without SPLITK): CTAs that share a tile's K loop, 1: none
+    int csplit;
     int4* slabs;          // [split item][chunk][16-byte group][row]: one part's accumulators
     unsigned* counters;   // [split tile] parts finished; zero between launches
 };
@@ -100,9 +101,14 @@ struct WorkItem {
 };
 
 template <bool SPLITK>
-__device__ __forceinline__ WorkItem decode_item(const UmmaConvParams& p, int item) {
+__device__ __forceinline__ WorkItem decode_item(const UmmaConvParams& p, int item, int rank) {
     WorkItem w;
-    if (!SPLITK || item < p.full_tiles) {
+    if (!SPLITK && p.csplit > 1) {
+        w.tile = item;
+        w.k0 = p.k_iters * rank / p.csplit;
+        w.k1 = p.k_iters * (rank + 1) / p.csplit;
+        w.slot = -1;
+    } else if (!SPLITK || item < p.full_tiles) {
         w.tile = item;
         w.k0 = 0;
         w.k1 = p.k_iters;
@@ -130,7 +136,7 @@ struct SmemLayout {
     static constexpr int kDynamic = kTotal + 1024;  // room to align the tiles to 1024 bytes
 };
 
-template <int BN, int GEOM, bool SPLITK = false>
+template <int BN, int GEOM, bool SPLITK = false, int FORM = FORM_ANY>
 __global__ void __launch_bounds__(Shape<BN>::kThreads, Shape<BN>::kMinCtas) conv_umma_kernel(
         const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b,
         const UmmaConvParams p) {
@@ -138,6 +144,8 @@ __global__ void __launch_bounds__(Shape<BN>::kThreads, Shape<BN>::kMinCtas) conv
     constexpr int kBKc = Geom<BN, GEOM>::kBKg;
     constexpr int kSt = Geom<BN, GEOM>::kStagesG;
     constexpr int kEpilogueWarps = Shape<BN>::kEpilogueWarps;
+    constexpr int kPartPitch = BN + 4;  // int32 per row of a split tile's share
+    static_assert(SPLITK || BN == 256 || kBM * kPartPitch * 4 <= L::kTiles, "the share takes the stages' place");
     extern __shared__ uint8_t smem_raw[];
     uint8_t* smem = (uint8_t*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
     uint8_t* tiles_a = smem;
@@ -154,6 +162,10 @@ __global__ void __launch_bounds__(Shape<BN>::kThreads, Shape<BN>::kMinCtas) conv
 
     const int warp = uniform_warp_index(), lane = threadIdx.x & 31;
     const int total_tiles = SPLITK ? p.total_items : p.m_tiles * p.n_tiles;
+    // split over a cluster: one tile per cluster, a K range per CTA
+    const int rank = !SPLITK && p.csplit > 1 ? (int)cluster_rank() : 0;
+    const int first_item = SPLITK ? (int)blockIdx.x : (int)blockIdx.x / p.csplit;
+    const int item_step = !SPLITK && p.csplit > 1 ? total_tiles : (int)gridDim.x;
 
     if (threadIdx.x == 0) {
         for (int s = 0; s < kStages; ++s) {
@@ -168,6 +180,9 @@ __global__ void __launch_bounds__(Shape<BN>::kThreads, Shape<BN>::kMinCtas) conv
         mbar_init(ep_bar, 32 * kEpilogueWarps);
         *abort_flag = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    } else if (threadIdx.x == 32 * 2) {
+        tma_prefetch_map(&map_a);
+        tma_prefetch_map(&map_b);
     }
     if (warp == 1) {
         asm volatile(
@@ -181,7 +196,7 @@ __global__ void __launch_bounds__(Shape<BN>::kThreads, Shape<BN>::kMinCtas) conv
     __syncthreads();
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     const uint32_t tmem_base = *tmem_slot;
-    pdl_start();  // set-up done: from here on the kernel touches global memory
+    pdl_release();  // set-up done: the next kernel may take the SMs this one leaves free
 
     if (warp == 0) {
         // ---------------- TMA producer ----------------
@@ -191,8 +206,8 @@ __global__ void __launch_bounds__(Shape<BN>::kThreads, Shape<BN>::kMinCtas) conv
             int s = 0;
             uint32_t phase = 0;
             bool ok = true;
-            for (int item = blockIdx.x; item < total_tiles && ok; item += gridDim.x) {
-                const WorkItem w = decode_item<SPLITK>(p, item);
+            for (int item = first_item; item < total_tiles && ok; item += item_step) {
+                const WorkItem w = decode_item<SPLITK>(p, item, rank);
                 const int tile = w.tile;
                 const int tile_n = tile % p.n_tiles, tile_m = tile / p.n_tiles;
                 const int m0 = tile_m * kBM, n0 = tile_n * BN;
@@ -201,13 +216,15 @@ __global__ void __launch_bounds__(Shape<BN>::kThreads, Shape<BN>::kMinCtas) conv
                 const int oy = rem / p.ow, ox = rem - oy * p.ow;
                 const int base_w = ox * p.sw + p.base_w, base_h = oy * p.sh + p.base_h;
                 int cb = 0, fx = 0, fy = 0;
-                if (SPLITK && w.k0 != 0) {
+                if (w.k0 != 0) {
                     // a later part of a split tile starts in the middle of the filter
                     cb = w.k0 % p.cblocks;
                     const int tap = w.k0 / p.cblocks;
                     fy = tap / p.taps_w;
                     fx = tap - fy * p.taps_w;
                 }
+                if (item == first_item)
+                    pdl_wait();  // (the first tile is worked out before the wait)
                 for (int it = w.k0; it < w.k1; ++it) {
                     if (!mbar_wait(&empty_bar[s], phase ^ 1u, abort_flag, p.wait_cycles)) {
                         if (!*abort_flag) {
@@ -288,8 +305,8 @@ __global__ void __launch_bounds__(Shape<BN>::kThreads, Shape<BN>::kMinCtas) conv
         uint32_t phase = 0, buf = 0, acc_parity = 1;
         int s = 0;
         bool ok = true;
-        for (int item = blockIdx.x; item < total_tiles && ok; item += gridDim.x) {
-            const WorkItem w = decode_item<SPLITK>(p, item);
+        for (int item = first_item; item < total_tiles && ok; item += item_step) {
+            const WorkItem w = decode_item<SPLITK>(p, item, rank);
             // the epilogue must have drained this accumulator buffer
             ok = mbar_wait_u32(acc_empty_a + 8 * buf, acc_parity, abort_flag, p.wait_cycles);
             if (!ok) {
@@ -340,9 +357,10 @@ __global__ void __launch_bounds__(Shape<BN>::kThreads, Shape<BN>::kMinCtas) conv
         int local = 0;
         bool ok = true;
         uint32_t ep_phase = 0;  // parity of the epilogue's own rendezvous (split-K)
-        const bool overlap_ok = p.overlap && epilogue_chunk_overlappable(p.ep, p.dst, 0);
-        for (int item = blockIdx.x; item < total_tiles && ok; item += gridDim.x, ++local) {
-            const WorkItem w = decode_item<SPLITK>(p, item);
+        pdl_wait();  // before the first read of z and the first store
+        const bool unbounded = FORM >= FORM_CHAIN_RELU && chain_unbounded(p.ep);
+        for (int item = first_item; item < total_tiles && ok; item += item_step, ++local) {
+            const WorkItem w = decode_item<SPLITK>(p, item, rank);
             const int tile = w.tile;
             const int buf = local & 1;
             const uint32_t acc_phase = (uint32_t)(local >> 1) & 1u;
@@ -436,30 +454,84 @@ __global__ void __launch_bounds__(Shape<BN>::kThreads, Shape<BN>::kMinCtas) conv
                 }
                 continue;
             }
+            if (!SPLITK && p.csplit > 1) {
+                // This CTA's share of the K loop: raw accumulators into shared memory in place
+                // of the stages (every load has been consumed, every MMA has retired); the
+                // cluster adds the shares up below.
+                int4* part = reinterpret_cast<int4*>(smem + (size_t)row * (kPartPitch * 4));
+#pragma unroll 1
+                for (int c = half * kChunksPerWarp; c < (half + 1) * kChunksPerWarp; ++c) {
+                    uint32_t v[32];
+                    tmem_ld32(taddr + (uint32_t)(c * 32), v);
+#pragma unroll
+                    for (int k = 0; k < 8; ++k)
+                        part[c * 8 + k] = make_int4((int)v[4 * k], (int)v[4 * k + 1],
+                                                    (int)v[4 * k + 2], (int)v[4 * k + 3]);
+                }
+                continue;
+            }
 #pragma unroll 1
             for (int c = half * kChunksPerWarp; c < (half + 1) * kChunksPerWarp; ++c) {
-                if (overlap_ok && n0 + c * 32 + 32 <= p.oc) {
-                    // a verified short form: the chunk's second 16 columns are fetched while
-                    // the first are requantised (conv_epilogue.cuh)
+                if constexpr (FORM != FORM_ANY) {
+                    // (the channel count is a multiple of 32: a chunk exists as a whole or not)
                     const int ch0 = n0 + c * 32;
-                    epilogue_chunk_overlapped(
-                            taddr + (uint32_t)(c * 32), p.ep, p.dst, (size_t)m * p.oc + ch0, ch0,
-                            m < p.m_total,
-                            c + 1 == (half + 1) * kChunksPerWarp ? &acc_empty[buf] : nullptr);
-                    continue;
+                    uint64_t* release =
+                            c + 1 == (half + 1) * kChunksPerWarp ? &acc_empty[buf] : nullptr;
+                    if (ch0 < p.oc) {
+                        epilogue_form_chunk<FORM>(taddr + (uint32_t)(c * 32), p.ep, p.dst,
+                                                  (size_t)m * p.oc + ch0, ch0, m < p.m_total,
+                                                  unbounded, release);
+                    } else if (release) {
+                        mbar_arrive(release);
+                    }
+                } else {
+                    uint32_t v[32];
+                    tmem_ld32(taddr + (uint32_t)(c * 32), v);
+                    if (c + 1 == (half + 1) * kChunksPerWarp) {
+                        // all of this thread's accumulators are in registers: hand the buffer back
+                        asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+                        mbar_arrive(&acc_empty[buf]);
+                    }
+                    const int ch0 = n0 + c * 32;
+                    if (m < p.m_total && ch0 < p.oc)
+                        epilogue_store<32>(v, p.ep, p.dst, (size_t)m * p.oc + ch0, ch0);
                 }
-                uint32_t v[32];
-                tmem_ld32(taddr + (uint32_t)(c * 32), v);
-                if (c + 1 == (half + 1) * kChunksPerWarp) {
-                    // all of this thread's accumulators are in registers: hand the buffer back
-                    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-                    mbar_arrive(&acc_empty[buf]);
-                }
-                const int ch0 = n0 + c * 32;
-                if (m < p.m_total && ch0 < p.oc)
-                    epilogue_store<32>(v, p.ep, p.dst, (size_t)m * p.oc + ch0, ch0);
             }
         }
+    }
+
+    if (!SPLITK && p.csplit > 1) {
+        // every CTA of the cluster comes here, whatever became of its waits; each finishes an
+        // equal share of the rows
+        __syncwarp();
+        cluster_barrier();  // the shares are in place
+        const int et = (int)threadIdx.x - 64;
+        if (et >= 0 && !*abort_flag) {
+            const int rows = kBM / p.csplit;
+            const int tile_n = first_item % p.n_tiles, tile_m = first_item / p.n_tiles;
+            for (int u = et; u < rows * (BN / 4); u += 32 * kEpilogueWarps) {
+                const int r = rank * rows + u / (BN / 4), c = (u % (BN / 4)) * 4;
+                const int m = tile_m * kBM + r, ch = tile_n * BN + c;
+                if (m >= p.m_total || ch >= p.oc)
+                    continue;
+                const uint32_t at = smem_u32(smem) + (uint32_t)((r * kPartPitch + c) * 4);
+                uint4 x[8];
+#pragma unroll
+                for (int i = 0; i < 8; ++i)  // all shares' loads in flight together
+                    x[i] = i < p.csplit ? ld_cluster_v4(at, i) : make_uint4(0, 0, 0, 0);
+                int v[4] = {0, 0, 0, 0};
+#pragma unroll
+                for (int i = 0; i < 8; ++i) {
+                    v[0] += (int)x[i].x;
+                    v[1] += (int)x[i].y;
+                    v[2] += (int)x[i].z;
+                    v[3] += (int)x[i].w;
+                }
+                epilogue_quad(v, p.ep, p.dst, (size_t)m * p.oc + ch, ch);
+            }
+        }
+        __syncwarp();
+        cluster_barrier();  // nobody leaves while its share may still be read
     }
 
     // ---------------- teardown ----------------
@@ -492,28 +564,97 @@ __global__ void __launch_bounds__(Shape<BN>::kThreads, Shape<BN>::kMinCtas) conv
 // ------------------------------------------------------------------------------------------
 // host side: tensor maps and launch
 // ------------------------------------------------------------------------------------------
-template <int BN, int GEOM, bool SPLITK = false>
-int launch_kernel(
+template <int BN, int GEOM, bool SPLITK = false, int FORM = FORM_ANY>
+bool umma_kernel_ready() {
+    static KernelReady ready;
+    return ready.smem(conv_umma_kernel<BN, GEOM, SPLITK, FORM>, SmemLayout<BN, GEOM>::kDynamic);
+}
+
+template <int BN, int GEOM, bool SPLITK = false, int FORM = FORM_ANY>
+int launch_form(
         const CUtensorMap& ma, const CUtensorMap& mb, const UmmaConvParams& p, cudaStream_t st) {
-    if (cudaFuncSetAttribute(
-                conv_umma_kernel<BN, GEOM, SPLITK>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                SmemLayout<BN, GEOM>::kDynamic) != cudaSuccess)
+    if (!umma_kernel_ready<BN, GEOM, SPLITK, FORM>())
         return check_launch("conv_umma smem attribute");
     // persistent CTAs: as many as the SM holds at once
     constexpr int kThreads = Shape<BN>::kThreads;
-    const int per_sm = resident_ctas_per_sm(
-            conv_umma_kernel<BN, GEOM, SPLITK>, kThreads, SmemLayout<BN, GEOM>::kDynamic, 2 * BN);
+    static ResidentCtas resident;
+    const int per_sm = resident.per_sm(conv_umma_kernel<BN, GEOM, SPLITK, FORM>, kThreads,
+                                       SmemLayout<BN, GEOM>::kDynamic, 2 * BN);
     const int total = SPLITK ? p.total_items : p.m_tiles * p.n_tiles;
     int grid = sm_count() * per_sm;
-    if (grid > total)
-        grid = total;
+    if (grid > total || p.csplit > 1)
+        grid = total * p.csplit;
     if (tuning().debug)
-        fprintf(stderr, "conv_umma<%d,%d,%d>: per_sm %d grid %d items %d (whole tiles %d, split %d) smem %d\n",
-                BN, GEOM, (int)SPLITK, per_sm, grid, total, SPLITK ? p.full_tiles : total,
+        fprintf(stderr, "conv_umma<%d,%d,%d,%d>: csplit %d per_sm %d grid %d items %d (whole tiles %d, split %d) smem %d\n",
+                BN, GEOM, (int)SPLITK, FORM, p.csplit, per_sm, grid, total, SPLITK ? p.full_tiles : total,
                 SPLITK ? p.split : 1, SmemLayout<BN, GEOM>::kDynamic);
-    launch_pdl(conv_umma_kernel<BN, GEOM, SPLITK>, dim3(grid), dim3(kThreads),
-               (size_t)SmemLayout<BN, GEOM>::kDynamic, st, ma, mb, p);
+    launch_pdl_cluster(conv_umma_kernel<BN, GEOM, SPLITK, FORM>, dim3(grid), dim3(kThreads),
+                       (size_t)SmemLayout<BN, GEOM>::kDynamic, p.csplit, st, ma, mb, p);
     return check_launch("conv_umma");
+}
+
+// the instantiation with the launch's epilogue (a split tile has its own, epilogue_quad)
+template <int BN, int GEOM>
+int launch_kernel(
+        const CUtensorMap& ma, const CUtensorMap& mb, const UmmaConvParams& p, cudaStream_t st) {
+    switch (p.csplit > 1 || !tuning().epilogue_forms ? FORM_ANY : epilogue_form(p.ep, p.dst)) {
+        case FORM_FMA_RELU: return launch_form<BN, GEOM, false, FORM_FMA_RELU>(ma, mb, p, st);
+        case FORM_FMA_NONE: return launch_form<BN, GEOM, false, FORM_FMA_NONE>(ma, mb, p, st);
+        case FORM_FMA_ADD_RELU: return launch_form<BN, GEOM, false, FORM_FMA_ADD_RELU>(ma, mb, p, st);
+        case FORM_CHAIN_RELU: return launch_form<BN, GEOM, false, FORM_CHAIN_RELU>(ma, mb, p, st);
+        case FORM_CHAIN_NONE: return launch_form<BN, GEOM, false, FORM_CHAIN_NONE>(ma, mb, p, st);
+        case FORM_CHAIN_ADD_RELU:
+            return launch_form<BN, GEOM, false, FORM_CHAIN_ADD_RELU>(ma, mb, p, st);
+        default: return launch_form<BN, GEOM>(ma, mb, p, st);
+    }
+}
+
+template <int BN, int GEOM>
+int umma_clusters(int size) {
+    static ClusterCapacity capacity;
+    if (!umma_kernel_ready<BN, GEOM>())
+        return 0;
+    return capacity.clusters(conv_umma_kernel<BN, GEOM>, size, Shape<BN>::kThreads,
+                             SmemLayout<BN, GEOM>::kDynamic);
+}
+
+// A layer with fewer tiles than SMs (a small batch): 64- or 128-column tiles, and how many CTAs
+// of a cluster share a tile's K loop. The pair with the shortest estimated chain of its
+// busiest CTA, in clocks: a pipeline step of 128-byte rows (half of that for 64-byte ones) costs
+// 300 with 64 columns and 380 with 128, a tile's end 1200 and 1800; the exchange of the shares
+// over the cluster 1600 and 350 for every four channels that a thread then finishes. A split
+// has to promise a sixth less: 512 -> 512 3x3 over 37 images of 7 x 7 took 30 us as 60 tiles
+// split in two and 26 us unsplit, one image 23 us unsplit and 8 us as 8 tiles split in eight.
+void choose_split(int m_tiles, int oc, int k_iters, bool wide128, int* bn, int* csplit) {
+    long long best = -1;
+    const int bn_first = *bn;
+    for (int b = 64; b <= 128; b *= 2) {
+        if (b > 64 && oc <= 64)
+            break;
+        const long long tiles = (long long)m_tiles * ((oc + b - 1) / b);
+        const int step = (b == 128 ? 380 : 300) / (wide128 ? 1 : 2);
+        for (int s = 1; s <= 8; s *= 2) {
+            if (s > 1) {
+                const int fit = wide128 ? (b == 64 ? umma_clusters<64, GEOM_WIDE128>(s)
+                                                   : umma_clusters<128, GEOM_WIDE128>(s))
+                                        : (b == 64 ? umma_clusters<64, GEOM_WIDE>(s)
+                                                   : umma_clusters<128, GEOM_WIDE>(s));
+                if (k_iters / s < 2 || tiles > fit || tiles * s > sm_count())
+                    break;
+            }
+            const long long waves = (tiles * s + sm_count() - 1) / sm_count();
+            const long long steps = (long long)((k_iters + s - 1) / s) * step;
+            const int quads = b / (8 * s) > 1 ? b / (8 * s) : 1;
+            const long long clocks = s > 1 ? (steps + 1600 + 350 * quads) * 6 / 5
+                                           : waves * (steps + (b == 128 ? 1800 : 1200));
+            // (a tie goes to the width the caller had chosen)
+            if (best < 0 || clocks < best || (clocks == best && b == bn_first && s == 1)) {
+                best = clocks;
+                *bn = b;
+                *csplit = s;
+            }
+        }
+    }
 }
 
 // ------------------------------------------------------------------------------------------
@@ -655,7 +796,7 @@ int launch_conv_umma_geom(
             return launch_conv_pair(a, src, flt, bias, flt_scales, dst, st);
     }
     const int chans = geom == GEOM_WIDE128 ? 128 : geom == GEOM_WIDE ? kBK : 16;
-    int bn = a.oc <= 64 ? 64 : 128;
+    int bn = a.oc <= 64 ? 64 : 128, csplit = 1;
     {
         // 256 output channels per tile when the K loop is long enough to hide the epilogue
         // of a single CTA per SM and there are tiles for every SM
@@ -672,6 +813,15 @@ int launch_conv_umma_geom(
         // the TMEM, so three CTAs (24 epilogue warps) fit an SM instead of two
         if (force == 64 || (force == 0 && k_bytes <= 256 && bn == 128))
             bn = 64;
+        // fewer tiles than SMs: narrower tiles, K split over clusters
+        const long long tiles = (long long)((a.m + kBM - 1) / kBM) * ((a.oc + bn - 1) / bn);
+        const int k_iters = geom == GEOM_TAP16 ? taps / 4 : taps * ((a.ic + chans - 1) / chans);
+        if (geom != GEOM_TAP16 && bn <= 128 && force == 0 && a.test_wait_cycles == 0 &&
+            tiles <= sm_count())
+            choose_split((a.m + kBM - 1) / kBM, a.oc, k_iters, geom == GEOM_WIDE128, &bn, &csplit);
+        const int fs = tuning().conv_csplit;
+        if ((fs == 1 || fs == 2 || fs == 4 || fs == 8) && geom != GEOM_TAP16 && bn <= 128)
+            csplit = k_iters >= fs ? fs : 1;
     }
     const CUtensorMapSwizzle swz = geom == GEOM_WIDE128 ? CU_TENSOR_MAP_SWIZZLE_128B
                                    : geom == GEOM_WIDE  ? CU_TENSOR_MAP_SWIZZLE_64B
@@ -763,7 +913,7 @@ int launch_conv_umma_geom(
     p.ep.z_scale = a.z_scale;
     p.ep.z_div = 1.0f / a.z_out_scale;  // the reference's scale_div = 1.f / scale_dst
     p.ep.z_fast_a = p.ep.z_fast_b = 0.f;
-    if (p.ep.z_mode != 0 && p.ep.fast_ops != 0)
+    if (p.ep.z_mode != 0)
         residual_fast_constants(a.s_dst, a.z_scale, a.z_out_scale, p.ep.z_mode, &p.ep.z_fast_a,
                                 &p.ep.z_fast_b);
     if (tuning().debug)
@@ -782,7 +932,7 @@ int launch_conv_umma_geom(
     p.split = 1;
     p.k_per_part = p.k_iters;
     p.slabs = nullptr;
-    p.overlap = tuning().overlap_loads;
+    p.csplit = csplit;
     p.counters = nullptr;
     if (geom == GEOM_WIDE128) {
         if (bn == 256) {
@@ -795,7 +945,7 @@ int launch_conv_umma_geom(
                 p.total_items = sp.total_items;
                 p.counters = (unsigned*)scratch;
                 p.slabs = (int4*)((uint8_t*)scratch + kCounterBytes);
-                return launch_kernel<256, GEOM_WIDE128, true>(map_a, map_b, p, st);
+                return launch_form<256, GEOM_WIDE128, true>(map_a, map_b, p, st);
             }
             return launch_kernel<256, GEOM_WIDE128>(map_a, map_b, p, st);
         }
@@ -805,8 +955,8 @@ int launch_conv_umma_geom(
     if (geom == GEOM_WIDE)
         return bn == 64 ? launch_kernel<64, GEOM_WIDE>(map_a, map_b, p, st)
                         : launch_kernel<128, GEOM_WIDE>(map_a, map_b, p, st);
-    return bn == 64 ? launch_kernel<64, GEOM_TAP16>(map_a, map_b, p, st)
-                    : launch_kernel<128, GEOM_TAP16>(map_a, map_b, p, st);
+    return bn == 64 ? launch_form<64, GEOM_TAP16>(map_a, map_b, p, st)
+                    : launch_form<128, GEOM_TAP16>(map_a, map_b, p, st);
 }
 
 int launch_conv_umma(

@@ -13,7 +13,8 @@ struct Tuning {
     int patch_ctas = 0;     // MB200_PATCH_CTAS     1..3 = resident CTAs the patch kernel tries first
     int patch_alone = 0;    // MB200_PATCH_ALONE    1 = patch kernel even with one CTA per SM
     int patch_plain = 0;    // MB200_PATCH_PLAIN    1 = 16-channel planes for 64-channel layers
-    int overlap_loads = 1;  // MB200_OVERLAP_LOADS  0 = one 32-column TMEM load per chunk in the halo-patch epilogue
+    int epilogue_forms = 1; // MB200_EPILOGUE_FORMS 0 = the kernels with every epilogue variant at run time
+    int conv_csplit = 0;    // MB200_CONV_CSPLIT    0 = by shape, 1 | 2 | 4 | 8 = CTAs of a cluster per tile's K loop
     int f32_bn = 0;         // MB200_F32_BN         0 = by shape, 32 | 64 | 128 = that fp32 tile width
     int f32_split = 0;      // MB200_F32_SPLIT      0 = by shape, 1 | 2 | 4 | 8 = CTAs per tile's K loop
     int dw_tensor = 1;      // MB200_DW_TENSOR      0 = depthwise 3x3/1 on the CUDA cores only

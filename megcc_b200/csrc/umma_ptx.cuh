@@ -153,6 +153,29 @@ __device__ __forceinline__ void tma_prefetch_map(const CUtensorMap* map) {
     asm volatile("prefetch.tensormap [%0];" ::"l"((uint64_t)map) : "memory");
 }
 
+// ---- thread-block clusters ----
+__device__ __forceinline__ uint32_t cluster_rank() {
+    uint32_t r;
+    asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
+    return r;
+}
+// every thread of every CTA of the cluster
+__device__ __forceinline__ void cluster_barrier() {
+    asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+    asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+// 16 bytes at the shared-memory address `local` of CTA `rank`
+__device__ __forceinline__ uint4 ld_cluster_v4(uint32_t local, int rank) {
+    uint32_t addr;
+    uint4 v;
+    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(addr) : "r"(local), "r"(rank));
+    asm volatile("ld.shared::cluster.v4.u32 {%0, %1, %2, %3}, [%4];"
+                 : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w)
+                 : "r"(addr)
+                 : "memory");
+    return v;
+}
+
 __device__ __forceinline__ void tma_load_2d(
         void* smem, const CUtensorMap* map, uint64_t* bar, int c0, int c1) {
     asm volatile(
@@ -436,6 +459,24 @@ inline int resident_ctas_per_sm(Kernel kernel, int threads, int dynamic_smem, in
     n = n < by_tmem ? n : by_tmem;
     return n < 1 ? 1 : n;
 }
+
+// resident_ctas_per_sm, asked once per kernel, shared-memory size and device (a function-attribute
+// query on every launch costs it about a microsecond)
+struct ResidentCtas {
+    std::atomic<long long> known[64] = {};  // shared memory << 8 | CTAs
+    template <class Kernel>
+    int per_sm(Kernel kernel, int threads, int dynamic_smem, int tmem_cols) {
+        int dev = 0;
+        if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64)
+            return resident_ctas_per_sm(kernel, threads, dynamic_smem, tmem_cols);
+        const long long k = known[dev].load(std::memory_order_relaxed);
+        if (k && (k >> 8) == dynamic_smem)
+            return (int)(k & 255);
+        const int n = resident_ctas_per_sm(kernel, threads, dynamic_smem, tmem_cols);
+        known[dev].store(((long long)dynamic_smem << 8) | n, std::memory_order_relaxed);
+        return n;
+    }
+};
 
 }  // namespace umma
 }  // namespace mb200
