@@ -32,7 +32,9 @@ int check_launch(const char* what) {
 
 // One status word per (device, stream): a kernel whose bounded wait runs out records its
 // code in the word of the stream it was launched on, so that a network waiting on its own
-// stream never consumes another network's error. The words of a device come from one small
+// stream never consumes another network's error. The words are mapped page-locked host memory:
+// kernels only ever write them (when something went wrong), and a host that has waited for the
+// stream reads its word without a transfer. A device's words come from one small
 // allocation made at first use; a stream first seen while it is capturing (no set-up may
 // happen then) and streams beyond the pool's capacity share word 0.
 int* device_status_word(cudaStream_t st) {
@@ -58,13 +60,15 @@ int* device_status_word(cudaStream_t st) {
             set_error(ST_RUNTIME, "first use of the library on this device during stream capture");
             return nullptr;
         }
+        // (unified addressing: the host address is the device address)
         int* p = nullptr;
-        if (cudaMalloc(&p, kWords * sizeof(int)) != cudaSuccess ||
-            cudaMemset(p, 0, kWords * sizeof(int)) != cudaSuccess) {
+        if (cudaHostAlloc((void**)&p, kWords * sizeof(int),
+                          cudaHostAllocMapped | cudaHostAllocPortable) != cudaSuccess) {
             cudaGetLastError();
             set_error(ST_MALLOC, "cannot allocate the device status words");
             return nullptr;
         }
+        memset(p, 0, kWords * sizeof(int));
         pool.base = p;
     }
     auto it = pool.index.find(st);
@@ -266,14 +270,12 @@ int mb200_device_status(void* stream, int* status_host) {
     int* w = device_status_word(st);
     if (!w)
         return ST_MALLOC;
-    int v = 0;
-    if (cudaMemcpyAsync(&v, w, sizeof(int), cudaMemcpyDeviceToHost, st) != cudaSuccess ||
-        cudaStreamSynchronize(st) != cudaSuccess)
-        return set_error(ST_RUNTIME, "reading the device status word failed: %s",
+    if (cudaStreamSynchronize(st) != cudaSuccess)
+        return set_error(ST_RUNTIME, "waiting for the stream failed: %s",
                          cudaGetErrorString(cudaGetLastError()));
-    if (v != 0)
-        cudaMemsetAsync(w, 0, sizeof(int), st);
-    *status_host = v;
+    *status_host = *(volatile int*)w;
+    if (*status_host != 0)
+        *(volatile int*)w = 0;
     return ST_SUCCESS;
 }
 

@@ -161,6 +161,8 @@ int launch_typecvt_qs8_f32(
 int launch_typecvt_qs32_qs8(
         const int32_t* src, int8_t* dst, size_t nr_elem, float s_src, float s_dst,
         cudaStream_t st);
+// plain copy by a kernel (src may be page-locked host memory)
+int launch_copy_bytes(const void* src, void* dst, size_t bytes, cudaStream_t st);
 int launch_transpose_s8(
         const int8_t* src, int8_t* dst, int batch, int rows, int cols, cudaStream_t st);
 

@@ -138,6 +138,8 @@ struct IoSlot {
     Tensor* tensor = nullptr;
     void* user_ptr = nullptr;   // what LITE_reset_tensor_memory was given (inputs)
     bool user_is_device = false;
+    const void* user_mapped = nullptr;  // page-locked host memory: its address for kernels
+    bool written_mapped = false;  // an output its kernel writes straight into host_stage
     bool want_device = false;   // LiteIO.is_host == 0
     void* host_stage = nullptr; // pinned copy of an output
     size_t bytes = 0;
@@ -210,6 +212,7 @@ struct ComputeLane {
     std::mutex mu;
     cudaEvent_t done = nullptr;
     bool recorded = false;
+    cudaStream_t last = nullptr;  // the stream `done` was recorded on (its own order needs no wait)
 };
 // Defaults of a new network, taken from the environment once per process
 // (MB200_NO_GRAPH=1, MB200_PROFILE=1, MB200_LITE_SERIAL_COMPUTE=0); a network's own settings
@@ -238,6 +241,9 @@ ComputeLane* compute_lane(int device) {
         return nullptr;
     return &lanes[device];
 }
+
+constexpr size_t kKernelCopyBytes = 512u << 10;
+constexpr size_t kMappedOutputBytes = 2u << 20;
 
 // Host -> device copy of one input, ordered after what `net->stream` holds so far and before
 // what it is given next. Pieces of at least 2 MiB go to the side streams.
@@ -1405,6 +1411,25 @@ int init_model_memory(Network* net) {
         if (!o.host_stage && !o.want_device &&
             (e = cudaMallocHost(&o.host_stage, o.bytes ? o.bytes : 1)) != cudaSuccess)
             return cuda_fail(e, "cudaMallocHost(output)");
+        // An output that no other instruction reads is written where the caller looks for it:
+        // its kernel stores over PCIe and the copy behind the graph goes away. (Up to 2 MiB: a
+        // large batch's results leave faster through the copy engine.)
+        bool read_here = false;
+        for (auto& ins : m.instrs) {
+            if (ins.is_opr)
+                for (const Tensor* t : ins.op.inputs)
+                    read_here |= t == o.tensor;
+            else
+                read_here |= ins.mf.in == o.tensor || ins.mf.out == o.tensor;
+        }
+        void* mapped = nullptr;
+        if (o.host_stage && !read_here && o.bytes <= kMappedOutputBytes &&
+            cudaHostGetDevicePointer(&mapped, o.host_stage, 0) == cudaSuccess) {
+            o.tensor->ptr = mapped;
+            o.written_mapped = true;
+        } else {
+            cudaGetLastError();
+        }
     }
     m.memory_ready = true;
     return TinyNN_SUCCESS;
@@ -1467,7 +1492,12 @@ int forward(Network* net) {
             s.tensor->ptr = s.user_ptr;
         } else {
             s.tensor->ptr = (uint8_t*)net->arena->ptr + s.tensor->offset;
-            if ((e = copy_input(net, s.tensor->ptr, s.user_ptr, s.bytes)) != cudaSuccess)
+            // A small page-locked input is fetched by a kernel: a copy-engine transfer in front of
+            // the graph costs two hand-overs between engines, more than the transfer itself.
+            if (s.user_mapped && s.bytes <= kKernelCopyBytes) {
+                if ((rc = mb200::launch_copy_bytes(s.user_mapped, s.tensor->ptr, s.bytes, net->stream)))
+                    return fail(rc, "input copy: %s", mb200_last_error());
+            } else if ((e = copy_input(net, s.tensor->ptr, s.user_ptr, s.bytes)) != cudaSuccess)
                 return cuda_fail(e, "cudaMemcpyAsync(input)");
         }
         in_ptrs.push_back(s.tensor->ptr);
@@ -1480,7 +1510,7 @@ int forward(Network* net) {
         if (!lane->done &&
             (e = cudaEventCreateWithFlags(&lane->done, cudaEventDisableTiming)) != cudaSuccess)
             return cuda_fail(e, "cudaEventCreate");
-        if (lane->recorded &&
+        if (lane->recorded && lane->last != net->stream &&
             (e = cudaStreamWaitEvent(net->stream, lane->done, 0)) != cudaSuccess)
             return cuda_fail(e, "cudaStreamWaitEvent");
     }
@@ -1537,10 +1567,11 @@ int forward(Network* net) {
         if ((e = cudaEventRecord(lane->done, net->stream)) != cudaSuccess)
             return cuda_fail(e, "cudaEventRecord");
         lane->recorded = true;
+        lane->last = net->stream;
         lane_lock.unlock();
     }
     for (auto& o : m.outputs) {
-        if (o.want_device)
+        if (o.want_device || o.written_mapped)
             continue;
         if ((e = cudaMemcpyAsync(o.host_stage, o.tensor->ptr, o.bytes, cudaMemcpyDeviceToHost,
                                  net->stream)) != cudaSuccess)
@@ -1774,7 +1805,7 @@ int LITE_reset_tensor_memory(LiteTensor tensor, void* prepared_data, size_t data
                     data_length_in_byte, s->bytes);
     if (!h->is_input)
         return fail(TinyNN_ERROR_NO_IMPLEMENT, "only input tensors take user memory");
-    cudaPointerAttributes attr;
+    cudaPointerAttributes attr = {};
     bool is_dev = false;
     if (cudaPointerGetAttributes(&attr, prepared_data) == cudaSuccess)
         is_dev = attr.type == cudaMemoryTypeDevice || attr.type == cudaMemoryTypeManaged;
@@ -1784,6 +1815,7 @@ int LITE_reset_tensor_memory(LiteTensor tensor, void* prepared_data, size_t data
         return fail(TinyNN_ERROR_INVALID_LAYOUT, "device input must be 16-byte aligned");
     s->user_ptr = prepared_data;
     s->user_is_device = is_dev;
+    s->user_mapped = attr.type == cudaMemoryTypeHost ? attr.devicePointer : nullptr;
     return TinyNN_SUCCESS;
 }
 

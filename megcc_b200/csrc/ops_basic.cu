@@ -509,6 +509,22 @@ __global__ void __launch_bounds__(256) typecvt_qs32_qs8_kernel(
 }
 
 // ------------------------------------------------------------------------------------------
+// plain copy, for small transfers out of page-locked host memory: 16 bytes per thread, all of
+// them in flight at once (latency-bound over PCIe)
+// ------------------------------------------------------------------------------------------
+__global__ void __launch_bounds__(256) copy_bytes_kernel(
+        const uint8_t* src, uint8_t* dst, size_t bytes, int vec_ok) {
+    pdl_start();
+    const size_t tid = blockIdx.x * (size_t)blockDim.x + threadIdx.x;
+    const size_t nthr = (size_t)gridDim.x * blockDim.x;
+    const size_t vecs = vec_ok ? bytes / 16 : 0;
+    for (size_t i = tid; i < vecs; i += nthr)
+        reinterpret_cast<uint4*>(dst)[i] = reinterpret_cast<const uint4*>(src)[i];
+    for (size_t i = vecs * 16 + tid; i < bytes; i += nthr)
+        dst[i] = src[i];
+}
+
+// ------------------------------------------------------------------------------------------
 // [R][C] -> [C][R] byte transpose per batch item, 32x32 tiles through shared memory
 // ------------------------------------------------------------------------------------------
 __global__ void __launch_bounds__(256) transpose_s8_kernel(
@@ -657,6 +673,15 @@ int launch_typecvt_qs32_qs8(
     typecvt_qs32_qs8_kernel<<<grid_for(nr_elem, 256), 256, 0, st>>>(
             src, dst, nr_elem, s_src, s_dst);
     return check_launch("typecvt_qs32_qs8");
+}
+
+int launch_copy_bytes(const void* src, void* dst, size_t bytes, cudaStream_t st) {
+    if (bytes == 0)
+        return 0;
+    const int vec_ok = ((((uintptr_t)src | (uintptr_t)dst) & 15) == 0) ? 1 : 0;
+    launch_pdl(copy_bytes_kernel, dim3(grid_for(vec_ok ? bytes / 16 + 15 : bytes, 256)), dim3(256), 0,
+               st, (const uint8_t*)src, (uint8_t*)dst, bytes, vec_ok);
+    return check_launch("copy_bytes");
 }
 
 int launch_transpose_s8(
