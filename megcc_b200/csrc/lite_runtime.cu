@@ -162,6 +162,12 @@ struct DevModel {
     std::vector<CapturedGraph> graphs;
     bool memory_ready = false;
     bool ran_eager = false;
+    // independent instructions are captured side by side (see spread_small_model)
+    bool side_by_side = false;
+    // where tensors and workspaces really lie in the arena: as planned, or each on its own
+    size_t arena_bytes = 0;
+    std::vector<size_t> tensor_place, ws_place;
+    std::vector<cudaEvent_t> marks;  // one per instruction, for capture only
 };
 
 struct Network;
@@ -198,6 +204,9 @@ struct Network {
     // measured 40 GB/s over PCIe gen5 x16, four concurrent pieces 54 GB/s.
     static constexpr int kCopyStreams = 3;
     cudaStream_t copy_stream[kCopyStreams] = {nullptr, nullptr, nullptr};
+    // lanes beside `stream` that branches of a small model are captured on
+    static constexpr int kLanes = 5;
+    cudaStream_t lane_stream[kLanes] = {nullptr, nullptr, nullptr, nullptr, nullptr};
     cudaEvent_t copy_fork = nullptr, copy_join[kCopyStreams] = {nullptr, nullptr, nullptr};
 };
 
@@ -1009,6 +1018,68 @@ bool read_layout(const fb::Table& t, Layout* out) {
     return true;
 }
 
+// May the two instructions run at the same time? (by the tensors they name: outputs and
+// workspaces have memory of their own here)
+bool conflicts(const Instr& a, const Instr& b) {
+    auto touches = [](const Instr& i, const Tensor* t) {
+        for (const Tensor* x : i.op.inputs)
+            if (x == t)
+                return true;
+        for (const Tensor* x : i.op.outputs)
+            if (x == t)
+                return true;
+        return false;
+    };
+    for (const Tensor* t : a.op.outputs)
+        if (touches(b, t))
+            return true;
+    for (const Tensor* t : b.op.outputs)
+        if (touches(a, t))
+            return true;
+    return false;
+}
+
+// A small model (a batch of one) is bound by the latency of its instructions one after the
+// other, each of which leaves most SMs idle. Where it has branches (the heads of a detector,
+// the two arms of a residual block) and all its tensors fit the L2 together, every tensor gets
+// memory of its own instead of the planned reuse, so that nothing but data ties two
+// instructions, and independent instructions are captured on parallel branches of the graph.
+void spread_small_model(DevModel& m) {
+    constexpr size_t kMost = 48u << 20;
+    m.arena_bytes = m.tensor_memory;
+    m.tensor_place.clear();
+    for (auto& t : m.tensors)
+        m.tensor_place.push_back(t.offset);
+    m.ws_place.clear();
+    for (auto& ins : m.instrs)
+        m.ws_place.push_back(ins.is_opr ? ins.op.ws.offset : 0);
+    size_t total = 0;
+    auto up = [](size_t v) { return (v + 255) / 256 * 256; };
+    for (auto& t : m.tensors)
+        total += up(t.size);
+    bool branches = false;
+    for (size_t i = 0; i < m.instrs.size(); ++i) {
+        if (!m.instrs[i].is_opr)
+            return;  // an alias of another tensor: keep the plan
+        total += up(m.instrs[i].op.ws.size);
+        branches |= i > 0 && !conflicts(m.instrs[i - 1], m.instrs[i]);
+    }
+    if (!branches || total > kMost)
+        return;
+    size_t off = 0;
+    for (size_t i = 0; i < m.tensors.size(); ++i) {
+        m.tensor_place[i] = off;
+        off += up(m.tensors[i].size);
+    }
+    for (size_t i = 0; i < m.instrs.size(); ++i)
+        if (m.instrs[i].op.ws.size) {
+            m.ws_place[i] = off;
+            off += up(m.instrs[i].op.ws.size);
+        }
+    m.arena_bytes = off > m.tensor_memory ? off : m.tensor_memory;
+    m.side_by_side = true;
+}
+
 int parse_model(Network* net, const void* mem, size_t size) {
     fb::Buffer buf;  // Tables keep a pointer to it; none outlives this call
     buf.data = (const uint8_t*)mem;
@@ -1226,8 +1297,9 @@ int parse_model(Network* net, const void* mem, size_t size) {
             }
             m.instrs.push_back(std::move(ins));
         }
-        if (m.tensor_memory > net->arena_need)
-            net->arena_need = m.tensor_memory;
+        spread_small_model(m);
+        if (m.arena_bytes > net->arena_need)
+            net->arena_need = m.arena_bytes;
     }
     if (buf.failed)
         return fail(TinyNN_ERROR_MODEL_PARSE, "model buffer is truncated or corrupt");
@@ -1399,11 +1471,12 @@ int init_model_memory(Network* net) {
             return cuda_fail(e, "cudaMemset(arena slack)");
         mb200_register_readable_range(a.ptr, total);
     }
-    for (auto& t : m.tensors)
-        t.ptr = (uint8_t*)a.ptr + t.offset;
-    for (auto& ins : m.instrs) {
+    for (size_t i = 0; i < m.tensors.size(); ++i)
+        m.tensors[i].ptr = (uint8_t*)a.ptr + m.tensor_place[i];
+    for (size_t i = 0; i < m.instrs.size(); ++i) {
+        Instr& ins = m.instrs[i];
         if (ins.is_opr)
-            ins.op.ws.ptr = ins.op.ws.size ? (uint8_t*)a.ptr + ins.op.ws.offset : nullptr;
+            ins.op.ws.ptr = ins.op.ws.size ? (uint8_t*)a.ptr + m.ws_place[i] : nullptr;
         else
             ins.mf.out->ptr = (uint8_t*)ins.mf.in->ptr + ins.mf.offset;
     }
@@ -1470,6 +1543,124 @@ int issue_instructions(Network* net, DevModel& m, bool timed) {
     return TinyNN_SUCCESS;
 }
 
+// The instructions as branches of the graph under capture: each goes to the lane whose last
+// instruction it depends on, or to one whose work it follows anyway, or to a free one.
+int issue_side_by_side(Network* net, DevModel& m) {
+    constexpr int kLanes = Network::kLanes + 1;
+    cudaStream_t lanes[kLanes] = {net->stream};
+    for (int l = 1; l < kLanes; ++l)
+        lanes[l] = net->lane_stream[l - 1];
+    const int n = (int)m.instrs.size();
+    std::vector<int> lane_of(n, 0);
+    int tail[kLanes];               // last instruction of each lane, -1: none
+    int seen[kLanes][kLanes];       // seen[a][b]: last instruction of lane b that lane a follows
+    for (int a = 0; a < kLanes; ++a) {
+        tail[a] = -1;
+        for (int b = 0; b < kLanes; ++b)
+            seen[a][b] = -1;
+    }
+    cudaEvent_t fork = m.marks[n];
+    cudaError_t e = cudaEventRecord(fork, net->stream);
+    bool started[kLanes] = {true};
+    for (int i = 0; i < n && e == cudaSuccess; ++i) {
+        int need[kLanes];  // latest dependency on each lane
+        for (int l = 0; l < kLanes; ++l)
+            need[l] = -1;
+        for (int j = i - 1; j >= 0; --j)
+            if (need[lane_of[j]] < 0 && conflicts(m.instrs[j], m.instrs[i]))
+                need[lane_of[j]] = j;
+        int best = -1, free_lane = -1, any = 0;
+        for (int l = 0; l < kLanes; ++l) {
+            if (tail[l] >= 0 && need[l] == tail[l] && (best < 0 || tail[l] > tail[best]))
+                best = l;  // continues this lane's chain
+            if (tail[l] < 0 && free_lane < 0)
+                free_lane = l;
+            if (tail[l] < tail[any])
+                any = l;
+        }
+        if (best < 0)
+            for (int l = 0; l < kLanes && best < 0; ++l) {
+                // a lane whose last instruction is an ancestor through the dependencies
+                bool behind = tail[l] >= 0;
+                bool follows = false;
+                for (int d = 0; d < kLanes && behind; ++d)
+                    if (need[d] >= 0 && d != l && need[d] == tail[d] && seen[d][l] >= tail[l])
+                        follows = true;
+                if (behind && follows)
+                    best = l;
+            }
+        if (best < 0)
+            best = free_lane >= 0 ? free_lane : any;
+        if (!started[best]) {
+            e = cudaStreamWaitEvent(lanes[best], fork, 0);
+            started[best] = true;
+        }
+        for (int d = 0; d < kLanes && e == cudaSuccess; ++d) {
+            if (d == best || need[d] <= seen[best][d])
+                continue;
+            e = cudaStreamWaitEvent(lanes[best], m.marks[need[d]], 0);
+            seen[best][d] = need[d];
+            for (int b = 0; b < kLanes; ++b)  // (what the awaited lane follows now is no later
+                if (need[d] == tail[d] && seen[d][b] > seen[best][b])  // than what it had then)
+                    seen[best][b] = seen[d][b];
+        }
+        if (e != cudaSuccess)
+            break;
+        RuntimeOpt opt = net->opt;
+        opt.opr = &m.instrs[i].op;
+        opt.stream = lanes[best];
+        OpPlan& op = m.instrs[i].op;
+        const int rc = op.kernel_fn(op.inputs.data(), (int)op.inputs.size(), op.outputs.data(),
+                                    (int)op.outputs.size(), &op.ws, &opt);
+        if (rc)
+            return fail(rc, "kernel %s: %s", op.symbol.c_str(), mb200_last_error());
+        e = cudaEventRecord(m.marks[i], lanes[best]);
+        lane_of[i] = best;
+        tail[best] = i;
+        seen[best][best] = i;
+    }
+    for (int l = 1; l < kLanes && e == cudaSuccess; ++l)
+        if (tail[l] >= 0)
+            e = cudaStreamWaitEvent(net->stream, m.marks[tail[l]], 0);
+    return e == cudaSuccess ? TinyNN_SUCCESS : cuda_fail(e, "capturing parallel branches");
+}
+
+// What capturing side by side needs beforehand (nothing may be set up during a capture).
+bool ready_side_by_side(Network* net, DevModel& m) {
+    for (int l = 0; l < Network::kLanes; ++l) {
+        if (!net->lane_stream[l] &&
+            cudaStreamCreateWithFlags(&net->lane_stream[l], cudaStreamNonBlocking) != cudaSuccess)
+            return false;
+        if (!mb200::device_status_word(net->lane_stream[l]))
+            return false;
+    }
+    while (m.marks.size() < m.instrs.size() + 1) {
+        cudaEvent_t e;
+        if (cudaEventCreateWithFlags(&e, cudaEventDisableTiming) != cudaSuccess)
+            return false;
+        m.marks.push_back(e);
+    }
+    return true;
+}
+
+// The model's instructions as an executable graph.
+int capture(Network* net, DevModel& m, bool side_by_side, cudaGraphExec_t* exec) {
+    cudaGraph_t graph = nullptr;
+    cudaError_t e = cudaStreamBeginCapture(net->stream, cudaStreamCaptureModeThreadLocal);
+    if (e != cudaSuccess)
+        return cuda_fail(e, "cudaStreamBeginCapture");
+    const int rc =
+            side_by_side ? issue_side_by_side(net, m) : issue_instructions(net, m, false);
+    e = cudaStreamEndCapture(net->stream, &graph);
+    if (!rc && e == cudaSuccess)
+        e = cudaGraphInstantiate(exec, graph, 0);
+    if (graph)
+        cudaGraphDestroy(graph);
+    if (rc)
+        return rc;
+    return e == cudaSuccess ? TinyNN_SUCCESS : cuda_fail(e, "capturing the model's graph");
+}
+
 int forward(Network* net) {
     if (!net->loaded)
         return fail(TinyNN_ERROR, "LITE_forward before a model was loaded");
@@ -1491,7 +1682,7 @@ int forward(Network* net) {
         if (s.user_is_device) {
             s.tensor->ptr = s.user_ptr;
         } else {
-            s.tensor->ptr = (uint8_t*)net->arena->ptr + s.tensor->offset;
+            s.tensor->ptr = (uint8_t*)net->arena->ptr + m.tensor_place[s.tensor - m.tensors.data()];
             // A small page-locked input is fetched by a kernel: a copy-engine transfer in front of
             // the graph costs two hand-overs between engines, more than the transfer itself.
             if (s.user_mapped && s.bytes <= kKernelCopyBytes) {
@@ -1539,24 +1730,14 @@ int forward(Network* net) {
                     cudaGraphExecDestroy(m.graphs.back().exec);
                     m.graphs.pop_back();
                 }
-                cudaGraph_t graph = nullptr;
-                if ((e = cudaStreamBeginCapture(net->stream, cudaStreamCaptureModeThreadLocal)) !=
-                    cudaSuccess)
-                    return cuda_fail(e, "cudaStreamBeginCapture");
-                rc = issue_instructions(net, m, false);
-                e = cudaStreamEndCapture(net->stream, &graph);
-                if (rc) {
-                    if (graph)
-                        cudaGraphDestroy(graph);
-                    return rc;
-                }
-                if (e != cudaSuccess)
-                    return cuda_fail(e, "cudaStreamEndCapture");
                 cudaGraphExec_t exec = nullptr;
-                e = cudaGraphInstantiate(&exec, graph, 0);
-                cudaGraphDestroy(graph);
-                if (e != cudaSuccess)
-                    return cuda_fail(e, "cudaGraphInstantiate");
+                if (m.side_by_side &&
+                    (!ready_side_by_side(net, m) || capture(net, m, true, &exec))) {
+                    cudaGetLastError();  // then one instruction after the other
+                    m.side_by_side = false;
+                }
+                if (!exec && (rc = capture(net, m, false, &exec)))
+                    return rc;
                 m.graphs.insert(m.graphs.begin(), DevModel::CapturedGraph{in_ptrs, exec});
             }
             if ((e = cudaGraphLaunch(m.graphs.front().exec, net->stream)) != cudaSuccess)
@@ -1587,7 +1768,10 @@ int wait(Network* net) {
     net->pending = false;
     cudaSetDevice(net->device_id);
     int status = 0;
-    const int rc = mb200_device_status(net->stream, &status);  // synchronises the stream
+    int rc = mb200_device_status(net->stream, &status);  // synchronises the stream
+    for (int l = 0; l < Network::kLanes && !rc && !status; ++l)
+        if (net->lane_stream[l])  // (captured branches record under their lane's stream)
+            rc = mb200_device_status(net->lane_stream[l], &status);
     if (rc)
         return fail(rc, "%s", mb200_last_error());
     if (status)
@@ -1997,6 +2181,12 @@ int LITE_destroy_network(LiteNetwork network) {
     }
     if (net->copy_fork)
         cudaEventDestroy(net->copy_fork);
+    for (int l = 0; l < Network::kLanes; ++l)
+        if (net->lane_stream[l])
+            cudaStreamDestroy(net->lane_stream[l]);
+    for (auto& m : net->models)
+        for (cudaEvent_t e : m.marks)
+            cudaEventDestroy(e);
     if (net->stream)
         cudaStreamDestroy(net->stream);
     delete net;
