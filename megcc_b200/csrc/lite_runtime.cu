@@ -1045,7 +1045,7 @@ bool conflicts(const Instr& a, const Instr& b) {
 // memory of its own instead of the planned reuse, so that nothing but data ties two
 // instructions, and independent instructions are captured on parallel branches of the graph.
 void spread_small_model(DevModel& m) {
-    constexpr size_t kMost = 48u << 20;
+    constexpr size_t kMost = 96u << 20;
     m.arena_bytes = m.tensor_memory;
     m.tensor_place.clear();
     for (auto& t : m.tensors)

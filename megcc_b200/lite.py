@@ -241,4 +241,4 @@ class Network:
         """Host copy of an output as a flat numpy array."""
         n = self.tensor_bytes(name, LITE_OUTPUT)
         p = self.output_ptr(name)
-        return np.frombuffer(C.string_at(p, n), dtype=dtype).copy()
+        return np.frombuffer((C.c_char * n).from_address(p), dtype=dtype).copy()
