@@ -186,14 +186,24 @@ struct F32Epilogue {
     long long dst_pitch;  // floats between consecutive pixels of dst (>= oc)
 };
 
+// 1 / (1 + 2^(-x log2 e)) from the hardware's two approximations (2 and 1 ulp), without the range
+// handling that the general exponential and quotient put around them: a subnormal power is lost
+// beside the 1 anyway, and an infinite one gives the right 0. 5 instructions instead of some 25.
+__device__ __forceinline__ float sigmoid_f32(float x) {
+    float e, r;
+    asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(e) : "f"(x * -1.442695041f));
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(1.f + e));
+    return r;
+}
+
 template <int ACT>
 __device__ __forceinline__ float act_f32(float x) {
     if (ACT == MB200_F32_RELU)
         return x > 0.f ? x : 0.f;
     if (ACT == MB200_F32_SIGMOID)
-        return __fdividef(1.f, 1.f + __expf(-x));
+        return sigmoid_f32(x);
     if (ACT == MB200_F32_SILU)
-        return __fdividef(x, 1.f + __expf(-x));
+        return x * sigmoid_f32(x);
     if (ACT == MB200_F32_H_SWISH) {
         float t = x + 3.f;
         t = t > 0.f ? t : 0.f;
@@ -217,66 +227,55 @@ __device__ __forceinline__ void with_act(int act, F&& f) {
     }
 }
 
-// NC consecutive channels (from ch0) of pixel `m`
-template <int NC, int ACT>
-__device__ __forceinline__ void store_f32_chunk_t(
-        const float (&v)[NC], const F32Epilogue& e, size_t m, int ch0) {
+// One pixel's channels of a finished tile (a row per lane): bias, activation, residual, stores.
+// With a short K loop (1x1 filters) this is the kernel's longest chain. So the bias lies in
+// shared memory (fetched once per tile column: from global memory each eight channels waited
+// for their load behind the stores before them), the residual is brought into the L2 while the tile
+// is computed, and stores are whole 32-byte sectors. 32 x 80 x 80 pixels of 128 channels to 80:
+// 96 us before, 48 now (floor 26 by its bytes); 128 to 128: 66 -> 54. (Turning the tile round in shared memory, so that a warp
+// stores 64-byte pieces of 16 rows instead of sectors of 32, measured the same within 3 %
+// either way and costs 16 KB of the ring.)
+template <int COLS, int ACT>
+__device__ __forceinline__ void store_f32_row(
+        const float (&sum)[COLS], const F32Epilogue& e, const float4* bias, size_t m, int ch0,
+        bool vec4, bool vec8) {
     float* out = e.dst + m * e.dst_pitch + ch0;
     const float* zin = e.z ? e.z + m * e.z_pitch + ch0 : nullptr;
-    const bool vec = ch0 + NC <= e.oc && (((uintptr_t)out | (uintptr_t)zin) & 15) == 0 &&
-                     (!e.bias || ((uintptr_t)(e.bias + ch0) & 15) == 0);
-    if (vec) {
-        // a thread's channels are whole 32-byte sectors when the pixel starts on one: 256-bit
-        // stores, so that no sector is written in two halves
-        const bool sector = ((uintptr_t)out & 31) == 0;
 #pragma unroll
-        for (int j = 0; j < NC / 8; ++j) {
-            float r[8];
+    for (int c = 0; c < COLS / 8; ++c) {
+        if (ch0 + 8 * c >= e.oc)
+            break;  // (also keeps the steps apart: run together they need too many registers)
+        const bool whole = vec4 && ch0 + 8 * c + 8 <= e.oc;
+        const float4 b0 = bias[2 * c], b1 = bias[2 * c + 1];
+        const float b[8] = {b0.x, b0.y, b0.z, b0.w, b1.x, b1.y, b1.z, b1.w};
+        float v[8];
 #pragma unroll
-            for (int h = 0; h < 2; ++h) {
-                float4 b = make_float4(0.f, 0.f, 0.f, 0.f);
-                if (e.bias)
-                    b = __ldg(reinterpret_cast<const float4*>(e.bias + ch0) + 2 * j + h);
-                r[4 * h + 0] = act_f32<ACT>(v[8 * j + 4 * h + 0] + b.x);
-                r[4 * h + 1] = act_f32<ACT>(v[8 * j + 4 * h + 1] + b.y);
-                r[4 * h + 2] = act_f32<ACT>(v[8 * j + 4 * h + 2] + b.z);
-                r[4 * h + 3] = act_f32<ACT>(v[8 * j + 4 * h + 3] + b.w);
-                if (zin) {
-                    const float4 zz = *(reinterpret_cast<const float4*>(zin) + 2 * j + h);
-                    r[4 * h + 0] += zz.x;
-                    r[4 * h + 1] += zz.y;
-                    r[4 * h + 2] += zz.z;
-                    r[4 * h + 3] += zz.w;
-                }
+        for (int j = 0; j < 8; ++j)
+            v[j] = act_f32<ACT>(sum[8 * c + j] + b[j]);
+        if (whole) {
+            if (zin) {
+                const float4 z0 = *(reinterpret_cast<const float4*>(zin) + 2 * c);
+                const float4 z1 = *(reinterpret_cast<const float4*>(zin) + 2 * c + 1);
+                v[0] += z0.x, v[1] += z0.y, v[2] += z0.z, v[3] += z0.w;
+                v[4] += z1.x, v[5] += z1.y, v[6] += z1.z, v[7] += z1.w;
             }
-            if (sector) {
+            if (vec8) {
                 asm volatile("st.global.v8.f32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"l"(
-                                     out + 8 * j),
-                             "f"(r[0]), "f"(r[1]), "f"(r[2]), "f"(r[3]), "f"(r[4]), "f"(r[5]),
-                             "f"(r[6]), "f"(r[7])
+                                     out + 8 * c),
+                             "f"(v[0]), "f"(v[1]), "f"(v[2]), "f"(v[3]), "f"(v[4]), "f"(v[5]),
+                             "f"(v[6]), "f"(v[7])
                              : "memory");
             } else {
-                reinterpret_cast<float4*>(out)[2 * j] = make_float4(r[0], r[1], r[2], r[3]);
-                reinterpret_cast<float4*>(out)[2 * j + 1] = make_float4(r[4], r[5], r[6], r[7]);
+                reinterpret_cast<float4*>(out)[2 * c] = make_float4(v[0], v[1], v[2], v[3]);
+                reinterpret_cast<float4*>(out)[2 * c + 1] = make_float4(v[4], v[5], v[6], v[7]);
             }
-        }
-    } else {
+        } else {
 #pragma unroll
-        for (int i = 0; i < NC; ++i) {
-            if (ch0 + i < e.oc) {
-                float r = act_f32<ACT>(v[i] + (e.bias ? e.bias[ch0 + i] : 0.f));
-                if (zin)
-                    r += zin[i];
-                out[i] = r;
-            }
+            for (int j = 0; j < 8; ++j)
+                if (ch0 + 8 * c + j < e.oc)
+                    out[8 * c + j] = zin ? v[j] + zin[8 * c + j] : v[j];
         }
     }
-}
-
-template <int NC>
-__device__ __forceinline__ void store_f32_chunk(
-        const float (&v)[NC], const F32Epilogue& e, size_t m, int ch0) {
-    with_act(e.act, [&](auto a) { store_f32_chunk_t<NC, decltype(a)::value>(v, e, m, ch0); });
 }
 
 // ------------------------------------------------------------------------------------------
@@ -299,6 +298,8 @@ struct F32ConvParams {
     long long wait_cycles;
 };
 
+constexpr int kF32EpilogueWarps = 8;
+
 template <int BN, int ROWB>
 struct F32Cfg {
     static constexpr int kChans = ROWB / 4;  // floats per row = TMEM columns of an A plane
@@ -310,14 +311,18 @@ struct F32Cfg {
     static constexpr int kSegIters = 256 / ROWB;  // stages per segment: eight K = 8 steps
     static constexpr int kABytes = kBM * ROWB;
     static constexpr int kBBytes = 2 * BN * ROWB;  // both planes of a filter tile
-    static constexpr int kBarBytes = 1024;         // barriers, in front of the tiles
+    static constexpr int kBarBytes = 1024;         // barriers, in front of everything
+    // each epilogue warp's copy of its columns' bias, behind the barriers
+    static constexpr int kBiasBytes = (kF32EpilogueWarps * BN / 2 * 4 + 1023) / 1024 * 1024;
+    // shared memory for tiles: a CTA's 227 KB less alignment slack, barriers and bias
+    static constexpr int kTileBudget = 227 * 1024 - 1024 - kBarBytes - kBiasBytes;
+    static constexpr int kDynamic = kTileBudget + 1024 + kBarBytes + kBiasBytes;
     static constexpr int kPartPitch = BN + 4;      // floats per row of a split part's tile
 };
 
 // Eight epilogue warps, and one converter group of four warps for 128 columns (its epilogue holds
 // 64 sums per thread: with 14 warps in the block a thread may have 128 registers), two groups
 // that take turns for the narrower tiles, whose steps are shorter.
-constexpr int kF32EpilogueWarps = 8;
 __host__ __device__ constexpr int f32_groups(int bn) { return bn == 128 ? 1 : 2; }
 __host__ __device__ constexpr int f32_threads(int bn) {
     return 64 + 32 * kF32EpilogueWarps + 128 * f32_groups(bn);
@@ -352,7 +357,7 @@ __global__ void __launch_bounds__(f32_threads(BN), 1) conv_f32_umma_kernel(
     uint64_t* drain_bar = b_full + 1;
     uint32_t* tmem_slot = (uint32_t*)(drain_bar + 1);
     volatile int* abort_flag = (volatile int*)(tmem_slot + 1);
-    uint8_t* tiles = smem + C::kBarBytes;
+    uint8_t* tiles = smem + C::kBarBytes + C::kBiasBytes;
     uint8_t* tiles_b = tiles;  // resident filter (if any), then the ring
     uint8_t* ring = tiles + (p.b_resident ? p.k_iters * C::kBBytes : 0);
     const int stage_bytes = C::kABytes + (p.b_resident ? 0 : C::kBBytes);
@@ -418,78 +423,83 @@ __global__ void __launch_bounds__(f32_threads(BN), 1) conv_f32_umma_kernel(
     };
 
     if (warp == 0) {
-        // ---------------- TMA producer ----------------
-        if (lane == 0) {
-            // where the first tile starts is worked out before the wait for the previous kernel
-            int tile_n = first_tile % p.n_tiles, tile_m = first_tile / p.n_tiles;
-            int img = tile_m * kBM / (p.oh * p.ow);
-            int rem = tile_m * kBM - img * (p.oh * p.ow);
-            int oy = rem / p.ow, ox = rem - oy * p.ow;
-            int cb = 0, fx = 0, fy = 0;
-            if (kb != 0) {  // a later part of a split tile starts inside the filter
-                const int tap = kb / p.cblocks;
-                cb = kb - tap * p.cblocks;
-                fy = tap / p.taps_w;
-                fx = tap - fy * p.taps_w;
+        // ---------------- TMA producer (a converged warp, one lane issues) ----------------
+        const uint32_t leader = elect_one() ? 1u : 0u;
+        const uint32_t full_a = smem_u32(full_bar), empty_a = smem_u32(empty_bar);
+        const uint32_t ring_a = smem_u32(ring);
+        const int pixels = p.oh * p.ow;
+        // where the first tile starts is worked out before the wait for the previous kernel
+        int tile_n = first_tile % p.n_tiles, tile_m = first_tile / p.n_tiles;
+        int img = tile_m * kBM / pixels;
+        int rem = tile_m * kBM - img * pixels;
+        int oy = rem / p.ow, ox = rem - oy * p.ow;
+        int cb = 0, fx = 0, fy = 0;
+        if (kb != 0) {  // a later part of a split tile starts inside the filter
+            const int tap = kb / p.cblocks;
+            cb = kb - tap * p.cblocks;
+            fy = tap / p.taps_w;
+            fx = tap - fy * p.taps_w;
+        }
+        pdl_wait();  // from here on the kernel touches global memory
+        if (p.b_resident) {
+            const uint32_t bar = smem_u32(b_full), b0 = smem_u32(tiles_b);
+            mbar_expect_tx_if(leader, bar, (uint32_t)(p.k_iters * C::kBBytes));
+            for (int it = 0; it < p.k_iters; ++it) {
+                const uint32_t b = b0 + it * C::kBBytes;
+                tma_load_2d_if(leader, b, &map_b, bar, it * kChans, 0);
+                tma_load_2d_if(leader, b + C::kBBytes / 2, &map_b, bar, it * kChans, p.b_lo_offset);
             }
-            pdl_wait();  // from here on the kernel touches global memory
-            if (p.b_resident) {
-                mbar_expect_tx(b_full, (uint32_t)(p.k_iters * C::kBBytes));
-                for (int it = 0; it < p.k_iters; ++it) {
-                    uint8_t* b = tiles_b + it * C::kBBytes;
-                    tma_load_2d(b, &map_b, b_full, it * kChans, 0);
-                    tma_load_2d(b + C::kBBytes / 2, &map_b, b_full, it * kChans, p.b_lo_offset);
-                }
+        }
+        int s = 0;
+        uint32_t parity = 1, slot = ring_a;
+        bool ok = true;
+        for (int tile = first_tile; tile < total_tiles && ok; tile += tile_step) {
+            if (tile != first_tile) {
+                tile_n = tile % p.n_tiles;
+                tile_m = tile / p.n_tiles;
+                img = tile_m * kBM / pixels;
+                rem = tile_m * kBM - img * pixels;
+                oy = rem / p.ow;
+                ox = rem - oy * p.ow;
+                cb = fx = fy = 0;
             }
-            const uint32_t tx = (uint32_t)stage_bytes;
-            int s = 0;
-            uint32_t phase = 0;
-            bool ok = true;
-            for (int tile = first_tile; tile < total_tiles && ok; tile += tile_step) {
-                if (tile != first_tile) {
-                    tile_n = tile % p.n_tiles;
-                    tile_m = tile / p.n_tiles;
-                    img = tile_m * kBM / (p.oh * p.ow);
-                    rem = tile_m * kBM - img * (p.oh * p.ow);
-                    oy = rem / p.ow;
-                    ox = rem - oy * p.ow;
-                    cb = fx = fy = 0;
+            const int m0 = tile_m * kBM, n0 = tile_n * BN;
+            const int base_w = ox * p.sw + p.base_w, base_h = oy * p.sh + p.base_h;
+            for (int it = kb; it < ke; ++it) {
+                ok = mbar_wait_u32(empty_a + 8 * s, parity, abort_flag, p.wait_cycles);
+                if (!ok)
+                    break;
+                const uint32_t bar = full_a + 8 * s;
+                mbar_expect_tx_if(leader, bar, (uint32_t)stage_bytes);
+                if (p.a_tiled)
+                    tma_load_2d_if(leader, slot, &map_a, bar, cb * kChans, m0);
+                else
+                    tma_load_im2col_4d_if(leader, slot, &map_a, bar, cb * kChans, base_w, base_h,
+                                          img, (uint16_t)fx, (uint16_t)fy);
+                if (!p.b_resident) {
+                    const uint32_t b = slot + C::kABytes;
+                    tma_load_2d_if(leader, b, &map_b, bar, it * kChans, n0);
+                    tma_load_2d_if(leader, b + C::kBBytes / 2, &map_b, bar, it * kChans,
+                                   n0 + p.b_lo_offset);
                 }
-                const int m0 = tile_m * kBM, n0 = tile_n * BN;
-                const int base_w = ox * p.sw + p.base_w, base_h = oy * p.sh + p.base_h;
-                for (int it = kb; it < ke; ++it) {
-                    if (!mbar_wait(&empty_bar[s], phase ^ 1u, abort_flag, p.wait_cycles)) {
-                        give_up(ERR_PRODUCER_WAIT);
-                        ok = false;
-                        break;
+                if (++cb == p.cblocks) {
+                    cb = 0;
+                    if (++fx == p.taps_w) {
+                        fx = 0;
+                        ++fy;
                     }
-                    mbar_expect_tx(&full_bar[s], tx);
-                    uint8_t* a = ring + s * stage_bytes;
-                    if (p.a_tiled)
-                        tma_load_2d(a, &map_a, &full_bar[s], cb * kChans, m0);
-                    else
-                        tma_load_im2col_4d(a, &map_a, &full_bar[s], cb * kChans, base_w, base_h,
-                                           img, (uint16_t)fx, (uint16_t)fy);
-                    if (!p.b_resident) {
-                        uint8_t* b = a + C::kABytes;
-                        tma_load_2d(b, &map_b, &full_bar[s], it * kChans, n0);
-                        tma_load_2d(b + C::kBBytes / 2, &map_b, &full_bar[s], it * kChans,
-                                    n0 + p.b_lo_offset);
-                    }
-                    if (++cb == p.cblocks) {
-                        cb = 0;
-                        if (++fx == p.taps_w) {
-                            fx = 0;
-                            ++fy;
-                        }
-                    }
-                    if (++s == p.stages) {
-                        s = 0;
-                        phase ^= 1u;
-                    }
+                }
+                slot += (uint32_t)stage_bytes;
+                if (++s == p.stages) {
+                    s = 0;
+                    slot = ring_a;
+                    parity ^= 1u;
                 }
             }
         }
+        if (!ok)
+            give_up(ERR_PRODUCER_WAIT);
+        __syncwarp();
     } else if (warp == 1) {
         // ---------------- MMA issuer (the whole warp waits, one lane issues) ----------------
         // The tensor pipe holds only a few MMAs beyond the one it executes, so every instruction
@@ -673,12 +683,34 @@ __global__ void __launch_bounds__(f32_threads(BN), 1) conv_f32_umma_kernel(
         const int half = (warp - 2) >> 2;
         constexpr int kCols = BN / 2;        // columns of this warp
         constexpr int kChunks = kCols / 16;  // ... in 16-column loads
+        float* bias_row = reinterpret_cast<float*>(smem + C::kBarBytes) + (warp - 2) * kCols;
+        const float4* bias = reinterpret_cast<const float4*>(bias_row);
+        // 16- and 32-byte accesses: every row starts on such a boundary when the first does
+        const bool vec4 = ((p.ep.dst_pitch | (p.ep.z ? p.ep.z_pitch : 0)) & 3) == 0 &&
+                          (((uintptr_t)p.ep.dst | (uintptr_t)p.ep.z) & 15) == 0;
+        const bool vec8 = vec4 && (p.ep.dst_pitch & 7) == 0 && ((uintptr_t)p.ep.dst & 31) == 0;
         int local = 0;
         bool ok = true;
         pdl_wait();  // before the first read of z and the first store
         for (int tile = first_tile; tile < total_tiles && ok; tile += tile_step) {
             const int tile_n = tile % p.n_tiles, tile_m = tile / p.n_tiles;
             const int m = tile_m * kBM + row, n0 = tile_n * BN;
+            if (p.n_tiles > 1 || tile == first_tile) {  // once, where one column covers the channels
+                __syncwarp();
+#pragma unroll
+                for (int j = lane; j < kCols; j += 32) {
+                    const int ch = n0 + half * kCols + j;
+                    bias_row[j] = p.ep.bias && ch < p.oc ? __ldg(p.ep.bias + ch) : 0.f;
+                }
+                __syncwarp();
+            }
+            if (p.ep.z && p.splits == 1 && m < p.m_total) {
+                const float* zin = p.ep.z + (size_t)m * p.ep.z_pitch + n0 + half * kCols;
+#pragma unroll
+                for (int j = 0; j < kCols; j += 32)
+                    if (n0 + half * kCols + j < p.oc)
+                        asm volatile("prefetch.global.L2 [%0];" ::"l"(zin + j));
+            }
             // running fp32 sums of this thread's accumulators over the tile's segments
             float sum[kCols];
 #pragma unroll
@@ -736,7 +768,10 @@ __global__ void __launch_bounds__(f32_threads(BN), 1) conv_f32_umma_kernel(
                     reinterpret_cast<float4*>(part)[j] = make_float4(
                             sum[4 * j], sum[4 * j + 1], sum[4 * j + 2], sum[4 * j + 3]);
             } else if (m < p.m_total && n0 + half * kCols < p.oc) {
-                store_f32_chunk<kCols>(sum, p.ep, (size_t)m, n0 + half * kCols);
+                with_act(p.ep.act, [&](auto a) {
+                    store_f32_row<kCols, decltype(a)::value>(sum, p.ep, bias, (size_t)m,
+                                                             n0 + half * kCols, vec4, vec8);
+                });
             }
         }
     }
@@ -906,13 +941,10 @@ int grid_1d(size_t work, int block) {
     return g < 1 ? 1 : (int)g;
 }
 
-// The shared memory a CTA may ask for, less the alignment slack and the barriers.
-constexpr int kF32TileBudget = 227 * 1024 - 1024 - 1024;
-
 template <int BN, int ROWB>
 bool f32_kernel_ready() {
     static KernelReady ready;
-    return ready.smem(conv_f32_umma_kernel<BN, ROWB>, kF32TileBudget + 2048);
+    return ready.smem(conv_f32_umma_kernel<BN, ROWB>, F32Cfg<BN, ROWB>::kDynamic);
 }
 
 template <int BN, int ROWB>
@@ -921,23 +953,23 @@ int f32_clusters(int size) {
     if (!f32_kernel_ready<BN, ROWB>())
         return 0;
     return capacity.clusters(conv_f32_umma_kernel<BN, ROWB>, size, f32_threads(BN),
-                             kF32TileBudget + 2048);
+                             F32Cfg<BN, ROWB>::kDynamic);
 }
 
 template <int BN, int ROWB>
 int launch_f32_kernel(
         const CUtensorMap& ma, const CUtensorMap& mb, F32ConvParams& p, cudaStream_t st) {
     using C = F32Cfg<BN, ROWB>;
-    constexpr int kDynamic = kF32TileBudget + 2048;
     if (!f32_kernel_ready<BN, ROWB>())
         return check_launch("conv_f32_umma smem attribute");
-    // The filter stays resident where one tile column covers the channels and at least five
-    // A stages fit behind it (a TMA round trip is four to five stages of conversion).
+    // The filter stays resident where one tile column covers the channels and enough A stages
+    // fit behind it (a TMA round trip is four to five stages of conversion).
+    constexpr int kResidentStages = 5;
     const long long b_all = (long long)p.k_iters * C::kBBytes;
     p.b_resident = p.splits == 1 && p.n_tiles == 1 && p.m_tiles > sm_count() &&
-                   b_all + 5 * C::kABytes <= kF32TileBudget;
+                   b_all + kResidentStages * C::kABytes <= C::kTileBudget;
     const int stage = C::kABytes + (p.b_resident ? 0 : C::kBBytes);
-    int stages = (int)((kF32TileBudget - (p.b_resident ? b_all : 0)) / stage);
+    int stages = (int)((C::kTileBudget - (p.b_resident ? b_all : 0)) / stage);
     p.stages = stages > kMaxStages ? kMaxStages : stages;
     const int total = p.m_tiles * p.n_tiles;
     int grid = total * p.splits;
@@ -947,7 +979,7 @@ int launch_f32_kernel(
         fprintf(stderr, "conv_f32_umma<%d,%d>: grid %d tiles %d k_iters %d stages %d resident %d "
                 "splits %d\n", BN, ROWB, grid, total, p.k_iters, p.stages, p.b_resident, p.splits);
     launch_pdl_cluster(conv_f32_umma_kernel<BN, ROWB>, dim3(grid), dim3(f32_threads(BN)),
-                       (size_t)kDynamic, p.splits, st, ma, mb, p);
+                       (size_t)C::kDynamic, p.splits, st, ma, mb, p);
     return check_launch("conv_f32_umma");
 }
 

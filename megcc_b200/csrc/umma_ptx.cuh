@@ -223,6 +223,37 @@ __device__ __forceinline__ void tma_load_im2col_4d(
             : "memory");
 }
 
+// The same from a converged warp: carried out by the lane whose `leader` is non-zero. A role that
+// runs as a whole warp keeps its addresses and coordinates in uniform registers, where the
+// instruction wants them; inside a one-lane branch each is moved there first.
+__device__ __forceinline__ void mbar_expect_tx_if(uint32_t leader, uint32_t bar, uint32_t bytes) {
+    asm volatile(
+            "{\n\t.reg .pred q;\n\tsetp.ne.b32 q, %2, 0;\n\t"
+            "@q mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;\n\t}" ::"r"(bar),
+            "r"(bytes), "r"(leader)
+            : "memory");
+}
+__device__ __forceinline__ void tma_load_2d_if(
+        uint32_t leader, uint32_t smem, const CUtensorMap* map, uint32_t bar, int c0, int c1) {
+    asm volatile(
+            "{\n\t.reg .pred q;\n\tsetp.ne.b32 q, %5, 0;\n\t"
+            "@q cp.async.bulk.tensor.2d.shared::cluster.global.tile.mbarrier::complete_tx::bytes"
+            " [%0], [%1, {%3, %4}], [%2];\n\t}" ::"r"(smem),
+            "l"((uint64_t)map), "r"(bar), "r"(c0), "r"(c1), "r"(leader)
+            : "memory");
+}
+__device__ __forceinline__ void tma_load_im2col_4d_if(
+        uint32_t leader, uint32_t smem, const CUtensorMap* map, uint32_t bar, int c, int w, int h,
+        int n, uint16_t off_w, uint16_t off_h) {
+    asm volatile(
+            "{\n\t.reg .pred q;\n\tsetp.ne.b32 q, %9, 0;\n\t"
+            "@q cp.async.bulk.tensor.4d.shared::cluster.global.im2col.mbarrier::complete_tx::bytes"
+            " [%0], [%1, {%3, %4, %5, %6}], [%2], {%7, %8};\n\t}" ::"r"(smem),
+            "l"((uint64_t)map), "r"(bar), "r"(c), "r"(w), "r"(h), "r"(n), "h"(off_w), "h"(off_h),
+            "r"(leader)
+            : "memory");
+}
+
 // Shared-memory matrix descriptor of a K-major operand tile.
 //   swizzled (64 B): rows of 64 bytes, 8-row groups `sbo` bytes apart, `lbo` unused
 //   plain:           8x16-byte core matrices; `lbo` = distance between the two 16-byte K
