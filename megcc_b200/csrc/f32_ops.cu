@@ -213,6 +213,46 @@ __global__ void __launch_bounds__(256) pooling_f32_kernel(
     }
 }
 
+// Max pooling with stride 1 and a large window (the 5, 9 and 13 wide pools of a detector's
+// spatial pyramid): a maximum over a window is a maximum of row maxima. One CTA keeps an image's
+// `cv` float4 of channels in shared memory, takes the maxima along the rows into a second buffer
+// and then along the columns: wh + ww reads per output instead of wh * ww, each input read from
+// memory once. 32 x 20 x 20 x 256, window 13: 157 us with a thread per window.
+__global__ void __launch_bounds__(256) maxpool_rows_f32_kernel(
+        const float4* __restrict__ src, float4* __restrict__ dst, int c4, int cv, int ih, int iw,
+        int oh, int ow, int wh, int ww, int ph, int pw) {
+    pdl_start();
+    extern __shared__ float4 pool_smem[];
+    float4* rows = pool_smem + (size_t)ih * iw * cv;  // [ih][ow][cv]
+    const float low = -3.402823466e38f;
+    const size_t in0 = (size_t)blockIdx.y * ih * iw * c4 + (size_t)blockIdx.x * cv;
+    const size_t out0 = (size_t)blockIdx.y * oh * ow * c4 + (size_t)blockIdx.x * cv;
+    auto larger = [](float4& a, const float4& v) {
+        a.x = fmaxf(a.x, v.x); a.y = fmaxf(a.y, v.y);
+        a.z = fmaxf(a.z, v.z); a.w = fmaxf(a.w, v.w);
+    };
+    for (int i = threadIdx.x; i < ih * iw * cv; i += blockDim.x)
+        pool_smem[i] = __ldg(src + in0 + (size_t)(i / cv) * c4 + i % cv);
+    __syncthreads();
+    for (int i = threadIdx.x; i < ih * ow * cv; i += blockDim.x) {
+        const int ch = i % cv, x = i / cv % ow, y = i / cv / ow;
+        const int x0 = max(x - pw, 0), x1 = min(x - pw + ww, iw);
+        float4 acc = make_float4(low, low, low, low);
+        for (int ix = x0; ix < x1; ++ix)
+            larger(acc, pool_smem[(y * iw + ix) * cv + ch]);
+        rows[i] = acc;
+    }
+    __syncthreads();
+    for (int i = threadIdx.x; i < oh * ow * cv; i += blockDim.x) {
+        const int ch = i % cv, x = i / cv % ow, y = i / cv / ow;
+        const int y0 = max(y - ph, 0), y1 = min(y - ph + wh, ih);
+        float4 acc = make_float4(low, low, low, low);
+        for (int iy = y0; iy < y1; ++iy)
+            larger(acc, rows[(iy * ow + x) * cv + ch]);
+        dst[out0 + (size_t)(i / cv) * c4 + ch] = acc;
+    }
+}
+
 // Focus: out[b][y][x][k * C + ch] = in[b][ch][2y + dy_k][2x + dx_k] with the slice order
 // (dy, dx) = (0,0), (1,0), (0,1), (1,1); output channels beyond 4 * C are written as zeros so
 // that the 16-channel rows the first ConvBias loads hold no stale data. One thread per
@@ -238,6 +278,42 @@ __global__ void __launch_bounds__(256) focus_f32_kernel(
         }
         for (int ch = 4 * c; ch < c_out; ++ch)
             o[ch] = 0.f;
+    }
+}
+
+// The same for images of three channels and 16-channel rows: a thread reads its pixel's two
+// columns of each plane row as one 8-byte load (a warp: 256 bytes) and writes the 64-byte row in
+// two whole sectors. Bound by HBM: 32 images of 640 x 640 took 250 us with single floats.
+__global__ void __launch_bounds__(256) focus_rgb_f32_kernel(
+        const float* __restrict__ src, float* __restrict__ dst, int n, int h, int w) {
+    pdl_start();
+    const int h2 = h / 2, w2 = w / 2;
+    const size_t total = (size_t)n * h2 * w2, plane = (size_t)h * w;
+    for (size_t idx = blockIdx.x * (size_t)blockDim.x + threadIdx.x; idx < total;
+         idx += (size_t)gridDim.x * blockDim.x) {
+        const int x = (int)(idx % w2);
+        const size_t t = idx / w2;
+        const int y = (int)(t % h2);
+        const float* s = src + (t / h2) * 3 * plane + (size_t)(2 * y) * w + 2 * x;
+        float v[16];
+#pragma unroll
+        for (int ch = 0; ch < 3; ++ch)
+#pragma unroll
+            for (int dy = 0; dy < 2; ++dy) {
+                const float2 two = __ldg(reinterpret_cast<const float2*>(s + ch * plane + (size_t)dy * w));
+                v[dy * 3 + ch] = two.x;
+                v[(2 + dy) * 3 + ch] = two.y;
+            }
+#pragma unroll
+        for (int j = 12; j < 16; ++j)
+            v[j] = 0.f;
+        float* o = dst + idx * 16;
+#pragma unroll
+        for (int j = 0; j < 16; j += 8)
+            asm volatile("st.global.v8.f32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"l"(o + j),
+                         "f"(v[j]), "f"(v[j + 1]), "f"(v[j + 2]), "f"(v[j + 3]), "f"(v[j + 4]),
+                         "f"(v[j + 5]), "f"(v[j + 6]), "f"(v[j + 7])
+                         : "memory");
     }
 }
 
@@ -313,6 +389,26 @@ int launch_pooling_f32(
         int sh, int sw, int ph, int pw, cudaStream_t st) {
     const int oh = (ih + 2 * ph - wh) / sh + 1, ow = (iw + 2 * pw - ww) / sw + 1;
     const int vec = (c % 4 == 0 && ((((uintptr_t)src | (uintptr_t)dst) & 15) == 0)) ? 1 : 0;
+    // Row maxima pay from about a 3 x 3 window on; the image's channels of a CTA, raw and reduced,
+    // have to fit shared memory. 32 channels per CTA (128-byte rows) while that gives every SM
+    // one, else 8 (a sector).
+    if (mode == 0 && vec && sh == 1 && sw == 1 && wh * ww > 9 && n <= 65535 && c / 4 <= 65535) {
+        constexpr size_t kMost = 100 * 1024;  // two CTAs on an SM
+        const size_t per_cv = ((size_t)ih * iw + (size_t)ih * ow) * 16;
+        for (int cv = 8; cv >= 1; cv /= 2) {
+            if ((c / 4) % cv || per_cv * cv > kMost)
+                continue;
+            if (cv > 2 && (size_t)n * (c / 4 / cv) < (size_t)umma::sm_count() && (c / 4) % (cv / 2) == 0)
+                continue;
+            static umma::KernelReady ready;
+            if (!ready.smem(maxpool_rows_f32_kernel, (int)kMost))
+                return check_launch("maxpool_rows_f32 smem attribute");
+            launch_pdl(maxpool_rows_f32_kernel, dim3(c / 4 / cv, n), dim3(256), per_cv * cv, st,
+                       reinterpret_cast<const float4*>(src), reinterpret_cast<float4*>(dst), c / 4,
+                       cv, ih, iw, oh, ow, wh, ww, ph, pw);
+            return check_launch("maxpool_rows_f32");
+        }
+    }
     const size_t work = (size_t)n * oh * ow * (c / (vec ? 4 : 1));
     launch_pdl(pooling_f32_kernel, dim3(grid_for_f32(work, 256)), dim3(256), 0, st, src, dst, mode, n,
                c, ih, iw, oh, ow, wh, ww, sh, sw, ph, pw, vec);
@@ -323,6 +419,13 @@ int launch_focus_f32(
         const float* src_nchw, float* dst_nhwc, int n, int c, int h, int w, int c_out,
         cudaStream_t st) {
     const size_t work = (size_t)n * (h / 2) * (w / 2);
+    // whole columns of two: an even width and planes that start on 8 bytes; rows of two sectors
+    if (c == 3 && c_out == 16 && w % 2 == 0 && h % 2 == 0 && ((uintptr_t)src_nchw & 7) == 0 &&
+        ((uintptr_t)dst_nhwc & 31) == 0) {
+        launch_pdl(focus_rgb_f32_kernel, dim3(grid_for_f32(work, 256)), dim3(256), 0, st, src_nchw,
+                   dst_nhwc, n, h, w);
+        return check_launch("focus_rgb_f32");
+    }
     launch_pdl(focus_f32_kernel, dim3(grid_for_f32(work, 256)), dim3(256), 0, st, src_nchw, dst_nhwc,
                n, c, h, w, c_out);
     return check_launch("focus_f32");
