@@ -57,6 +57,43 @@ size_t plain_filter_bytes(const ConvF32Args& a) {
 
 }  // namespace
 
+namespace mb200 {
+
+int conv_bias_f32_pitched(
+        const mb200_conv_f32_param* p, const float* src, long long src_pitch,
+        const float* flt_packed, const float* bias, const float* z, long long z_pitch, float* dst,
+        long long dst_pitch, void* workspace, size_t workspace_bytes, int algo, cudaStream_t st) {
+    ConvF32Args a{};
+    int rc = make_f32_args(p, dst_pitch, &a);
+    if (rc)
+        return rc;
+    if (src_pitch > 0)
+        a.src_pitch = src_pitch;
+    if (z_pitch > 0)
+        a.z_pitch = z_pitch;
+    if (!src || !flt_packed || !dst)
+        return set_error(ST_NULL_PTR, "conv tensor pointer is NULL");
+    if (((uintptr_t)src | (uintptr_t)flt_packed | (uintptr_t)dst | (uintptr_t)bias |
+         (uintptr_t)z) & 3)
+        return set_error(ST_INVALID_LAYOUT, "fp32 operands must be 4-byte aligned");
+    const bool umma_ok = conv_f32_umma_supported(a, src, dst) &&
+                         workspace_bytes >= conv_f32_workspace_bytes(a) &&
+                         (((uintptr_t)workspace | (uintptr_t)flt_packed | (uintptr_t)bias |
+                           (uintptr_t)z) & 15) == 0;
+    if (algo == MB200_ALGO_UMMA && !umma_ok)
+        return set_error(ST_NO_IMPLEMENT,
+                         "tensor-core fp32 ConvBias needs a dense filter, ic %% 4 == 0 (with a spatial "
+                         "filter ic == 16 or ic >= 32), 16-byte aligned operands and, with a spatial "
+                         "filter, >= 128 KiB of readable memory from the input on");
+    if (algo == MB200_ALGO_UMMA || (algo == MB200_ALGO_AUTO && umma_ok))
+        return launch_conv_f32_umma(a, src, flt_packed, bias, z, dst, workspace, st);
+    if (algo != MB200_ALGO_AUTO && algo != MB200_ALGO_DIRECT)
+        return set_error(ST_OUT_OF_RANGE, "unknown algo %d", algo);
+    return launch_conv_f32_direct(a, src, flt_packed, bias, z, dst, st);
+}
+
+}  // namespace mb200
+
 extern "C" {
 
 size_t mb200_conv_f32_packed_filter_bytes(const mb200_conv_f32_param* p) {
@@ -93,30 +130,8 @@ int mb200_conv_bias_f32_nhwc(
         const mb200_conv_f32_param* p, const float* src, const float* flt_packed,
         const float* bias, const float* z, float* dst, long long dst_pitch, void* workspace,
         size_t workspace_bytes, int algo, void* stream) {
-    ConvF32Args a{};
-    int rc = make_f32_args(p, dst_pitch, &a);
-    if (rc)
-        return rc;
-    if (!src || !flt_packed || !dst)
-        return set_error(ST_NULL_PTR, "conv tensor pointer is NULL");
-    if (((uintptr_t)src | (uintptr_t)flt_packed | (uintptr_t)dst | (uintptr_t)bias |
-         (uintptr_t)z) & 3)
-        return set_error(ST_INVALID_LAYOUT, "fp32 operands must be 4-byte aligned");
-    cudaStream_t st = (cudaStream_t)stream;
-    const bool umma_ok = conv_f32_umma_supported(a, src, dst) &&
-                         workspace_bytes >= conv_f32_workspace_bytes(a) &&
-                         (((uintptr_t)workspace | (uintptr_t)flt_packed | (uintptr_t)bias |
-                           (uintptr_t)z) & 15) == 0;
-    if (algo == MB200_ALGO_UMMA && !umma_ok)
-        return set_error(ST_NO_IMPLEMENT,
-                         "tensor-core fp32 ConvBias needs a dense filter, ic %% 4 == 0 (with a spatial "
-                         "filter ic == 16 or ic >= 32), 16-byte aligned operands and, with a spatial "
-                         "filter, >= 128 KiB of readable memory from the input on");
-    if (algo == MB200_ALGO_UMMA || (algo == MB200_ALGO_AUTO && umma_ok))
-        return launch_conv_f32_umma(a, src, flt_packed, bias, z, dst, workspace, st);
-    if (algo != MB200_ALGO_AUTO && algo != MB200_ALGO_DIRECT)
-        return set_error(ST_OUT_OF_RANGE, "unknown algo %d", algo);
-    return launch_conv_f32_direct(a, src, flt_packed, bias, z, dst, st);
+    return conv_bias_f32_pitched(p, src, 0, flt_packed, bias, z, 0, dst, dst_pitch, workspace,
+                                 workspace_bytes, algo, (cudaStream_t)stream);
 }
 
 // ---- fp32 matrix product: a 1x1 ConvBias over M "pixels" with K channels ----
@@ -202,7 +217,7 @@ int mb200_concat_f32_nhwc(
         return set_error(ST_NULL_PTR, "concat pointer is NULL");
     if (pixels == 0)
         return ST_SUCCESS;
-    return launch_concat_f32(srcs, channels, nr_inputs, dst, pixels, (cudaStream_t)stream);
+    return launch_concat_f32(srcs, channels, nullptr, nr_inputs, dst, pixels, (cudaStream_t)stream);
 }
 
 int mb200_resize_nearest_f32_nhwc(
@@ -211,7 +226,7 @@ int mb200_resize_nearest_f32_nhwc(
         return set_error(ST_NULL_PTR, "resize tensor pointer is NULL");
     if (n <= 0 || c <= 0 || ih <= 0 || iw <= 0 || oh <= 0 || ow <= 0)
         return set_error(ST_INVALID_LAYOUT, "resize extents must be positive");
-    return launch_resize_nearest_f32(src, dst, n, c, ih, iw, oh, ow, (cudaStream_t)stream);
+    return launch_resize_nearest_f32(src, dst, n, c, ih, iw, oh, ow, c, c, (cudaStream_t)stream);
 }
 
 int mb200_pooling_f32_nhwc(
@@ -227,7 +242,7 @@ int mb200_pooling_f32_nhwc(
         pad_w >= window_w)
         return set_error(ST_INVALID_LAYOUT, "pooling extents are invalid");
     return launch_pooling_f32(src, dst, mode, n, c, ih, iw, window_h, window_w, stride_h,
-                              stride_w, pad_h, pad_w, (cudaStream_t)stream);
+                              stride_w, pad_h, pad_w, c, c, (cudaStream_t)stream);
 }
 
 int mb200_focus_f32(

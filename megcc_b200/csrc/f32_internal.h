@@ -42,15 +42,22 @@ int launch_conv_f32_umma(
 
 int launch_elemwise_f32(
         int mode, const float* a, const float* b, float* dst, size_t nr_elem, cudaStream_t st);
+// (pitches: floats between consecutive pixels; concat: null for dense inputs, an input that lies
+// in its place of dst already is left alone)
 int launch_concat_f32(
-        const float* const* srcs, const int* channels, int nr, float* dst, size_t pixels,
-        cudaStream_t st);
+        const float* const* srcs, const int* channels, const long long* pitches, int nr, float* dst,
+        size_t pixels, cudaStream_t st);
 int launch_resize_nearest_f32(
         const float* src, float* dst, int n, int c, int ih, int iw, int oh, int ow,
-        cudaStream_t st);
+        long long src_pitch, long long dst_pitch, cudaStream_t st);
 int launch_pooling_f32(
         const float* src, float* dst, int mode, int n, int c, int ih, int iw, int wh, int ww,
-        int sh, int sw, int ph, int pw, cudaStream_t st);
+        int sh, int sw, int ph, int pw, long long src_pitch, long long dst_pitch, cudaStream_t st);
+// mb200_conv_bias_f32_nhwc over operands that are slices of wider pixels (0: dense)
+int conv_bias_f32_pitched(
+        const mb200_conv_f32_param* p, const float* src, long long src_pitch,
+        const float* flt_packed, const float* bias, const float* z, long long z_pitch, float* dst,
+        long long dst_pitch, void* workspace, size_t workspace_bytes, int algo, cudaStream_t st);
 int launch_focus_f32(
         const float* src_nchw, float* dst_nhwc, int n, int c, int h, int w, int c_out,
         cudaStream_t st);

@@ -98,8 +98,9 @@ __global__ void __launch_bounds__(256) elemwise_f32_kernel(
 constexpr int kMaxConcat = 8;
 struct ConcatArgs {
     const float* src[kMaxConcat];
-    int channels[kMaxConcat];
+    int pitch[kMaxConcat];   // floats between consecutive pixels of input i
     int offset[kMaxConcat];  // first output channel of input i
+    int skip[kMaxConcat];    // input i lies in dst already
     int nr, c_out, vec;
 };
 
@@ -119,7 +120,9 @@ __global__ void __launch_bounds__(256) concat_f32_kernel(ConcatArgs a, float* __
         for (int i = 1; i < kMaxConcat; ++i)
             if (i < a.nr && ch >= a.offset[i])
                 k = i;
-        const float* s = a.src[k] + px * (size_t)a.channels[k] + (ch - a.offset[k]);
+        if (a.skip[k])
+            continue;
+        const float* s = a.src[k] + px * (size_t)a.pitch[k] + (ch - a.offset[k]);
         float* d = dst + px * (size_t)a.c_out + ch;
         if (a.vec)
             *reinterpret_cast<float4*>(d) = __ldg(reinterpret_cast<const float4*>(s));
@@ -130,7 +133,7 @@ __global__ void __launch_bounds__(256) concat_f32_kernel(ConcatArgs a, float* __
 
 __global__ void __launch_bounds__(256) resize_nearest_f32_kernel(
         const float* __restrict__ src, float* __restrict__ dst, int n, int c, int ih, int iw,
-        int oh, int ow, float scale_h, float scale_w, int vec) {
+        int oh, int ow, float scale_h, float scale_w, int vec, int src_pitch, int dst_pitch) {
     pdl_start();
     const int step = vec ? 4 : 1;
     const int cv = c / step;
@@ -149,8 +152,8 @@ __global__ void __launch_bounds__(256) resize_nearest_f32_kernel(
         int sx = (int)((float)x / scale_w);
         sy = sy < ih - 1 ? sy : ih - 1;
         sx = sx < iw - 1 ? sx : iw - 1;
-        const float* s = src + (((size_t)b * ih + sy) * iw + sx) * c + ch;
-        float* d = dst + (((size_t)b * oh + y) * ow + x) * c + ch;
+        const float* s = src + (((size_t)b * ih + sy) * iw + sx) * src_pitch + ch;
+        float* d = dst + (((size_t)b * oh + y) * ow + x) * dst_pitch + ch;
         if (vec)
             *reinterpret_cast<float4*>(d) = __ldg(reinterpret_cast<const float4*>(s));
         else
@@ -161,7 +164,8 @@ __global__ void __launch_bounds__(256) resize_nearest_f32_kernel(
 // mode 0 MAX, 1 AVERAGE (divide by the window), 2 AVERAGE_COUNT_EXCLUDE_PADDING
 __global__ void __launch_bounds__(256) pooling_f32_kernel(
         const float* __restrict__ src, float* __restrict__ dst, int mode, int n, int c, int ih,
-        int iw, int oh, int ow, int wh, int ww, int sh, int sw, int ph, int pw, int vec) {
+        int iw, int oh, int ow, int wh, int ww, int sh, int sw, int ph, int pw, int vec,
+        int src_pitch, int dst_pitch) {
     pdl_start();
     const int step = vec ? 4 : 1;
     const int cv = c / step;
@@ -186,7 +190,7 @@ __global__ void __launch_bounds__(256) pooling_f32_kernel(
                 const int ix = x * sw + fx - pw;
                 if ((unsigned)ix >= (unsigned)iw)
                     continue;
-                const float* s = src + (((size_t)b * ih + iy) * iw + ix) * c + ch;
+                const float* s = src + (((size_t)b * ih + iy) * iw + ix) * src_pitch + ch;
                 float4 v;
                 if (vec)
                     v = __ldg(reinterpret_cast<const float4*>(s));
@@ -205,7 +209,7 @@ __global__ void __launch_bounds__(256) pooling_f32_kernel(
             const float d = mode == 1 ? (float)(wh * ww) : (float)count;
             acc.x /= d; acc.y /= d; acc.z /= d; acc.w /= d;
         }
-        float* o = dst + (((size_t)b * oh + y) * ow + x) * c + ch;
+        float* o = dst + (((size_t)b * oh + y) * ow + x) * dst_pitch + ch;
         if (vec)
             *reinterpret_cast<float4*>(o) = acc;
         else
@@ -219,20 +223,20 @@ __global__ void __launch_bounds__(256) pooling_f32_kernel(
 // and then along the columns: wh + ww reads per output instead of wh * ww, each input read from
 // memory once. 32 x 20 x 20 x 256, window 13: 157 us with a thread per window.
 __global__ void __launch_bounds__(256) maxpool_rows_f32_kernel(
-        const float4* __restrict__ src, float4* __restrict__ dst, int c4, int cv, int ih, int iw,
-        int oh, int ow, int wh, int ww, int ph, int pw) {
+        const float4* __restrict__ src, float4* __restrict__ dst, int src_pitch4, int dst_pitch4,
+        int cv, int ih, int iw, int oh, int ow, int wh, int ww, int ph, int pw) {
     pdl_start();
     extern __shared__ float4 pool_smem[];
     float4* rows = pool_smem + (size_t)ih * iw * cv;  // [ih][ow][cv]
     const float low = -3.402823466e38f;
-    const size_t in0 = (size_t)blockIdx.y * ih * iw * c4 + (size_t)blockIdx.x * cv;
-    const size_t out0 = (size_t)blockIdx.y * oh * ow * c4 + (size_t)blockIdx.x * cv;
+    const size_t in0 = (size_t)blockIdx.y * ih * iw * src_pitch4 + (size_t)blockIdx.x * cv;
+    const size_t out0 = (size_t)blockIdx.y * oh * ow * dst_pitch4 + (size_t)blockIdx.x * cv;
     auto larger = [](float4& a, const float4& v) {
         a.x = fmaxf(a.x, v.x); a.y = fmaxf(a.y, v.y);
         a.z = fmaxf(a.z, v.z); a.w = fmaxf(a.w, v.w);
     };
     for (int i = threadIdx.x; i < ih * iw * cv; i += blockDim.x)
-        pool_smem[i] = __ldg(src + in0 + (size_t)(i / cv) * c4 + i % cv);
+        pool_smem[i] = __ldg(src + in0 + (size_t)(i / cv) * src_pitch4 + i % cv);
     __syncthreads();
     for (int i = threadIdx.x; i < ih * ow * cv; i += blockDim.x) {
         const int ch = i % cv, x = i / cv % ow, y = i / cv / ow;
@@ -249,7 +253,7 @@ __global__ void __launch_bounds__(256) maxpool_rows_f32_kernel(
         float4 acc = make_float4(low, low, low, low);
         for (int iy = y0; iy < y1; ++iy)
             larger(acc, rows[(iy * ow + x) * cv + ch]);
-        dst[out0 + (size_t)(i / cv) * c4 + ch] = acc;
+        dst[out0 + (size_t)(i / cv) * dst_pitch4 + ch] = acc;
     }
 }
 
@@ -347,8 +351,8 @@ int launch_elemwise_f32(
 }
 
 int launch_concat_f32(
-        const float* const* srcs, const int* channels, int nr, float* dst, size_t pixels,
-        cudaStream_t st) {
+        const float* const* srcs, const int* channels, const long long* pitches, int nr, float* dst,
+        size_t pixels, cudaStream_t st) {
     if (nr < 1 || nr > kMaxConcat)
         return set_error(ST_OUT_OF_RANGE, "concat takes 1..%d inputs, not %d", kMaxConcat, nr);
     ConcatArgs a;
@@ -357,16 +361,19 @@ int launch_concat_f32(
     a.vec = (((uintptr_t)dst & 15) == 0) ? 1 : 0;
     for (int i = 0; i < kMaxConcat; ++i) {
         a.src[i] = i < nr ? srcs[i] : nullptr;
-        a.channels[i] = i < nr ? channels[i] : 0;
+        a.pitch[i] = i < nr ? (int)(pitches ? pitches[i] : channels[i]) : 0;
         a.offset[i] = a.c_out;
+        a.skip[i] = i < nr && srcs[i] == dst + a.c_out;
         if (i < nr) {
             if (channels[i] <= 0 || !srcs[i])
                 return set_error(ST_INVALID_LAYOUT, "concat input %d is empty", i);
             a.c_out += channels[i];
-            if ((channels[i] & 3) || ((uintptr_t)srcs[i] & 15))
+            if (((channels[i] | a.pitch[i]) & 3) || ((uintptr_t)srcs[i] & 15))
                 a.vec = 0;
         }
     }
+    for (int i = 0; i < nr; ++i)
+        a.skip[i] = a.skip[i] && a.pitch[i] == a.c_out && nr > 1;
     const size_t work = pixels * (size_t)(a.c_out / (a.vec ? 4 : 1));
     launch_pdl(concat_f32_kernel, dim3(grid_for_f32(work, 256)), dim3(256), 0, st, a, dst, pixels);
     return check_launch("concat_f32");
@@ -374,21 +381,22 @@ int launch_concat_f32(
 
 int launch_resize_nearest_f32(
         const float* src, float* dst, int n, int c, int ih, int iw, int oh, int ow,
-        cudaStream_t st) {
-    const int vec = (c % 4 == 0 && ((((uintptr_t)src | (uintptr_t)dst) & 15) == 0)) ? 1 : 0;
+        long long src_pitch, long long dst_pitch, cudaStream_t st) {
+    const int vec = ((c | src_pitch | dst_pitch) % 4 == 0 && ((((uintptr_t)src | (uintptr_t)dst) & 15) == 0)) ? 1 : 0;
     // scale = (float)out / in, the reference's own float expression
     const float scale_h = (float)oh / ih, scale_w = (float)ow / iw;
     const size_t work = (size_t)n * oh * ow * (c / (vec ? 4 : 1));
     launch_pdl(resize_nearest_f32_kernel, dim3(grid_for_f32(work, 256)), dim3(256), 0, st, src, dst,
-               n, c, ih, iw, oh, ow, scale_h, scale_w, vec);
+               n, c, ih, iw, oh, ow, scale_h, scale_w, vec, (int)src_pitch, (int)dst_pitch);
     return check_launch("resize_nearest_f32");
 }
 
 int launch_pooling_f32(
         const float* src, float* dst, int mode, int n, int c, int ih, int iw, int wh, int ww,
-        int sh, int sw, int ph, int pw, cudaStream_t st) {
+        int sh, int sw, int ph, int pw, long long src_pitch, long long dst_pitch, cudaStream_t st) {
     const int oh = (ih + 2 * ph - wh) / sh + 1, ow = (iw + 2 * pw - ww) / sw + 1;
-    const int vec = (c % 4 == 0 && ((((uintptr_t)src | (uintptr_t)dst) & 15) == 0)) ? 1 : 0;
+    const int vec = ((c | src_pitch | dst_pitch) % 4 == 0 &&
+                     ((((uintptr_t)src | (uintptr_t)dst) & 15) == 0)) ? 1 : 0;
     // Row maxima pay from about a 3 x 3 window on; the image's channels of a CTA, raw and reduced,
     // have to fit shared memory. 32 channels per CTA (128-byte rows) while that gives every SM
     // one, else 8 (a sector).
@@ -404,14 +412,14 @@ int launch_pooling_f32(
             if (!ready.smem(maxpool_rows_f32_kernel, (int)kMost))
                 return check_launch("maxpool_rows_f32 smem attribute");
             launch_pdl(maxpool_rows_f32_kernel, dim3(c / 4 / cv, n), dim3(256), per_cv * cv, st,
-                       reinterpret_cast<const float4*>(src), reinterpret_cast<float4*>(dst), c / 4,
-                       cv, ih, iw, oh, ow, wh, ww, ph, pw);
+                       reinterpret_cast<const float4*>(src), reinterpret_cast<float4*>(dst),
+                       (int)(src_pitch / 4), (int)(dst_pitch / 4), cv, ih, iw, oh, ow, wh, ww, ph, pw);
             return check_launch("maxpool_rows_f32");
         }
     }
     const size_t work = (size_t)n * oh * ow * (c / (vec ? 4 : 1));
     launch_pdl(pooling_f32_kernel, dim3(grid_for_f32(work, 256)), dim3(256), 0, st, src, dst, mode, n,
-               c, ih, iw, oh, ow, wh, ww, sh, sw, ph, pw, vec);
+               c, ih, iw, oh, ow, wh, ww, sh, sw, ph, pw, vec, (int)src_pitch, (int)dst_pitch);
     return check_launch("pooling_f32");
 }
 

@@ -26,6 +26,7 @@
 #include "../../include/megcc_b200.h"
 #include "../../include/megcc_b200_lite.h"
 #include "../../include/megcc_b200_runtime.h"
+#include "f32_internal.h"
 #include "internal.h"
 #include "tinynn_format.h"
 
@@ -115,6 +116,7 @@ struct MemForwardPlan {
 
 struct Instr {
     bool is_opr;
+    bool in_place = false;  // a concat whose inputs were all written into its output
     OpPlan op;
     MemForwardPlan mf;
 };
@@ -162,6 +164,9 @@ struct DevModel {
     std::vector<CapturedGraph> graphs;
     bool memory_ready = false;
     bool ran_eager = false;
+    // concat inputs that are written as channel slices of the concat's output (see join_concats)
+    std::vector<Tensor*> view_of;     // per tensor: the concat output, or null
+    std::vector<size_t> view_offset;  // ... and its first byte in there
     // independent instructions are captured side by side (see spread_small_model)
     bool side_by_side = false;
     // where tensors and workspaces really lie in the arena: as planned, or each on its own
@@ -546,6 +551,12 @@ int matrix_k(const Tensor* a) {
     return (int)(nr_elems(a) / (size_t)a->layout.dims[0]);
 }
 
+// floats between consecutive pixels of an NHWC tensor: its channels, or more for a slice
+long long pixel_pitch(const Tensor* t) {
+    const Layout& l = t->layout;
+    return l.stride[1] == 1 && l.stride[3] > (int)l.dims[1] ? l.stride[3] : (int)l.dims[1];
+}
+
 // The library's own KernelFunc: what the generated stub of op.symbol does
 // (megcc_b200/compiler/cuda_kernel_pack.cpp). One function serves every symbol; the
 // attributes a stub has baked in come from the Opr's parsed symbol, which the VM passes in
@@ -658,10 +669,11 @@ TinyNNStatus builtin_kernel(
             fill_conv_f32_param(op, inputs, &p);
             const float* bias = op.has_bias ? (const float*)inputs[2]->ptr : nullptr;
             const float* z = op.f32_z ? (const float*)inputs[nr_input - 1]->ptr : nullptr;
-            return (TinyNNStatus)mb200_conv_bias_f32_nhwc(
-                    &p, (const float*)inputs[0]->ptr, (const float*)inputs[1]->ptr, bias, z,
-                    (float*)dst->ptr, (long long)dst->layout.stride[3], ws->ptr, ws->size,
-                    MB200_ALGO_AUTO, st);
+            return (TinyNNStatus)mb200::conv_bias_f32_pitched(
+                    &p, (const float*)inputs[0]->ptr, pixel_pitch(inputs[0]),
+                    (const float*)inputs[1]->ptr, bias, z,
+                    z ? pixel_pitch(inputs[nr_input - 1]) : 0, (float*)dst->ptr, pixel_pitch(dst),
+                    ws->ptr, ws->size, MB200_ALGO_AUTO, (cudaStream_t)st);
         }
         case OP_MATMUL_F32: {
             const Tensor* a = inputs[0];
@@ -679,15 +691,18 @@ TinyNNStatus builtin_kernel(
         case OP_CONCAT_F32: {
             const float* srcs[8];
             int channels[8];
+            long long pitches[8];
             if (nr_input > 8)
                 return TinyNN_ERROR_OUT_OF_RANGE;
             for (int i = 0; i < nr_input; ++i) {
                 srcs[i] = (const float*)inputs[i]->ptr;
                 channels[i] = inputs[i]->layout.dims[1];
+                pitches[i] = pixel_pitch(inputs[i]);
             }
-            return (TinyNNStatus)mb200_concat_f32_nhwc(
-                    srcs, channels, nr_input, (float*)dst->ptr,
-                    (size_t)dst->layout.dims[0] * dst->layout.dims[2] * dst->layout.dims[3], st);
+            return (TinyNNStatus)mb200::launch_concat_f32(
+                    srcs, channels, pitches, nr_input, (float*)dst->ptr,
+                    (size_t)dst->layout.dims[0] * dst->layout.dims[2] * dst->layout.dims[3],
+                    (cudaStream_t)st);
         }
         case OP_FOCUS_F32: {
             const Tensor* s = inputs[0];
@@ -697,17 +712,19 @@ TinyNNStatus builtin_kernel(
         }
         case OP_RESIZE_F32: {
             const Tensor* s = inputs[0];
-            return (TinyNNStatus)mb200_resize_nearest_f32_nhwc(
+            return (TinyNNStatus)mb200::launch_resize_nearest_f32(
                     (const float*)s->ptr, (float*)dst->ptr, s->layout.dims[0], s->layout.dims[1],
                     s->layout.dims[2], s->layout.dims[3], dst->layout.dims[2], dst->layout.dims[3],
-                    st);
+                    pixel_pitch(s), pixel_pitch(dst), (cudaStream_t)st);
         }
         case OP_POOL_F32: {
             const Tensor* s = inputs[0];
-            return (TinyNNStatus)mb200_pooling_f32_nhwc(
+            if (op.sh <= 0 || op.sw <= 0 || op.kh <= 0 || op.kw <= 0)
+                return TinyNN_ERROR_INVALID_LAYOUT;
+            return (TinyNNStatus)mb200::launch_pooling_f32(
                     (const float*)s->ptr, (float*)dst->ptr, op.mode, s->layout.dims[0],
                     s->layout.dims[1], s->layout.dims[2], s->layout.dims[3], op.kh, op.kw, op.sh,
-                    op.sw, op.ph, op.pw, st);
+                    op.sw, op.ph, op.pw, pixel_pitch(s), pixel_pitch(dst), (cudaStream_t)st);
         }
         case OP_EXTERNAL:
             break;
@@ -1018,15 +1035,24 @@ bool read_layout(const fb::Table& t, Layout* out) {
     return true;
 }
 
-// May the two instructions run at the same time? (by the tensors they name: outputs and
+// Do the tensors share memory by intent (equal, or a slice and the whole)?
+bool same_memory(const DevModel& m, const Tensor* a, const Tensor* b) {
+    auto whole = [&](const Tensor* t) -> const Tensor* {
+        const size_t i = t - m.tensors.data();  // (a weight is not one of the model's tensors)
+        return t >= m.tensors.data() && i < m.view_of.size() ? m.view_of[i] : nullptr;
+    };
+    return a == b || whole(a) == b || whole(b) == a;
+}
+
+// May the two instructions not run at the same time? (by the tensors they name: outputs and
 // workspaces have memory of their own here)
-bool conflicts(const Instr& a, const Instr& b) {
-    auto touches = [](const Instr& i, const Tensor* t) {
+bool conflicts(const DevModel& m, const Instr& a, const Instr& b) {
+    auto touches = [&](const Instr& i, const Tensor* t) {
         for (const Tensor* x : i.op.inputs)
-            if (x == t)
+            if (same_memory(m, x, t))
                 return true;
         for (const Tensor* x : i.op.outputs)
-            if (x == t)
+            if (same_memory(m, x, t))
                 return true;
         return false;
     };
@@ -1039,13 +1065,8 @@ bool conflicts(const Instr& a, const Instr& b) {
     return false;
 }
 
-// A small model (a batch of one) is bound by the latency of its instructions one after the
-// other, each of which leaves most SMs idle. Where it has branches (the heads of a detector,
-// the two arms of a residual block) and all its tensors fit the L2 together, every tensor gets
-// memory of its own instead of the planned reuse, so that nothing but data ties two
-// instructions, and independent instructions are captured on parallel branches of the graph.
-void spread_small_model(DevModel& m) {
-    constexpr size_t kMost = 96u << 20;
+// Tensors and workspaces where the model file's memory plan puts them.
+void place_as_planned(DevModel& m) {
     m.arena_bytes = m.tensor_memory;
     m.tensor_place.clear();
     for (auto& t : m.tensors)
@@ -1053,31 +1074,195 @@ void spread_small_model(DevModel& m) {
     m.ws_place.clear();
     for (auto& ins : m.instrs)
         m.ws_place.push_back(ins.is_opr ? ins.op.ws.offset : 0);
+    m.view_of.assign(m.tensors.size(), nullptr);
+    m.view_offset.assign(m.tensors.size(), 0);
+}
+
+constexpr size_t kPlaceAlign = 256;
+size_t place_up(size_t v) {
+    return (v + kPlaceAlign - 1) / kPlaceAlign * kPlaceAlign;
+}
+
+// Concats along channels without the copy: an input whose producer and readers all take a pixel
+// pitch (ConvBias, nearest resize, pooling) becomes a slice of the concat's output, written there
+// in the first place. A copy costs a read and a write of the whole output and one more link
+// in a small batch's chain (a detector of 32 frames spends 0.43 of 7 ms on them). Slices start
+// on 16 bytes, as the tensor-core path asks. Only the library's own kernels read the pitch.
+bool join_concats(DevModel& m) {
+    for (auto& ins : m.instrs)
+        if (!ins.is_opr || ins.op.kernel_fn != builtin_kernel)
+            return false;
+    auto index = [&](const Tensor* t) {
+        return t >= m.tensors.data() && t < m.tensors.data() + m.tensors.size()
+                       ? (int)(t - m.tensors.data())
+                       : -1;
+    };
+    std::vector<char> fixed(m.tensors.size(), 0);  // the caller sees it
+    for (auto& s : m.inputs)
+        fixed[s.tensor - m.tensors.data()] = 1;
+    for (auto& s : m.outputs)
+        fixed[s.tensor - m.tensors.data()] = 1;
+    std::vector<char> whole(m.tensors.size(), 0);  // has slices of its own
+    bool any = false;
+    for (auto& ins : m.instrs) {
+        OpPlan& cat = ins.op;
+        if (cat.kind != OP_CONCAT_F32)
+            continue;
+        Tensor* out = cat.outputs[0];
+        const int oi = index(out);
+        if (oi < 0 || m.view_of[oi] || fixed[oi] || out->layout.dims[1] % 4 ||
+            out->layout.stride[1] != 1)
+            continue;
+        bool all = true;
+        size_t channel = 0;
+        for (Tensor* t : cat.inputs) {
+            const size_t at = channel;
+            channel += t->layout.dims[1];
+            const int ti = index(t);
+            bool ok = ti >= 0 && !fixed[ti] && !m.view_of[ti] && !whole[ti] && at % 4 == 0 &&
+                      t->layout.dims[1] % 4 == 0 && t->layout.stride[1] == 1;
+            int written = 0, taken = 0;
+            for (auto& other : m.instrs) {
+                const OpPlan& o = other.op;
+                const bool pitched = o.kind == OP_CONV_F32 || o.kind == OP_RESIZE_F32 ||
+                                     o.kind == OP_POOL_F32;
+                for (const Tensor* x : o.outputs)
+                    if (x == t) {
+                        ++written;
+                        ok &= pitched;
+                    }
+                for (const Tensor* x : o.inputs)
+                    if (x == t) {
+                        taken += &other == &ins;
+                        ok &= pitched || o.kind == OP_CONCAT_F32;
+                    }
+            }
+            if (!ok || written != 1 || taken != 1) {
+                all = false;
+                continue;
+            }
+            m.view_of[ti] = out;
+            m.view_offset[ti] = at * sizeof(float);
+            for (int d : {0, 2, 3})
+                t->layout.stride[d] = out->layout.stride[d];
+            whole[oi] = 1;
+            any = true;
+        }
+        ins.in_place = all;
+    }
+    return any;
+}
+
+// A memory plan of the model with its slices: the largest tensor first, each at the lowest
+// place where no tensor that lives at the same time lies.
+void plan_memory(DevModel& m) {
+    const int n = (int)m.instrs.size(), nt = (int)m.tensors.size();
+    struct Block {
+        size_t bytes, at;
+        int first, last, tensor, ws;
+    };
+    std::vector<Block> blocks;
+    std::vector<int> block_of(nt);
+    for (int t = 0; t < nt; ++t) {
+        block_of[t] = (int)blocks.size();
+        blocks.push_back({place_up(m.tensors[t].size), 0, n, -1, t, -1});
+    }
+    auto live = [&](const Tensor* t, int at) {
+        if (t < m.tensors.data() || t >= m.tensors.data() + nt)
+            return;
+        int i = (int)(t - m.tensors.data());
+        if (m.view_of[i])
+            i = (int)(m.view_of[i] - m.tensors.data());
+        Block& b = blocks[block_of[i]];
+        b.first = std::min(b.first, at);
+        b.last = std::max(b.last, at);
+    };
+    for (auto& s : m.inputs)
+        live(s.tensor, -1);
+    for (auto& s : m.outputs)
+        live(s.tensor, n);
+    for (int i = 0; i < n; ++i) {
+        for (const Tensor* t : m.instrs[i].op.inputs)
+            live(t, i);
+        for (const Tensor* t : m.instrs[i].op.outputs)
+            live(t, i);
+        if (m.instrs[i].op.ws.size)
+            blocks.push_back({place_up(m.instrs[i].op.ws.size), 0, i, i, -1, i});
+    }
+    std::vector<Block*> order;
+    for (auto& b : blocks)
+        if (b.last >= b.first && !(b.tensor >= 0 && m.view_of[b.tensor]))
+            order.push_back(&b);
+    std::stable_sort(order.begin(), order.end(),
+                     [](const Block* a, const Block* b) { return a->bytes > b->bytes; });
+    std::vector<Block*> placed;  // by address
+    m.arena_bytes = 0;
+    for (Block* b : order) {
+        size_t at = 0;
+        for (const Block* p : placed) {
+            if (p->last < b->first || b->last < p->first)
+                continue;
+            if (at + b->bytes <= p->at)
+                break;
+            at = std::max(at, p->at + p->bytes);
+        }
+        b->at = at;
+        placed.insert(std::upper_bound(placed.begin(), placed.end(), b,
+                                       [](const Block* x, const Block* y) { return x->at < y->at; }),
+                      b);
+        m.arena_bytes = std::max(m.arena_bytes, at + b->bytes);
+        if (b->tensor >= 0)
+            m.tensor_place[b->tensor] = at;
+        else
+            m.ws_place[b->ws] = at;
+    }
+}
+
+// A small model (a batch of one) is bound by the latency of its instructions one after the
+// other, each of which leaves most SMs idle. Where it has branches (the heads of a detector,
+// the two arms of a residual block) and all its tensors fit the L2 together, every tensor gets
+// memory of its own instead of the planned reuse, so that nothing but data ties two
+// instructions, and independent instructions are captured on parallel branches of the graph.
+bool spread_small_model(DevModel& m) {
+    constexpr size_t kMost = 96u << 20;
     size_t total = 0;
-    auto up = [](size_t v) { return (v + 255) / 256 * 256; };
-    for (auto& t : m.tensors)
-        total += up(t.size);
+    for (size_t i = 0; i < m.tensors.size(); ++i)
+        total += m.view_of[i] ? 0 : place_up(m.tensors[i].size);
     bool branches = false;
     for (size_t i = 0; i < m.instrs.size(); ++i) {
         if (!m.instrs[i].is_opr)
-            return;  // an alias of another tensor: keep the plan
-        total += up(m.instrs[i].op.ws.size);
-        branches |= i > 0 && !conflicts(m.instrs[i - 1], m.instrs[i]);
+            return false;  // an alias of another tensor: keep the plan
+        total += place_up(m.instrs[i].op.ws.size);
+        branches |= i > 0 && !conflicts(m, m.instrs[i - 1], m.instrs[i]);
     }
     if (!branches || total > kMost)
-        return;
+        return false;
     size_t off = 0;
     for (size_t i = 0; i < m.tensors.size(); ++i) {
+        if (m.view_of[i])
+            continue;
         m.tensor_place[i] = off;
-        off += up(m.tensors[i].size);
+        off += place_up(m.tensors[i].size);
     }
     for (size_t i = 0; i < m.instrs.size(); ++i)
         if (m.instrs[i].op.ws.size) {
             m.ws_place[i] = off;
-            off += up(m.instrs[i].op.ws.size);
+            off += place_up(m.instrs[i].op.ws.size);
         }
-    m.arena_bytes = off > m.tensor_memory ? off : m.tensor_memory;
+    m.arena_bytes = off;
     m.side_by_side = true;
+    return true;
+}
+
+// What the runtime makes of the file's plan: slices, and room for parallel branches.
+void arrange_model(DevModel& m) {
+    const bool joined = join_concats(m);
+    if (!spread_small_model(m) && joined)
+        plan_memory(m);
+    for (size_t i = 0; i < m.tensors.size(); ++i)
+        if (m.view_of[i])
+            m.tensor_place[i] =
+                    m.tensor_place[m.view_of[i] - m.tensors.data()] + m.view_offset[i];
 }
 
 int parse_model(Network* net, const void* mem, size_t size) {
@@ -1297,7 +1482,7 @@ int parse_model(Network* net, const void* mem, size_t size) {
             }
             m.instrs.push_back(std::move(ins));
         }
-        spread_small_model(m);
+        place_as_planned(m);
         if (m.arena_bytes > net->arena_need)
             net->arena_need = m.arena_bytes;
     }
@@ -1515,7 +1700,7 @@ int issue_instructions(Network* net, DevModel& m, bool timed) {
         cudaEventCreate(&ev1);
     }
     for (auto& ins : m.instrs) {
-        if (!ins.is_opr)
+        if (!ins.is_opr || ins.in_place)
             continue;  // memforward is resolved when the arena is laid out
         if (timed)
             cudaEventRecord(ev0, net->stream);
@@ -1563,11 +1748,14 @@ int issue_side_by_side(Network* net, DevModel& m) {
     cudaError_t e = cudaEventRecord(fork, net->stream);
     bool started[kLanes] = {true};
     for (int i = 0; i < n && e == cudaSuccess; ++i) {
+        if (m.instrs[i].in_place)
+            continue;
         int need[kLanes];  // latest dependency on each lane
         for (int l = 0; l < kLanes; ++l)
             need[l] = -1;
         for (int j = i - 1; j >= 0; --j)
-            if (need[lane_of[j]] < 0 && conflicts(m.instrs[j], m.instrs[i]))
+            if (!m.instrs[j].in_place && need[lane_of[j]] < 0 &&
+                conflicts(m, m.instrs[j], m.instrs[i]))
                 need[lane_of[j]] = j;
         int best = -1, free_lane = -1, any = 0;
         for (int l = 0; l < kLanes; ++l) {
@@ -1910,7 +2098,14 @@ int LITE_load_model_from_mem(LiteNetwork network, void* model_mem, size_t size) 
     if (net->loaded)
         return fail(TinyNN_ERROR, "this network already holds a model");
     const int rc = parse_model(net, model_mem, size);
-    return rc ? rc : upload_weights(net);
+    if (rc)
+        return rc;
+    net->arena_need = 0;
+    for (auto& m : net->models) {
+        arrange_model(m);
+        net->arena_need = std::max(net->arena_need, m.arena_bytes);
+    }
+    return upload_weights(net);
 }
 
 int LITE_load_model_with_shared_mem(LiteNetwork network, void* model_mem, size_t size) {

@@ -273,3 +273,55 @@ def test_fp32_matmul_model_matches_oracle(ops, oracle):
         got = net.output(net.output_names()[0], dtype=np.float32).reshape(n, 200)
         close(got, want, RTOL, 3 * ATOL)
     net.close()
+
+
+# channels per CTA of the row-maxima kernel (1, 2 or 8 groups of four), no padding, the largest map
+# that fits shared memory and one that does not
+@pytest.mark.parametrize("shape,window,pad", [
+    ((1, 4, 7, 5), 4, 0), ((3, 12, 6, 31), 5, 2), ((40, 128, 5, 5), 5, 2), ((1, 64, 13, 13), 13, 6),
+    ((1, 8, 56, 56), 5, 2), ((1, 4, 80, 80), 4, 1)], ids=lambda v: str(v))
+def test_max_pooling_by_rows_is_exact(ops, oracle, shape, window, pad):
+    x = cases.rng_for(f"f32_rowmax_{shape}_{window}").standard_normal(shape).astype(np.float32)
+    got = ops.pooling_f32_nhwc(ops.nchw_to_nhwc_f32(dev(x)), "MAX", window, 1, pad)
+    assert (to_nchw(got) == oracle.pooling_f32(x, "MAX", window, 1, pad)).all()
+
+
+# concats whose inputs are written in place: all of them, some of them (an elementwise operator
+# writes dense pixels), a slice that other operators read, one input taken twice
+@pytest.mark.parametrize("batch", [1, 3, 160])
+@pytest.mark.parametrize("form", ["all", "some", "twice"])
+def test_concat_slices_in_place_match_oracle(ops, oracle, batch, form):
+    from megcc_b200 import lite
+    from megcc_b200.compiler import Graph
+    r = cases.rng_for(f"f32_slices_{form}")
+    f = {n: (r.standard_normal(s) / np.sqrt(s[1] * s[2] * s[3])).astype(np.float32) for n, s in (
+        ("a", (32, 16, 3, 3)), ("b", (64, 32, 1, 1)), ("c", (32, 64, 3, 3)), ("e", (40, 128, 1, 1)),
+        ("d", (32, 32, 3, 3)))}
+    g = Graph("slices")
+    x = g.input_f32("data", 16, 12, 10)
+    a = g.conv_f32("a", x, f["a"], None, 1, 1, "RELU")
+    b = g.conv_f32("b", a, f["b"], None, 1, 0, "SILU")
+    d = g.conv_f32("d", a, f["d"], None, 1, 1, "IDENTITY", z=a)
+    third = {"all": lambda: g.pooling("p", d, "MAX", 5, 1, 2),
+             "some": lambda: g.elemwise_f32("p", "RELU", d), "twice": lambda: a}[form]()
+    cat = g.concat("cat", [a, third, b])
+    y = g.conv_f32("e", cat, f["e"], None, 1, 0, "SIGMOID")
+    z = g.conv_f32("c", b, f["c"], None, 1, 1, "RELU", z=d)
+    g.mark_output(y)
+    g.mark_output(z)
+    src = r.standard_normal((batch, 16, 12, 10)).astype(np.float32)
+    conv = lambda v, n, pad, act, **k: oracle.conv_bias_f32(v, f[n], None, 1, pad, act, **k)
+    wa = conv(src, "a", 1, "RELU")
+    wb = conv(wa, "b", 0, "SILU")
+    wd = conv(wa, "d", 1, "IDENTITY", z=wa)
+    w3 = {"all": lambda: oracle.pooling_f32(wd, "MAX", 5, 1, 2),
+          "some": lambda: np.maximum(wd, 0), "twice": lambda: wa}[form]()
+    want = [conv(oracle.concat_f32([wa, w3, wb]), "e", 0, "SIGMOID"), conv(wb, "c", 1, "RELU", z=wd)]
+    net = lite.Network(g.compile([batch]))
+    for _ in range(3):
+        net.set_input("data", src)
+        net.forward()
+        net.wait()
+        for n, w in zip(net.output_names(), want):
+            close(net.output(n, dtype=np.float32).reshape(w.shape), w)
+    net.close()
