@@ -162,6 +162,94 @@ __global__ void __launch_bounds__(256) conv_dw_kernel(
 }
 
 // ------------------------------------------------------------------------------------------
+// one output pixel x 4 channels per thread: small layers
+// ------------------------------------------------------------------------------------------
+// A layer of a batch of one is a single chain of latencies: what counts is how long one thread's
+// work is, and 16 or 32 outputs of a thread are some 600 dependent instructions on a few of the
+// SMs (4.5 to 6.4 us from its input being ready to the next kernel's for MobileNetV1's layers).
+// Here a thread has about 100, the filter (36 adjacent bytes per thread, straight into registers),
+// bias and scales are fetched before the wait for the previous kernel, and there is no shared
+// memory and no barrier. Bytes are loaded 4 at a time, so it is no match for the forms above once
+// the GPU is full.
+__global__ void __launch_bounds__(128) conv_dw3x3_quad_kernel(
+        const DwParams p, const uint32_t* __restrict__ src, const uint32_t* __restrict__ flt,
+        const int32_t* __restrict__ bias, const float* __restrict__ flt_scales,
+        uint32_t* __restrict__ dst) {
+    const ConvArgs& a = p.a;
+    const unsigned c4 = (unsigned)p.c16 * 4;
+    const unsigned idx = blockIdx.x * blockDim.x + threadIdx.x;
+    pdl_release();
+    if (idx >= (unsigned)a.m * c4)
+        return;
+    const unsigned cq = idx % c4;
+    unsigned m = idx / c4;
+    const int ox = (int)(m % a.ow);
+    m /= a.ow;
+    const int oy = (int)(m % a.oh);
+    const int n = (int)(m / a.oh);
+    uint32_t f[9];
+#pragma unroll
+    for (int t = 0; t < 9; ++t)
+        f[t] = __ldg(flt + cq * 9 + t);
+    int4 b = make_int4(0, 0, 0, 0);
+    if (bias)
+        b = __ldg(reinterpret_cast<const int4*>(bias) + cq);
+    float4 s = make_float4(a.s_flt, a.s_flt, a.s_flt, a.s_flt);
+    if (flt_scales)
+        s = __ldg(reinterpret_cast<const float4*>(flt_scales) + cq);
+    const int iy0 = oy * a.sh - a.ph, ix0 = ox * a.sw - a.pw;
+    const uint32_t* base = src + (size_t)((unsigned)n * a.ih) * a.iw * c4 + cq;
+    pdl_wait();  // (everything above is parameters)
+    uint32_t v[9];
+#pragma unroll
+    for (int t = 0; t < 9; ++t) {
+        const int iy = iy0 + t / 3, ix = ix0 + t % 3;
+        v[t] = 0;
+        if ((unsigned)iy < (unsigned)a.ih && (unsigned)ix < (unsigned)a.iw)
+            v[t] = __ldg(base + ((size_t)iy * a.iw + ix) * c4);
+    }
+    uint32_t zw = 0;
+    if (a.z_mode != 0 && a.z)
+        zw = __ldg(reinterpret_cast<const uint32_t*>(a.z) + idx);
+    uint32_t t0[4], t1[4];  // per channel: taps 0..3, 4..7
+    transpose4x4(v[0], v[1], v[2], v[3], t0);
+    transpose4x4(v[4], v[5], v[6], v[7], t1);
+    const int bb[4] = {b.x, b.y, b.z, b.w};
+    const float ss[4] = {s.x, s.y, s.z, s.w};
+    int r[4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        // channel i's nine bytes start at byte 9 i of f
+        const int w = 9 * i / 4, sh = 9 * i % 4 * 8;
+        const uint32_t w0 = sh ? __funnelshift_r(f[w], f[w + 1], sh) : f[w];
+        const uint32_t w1 = sh ? __funnelshift_r(f[w + 1], f[w + 2], sh) : f[w + 1];
+        int acc = __dp4a((int)t0[i], (int)w0, bb[i]);
+        acc = __dp4a((int)t1[i], (int)w1, acc);
+        const int last = (int)(int8_t)(f[w + 2] >> sh), v8 = (int)(int8_t)(v[8] >> (8 * i));
+        acc += last * v8;
+        if (p.fast_ops == 1) {
+            const float x = __int2float_rn(acc);
+            const float y = __fmaf_rn(
+                    x, p.fast_mul, a.act == ACT_RELU ? p.fast_add : copysignf(p.fast_add, x));
+            asm("cvt.rzi.sat.s8.f32 %0, %1;" : "=r"(r[i]) : "f"(y));
+            if (a.act == ACT_RELU)
+                r[i] = max(r[i], 0);
+        } else {
+            r[i] = requant_conv_fast(acc, a.s_src, ss[i], a.s_dst, p.inv_dst, a.act);
+        }
+        if (a.z_mode != 0 && a.z) {
+            const int zi = (int)(int8_t)(zw >> (8 * i));
+            float t = __fadd_rn(__fmul_rn(a.s_dst, __int2float_rn(r[i])),
+                                __fmul_rn(a.z_scale, __int2float_rn(zi)));
+            if (a.z_mode == 2)
+                t = t > 0.f ? t : 0.f;
+            r[i] = fp32_to_int8(__fmul_rn(t, p.z_div));
+        }
+    }
+    dst[idx] = pack4(r[0], r[1], r[2], r[3]);
+}
+
+// ------------------------------------------------------------------------------------------
 // OUT (2 or 4) horizontally adjacent outputs per thread (3x3, stride 1 or 2, no fused residual step)
 // ------------------------------------------------------------------------------------------
 // The kernel above spends 41 instructions per output and is bound by instruction issue.
@@ -323,6 +411,14 @@ int launch_conv_dw(
             p.fast_ops = 0;
     }
     const size_t work = (size_t)a.m * p.c16;
+    // While a thread per 4 outputs still fits the GPU at once (2048 threads on each SM), the
+    // shortest thread wins; beyond that the instructions per output decide.
+    if (tuning().dw_out == 0 && !tuning().dw_one_output && work * 4 <= (size_t)148 * 2048 &&
+        ((uintptr_t)flt & 3) == 0) {
+        launch_pdl(conv_dw3x3_quad_kernel, dim3((unsigned)((work * 4 + 127) / 128)), dim3(128), 0, st,
+                   p, (const uint32_t*)src, (const uint32_t*)flt, bias, flt_scales, (uint32_t*)dst);
+        return check_launch("conv_dw_quad");
+    }
     size_t grid = (work + 255) / 256;
     const size_t cap = (size_t)148 * 8;
     if (grid > cap)
