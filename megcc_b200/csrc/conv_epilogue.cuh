@@ -424,23 +424,50 @@ __device__ __forceinline__ uint32_t epilogue_word(
 // Four consecutive channels (from ch0, a multiple of 4) of one output pixel, every epilogue: the
 // reference's float operations in their order. For the CTAs of a split tile, where a thread
 // finishes a few channels only and code that stays small matters more than operations saved.
-__device__ __forceinline__ void epilogue_quad(
-        const int (&acc)[4], const EpilogueParams& e, int8_t* dst, size_t off, int ch0) {
-    int r[4];
+// What does not depend on the accumulators is fetched beforehand (quad_params, quad_z).
+struct QuadParams {
+    int bias[4];
+    float scale[4];
+};
+__device__ __forceinline__ QuadParams quad_params(const EpilogueParams& e, int ch0) {
+    QuadParams q;
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
         const bool in = ch0 + i < e.oc;
-        const int a = acc[i] + (in && e.bias ? e.bias[ch0 + i] : 0);
+        q.bias[i] = in && e.bias ? __ldg(e.bias + ch0 + i) : 0;
+        q.scale[i] = in && e.flt_scales ? __ldg(e.flt_scales + ch0 + i) : e.s_flt;
+    }
+    return q;
+}
+// the fused step's operand, a byte per channel
+__device__ __forceinline__ uint32_t quad_z(const EpilogueParams& e, size_t off, int ch0) {
+    if (e.z_mode == 0)
+        return 0;
+    if ((e.oc & 3) == 0 && ((uintptr_t)e.z & 3) == 0)
+        return *reinterpret_cast<const uint32_t*>(e.z + off);
+    uint32_t w = 0;
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+        if (ch0 + i < e.oc)
+            w |= (uint32_t)(uint8_t)e.z[off + i] << (8 * i);
+    return w;
+}
+__device__ __forceinline__ void epilogue_quad(
+        const int (&acc)[4], const EpilogueParams& e, const QuadParams& q, uint32_t zw, int8_t* dst,
+        size_t off, int ch0) {
+    int r[4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        const int a = acc[i] + q.bias[i];
         if (e.acc_out) {
-            if (in)
+            if (ch0 + i < e.oc)
                 e.acc_out[off + i] = a;
             continue;
         }
-        const float s = in && e.flt_scales ? e.flt_scales[ch0 + i] : e.s_flt;
-        const float t = __fmul_rn(__fmul_rn(__int2float_rn(a), e.s_src), s);
+        const float t = __fmul_rn(__fmul_rn(__int2float_rn(a), e.s_src), q.scale[i]);
         r[i] = round_clamp_s8(apply_act(e.act, div_rn_by_const(t, e.s_dst, e.inv_dst)));
-        if (e.z_mode != 0 && in) {
-            const int zv = (int)e.z[off + i];
+        if (e.z_mode != 0) {
+            const int zv = (int)(int8_t)(zw >> (8 * i));
             r[i] = e.z_mode == 1 ? fuse_z<1>(r[i], zv, e) : fuse_z<2>(r[i], zv, e);
         }
     }
@@ -454,6 +481,24 @@ __device__ __forceinline__ void epilogue_quad(
             if (ch0 + i < e.oc)
                 dst[off + i] = (int8_t)r[i];
     }
+}
+
+// Brings the first tile's bias, channel scales and residual of a warp (`cols` channels from ch0,
+// a pixel per lane at element `off`) into the L1 while its MMAs run: behind them each load would
+// be a link of the tile's chain, most of what a small layer consists of.
+__device__ __forceinline__ uint32_t ask_for_params(
+        const EpilogueParams& e, int ch0, int cols, bool valid, size_t off) {
+    const int lane = threadIdx.x & 31;
+    uint32_t v = 0;
+    if (lane * 32 < cols && ch0 + lane * 32 < e.oc) {
+        if (e.bias)
+            v = umma::ask_for(e.bias + ch0 + lane * 32);
+        if (e.flt_scales)
+            v ^= umma::ask_for(e.flt_scales + ch0 + lane * 32);
+    }
+    if (e.z_mode != 0 && valid && ch0 < e.oc)
+        v ^= umma::ask_for((const void*)((uintptr_t)(e.z + off) & ~(uintptr_t)3));
+    return v;
 }
 
 // ---- epilogues fixed at compile time ----

@@ -777,68 +777,113 @@ __global__ void __launch_bounds__(f32_threads(BN), 1) conv_f32_umma_kernel(
     }
 
     if (p.splits > 1) {
-        // every CTA of the cluster comes here, whatever became of its waits
+        // Every CTA of the cluster comes here, whatever became of its waits. A thread's items lie
+        // 256 apart, in one channel quad: bias and residual are fetched while the partial tiles
+        // arrive, and the CTA says that it has read the others' before it activates and stores
+        // (an arrival behind the stores waits until they have been performed).
         __syncwarp();
-        cluster_barrier();  // the partial tiles are in place
+        cluster_arrive();
+        constexpr int kQuads = BN / 4, kRowStep = 32 * kF32EpilogueWarps / kQuads;
+        constexpr int kItems = kBM / 2 / kRowStep;  // at most (two CTAs)
         const int et = (int)threadIdx.x - 64;
-        if (et >= 0 && et < 32 * kF32EpilogueWarps && !*abort_flag) {
-            const int rows = kBM / p.splits;
-            const int tile_n = first_tile % p.n_tiles, tile_m = first_tile / p.n_tiles;
-            const uint32_t part = smem_u32(tiles);
-            for (int u = et; u < rows * (BN / 4); u += 32 * kF32EpilogueWarps) {
-                const int r = rank * rows + u / (BN / 4), c = (u % (BN / 4)) * 4;
-                const int m = tile_m * kBM + r, ch = tile_n * BN + c;
-                if (m >= p.m_total || ch >= p.oc)
-                    continue;
+        const bool worker = et >= 0 && et < 32 * kF32EpilogueWarps;
+        const int rows = kBM / p.splits;
+        const int tile_n = first_tile % p.n_tiles, tile_m = first_tile / p.n_tiles;
+        const int c = (et & (kQuads - 1)) * 4, ch = tile_n * BN + c;
+        const int r0 = rank * rows + et / kQuads;
+        const int m0 = tile_m * kBM + r0;
+        const int left = min(4, p.oc - ch);
+        const bool vec = left == 4 && ((p.ep.dst_pitch | (p.ep.z ? p.ep.z_pitch : 0)) & 3) == 0 &&
+                         (((uintptr_t)p.ep.dst | (uintptr_t)p.ep.z) & 15) == 0;
+        float bias[4] = {0.f, 0.f, 0.f, 0.f};
+        float4 v[kItems], zv[kItems];
+        int items = 0;
+        if (worker && left > 0) {
+#pragma unroll
+            for (int j = 0; j < 4; ++j)
+                if (j < left && p.ep.bias)
+                    bias[j] = __ldg(p.ep.bias + ch + j);
+#pragma unroll
+            for (int k = 0; k < kItems; ++k) {
+                zv[k] = make_float4(0.f, 0.f, 0.f, 0.f);
+                if (et / kQuads + k * kRowStep < rows && m0 + k * kRowStep < p.m_total) {
+                    items = k + 1;
+                    if (p.ep.z) {
+                        const float* zin = p.ep.z + (size_t)(m0 + k * kRowStep) * p.ep.z_pitch + ch;
+                        if (vec) {
+                            zv[k] = *reinterpret_cast<const float4*>(zin);
+                        } else {
+                            zv[k].x = zin[0];
+                            zv[k].y = left > 1 ? zin[1] : 0.f;
+                            zv[k].z = left > 2 ? zin[2] : 0.f;
+                            zv[k].w = left > 3 ? zin[3] : 0.f;
+                        }
+                    }
+                }
+            }
+        }
+        cluster_wait();  // the partial tiles are in place
+        if (*abort_flag)
+            items = 0;
+#pragma unroll
+        for (int k = 0; k < kItems; ++k) {
+            if (k < items) {
+                const uint32_t at = smem_u32(tiles) +
+                                    (uint32_t)(((r0 + k * kRowStep) * C::kPartPitch + c) * 4);
                 // all parts' loads are in flight together (a remote load takes some 250 clocks)
-                const uint32_t at = part + (uint32_t)((r * C::kPartPitch + c) * 4);
                 uint4 x[8];
 #pragma unroll
                 for (int i = 0; i < 8; ++i)
                     if (i < p.splits)
                         x[i] = ld_cluster_v4(at, i);
-                float v[4] = {__uint_as_float(x[0].x), __uint_as_float(x[0].y),
-                              __uint_as_float(x[0].z), __uint_as_float(x[0].w)};
+                v[k] = make_float4(__uint_as_float(x[0].x), __uint_as_float(x[0].y),
+                                   __uint_as_float(x[0].z), __uint_as_float(x[0].w));
 #pragma unroll
                 for (int i = 1; i < 8; ++i) {
                     if (i < p.splits) {
-                        v[0] = __fadd_rn(v[0], __uint_as_float(x[i].x));
-                        v[1] = __fadd_rn(v[1], __uint_as_float(x[i].y));
-                        v[2] = __fadd_rn(v[2], __uint_as_float(x[i].z));
-                        v[3] = __fadd_rn(v[3], __uint_as_float(x[i].w));
+                        v[k].x = __fadd_rn(v[k].x, __uint_as_float(x[i].x));
+                        v[k].y = __fadd_rn(v[k].y, __uint_as_float(x[i].y));
+                        v[k].z = __fadd_rn(v[k].z, __uint_as_float(x[i].z));
+                        v[k].w = __fadd_rn(v[k].w, __uint_as_float(x[i].w));
                     }
-                }
-                float* out = p.ep.dst + (size_t)m * p.ep.dst_pitch + ch;
-                const float* zin = p.ep.z ? p.ep.z + (size_t)m * p.ep.z_pitch + ch : nullptr;
-                const int left = min(4, p.oc - ch);
-#pragma unroll
-                for (int j = 0; j < 4; ++j)
-                    if (j < left) {
-                        v[j] += p.ep.bias ? p.ep.bias[ch + j] : 0.f;
-                    }
-                with_act(p.ep.act, [&](auto a) {
-#pragma unroll
-                    for (int j = 0; j < 4; ++j)
-                        v[j] = act_f32<decltype(a)::value>(v[j]);
-                });
-                if (zin) {
-#pragma unroll
-                    for (int j = 0; j < 4; ++j)
-                        if (j < left)
-                            v[j] += zin[j];
-                }
-                if (left == 4 && ((uintptr_t)out & 15) == 0) {
-                    *reinterpret_cast<float4*>(out) = make_float4(v[0], v[1], v[2], v[3]);
-                } else {
-#pragma unroll
-                    for (int j = 0; j < 4; ++j)
-                        if (j < left)
-                            out[j] = v[j];
                 }
             }
         }
         __syncwarp();
-        cluster_barrier();  // nobody leaves while its partial tile may still be read
+        cluster_arrive();  // (a release: the loads above are done)
+        with_act(p.ep.act, [&](auto a) {
+#pragma unroll
+            for (int k = 0; k < kItems; ++k) {
+                if (k < items) {
+                    constexpr int kAct = decltype(a)::value;
+                    float4 r;
+                    r.x = act_f32<kAct>(v[k].x + bias[0]);
+                    r.y = act_f32<kAct>(v[k].y + bias[1]);
+                    r.z = act_f32<kAct>(v[k].z + bias[2]);
+                    r.w = act_f32<kAct>(v[k].w + bias[3]);
+                    if (p.ep.z) {
+                        r.x += zv[k].x;
+                        r.y += zv[k].y;
+                        r.z += zv[k].z;
+                        r.w += zv[k].w;
+                    }
+                    float* out = p.ep.dst + (size_t)(m0 + k * kRowStep) * p.ep.dst_pitch + ch;
+                    if (vec) {
+                        *reinterpret_cast<float4*>(out) = r;
+                    } else {
+                        out[0] = r.x;
+                        if (left > 1)
+                            out[1] = r.y;
+                        if (left > 2)
+                            out[2] = r.z;
+                        if (left > 3)
+                            out[3] = r.w;
+                    }
+                }
+            }
+        });
+        __syncwarp();
+        cluster_wait();  // nobody leaves while its partial tile may still be read
     }
 
     // ---------------- teardown ----------------

@@ -422,6 +422,16 @@ __global__ void __launch_bounds__(64 + 32 * EW, EW == 16 ? 1 : 2) conv_patch_ker
         }
         const bool unbounded = FORM >= FORM_CHAIN_RELU && chain_unbounded(p.ep);
         PatchWalker at(m_first, p);
+        uint32_t asked = 0;
+        if (POOL == 0 && m_first < p.m_tiles) {
+            // the first tile's parameters and residual come while its MMAs run
+            const int ch0 = n0 + ((warp - 2) >> 2) * (BN / (kEpilogueWarps / 4));
+            const int oy = at.ty * kTH + py, ox = at.tx * kTW + px;
+            asked = ask_for_params(
+                    p.ep, (ROWS != 0 && p.dw_pairs) ? 0 : ch0, BN / (kEpilogueWarps / 4),
+                    oy < p.oh && ox < p.ow && !(ROWS != 0 && p.dw_pairs),
+                    (size_t)(((uint32_t)at.img * p.oh + oy) * p.ow + ox) * p.oc + ch0);
+        }
         for (int mt = m_first; mt < p.m_tiles && ok; mt += m_step, ++local, at.next(p)) {
             const int buf = local & 1;
             const uint32_t acc_phase = (uint32_t)(local >> 1) & 1u;
@@ -448,6 +458,7 @@ __global__ void __launch_bounds__(64 + 32 * EW, EW == 16 ? 1 : 2) conv_patch_ker
             }
             if (!ok)
                 break;
+            keep(asked);
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
             if constexpr (POOL != 0) {
                 // (1) this thread's pixel: 32 accumulators TMEM -> registers -> shared memory

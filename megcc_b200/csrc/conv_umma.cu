@@ -359,6 +359,13 @@ __global__ void __launch_bounds__(Shape<BN>::kThreads, Shape<BN>::kMinCtas) conv
         uint32_t ep_phase = 0;  // parity of the epilogue's own rendezvous (split-K)
         pdl_wait();  // before the first read of z and the first store
         const bool unbounded = FORM >= FORM_CHAIN_RELU && chain_unbounded(p.ep);
+        uint32_t asked = 0;
+        if (!SPLITK && p.csplit <= 1 && first_item < total_tiles) {
+            // the first tile's parameters and residual come while its MMAs run
+            const int n0 = first_item % p.n_tiles * BN, m = first_item / p.n_tiles * kBM + row;
+            const int ch0 = n0 + ((warp - 2) >> 2) * (BN / (kEpilogueWarps / 4));
+            asked = ask_for_params(p.ep, ch0, BN / (kEpilogueWarps / 4), m < p.m_total, (size_t)m * p.oc + ch0);
+        }
         for (int item = first_item; item < total_tiles && ok; item += item_step, ++local) {
             const WorkItem w = decode_item<SPLITK>(p, item, rank);
             const int tile = w.tile;
@@ -374,6 +381,7 @@ __global__ void __launch_bounds__(Shape<BN>::kThreads, Shape<BN>::kMinCtas) conv
             ok = __all_sync(0xffffffffu, ok);
             if (!ok)
                 break;
+            keep(asked);
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
             const uint32_t taddr = tmem_base + ((uint32_t)(q * 32) << 16) + (uint32_t)(buf * BN);
             const int half = (warp - 2) >> 2;
@@ -501,37 +509,68 @@ __global__ void __launch_bounds__(Shape<BN>::kThreads, Shape<BN>::kMinCtas) conv
     }
 
     if (!SPLITK && p.csplit > 1) {
-        // every CTA of the cluster comes here, whatever became of its waits; each finishes an
-        // equal share of the rows
+        // Every CTA of the cluster comes here, whatever became of its waits; each finishes an
+        // equal share of the rows. A thread's items lie 256 apart, in one channel quad: bias,
+        // scales and residual are fetched while the shares arrive, and the CTA says that it
+        // has read the others' shares before it stores (an arrival behind the stores waits for
+        // them to be performed: 3 to 4.5 us from the last MMA to the end with everything
+        // in line, on tiles of a batch of one).
         __syncwarp();
-        cluster_barrier();  // the shares are in place
+        cluster_arrive();
+        constexpr int kQuads = BN / 4, kRowStep = 32 * kEpilogueWarps / kQuads;
+        constexpr int kItems = kBM / 2 / kRowStep;  // at most (two CTAs)
         const int et = (int)threadIdx.x - 64;
-        if (et >= 0 && !*abort_flag) {
-            const int rows = kBM / p.csplit;
-            const int tile_n = first_item % p.n_tiles, tile_m = first_item / p.n_tiles;
-            for (int u = et; u < rows * (BN / 4); u += 32 * kEpilogueWarps) {
-                const int r = rank * rows + u / (BN / 4), c = (u % (BN / 4)) * 4;
-                const int m = tile_m * kBM + r, ch = tile_n * BN + c;
-                if (m >= p.m_total || ch >= p.oc)
-                    continue;
-                const uint32_t at = smem_u32(smem) + (uint32_t)((r * kPartPitch + c) * 4);
+        const int rows = kBM / p.csplit;
+        const int tile_n = first_item % p.n_tiles, tile_m = first_item / p.n_tiles;
+        const int c = (et & (kQuads - 1)) * 4, ch = tile_n * BN + c;
+        const int r0 = rank * rows + et / kQuads;
+        const int m0 = tile_m * kBM + r0;
+        QuadParams qp;
+        uint32_t zw[kItems];
+        int v[kItems][4];
+        int items = 0;
+        if (et >= 0 && ch < p.oc) {
+            qp = quad_params(p.ep, ch);
+#pragma unroll
+            for (int k = 0; k < kItems; ++k) {
+                zw[k] = 0;
+                if (et / kQuads + k * kRowStep < rows && m0 + k * kRowStep < p.m_total) {
+                    items = k + 1;
+                    zw[k] = quad_z(p.ep, (size_t)(m0 + k * kRowStep) * p.oc + ch, ch);
+                }
+            }
+        }
+        cluster_wait();  // the shares are in place
+        if (*abort_flag)
+            items = 0;
+#pragma unroll
+        for (int k = 0; k < kItems; ++k) {
+            if (k < items) {
+                const uint32_t at =
+                        smem_u32(smem) + (uint32_t)(((r0 + k * kRowStep) * kPartPitch + c) * 4);
                 uint4 x[8];
 #pragma unroll
                 for (int i = 0; i < 8; ++i)  // all shares' loads in flight together
                     x[i] = i < p.csplit ? ld_cluster_v4(at, i) : make_uint4(0, 0, 0, 0);
-                int v[4] = {0, 0, 0, 0};
+                v[k][0] = v[k][1] = v[k][2] = v[k][3] = 0;
 #pragma unroll
                 for (int i = 0; i < 8; ++i) {
-                    v[0] += (int)x[i].x;
-                    v[1] += (int)x[i].y;
-                    v[2] += (int)x[i].z;
-                    v[3] += (int)x[i].w;
+                    v[k][0] += (int)x[i].x;
+                    v[k][1] += (int)x[i].y;
+                    v[k][2] += (int)x[i].z;
+                    v[k][3] += (int)x[i].w;
                 }
-                epilogue_quad(v, p.ep, p.dst, (size_t)m * p.oc + ch, ch);
             }
         }
         __syncwarp();
-        cluster_barrier();  // nobody leaves while its share may still be read
+        cluster_arrive();  // (a release: the loads above are done)
+#pragma unroll
+        for (int k = 0; k < kItems; ++k)
+            if (k < items)
+                epilogue_quad(v[k], p.ep, qp, zw[k], p.dst, (size_t)(m0 + k * kRowStep) * p.oc + ch,
+                              ch);
+        __syncwarp();
+        cluster_wait();  // nobody leaves while its share may still be read
     }
 
     // ---------------- teardown ----------------

@@ -164,6 +164,23 @@ __device__ __forceinline__ void cluster_barrier() {
     asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
     asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
+// its two halves, for work in between that needs nobody
+__device__ __forceinline__ void cluster_arrive() {
+    asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+}
+__device__ __forceinline__ void cluster_wait() {
+    asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+// Asks for the line of `p` ahead of its use: the value is thrown away, its line stays in the L1.
+// keep() takes it (the load is not dropped, and is not waited for before that).
+__device__ __forceinline__ uint32_t ask_for(const void* p) {
+    uint32_t v;
+    asm volatile("ld.global.b32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
+    return v;
+}
+__device__ __forceinline__ void keep(uint32_t v) {
+    asm volatile("" ::"r"(v) : "memory");
+}
 // 16 bytes at the shared-memory address `local` of CTA `rank`
 __device__ __forceinline__ uint4 ld_cluster_v4(uint32_t local, int rank) {
     uint32_t addr;
