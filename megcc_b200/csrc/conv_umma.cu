@@ -664,6 +664,10 @@ int umma_clusters(int size) {
 // over the cluster 1600 and 350 for every four channels that a thread then finishes. A split
 // has to promise a sixth less: 512 -> 512 3x3 over 37 images of 7 x 7 took 30 us as 60 tiles
 // split in two and 26 us unsplit, one image 23 us unsplit and 8 us as 8 tiles split in eight.
+// Clusters on more than half of the SMs cost another 4500: the next kernel's cannot be placed
+// beside them and start late (128 -> 128 3x3 over 28 x 28: one image 4.8 us as 56 CTAs against
+// 5.1 unsplit, two images 6.1 as 104 CTAs against 5.3). Channels that are no multiple of
+// 32 take the general epilogue, 2000 more for a whole tile and nothing for a split one.
 void choose_split(int m_tiles, int oc, int k_iters, bool wide128, int* bn, int* csplit) {
     long long best = -1;
     const int bn_first = *bn;
@@ -684,8 +688,10 @@ void choose_split(int m_tiles, int oc, int k_iters, bool wide128, int* bn, int* 
             const long long waves = (tiles * s + sm_count() - 1) / sm_count();
             const long long steps = (long long)((k_iters + s - 1) / s) * step;
             const int quads = b / (8 * s) > 1 ? b / (8 * s) : 1;
-            const long long clocks = s > 1 ? (steps + 1600 + 350 * quads) * 6 / 5
-                                           : waves * (steps + (b == 128 ? 1800 : 1200));
+            const int crowded = 2 * tiles * s > sm_count() ? 4500 : 0;
+            const int end = (b == 128 ? 1800 : 1200) + (oc % 32 ? 2000 : 0);
+            const long long clocks = s > 1 ? (steps + 1600 + 350 * quads + crowded) * 6 / 5
+                                           : waves * (steps + end);
             // (a tie goes to the width the caller had chosen)
             if (best < 0 || clocks < best || (clocks == best && b == bn_first && s == 1)) {
                 best = clocks;
