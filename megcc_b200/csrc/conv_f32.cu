@@ -1041,8 +1041,10 @@ int f32_cluster_capacity(int bn, int rowb, int size) {
 // Tile width and K split for a problem of `m_tiles` x `oc` with `k_iters` steps of `rowb` bytes:
 // the pair with the shortest estimated time of its busiest SM. Clocks per step and tile: 12
 // MMAs of 64 clocks for 128 columns, half that for 64, and for 32 what the handshakes of a step
-// cost. A split adds the
-// exchange of the partial tiles; it is taken only where the clusters all run at once.
+// cost. A tile that is its CTA's only one has nothing to hide its end behind: wide tiles cost
+// more there (128 -> 128 1x1 over 52 x 52: 4.6 us with 32 columns, 5.3 with 64, 7.8 with 128). A
+// split adds the exchange of the partial tiles; it is taken only where the clusters all run at
+// once. (512 -> 128 1x1 over 26 x 26: 5.8 us as 24 tiles split in four, 6.8 as 12 in eight.)
 void choose_f32_tile(int m_tiles, int oc, int k_iters, int rowb, int* bn, int* splits) {
     const int sms = sm_count();
     long long best = -1;
@@ -1056,8 +1058,10 @@ void choose_f32_tile(int m_tiles, int oc, int k_iters, int rowb, int* bn, int* s
             if (s > 1 && (k_iters / s < 2 || tiles > sms / s || tiles > f32_cluster_capacity(b, rowb, s)))
                 break;
             const long long waves = s > 1 ? 1 : (tiles + sms - 1) / sms;
+            const int alone = waves > 1 ? 0 : b == 128 ? 3000 : b == 64 ? 900 : 0;
             const long long clocks =
-                    waves * ((long long)((k_iters + s - 1) / s) * step + tile_end) + (s > 1 ? 2500 : 0);
+                    waves * ((long long)((k_iters + s - 1) / s) * step + tile_end + alone) +
+                    (s > 1 ? 2500 : 0);
             if (best < 0 || clocks < best) {
                 best = clocks;
                 *bn = b;
