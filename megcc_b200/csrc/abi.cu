@@ -604,9 +604,7 @@ int mb200_conv_bias_qs8_nchw(
     int8_t* ws_dst = ws_src + align_up((size_t)a.n * a.ih * a.iw * a.ic, 256);
     int8_t* ws_flt = ws_dst + align_up((size_t)a.m * a.oc, 256);
     // NCHW -> NHWC is a [C][HW] -> [HW][C] transpose per image
-    if ((rc = launch_transpose_s8(src, ws_src, a.n, a.ic, a.ih * a.iw, st)))
-        return rc;
-    if ((rc = launch_pack_filter(a, flt_oihw, ws_flt, st)))
+    if ((rc = launch_transpose_pack_s8(src, ws_src, a.n, a.ic, a.ih * a.iw, a, flt_oihw, ws_flt, st)))
         return rc;
     if ((rc = mb200_conv_bias_qs8_nhwc(p, ws_src, 0, ws_flt, bias, flt_scales, ws_dst, algo, st)))
         return rc;

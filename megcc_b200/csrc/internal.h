@@ -163,6 +163,10 @@ int launch_typecvt_qs32_qs8(
         cudaStream_t st);
 // plain copy by a kernel (src may be page-locked host memory)
 int launch_copy_bytes(const void* src, void* dst, size_t bytes, cudaStream_t st);
+// launch_transpose_s8 and launch_pack_filter, as one kernel where the shape allows
+int launch_transpose_pack_s8(
+        const int8_t* src, int8_t* dst, int batch, int rows, int cols, const ConvArgs& a,
+        const int8_t* flt, int8_t* packed, cudaStream_t st);
 int launch_transpose_s8(
         const int8_t* src, int8_t* dst, int batch, int rows, int cols, cudaStream_t st);
 

@@ -9,21 +9,25 @@ namespace mb200 {
 // ------------------------------------------------------------------------------------------
 // filter packing: OIHW (dense) or [G][OCpg][ICpg][KH][KW] (group) -> [OC][KH][KW][ICpg]
 // ------------------------------------------------------------------------------------------
+// byte i of the packed filter [o][fy][fx][c]
+__device__ __forceinline__ int8_t pack_filter_byte(
+        const int8_t* src, size_t i, int icpg, int kh, int kw) {
+    const int c = (int)(i % icpg);
+    size_t t = i / icpg;
+    const int fx = (int)(t % kw);
+    t /= kw;
+    const int fy = (int)(t % kh);
+    const int o = (int)(t / kh);
+    return __ldg(src + (((size_t)o * icpg + c) * kh + fy) * kw + fx);
+}
+
 __global__ void pack_filter_kernel(
         const int8_t* __restrict__ src, int8_t* __restrict__ dst, int oc, int icpg, int kh,
         int kw) {
     const size_t total = (size_t)oc * icpg * kh * kw;
     for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < total;
-         i += (size_t)gridDim.x * blockDim.x) {
-        // i indexes dst: [o][fy][fx][c]
-        int c = (int)(i % icpg);
-        size_t t = i / icpg;
-        int fx = (int)(t % kw);
-        t /= kw;
-        int fy = (int)(t % kh);
-        int o = (int)(t / kh);
-        dst[i] = src[(((size_t)o * icpg + c) * kh + fy) * kw + fx];
-    }
+         i += (size_t)gridDim.x * blockDim.x)
+        dst[i] = pack_filter_byte(src, i, icpg, kh, kw);
 }
 
 // ------------------------------------------------------------------------------------------
@@ -546,6 +550,57 @@ __global__ void __launch_bounds__(256) transpose_s8_kernel(
     }
 }
 
+// The same where rows and columns are multiples of 4: tiles of 64 x 64, a thread turns a 4 x 4 block
+// in registers and every access of memory is a word, 64 contiguous bytes per tile row (the byte
+// form above moves 32 bytes per warp instruction). Blocks behind the tiles, if any, pack a
+// ConvBias filter: the two steps in front of an NCHW ConvBias as one launch, a sixth of its host
+// time at small sizes. No early release of the next kernel: it may fetch the packed filter
+// before its own wait.
+__global__ void __launch_bounds__(256) transpose4_s8_kernel(
+        const int8_t* __restrict__ src, int8_t* __restrict__ dst, int rows, int cols, int tiles_c,
+        int tiles_r, int tiles, const int8_t* __restrict__ flt, int8_t* __restrict__ packed, int oc,
+        int icpg, int kh, int kw) {
+    __shared__ uint32_t turned[64][17];  // [column][four rows]
+    if (!flt)
+        pdl_release();
+    pdl_wait();
+    const int t = threadIdx.x;
+    if ((int)blockIdx.x >= tiles) {
+        const size_t total = (size_t)oc * icpg * kh * kw;
+        for (size_t i = (blockIdx.x - tiles) * (size_t)blockDim.x + t; i < total;
+             i += (size_t)(gridDim.x - tiles) * blockDim.x)
+            packed[i] = pack_filter_byte(flt, i, icpg, kh, kw);
+        return;
+    }
+    const int tc = (int)blockIdx.x % tiles_c, tr = (int)blockIdx.x / tiles_c % tiles_r;
+    const size_t base = (size_t)((int)blockIdx.x / tiles_c / tiles_r) * rows * cols;
+    const int c0 = tc * 64, r0 = tr * 64;
+    {
+        const int j = t & 15, g = t >> 4;  // column word, row group
+        const int c = c0 + 4 * j, r = r0 + 4 * g;
+        if (c < cols && r < rows) {
+            uint32_t v[4];
+#pragma unroll
+            for (int i = 0; i < 4; ++i)
+                v[i] = __ldg(reinterpret_cast<const uint32_t*>(src + base + (size_t)(r + i) * cols + c));
+            const uint32_t ab_lo = __byte_perm(v[0], v[1], 0x5140), cd_lo = __byte_perm(v[2], v[3], 0x5140);
+            const uint32_t ab_hi = __byte_perm(v[0], v[1], 0x7362), cd_hi = __byte_perm(v[2], v[3], 0x7362);
+            turned[4 * j][g] = __byte_perm(ab_lo, cd_lo, 0x5410);
+            turned[4 * j + 1][g] = __byte_perm(ab_lo, cd_lo, 0x7632);
+            turned[4 * j + 2][g] = __byte_perm(ab_hi, cd_hi, 0x5410);
+            turned[4 * j + 3][g] = __byte_perm(ab_hi, cd_hi, 0x7632);
+        }
+    }
+    __syncthreads();
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        const int c = c0 + (t >> 4) + 16 * i, r = r0 + 4 * (t & 15);
+        if (c < cols && r < rows)
+            *reinterpret_cast<uint32_t*>(dst + base + (size_t)c * rows + r) =
+                    turned[(t >> 4) + 16 * i][t & 15];
+    }
+}
+
 // ------------------------------------------------------------------------------------------
 // host launchers
 // ------------------------------------------------------------------------------------------
@@ -684,12 +739,41 @@ int launch_copy_bytes(const void* src, void* dst, size_t bytes, cudaStream_t st)
     return check_launch("copy_bytes");
 }
 
+// the word form: every row of source and destination starts on a word
+static bool transpose_by_words(
+        const int8_t* src, const int8_t* dst, int batch, int rows, int cols) {
+    const long long tiles = (long long)((cols + 63) / 64) * ((rows + 63) / 64) * batch;
+    return rows % 4 == 0 && cols % 4 == 0 && (((uintptr_t)src | (uintptr_t)dst) & 3) == 0 &&
+           tiles < (1 << 30);
+}
+
+int launch_transpose_pack_s8(
+        const int8_t* src, int8_t* dst, int batch, int rows, int cols, const ConvArgs& a,
+        const int8_t* flt, int8_t* packed, cudaStream_t st) {
+    if (batch <= 0 || rows <= 0 || cols <= 0 || !transpose_by_words(src, dst, batch, rows, cols)) {
+        const int rc = launch_transpose_s8(src, dst, batch, rows, cols, st);
+        return rc ? rc : launch_pack_filter(a, flt, packed, st);
+    }
+    const int tc = (cols + 63) / 64, tr = (rows + 63) / 64, tiles = tc * tr * batch;
+    const int icpg = a.ic / a.groups;
+    const int packers = grid_for((size_t)a.oc * icpg * a.kh * a.kw, 256);
+    launch_pdl(transpose4_s8_kernel, dim3(tiles + packers), dim3(256), 0, st, src, dst, rows, cols, tc,
+               tr, tiles, flt, packed, a.oc, icpg, a.kh, a.kw);
+    return check_launch("transpose_pack_s8");
+}
+
 int launch_transpose_s8(
         const int8_t* src, int8_t* dst, int batch, int rows, int cols, cudaStream_t st) {
     if (batch <= 0 || rows <= 0 || cols <= 0)
         return 0;
     if (batch > 65535)
         return set_error(4, "transpose: batch %d exceeds the grid z limit", batch);
+    if (transpose_by_words(src, dst, batch, rows, cols)) {
+        const int tc = (cols + 63) / 64, tr = (rows + 63) / 64, tiles = tc * tr * batch;
+        launch_pdl(transpose4_s8_kernel, dim3(tiles), dim3(256), 0, st, src, dst, rows, cols, tc, tr,
+                   tiles, (const int8_t*)nullptr, (int8_t*)nullptr, 0, 1, 1, 1);
+        return check_launch("transpose4_s8");
+    }
     dim3 grid((cols + 31) / 32, (rows + 31) / 32, batch), block(32, 8);
     launch_pdl(transpose_s8_kernel, grid, block, 0, st, src, dst, rows, cols);
     return check_launch("transpose_s8");
