@@ -37,7 +37,16 @@ int check_launch(const char* what) {
 // stream reads its word without a transfer. A device's words come from one small
 // allocation made at first use; a stream first seen while it is capturing (no set-up may
 // happen then) and streams beyond the pool's capacity share word 0.
+static thread_local int* borrowed_status_word = nullptr;
+int* borrow_status_word(int* word) {
+    int* before = borrowed_status_word;
+    borrowed_status_word = word;
+    return before;
+}
+
 int* device_status_word(cudaStream_t st) {
+    if (borrowed_status_word)
+        return borrowed_status_word;
     constexpr int kWords = 4096;
     struct Pool {
         int* base = nullptr;

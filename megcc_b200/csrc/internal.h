@@ -73,6 +73,8 @@ int check_launch(const char* what);
 // the int that kernels launched on `st` set when a bounded wait runs out (one per device
 // and stream, see abi.cu)
 int* device_status_word(cudaStream_t st);
+// this thread's launches use `word` whatever their stream, until given null; returns the word before
+int* borrow_status_word(int* word);
 
 int launch_pack_filter(const ConvArgs& a, const int8_t* src, int8_t* dst, cudaStream_t st);
 int launch_filter_nchw44_to_oihw(

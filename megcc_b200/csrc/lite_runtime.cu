@@ -209,10 +209,44 @@ struct Network {
     // measured 40 GB/s over PCIe gen5 x16, four concurrent pieces 54 GB/s.
     static constexpr int kCopyStreams = 3;
     cudaStream_t copy_stream[kCopyStreams] = {nullptr, nullptr, nullptr};
-    // lanes beside `stream` that branches of a small model are captured on
-    static constexpr int kLanes = 5;
-    cudaStream_t lane_stream[kLanes] = {nullptr, nullptr, nullptr, nullptr, nullptr};
+    bool uses_lanes = false;  // (see CaptureLanes)
     cudaEvent_t copy_fork = nullptr, copy_join[kCopyStreams] = {nullptr, nullptr, nullptr};
+};
+
+// The streams beside a network's own that branches of a small model are captured on. Nothing runs
+// on them (a graph is launched on the network's stream), so the networks of a device share one
+// set, the mutex held for a capture; it is created with the first capture that wants it (0.1 ms
+// per stream, which every network would pay) and given back with the last network that used it.
+struct CaptureLanes {
+    static constexpr int kLanes = 5;
+    std::mutex mu;
+    int users = 0;
+    cudaStream_t stream[kLanes] = {nullptr, nullptr, nullptr, nullptr, nullptr};
+
+    static CaptureLanes* of(int device) {
+        static CaptureLanes lanes[64];
+        return device >= 0 && device < 64 ? &lanes[device] : nullptr;
+    }
+    // with mu held
+    bool ready(Network* net) {
+        for (auto& s : stream)
+            if (!s && cudaStreamCreateWithFlags(&s, cudaStreamNonBlocking) != cudaSuccess) {
+                s = nullptr;
+                return false;
+            }
+        users += !net->uses_lanes;
+        net->uses_lanes = true;
+        return true;
+    }
+    void leave(Network* net) {
+        std::lock_guard<std::mutex> lock(mu);
+        if (!net->uses_lanes || --users)
+            return;
+        for (auto& s : stream) {
+            cudaStreamDestroy(s);
+            s = nullptr;
+        }
+    }
 };
 
 // Networks on one device run their instruction sequences one after the other, in the order of
@@ -1731,10 +1765,15 @@ int issue_instructions(Network* net, DevModel& m, bool timed) {
 // The instructions as branches of the graph under capture: each goes to the lane whose last
 // instruction it depends on, or to one whose work it follows anyway, or to a free one.
 int issue_side_by_side(Network* net, DevModel& m) {
-    constexpr int kLanes = Network::kLanes + 1;
+    constexpr int kLanes = CaptureLanes::kLanes + 1;
     cudaStream_t lanes[kLanes] = {net->stream};
     for (int l = 1; l < kLanes; ++l)
-        lanes[l] = net->lane_stream[l - 1];
+        lanes[l] = CaptureLanes::of(net->device_id)->stream[l - 1];
+    // every branch reports to the network's own status word
+    struct Borrow {
+        int* before;
+        ~Borrow() { mb200::borrow_status_word(before); }
+    } borrow{mb200::borrow_status_word(mb200::device_status_word(net->stream))};
     const int n = (int)m.instrs.size();
     std::vector<int> lane_of(n, 0);
     int tail[kLanes];               // last instruction of each lane, -1: none
@@ -1814,14 +1853,9 @@ int issue_side_by_side(Network* net, DevModel& m) {
 }
 
 // What capturing side by side needs beforehand (nothing may be set up during a capture).
-bool ready_side_by_side(Network* net, DevModel& m) {
-    for (int l = 0; l < Network::kLanes; ++l) {
-        if (!net->lane_stream[l] &&
-            cudaStreamCreateWithFlags(&net->lane_stream[l], cudaStreamNonBlocking) != cudaSuccess)
-            return false;
-        if (!mb200::device_status_word(net->lane_stream[l]))
-            return false;
-    }
+bool ready_side_by_side(Network* net, DevModel& m, CaptureLanes* lanes) {
+    if (!lanes->ready(net))
+        return false;
     while (m.marks.size() < m.instrs.size() + 1) {
         cudaEvent_t e;
         if (cudaEventCreateWithFlags(&e, cudaEventDisableTiming) != cudaSuccess)
@@ -1919,10 +1953,16 @@ int forward(Network* net) {
                     m.graphs.pop_back();
                 }
                 cudaGraphExec_t exec = nullptr;
-                if (m.side_by_side &&
-                    (!ready_side_by_side(net, m) || capture(net, m, true, &exec))) {
-                    cudaGetLastError();  // then one instruction after the other
-                    m.side_by_side = false;
+                if (m.side_by_side) {
+                    CaptureLanes* lanes = CaptureLanes::of(net->device_id);
+                    std::unique_lock<std::mutex> lock;
+                    if (lanes)
+                        lock = std::unique_lock<std::mutex>(lanes->mu);
+                    if (!lanes || !ready_side_by_side(net, m, lanes) ||
+                        capture(net, m, true, &exec)) {
+                        cudaGetLastError();  // then one instruction after the other
+                        m.side_by_side = false;
+                    }
                 }
                 if (!exec && (rc = capture(net, m, false, &exec)))
                     return rc;
@@ -1956,10 +1996,7 @@ int wait(Network* net) {
     net->pending = false;
     cudaSetDevice(net->device_id);
     int status = 0;
-    int rc = mb200_device_status(net->stream, &status);  // synchronises the stream
-    for (int l = 0; l < Network::kLanes && !rc && !status; ++l)
-        if (net->lane_stream[l])  // (captured branches record under their lane's stream)
-            rc = mb200_device_status(net->lane_stream[l], &status);
+    const int rc = mb200_device_status(net->stream, &status);  // synchronises the stream
     if (rc)
         return fail(rc, "%s", mb200_last_error());
     if (status)
@@ -2376,9 +2413,8 @@ int LITE_destroy_network(LiteNetwork network) {
     }
     if (net->copy_fork)
         cudaEventDestroy(net->copy_fork);
-    for (int l = 0; l < Network::kLanes; ++l)
-        if (net->lane_stream[l])
-            cudaStreamDestroy(net->lane_stream[l]);
+    if (net->uses_lanes)
+        CaptureLanes::of(net->device_id)->leave(net);
     for (auto& m : net->models)
         for (cudaEvent_t e : m.marks)
             cudaEventDestroy(e);
