@@ -827,3 +827,70 @@ def test_bad_arguments_return_status_not_trap(ops):
                                torch.zeros(216, dtype=torch.int8, device="cuda"), None,
                                algo="umma")
     assert e.value.status == 6
+
+
+def check_small_conv(ops, oracle, n, ic, oc, h, w, k, stride, pad, groups, form, algo="auto"):
+    """One ConvBias as bytes against the oracle: `fast` per-tensor scales, `channel` scales, or a
+    `residual` step; the input lies in a registered range, as a network's arena does."""
+    from megcc_b200._lib import check, lib
+    r = cases.rng_for(f"small_{n}_{ic}_{oc}_{h}_{w}_{k}_{stride}_{groups}_{form}")
+    src = r.integers(-128, 128, (n, ic, h, w)).astype(np.int8)
+    flt = r.integers(-127, 128, (oc, ic, k, k) if groups == 1 else (groups, 1, 1, k, k)).astype(np.int8)
+    bias = r.integers(-1000, 1001, (oc,)).astype(np.int32)
+    act = "IDENTITY" if form == "residual" else "RELU"
+    s_flt = (r.uniform(0.005, 0.02, oc) if form == "channel" else np.float64(0.01)).astype(np.float32)
+    s_dst = np.float32(0.3 * (ic // groups * k * k / 576.0) ** 0.5 + 0.1)
+    p = ops.conv_param(n, ic, h, w, oc, k, k, stride, pad, groups, act, 0.05, 0.01, float(s_dst))
+    want = oracle.conv_bias_qs8(src, flt, bias, stride, pad, 0.05, s_flt, s_dst, act, groups=groups)
+    room = torch.zeros(src.size + (1 << 18), dtype=torch.int8, device="cuda")
+    x = room[:src.size].view(n, h, w, ic)
+    x.copy_(dev(src.transpose(0, 2, 3, 1)))
+    check(lib().mb200_register_readable_range(room.data_ptr(), room.numel()))
+    try:
+        packed = ops.pack_filter(p, dev(flt))
+        if form == "residual":
+            z = r.integers(-128, 128, want.shape).astype(np.int8)
+            want = oracle.qelemwise("QFUSE_ADD_RELU", want, z, s_dst, 0.7, 1.3)
+            got = ops.conv_bias_qs8_nhwc_fused(p, x, packed, dev(bias), dev(z.transpose(0, 2, 3, 1)),
+                                               "QFUSE_ADD_RELU", 0.7, 1.3, algo=algo)
+        else:
+            got = ops.conv_bias_qs8_nhwc(p, x, packed, dev(bias), algo=algo,
+                                         flt_scales=dev(s_flt) if form == "channel" else None)
+        torch.cuda.synchronize()
+    finally:
+        lib().mb200_unregister_readable_range(room.data_ptr())
+    assert (got.cpu().numpy().transpose(0, 3, 1, 2) == want).all()
+    assert ops.device_status() == 0
+
+
+# depthwise layers small enough for a thread per four outputs, and the first size beyond: odd
+# extents, both strides, residual step, per-channel scales
+@pytest.mark.parametrize("n,c,h,w,stride,pad", [(1, 16, 1, 1, 1, 1), (1, 48, 7, 5, 2, 1), (3, 64, 13, 9, 1, 0),
+                                                (1, 32, 195, 194, 1, 1), (1, 32, 195, 195, 1, 1)])
+@pytest.mark.parametrize("form", ["fast", "channel", "residual"])
+def test_depthwise_quads_match_oracle(ops, oracle, n, c, h, w, stride, pad, form):
+    check_small_conv(ops, oracle, n, c, c, h, w, 3, stride, pad, c, form)
+
+
+# int8 tiles split over a cluster: every share count, tile ends inside a share, a K range that is no
+# multiple of the shares, channel counts that take the general store, residual and channel scales
+@pytest.mark.parametrize("split", [2, 4, 8])
+@pytest.mark.parametrize("n,ic,oc,h,w,k,stride", [(1, 64, 64, 9, 15, 3, 1), (1, 192, 100, 6, 7, 3, 2),
+                                                  (2, 128, 130, 12, 11, 3, 1), (1, 1024, 72, 1, 1, 1, 1)])
+@pytest.mark.parametrize("form", ["fast", "channel", "residual"])
+def test_split_tiles_match_oracle(ops, oracle, split, n, ic, oc, h, w, k, stride, form):
+    old = ops.set_option("conv_csplit", split)
+    try:
+        check_small_conv(ops, oracle, n, ic, oc, h, w, k, stride, k // 2, 1, form, "umma")
+    finally:
+        ops.set_option("conv_csplit", old)
+
+
+# transposes by words (64 x 64 tiles) and their neighbours that go byte by byte
+@pytest.mark.parametrize("n,c,h,w", [(1, 4, 2, 2), (2, 64, 8, 8), (3, 68, 7, 12), (1, 132, 9, 4), (2, 6, 8, 8),
+                                     (2, 64, 7, 7)])
+def test_relayout_by_words_is_exact(ops, n, c, h, w):
+    x = cases.rng_for(f"words_{n}_{c}_{h}_{w}").integers(-128, 128, (n, c, h, w)).astype(np.int8)
+    y = ops.nchw_to_nhwc(torch.from_numpy(x).cuda())
+    assert (y.cpu().numpy() == x.transpose(0, 2, 3, 1)).all()
+    assert (ops.nhwc_to_nchw(y).cpu().numpy() == x).all()
