@@ -660,14 +660,14 @@ int umma_clusters(int size) {
 // A layer with fewer tiles than SMs (a small batch): 64- or 128-column tiles, and how many CTAs
 // of a cluster share a tile's K loop. The pair with the shortest estimated chain of its
 // busiest CTA, in clocks: a pipeline step of 128-byte rows (half of that for 64-byte ones) costs
-// 300 with 64 columns and 380 with 128, a tile's end 1200 and 1800; the exchange of the shares
-// over the cluster 1600 and 350 for every four channels that a thread then finishes. A split
-// has to promise a sixth less: 512 -> 512 3x3 over 37 images of 7 x 7 took 30 us as 60 tiles
-// split in two and 26 us unsplit, one image 23 us unsplit and 8 us as 8 tiles split in eight.
-// Clusters on more than half of the SMs cost another 4500: the next kernel's cannot be placed
-// beside them and start late (128 -> 128 3x3 over 28 x 28: one image 4.8 us as 56 CTAs against
-// 5.1 unsplit, two images 6.1 as 104 CTAs against 5.3). Channels that are no multiple of
-// 32 take the general epilogue, 2000 more for a whole tile and nothing for a split one.
+// 300 with 64 columns and 380 with 128, a tile's end 1200 and 1800 (3000 more where the channels
+// are no multiple of 32 and take the general epilogue); the exchange of the shares over the
+// cluster 2200 and 350 for every four channels that a thread then finishes. A split has to
+// promise a sixth less, and only 64-column tiles are split: with 128 every exchange is twice as
+// long. Measured per call, 256 -> 256 3x3 with a residual step over five images of 14 x 14: 7.6 us as
+// 32 tiles of 64 columns split in four, 9.1 unsplit, 11.0 as 16 tiles of 128 split in four;
+// 512 -> 512 over one of 7 x 7: 5.8 split in eight, 13.9 unsplit; 128 -> 128 over two of 28 x 28: 6.1
+// split in four, 5.3 unsplit; a 512 -> 1000 classifier: 3.7 split in two, 4.9 unsplit.
 void choose_split(int m_tiles, int oc, int k_iters, bool wide128, int* bn, int* csplit) {
     long long best = -1;
     const int bn_first = *bn;
@@ -678,19 +678,18 @@ void choose_split(int m_tiles, int oc, int k_iters, bool wide128, int* bn, int* 
         const int step = (b == 128 ? 380 : 300) / (wide128 ? 1 : 2);
         for (int s = 1; s <= 8; s *= 2) {
             if (s > 1) {
-                const int fit = wide128 ? (b == 64 ? umma_clusters<64, GEOM_WIDE128>(s)
-                                                   : umma_clusters<128, GEOM_WIDE128>(s))
-                                        : (b == 64 ? umma_clusters<64, GEOM_WIDE>(s)
-                                                   : umma_clusters<128, GEOM_WIDE>(s));
+                if (b > 64)
+                    break;
+                const int fit = wide128 ? umma_clusters<64, GEOM_WIDE128>(s)
+                                        : umma_clusters<64, GEOM_WIDE>(s);
                 if (k_iters / s < 2 || tiles > fit || tiles * s > sm_count())
                     break;
             }
             const long long waves = (tiles * s + sm_count() - 1) / sm_count();
             const long long steps = (long long)((k_iters + s - 1) / s) * step;
             const int quads = b / (8 * s) > 1 ? b / (8 * s) : 1;
-            const int crowded = 2 * tiles * s > sm_count() ? 4500 : 0;
-            const int end = (b == 128 ? 1800 : 1200) + (oc % 32 ? 2000 : 0);
-            const long long clocks = s > 1 ? (steps + 1600 + 350 * quads + crowded) * 6 / 5
+            const int end = (b == 128 ? 1800 : 1200) + (oc % 32 ? 3000 : 0);
+            const long long clocks = s > 1 ? (steps + 2200 + 350 * quads) * 6 / 5
                                            : waves * (steps + end);
             // (a tie goes to the width the caller had chosen)
             if (best < 0 || clocks < best || (clocks == best && b == bn_first && s == 1)) {
