@@ -7,6 +7,7 @@ The shared objects land next to this file so that they travel with the source tr
 import os
 import subprocess
 import sys
+import sysconfig
 
 HERE = os.path.dirname(os.path.abspath(__file__))
 CSRC = os.path.join(HERE, "csrc")
@@ -23,6 +24,7 @@ NVCC_FLAGS = [
 
 COMPILER_DIR = os.path.join(HERE, "compiler")
 COMPILER_LIB = os.path.join(HERE, "libmegcc_b200_compiler.so")
+FASTCALL = os.path.join(HERE, "_fastcall.so")
 
 
 def _sources():
@@ -53,6 +55,23 @@ def build_compiler(verbose=False, force=False):
     return COMPILER_LIB
 
 
+def build_fastcall(verbose=False, force=False):
+    """The extension module through which operator calls reach the C ABI (plain C)."""
+    src = os.path.join(HERE, "fastcall", "fastcall.c")
+    deps = [src, os.path.join(os.path.dirname(HERE), "include", "megcc_b200.h")]
+    if not force and not _stale(FASTCALL, deps):
+        return FASTCALL
+    cc = "/usr/bin/gcc" if os.path.exists("/usr/bin/gcc") else os.environ.get("CC", "gcc")
+    cmd = [cc, "-std=c11", "-O2", "-fPIC", "-shared", "-fvisibility=hidden", "-Wall",
+           "-I" + sysconfig.get_paths()["include"], "-o", FASTCALL, src]
+    r = subprocess.run(cmd, stdout=subprocess.PIPE, stderr=subprocess.STDOUT, text=True)
+    if verbose or r.returncode:
+        sys.stderr.write(r.stdout)
+    if r.returncode:
+        raise RuntimeError("building the call extension failed")
+    return FASTCALL
+
+
 def _stale(target, deps):
     if not os.path.exists(target):
         return True
@@ -62,6 +81,7 @@ def _stale(target, deps):
 
 def build(verbose=False, force=False):
     build_compiler(verbose, force)
+    build_fastcall(verbose, force)
     nvcc = os.environ.get("NVCC", "/usr/local/cuda/bin/nvcc")
     srcs = _sources()
     deps = srcs + [os.path.join(CSRC, f) for f in os.listdir(CSRC) if f.endswith((".h", ".cuh"))]

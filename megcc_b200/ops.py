@@ -7,7 +7,7 @@ import ctypes as C
 
 import torch
 
-from ._lib import ConvParam, check, lib
+from ._lib import ConvF32Param, ConvFuse, ConvParam, check, fast, lib
 
 ACT = {"IDENTITY": 0, "RELU": 1, "H_SWISH": 2}
 POOL = {"MAX": 0, "AVERAGE": 1, "AVERAGE_COUNT_EXCLUDE_PADDING": 2}
@@ -23,6 +23,13 @@ def _stream():
 
 def _ptr(t):
     return None if t is None else t.data_ptr()
+
+
+def _at(p, kind=ConvParam):
+    """Address of a parameter struct that the caller keeps."""
+    if not isinstance(p, kind):
+        raise TypeError(f"expected a {kind.__name__}, not {type(p).__name__}")
+    return C.addressof(p)
 
 
 def conv_param(n, ic, ih, iw, oc, kh, kw, stride, pad, groups, act, s_src, s_flt, s_dst,
@@ -54,25 +61,24 @@ def pack_filter(p, flt_oihw):
 
 def conv_bias_qs8_nhwc(p, src, flt_packed, bias, dst=None, flt_scales=None, algo="auto",
                        src_is_nchw=False):
-    oh, ow = out_hw(p)
+    f, at = fast(), _at(p)
     if dst is None:
-        dst = src.new_empty((p.n, oh, ow, p.oc))
-    check(lib().mb200_conv_bias_qs8_nhwc(
-        C.byref(p), _ptr(src), int(src_is_nchw), _ptr(flt_packed), _ptr(bias), _ptr(flt_scales),
-        _ptr(dst), ALGO[algo], _stream()))
+        dst = src.new_empty(f.conv_shape(at))
+    check(f.mb200_conv_bias_qs8_nhwc(
+        at, _ptr(src), int(src_is_nchw), _ptr(flt_packed), _ptr(bias), _ptr(flt_scales),
+        dst.data_ptr(), ALGO[algo], _stream()))
     return dst
 
 
 def conv_bias_qs8_nhwc_fused(p, src, flt_packed, bias, z, mode, z_scale, out_scale, algo="auto"):
     """ConvBias (p.nonline must be IDENTITY) followed by QADD / QFUSE_ADD_RELU with the int8
     tensor z of the output's NHWC shape, in one kernel."""
-    from ._lib import ConvFuse
-    oh, ow = out_hw(p)
-    dst = src.new_empty((p.n, oh, ow, p.oc))
+    f, at = fast(), _at(p)
+    dst = src.new_empty(f.conv_shape(at))
     fuse = ConvFuse(z.data_ptr(), QELEM[mode], z_scale, out_scale)
-    check(lib().mb200_conv_bias_qs8_nhwc_fused(
-        C.byref(p), _ptr(src), 0, _ptr(flt_packed), _ptr(bias), None, C.byref(fuse), _ptr(dst),
-        ALGO[algo], _stream()))
+    check(f.mb200_conv_bias_qs8_nhwc_fused(
+        at, _ptr(src), 0, _ptr(flt_packed), _ptr(bias), None, C.addressof(fuse),
+        dst.data_ptr(), ALGO[algo], _stream()))
     return dst
 
 
@@ -86,14 +92,15 @@ def conv_acc_qs8_nhwc(p, src, flt_packed, bias):
 
 def conv_bias_qs8_nchw(p, src, flt_oihw, bias, flt_scales=None, algo="auto"):
     """ConvBias in the reference's own layouts (NCHW activations, OIHW filter)."""
-    oh, ow = out_hw(p)
-    dst = src.new_empty((p.n, p.oc, oh, ow))
+    f, at = fast(), _at(p)
+    n, oh, ow, oc = f.conv_shape(at)
+    dst = src.new_empty((n, oc, oh, ow))
     nbytes = lib().mb200_conv_bias_qs8_nchw_workspace(C.byref(p))
     ws = src.new_empty(nbytes + 256)
-    off = (-ws.data_ptr()) % 256
-    check(lib().mb200_conv_bias_qs8_nchw(
-        C.byref(p), _ptr(src), _ptr(flt_oihw), _ptr(bias), _ptr(flt_scales), _ptr(dst),
-        C.c_void_p(ws.data_ptr() + off), nbytes, ALGO[algo], _stream()))
+    base = ws.data_ptr()
+    check(f.mb200_conv_bias_qs8_nchw(
+        at, _ptr(src), _ptr(flt_oihw), _ptr(bias), _ptr(flt_scales), dst.data_ptr(),
+        base + (-base) % 256, nbytes, ALGO[algo], _stream()))
     return dst
 
 
@@ -117,8 +124,8 @@ def matmul_s8_qs8(a, b_packed, acc_scale, dst_scale):
     m, k = a.shape
     n = b_packed.shape[0]
     c = a.new_empty((m, n))
-    check(lib().mb200_matmul_s8_qs8(m, n, k, _ptr(a), _ptr(b_packed), _ptr(c), acc_scale,
-                                    dst_scale, _stream()))
+    check(fast().mb200_matmul_s8_qs8(m, n, k, _ptr(a), _ptr(b_packed), _ptr(c), acc_scale,
+                                     dst_scale, _stream()))
     return c
 
 
@@ -133,8 +140,8 @@ def pooling_qs8_nhwc(src, mode, window, stride, pad):
 
 def qelemwise_qs8(mode, a, b, s0, s1, s_dst):
     dst = torch.empty_like(a)
-    check(lib().mb200_qelemwise_qs8(_ptr(a), _ptr(b), _ptr(dst), QELEM[mode], a.numel(), s0, s1,
-                                    s_dst, _stream()))
+    check(fast().mb200_qelemwise_qs8(_ptr(a), _ptr(b), _ptr(dst), QELEM[mode], a.numel(), s0, s1,
+                                     s_dst, _stream()))
     return dst
 
 
@@ -188,7 +195,6 @@ ELEM = {"RELU": 0, "SIGMOID": 1, "SILU": 2, "H_SWISH": 3, "EXP": 4, "ADD": 16, "
 
 
 def conv_f32_param(n, ic, ih, iw, oc, kh, kw, stride, pad, groups=1, act="IDENTITY"):
-    from ._lib import ConvF32Param
     p = ConvF32Param()
     p.n, p.ic, p.ih, p.iw, p.oc, p.kh, p.kw = n, ic, ih, iw, oc, kh, kw
     p.stride_h = p.stride_w = stride
@@ -223,8 +229,8 @@ def conv_bias_f32_nhwc(p, src, flt_packed, bias=None, z=None, dst=None, dst_pitc
         dst = torch.empty((p.n, oh, ow, p.oc), dtype=torch.float32, device=src.device)
     nbytes = lib().mb200_conv_f32_workspace_bytes(C.byref(p))
     keep, ws = _scratch(nbytes, src.device)
-    check(lib().mb200_conv_bias_f32_nhwc(
-        C.byref(p), _ptr(src), _ptr(flt_packed), _ptr(bias), _ptr(z), _ptr(dst), dst_pitch,
+    check(fast().mb200_conv_bias_f32_nhwc(
+        _at(p, ConvF32Param), _ptr(src), _ptr(flt_packed), _ptr(bias), _ptr(z), _ptr(dst), dst_pitch,
         ws, nbytes, ALGO[algo], _stream()))
     return dst
 
@@ -235,11 +241,11 @@ def matmul_f32(a, b):
     n = b.shape[1]
     packed = torch.empty(lib().mb200_matmul_f32_packed_b_bytes(k, n) // 4, dtype=torch.float32,
                          device=a.device)
-    check(lib().mb200_matmul_f32_pack_b(k, n, _ptr(b), _ptr(packed), _stream()))
+    check(fast().mb200_matmul_f32_pack_b(k, n, _ptr(b), _ptr(packed), _stream()))
     c = a.new_empty((m, n))
     nbytes = lib().mb200_matmul_f32_workspace_bytes(m, k)
     keep, ws = _scratch(nbytes, a.device)
-    check(lib().mb200_matmul_f32(m, n, k, _ptr(a), _ptr(packed), _ptr(c), ws, nbytes, _stream()))
+    check(fast().mb200_matmul_f32(m, n, k, _ptr(a), _ptr(packed), _ptr(c), ws, nbytes, _stream()))
     return c
 
 
