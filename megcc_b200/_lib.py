@@ -124,7 +124,9 @@ def lib():
 # the functions behind the operator calls of a program's inner loop
 FAST = ("mb200_conv_bias_qs8_nhwc", "mb200_conv_bias_qs8_nhwc_fused", "mb200_conv_bias_qs8_nchw",
         "mb200_matmul_s8_qs8", "mb200_qelemwise_qs8", "mb200_conv_bias_f32_nhwc",
-        "mb200_matmul_f32_pack_b", "mb200_matmul_f32")
+        "mb200_conv_bias_qs8_nchw_workspace", "mb200_conv_f32_workspace_bytes",
+        "mb200_matmul_f32_packed_b_bytes", "mb200_matmul_f32_pack_b",
+        "mb200_matmul_f32_workspace_bytes", "mb200_matmul_f32", "mb200_elemwise_f32")
 _fast = None
 
 
@@ -141,7 +143,8 @@ def fast():
         f = types.SimpleNamespace(conv_shape=_fastcall.conv_shape)
         for name in FAST:
             fn = getattr(lib(), name)
-            kinds = "".join("f" if t is C.c_float else "i" for t in fn.argtypes)
+            kinds = ">" if fn.restype is C.c_size_t else ""
+            kinds += "".join("f" if t is C.c_float else "i" for t in fn.argtypes)
             setattr(f, name, _fastcall.bind(C.cast(fn, C.c_void_p).value, kinds))
         _fast = f
     return _fast

@@ -1,7 +1,7 @@
 /* Calls of the C ABI without ctypes. A ctypes call of nine arguments costs 1.3 us in conversions, a
  * tenth of a small operator's whole call; a bound function here costs 0.1. bind(address, kinds)
- * gives a callable for a function that returns int and takes, per character of `kinds`, an
- * integer or pointer ("i": int, or None for NULL) or a float ("f"). Integer and floating
+ * gives a callable for a function that returns int (size_t where `kinds` starts with ">") and takes,
+ * per character of `kinds`, an integer or pointer ("i": int, or None for NULL) or a float ("f"). Integer and floating
  * arguments travel in registers of their own (System V x86-64), so one prototype with all integers
  * in front of all floats calls every signature. The GIL is released during the call. */
 #define PY_SSIZE_T_CLEAN
@@ -18,14 +18,14 @@
 #define MAX_INTS 16
 #define MAX_FLOATS 8
 
-typedef int (*any_fn)(
+typedef uint64_t (*any_fn)(
         uint64_t, uint64_t, uint64_t, uint64_t, uint64_t, uint64_t, uint64_t, uint64_t, uint64_t,
         uint64_t, uint64_t, uint64_t, uint64_t, uint64_t, uint64_t, uint64_t, float, float, float,
         float, float, float, float, float);
 
 typedef struct {
     any_fn fn;
-    int n;
+    int n, wide;
     char kinds[MAX_INTS + MAX_FLOATS];
 } bound;
 
@@ -33,7 +33,8 @@ static PyObject* call(PyObject* self, PyObject* const* args, Py_ssize_t n) {
     const bound* b = (const bound*)PyBytes_AS_STRING(self);
     uint64_t v[MAX_INTS] = {0};
     float f[MAX_FLOATS] = {0};
-    int ni = 0, nf = 0, r;
+    int ni = 0, nf = 0;
+    uint64_t r;
     if (n != b->n) {
         PyErr_Format(PyExc_TypeError, "the function takes %d arguments (%zd given)", b->n, n);
         return NULL;
@@ -61,7 +62,8 @@ static PyObject* call(PyObject* self, PyObject* const* args, Py_ssize_t n) {
     r = b->fn(v[0], v[1], v[2], v[3], v[4], v[5], v[6], v[7], v[8], v[9], v[10], v[11], v[12],
               v[13], v[14], v[15], f[0], f[1], f[2], f[3], f[4], f[5], f[6], f[7]);
     Py_END_ALLOW_THREADS
-    return PyLong_FromLong(r);
+    /* (an int leaves the upper half of the register undefined) */
+    return b->wide ? PyLong_FromUnsignedLongLong(r) : PyLong_FromLong((long)(int)(uint32_t)r);
 }
 
 static PyMethodDef call_def = {"bound", (PyCFunction)(void*)call, METH_FASTCALL, NULL};
@@ -75,6 +77,10 @@ static PyObject* bind(PyObject* self, PyObject* args) {
     if (!PyArg_ParseTuple(args, "Ks", &address, &kinds))
         return NULL;
     memset(&b, 0, sizeof(b));
+    if (*kinds == '>') {
+        b.wide = 1;
+        ++kinds;
+    }
     for (; kinds[b.n]; ++b.n) {
         if (kinds[b.n] == 'f')
             ++nf;

@@ -95,7 +95,7 @@ def conv_bias_qs8_nchw(p, src, flt_oihw, bias, flt_scales=None, algo="auto"):
     f, at = fast(), _at(p)
     n, oh, ow, oc = f.conv_shape(at)
     dst = src.new_empty((n, oc, oh, ow))
-    nbytes = lib().mb200_conv_bias_qs8_nchw_workspace(C.byref(p))
+    nbytes = f.mb200_conv_bias_qs8_nchw_workspace(at)
     ws = src.new_empty(nbytes + 256)
     base = ws.data_ptr()
     check(f.mb200_conv_bias_qs8_nchw(
@@ -223,15 +223,16 @@ def pack_filter_f32(p, flt_oihw):
 
 def conv_bias_f32_nhwc(p, src, flt_packed, bias=None, z=None, dst=None, dst_pitch=0,
                        algo="auto"):
-    oh = (p.ih + 2 * p.pad_h - p.kh) // p.stride_h + 1
-    ow = (p.iw + 2 * p.pad_w - p.kw) // p.stride_w + 1
+    f, at = fast(), _at(p, ConvF32Param)
     if dst is None:
-        dst = torch.empty((p.n, oh, ow, p.oc), dtype=torch.float32, device=src.device)
-    nbytes = lib().mb200_conv_f32_workspace_bytes(C.byref(p))
+        oh = (p.ih + 2 * p.pad_h - p.kh) // p.stride_h + 1
+        ow = (p.iw + 2 * p.pad_w - p.kw) // p.stride_w + 1
+        dst = src.new_empty((p.n, oh, ow, p.oc), dtype=torch.float32)
+    nbytes = f.mb200_conv_f32_workspace_bytes(at)
     keep, ws = _scratch(nbytes, src.device)
-    check(fast().mb200_conv_bias_f32_nhwc(
-        _at(p, ConvF32Param), _ptr(src), _ptr(flt_packed), _ptr(bias), _ptr(z), _ptr(dst), dst_pitch,
-        ws, nbytes, ALGO[algo], _stream()))
+    check(f.mb200_conv_bias_f32_nhwc(
+        at, _ptr(src), _ptr(flt_packed), _ptr(bias), _ptr(z), _ptr(dst), dst_pitch, ws, nbytes,
+        ALGO[algo], _stream()))
     return dst
 
 
@@ -239,19 +240,19 @@ def matmul_f32(a, b):
     """C = A[M, K] @ B[K, N] (fp32 device tensors) through pack + product."""
     m, k = a.shape
     n = b.shape[1]
-    packed = torch.empty(lib().mb200_matmul_f32_packed_b_bytes(k, n) // 4, dtype=torch.float32,
-                         device=a.device)
-    check(fast().mb200_matmul_f32_pack_b(k, n, _ptr(b), _ptr(packed), _stream()))
+    f, st = fast(), _stream()
+    packed = a.new_empty(f.mb200_matmul_f32_packed_b_bytes(k, n) // 4, dtype=torch.float32)
+    check(f.mb200_matmul_f32_pack_b(k, n, _ptr(b), _ptr(packed), st))
     c = a.new_empty((m, n))
-    nbytes = lib().mb200_matmul_f32_workspace_bytes(m, k)
+    nbytes = f.mb200_matmul_f32_workspace_bytes(m, k)
     keep, ws = _scratch(nbytes, a.device)
-    check(fast().mb200_matmul_f32(m, n, k, _ptr(a), _ptr(packed), _ptr(c), ws, nbytes, _stream()))
+    check(f.mb200_matmul_f32(m, n, k, _ptr(a), _ptr(packed), _ptr(c), ws, nbytes, st))
     return c
 
 
 def elemwise_f32(mode, a, b=None):
     dst = torch.empty_like(a)
-    check(lib().mb200_elemwise_f32(ELEM[mode], _ptr(a), _ptr(b), _ptr(dst), a.numel(), _stream()))
+    check(fast().mb200_elemwise_f32(ELEM[mode], _ptr(a), _ptr(b), _ptr(dst), a.numel(), _stream()))
     return dst
 
 
