@@ -230,11 +230,11 @@ __device__ __forceinline__ void with_act(int act, F&& f) {
 // One pixel's channels of a finished tile (a row per lane): bias, activation, residual, stores.
 // With a short K loop (1x1 filters) this is the kernel's longest chain. So the bias lies in
 // shared memory (fetched once per tile column: from global memory each eight channels waited
-// for their load behind the stores before them), the residual is brought into the L2 while the tile
-// is computed, and stores are whole 32-byte sectors. 32 x 80 x 80 pixels of 128 channels to 80:
-// 96 us before, 48 now (floor 26 by its bytes); 128 to 128: 66 -> 54. (Turning the tile round in shared memory, so that a warp
-// stores 64-byte pieces of 16 rows instead of sectors of 32, measured the same within 3 %
-// either way and costs 16 KB of the ring.)
+// for their load behind the stores before them), the residual is brought into the L2 while the
+// tile is computed, and stores are whole 32-byte sectors. 32 x 80 x 80 pixels of 128 channels to
+// 80: 96 us before, 48 now (floor 26 by its bytes); 128 to 128: 66 -> 54. (Turning the tile round
+// in shared memory, so that a warp stores 64-byte pieces of 16 rows instead of sectors of 32,
+// measured the same within 3 % either way and costs 16 KB of the ring.)
 template <int COLS, int ACT>
 __device__ __forceinline__ void store_f32_row(
         const float (&sum)[COLS], const F32Epilogue& e, const float4* bias, size_t m, int ch0,
