@@ -177,7 +177,11 @@ LITE_API int mb200_lite_stream(const LiteNetwork network, void** stream);
  * runtime/src/vm/op.c:161-163 and runtime/src/init.c:29-131 do. NULL entries, and ids beyond
  * the tables, fall to the library's own implementation of the Opr's symbol; an Opr whose
  * symbol the library does not know runs only through a registered entry. The function types
- * are those of include/megcc_b200_runtime.h (void* here to keep this header free of it). */
+ * are those of include/megcc_b200_runtime.h (void* here to keep this header free of it).
+ * A registered KernelFunc is called for one instruction after the other, in the model's order,
+ * with the network's own stream (mb200_lite_stream) and with outputs in device memory: a model
+ * that holds one is not captured on parallel branches, and what a registered kernel writes
+ * is copied to the host behind it. */
 LITE_API int mb200_lite_set_kernel_tables(
         LiteNetwork network, const void* kernels, int nr_kernels, const void* init_kernels,
         int nr_init);

@@ -1257,6 +1257,8 @@ void plan_memory(DevModel& m) {
 // the two arms of a residual block) and all its tensors fit the L2 together, every tensor gets
 // memory of its own instead of the planned reuse, so that nothing but data ties two
 // instructions, and independent instructions are captured on parallel branches of the graph.
+// Only where every instruction is the library's own: a registered KernelFunc is promised one
+// stream and one instruction after the other, and may have scratch or state of its own.
 bool spread_small_model(DevModel& m) {
     constexpr size_t kMost = 96u << 20;
     size_t total = 0;
@@ -1266,6 +1268,8 @@ bool spread_small_model(DevModel& m) {
     for (size_t i = 0; i < m.instrs.size(); ++i) {
         if (!m.instrs[i].is_opr)
             return false;  // an alias of another tensor: keep the plan
+        if (m.instrs[i].op.kernel_fn != builtin_kernel)
+            return false;
         total += place_up(m.instrs[i].op.ws.size);
         branches |= i > 0 && !conflicts(m, m.instrs[i - 1], m.instrs[i]);
     }
@@ -1705,14 +1709,18 @@ int init_model_memory(Network* net) {
             return cuda_fail(e, "cudaMallocHost(output)");
         // An output that no other instruction reads is written where the caller looks for it:
         // its kernel stores over PCIe and the copy behind the graph goes away. (Up to 2 MiB: a
-        // large batch's results leave faster through the copy engine.)
+        // large batch's results leave faster through the copy engine.) Only the library's own
+        // kernels: a registered KernelFunc is promised device memory, which it may read back.
         bool read_here = false;
         for (auto& ins : m.instrs) {
-            if (ins.is_opr)
+            if (ins.is_opr) {
                 for (const Tensor* t : ins.op.inputs)
                     read_here |= t == o.tensor;
-            else
+                for (const Tensor* t : ins.op.outputs)
+                    read_here |= t == o.tensor && ins.op.kernel_fn != builtin_kernel;
+            } else {
                 read_here |= ins.mf.in == o.tensor || ins.mf.out == o.tensor;
+            }
         }
         void* mapped = nullptr;
         if (o.host_stage && !read_here && o.bytes <= kMappedOutputBytes &&

@@ -122,6 +122,72 @@ def test_a_symbol_the_library_does_not_know_runs_only_through_a_registered_table
     net.close()
 
 
+class _Tensor(C.Structure):  # the leading fields of include/megcc_b200_runtime.h's Tensor
+    _fields_ = [("name", C.c_char_p), ("type_enum", C.c_int), ("scale", C.c_float),
+                ("zero_point", C.c_uint8), ("nr_dim", C.c_int), ("dims", C.c_uint32 * 7),
+                ("stride", C.c_int * 7), ("format", C.c_int), ("ptr", C.c_void_p)]
+
+
+class _RuntimeOpt(C.Structure):
+    _fields_ = [("device", C.c_void_p), ("stream", C.c_void_p), ("device_id", C.c_int),
+                ("opr", C.c_void_p)]
+
+
+_KERNEL = C.CFUNCTYPE(C.c_int, C.POINTER(C.c_void_p), C.c_int, C.POINTER(C.POINTER(_Tensor)), C.c_int,
+                      C.c_void_p, C.POINTER(_RuntimeOpt))
+
+
+def test_registered_kernels_get_the_networks_stream_and_device_memory(oracle, tmp_path):
+    """A model with branches and a small host output, of which two kernels are a caller's own (the
+    others the library's): every call comes on the network's stream, in the model's order, and its
+    output is device memory."""
+    from megcc_b200 import lite, zoo
+    spec = zoo.resnet18(hw=64, classes=64, seed=9)
+    x = cases.rng_for("foreign_stream").integers(-128, 128, (1, 3, 64, 64), dtype=np.int8)
+    g = spec.to_graph()
+    model = g.compile([1])
+    symbols = g.kernel_symbols()
+    handle, n = build_kernel_library(g, str(tmp_path))
+    real = (C.c_void_p * n).in_dll(handle, "kernels")
+    init = (C.c_void_p * n).in_dll(handle, "init_kernels")
+    mine_k, mine_i, calls, keep = (C.c_void_p * n)(), (C.c_void_p * n)(), [], []
+    # the 3x3 layers (both arms of the residual blocks) and the 1x1 ones, the classifier among them
+    for k, s in enumerate(symbols):
+        if "_3x3_" not in s and "_1x1_" not in s or "conv2d" not in s:
+            continue
+        forward = _KERNEL(real[k])
+
+        def mine(inputs, ni, outputs, no, ws, opt, forward=forward):
+            calls.append((opt.contents.stream, outputs[0].contents.ptr, outputs[0].contents.name))
+            return forward(inputs, ni, outputs, no, ws, opt)
+
+        keep.append(_KERNEL(mine))
+        mine_k[k], mine_i[k] = C.cast(keep[-1], C.c_void_p).value, init[k]
+    net = lite.Network(model, kernel_tables=(C.addressof(mine_k), n, C.addressof(mine_i), n))
+    want = netwalk.run(spec, x, oracle).reshape(-1)
+    passes = []
+    for _ in range(3):  # eager, capture, replay
+        net.set_input("data", x)
+        net.forward()
+        net.wait()
+        assert (net.output(net.output_names()[0]) == want).all()
+        passes.append(list(calls))
+        calls.clear()
+    assert len(passes[0]) > 8 and passes[1] == passes[0] and not passes[2]
+    assert {s for s, _, _ in passes[0]} == {net.stream()}
+    assert net.output_names()[0].encode() in [name for _, _, name in passes[0]]
+    rt = C.CDLL("/usr/local/cuda/lib64/libcudart.so")
+
+    class Attributes(C.Structure):
+        _fields_ = [("type", C.c_int), ("device", C.c_int), ("dev", C.c_void_p), ("host", C.c_void_p)]
+
+    for _, p, name in passes[0]:
+        a = Attributes()
+        assert rt.cudaPointerGetAttributes(C.byref(a), C.c_void_p(p)) == 0
+        assert a.type == 2, name  # cudaMemoryTypeDevice
+    net.close()
+
+
 def test_c_program_written_against_the_reference_headers_runs_on_this_library(oracle, tmp_path):
     """oracle/_ref/lite_c_driver was compiled with -I <reference>/runtime/include and linked
     against libmegcc_b200.so where the reference tree was present; here it only runs."""
