@@ -1671,6 +1671,35 @@ int upload_weights(Network* net) {
 // ---------------------------------------------------------------------------------------
 // memory + execution
 // ---------------------------------------------------------------------------------------
+// May the tensor, an output, lie in page-locked host memory? Where one instruction writes it, one
+// of the library's own kernels (a registered KernelFunc is promised device memory, which it may
+// read back), no instruction reads it, and no other input or output of the model is the same
+// tensor: an input handed back as it is has no kernel that would write it.
+bool may_write_mapped(const DevModel& m, const Tensor* tensor) {
+    int named = 0, written = 0;
+    for (auto& s : m.inputs)
+        named += s.tensor == tensor;
+    for (auto& s : m.outputs)
+        named += s.tensor == tensor;
+    for (auto& ins : m.instrs) {
+        if (!ins.is_opr) {
+            if (ins.mf.in == tensor || ins.mf.out == tensor)
+                return false;
+            continue;
+        }
+        for (const Tensor* t : ins.op.inputs)
+            if (t == tensor)
+                return false;
+        for (const Tensor* t : ins.op.outputs)
+            if (t == tensor) {
+                if (ins.op.kernel_fn != builtin_kernel)
+                    return false;
+                ++written;
+            }
+    }
+    return named == 1 && written == 1;
+}
+
 int init_model_memory(Network* net) {
     DevModel& m = net->models[net->active];
     if (m.memory_ready)
@@ -1707,23 +1736,11 @@ int init_model_memory(Network* net) {
         if (!o.host_stage && !o.want_device &&
             (e = cudaMallocHost(&o.host_stage, o.bytes ? o.bytes : 1)) != cudaSuccess)
             return cuda_fail(e, "cudaMallocHost(output)");
-        // An output that no other instruction reads is written where the caller looks for it:
-        // its kernel stores over PCIe and the copy behind the graph goes away. (Up to 2 MiB: a
-        // large batch's results leave faster through the copy engine.) Only the library's own
-        // kernels: a registered KernelFunc is promised device memory, which it may read back.
-        bool read_here = false;
-        for (auto& ins : m.instrs) {
-            if (ins.is_opr) {
-                for (const Tensor* t : ins.op.inputs)
-                    read_here |= t == o.tensor;
-                for (const Tensor* t : ins.op.outputs)
-                    read_here |= t == o.tensor && ins.op.kernel_fn != builtin_kernel;
-            } else {
-                read_here |= ins.mf.in == o.tensor || ins.mf.out == o.tensor;
-            }
-        }
+        // An output is written where the caller looks for it, where may_write_mapped allows: its
+        // kernel stores over PCIe and the copy behind the graph goes away. (Up to 2 MiB: a
+        // large batch's results leave faster through the copy engine.)
         void* mapped = nullptr;
-        if (o.host_stage && !read_here && o.bytes <= kMappedOutputBytes &&
+        if (o.host_stage && o.bytes <= kMappedOutputBytes && may_write_mapped(m, o.tensor) &&
             cudaHostGetDevicePointer(&mapped, o.host_stage, 0) == cudaSuccess) {
             o.tensor->ptr = mapped;
             o.written_mapped = true;

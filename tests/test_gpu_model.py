@@ -191,6 +191,35 @@ def test_batch_variants_and_device_io(lite, oracle):
     net.close()
 
 
+@pytest.mark.parametrize("device_input", [False, True])
+def test_an_input_that_is_an_output_comes_back_as_it_was_given(lite, oracle, device_input):
+    """No kernel writes such an output: it is copied from where the input lies."""
+    from megcc_b200.compiler import Graph
+    r = cases.rng_for("passthrough")
+    g = Graph("passthrough")
+    x, extra = g.input("data", 64, 8, 8, 0.05), g.input("extra", 3, 4, 4, 0.05)
+    f = r.integers(-127, 128, (64, 64, 3, 3), dtype=np.int8)
+    g.mark_output(g.conv_bias("conv", x, f, None, 1, 1, 0.01, 0.9, "RELU"))
+    g.mark_output(extra)
+    net = lite.Network(g.compile([2]))
+    src = r.integers(-128, 128, (2, 64, 8, 8), dtype=np.int8)
+    want = oracle.conv_bias_qs8(src, f, None, 1, 1, 0.05, 0.01, 0.9, "RELU")
+    net.set_input("data", src)
+    for _ in range(4):  # eager, capture, replays: other values each time
+        e = r.integers(-128, 128, (2, 3, 4, 4), dtype=np.int8)
+        on_gpu = torch.from_numpy(e).cuda()
+        torch.cuda.synchronize()
+        if device_input:
+            net.set_input_ptr("extra", on_gpu.data_ptr(), e.nbytes)
+        else:
+            net.set_input("extra", e)
+        net.forward()
+        net.wait()
+        assert (net.output("extra").reshape(e.shape) == e).all()
+        assert (net.output("conv:out").reshape(want.shape) == want).all()
+    net.close()
+
+
 def test_api_errors(lite):
     from megcc_b200 import zoo
     model = zoo.single_conv(hw=16).to_graph().compile([1])
