@@ -140,7 +140,6 @@ struct IoSlot {
     Tensor* tensor = nullptr;
     void* user_ptr = nullptr;   // what LITE_reset_tensor_memory was given (inputs)
     bool user_is_device = false;
-    const void* user_mapped = nullptr;  // page-locked host memory: its address for kernels
     bool written_mapped = false;  // an output its kernel writes straight into host_stage
     bool want_device = false;   // LiteIO.is_host == 0
     void* host_stage = nullptr; // pinned copy of an output
@@ -292,6 +291,22 @@ ComputeLane* compute_lane(int device) {
 
 constexpr size_t kKernelCopyBytes = 512u << 10;
 constexpr size_t kMappedOutputBytes = 2u << 20;
+
+// The address under which kernels read the host memory [p, p + bytes), or null where they must
+// not: it is not page-locked, or not all of it. Asked on each forward (0.2 us): a program may
+// unlock its buffer after LITE_reset_tensor_memory, and a copy takes either kind.
+const void* mapped_host(const void* p, size_t bytes) {
+    cudaPointerAttributes first = {}, last = {};
+    if (bytes == 0 || cudaPointerGetAttributes(&first, p) != cudaSuccess ||
+        cudaPointerGetAttributes(&last, (const uint8_t*)p + bytes - 1) != cudaSuccess) {
+        cudaGetLastError();
+        return nullptr;
+    }
+    if (first.type != cudaMemoryTypeHost || last.type != cudaMemoryTypeHost || !first.devicePointer ||
+        (const uint8_t*)last.devicePointer != (const uint8_t*)first.devicePointer + bytes - 1)
+        return nullptr;
+    return first.devicePointer;
+}
 
 // Host -> device copy of one input, ordered after what `net->stream` holds so far and before
 // what it is given next. Pieces of at least 2 MiB go to the side streams.
@@ -1932,8 +1947,9 @@ int forward(Network* net) {
             s.tensor->ptr = (uint8_t*)net->arena->ptr + m.tensor_place[s.tensor - m.tensors.data()];
             // A small page-locked input is fetched by a kernel: a copy-engine transfer in front of
             // the graph costs two hand-overs between engines, more than the transfer itself.
-            if (s.user_mapped && s.bytes <= kKernelCopyBytes) {
-                if ((rc = mb200::launch_copy_bytes(s.user_mapped, s.tensor->ptr, s.bytes, net->stream)))
+            const void* mapped = s.bytes <= kKernelCopyBytes ? mapped_host(s.user_ptr, s.bytes) : nullptr;
+            if (mapped) {
+                if ((rc = mb200::launch_copy_bytes(mapped, s.tensor->ptr, s.bytes, net->stream)))
                     return fail(rc, "input copy: %s", mb200_last_error());
             } else if ((e = copy_input(net, s.tensor->ptr, s.user_ptr, s.bytes)) != cudaSuccess)
                 return cuda_fail(e, "cudaMemcpyAsync(input)");
@@ -2256,7 +2272,6 @@ int LITE_reset_tensor_memory(LiteTensor tensor, void* prepared_data, size_t data
         return fail(TinyNN_ERROR_INVALID_LAYOUT, "device input must be 16-byte aligned");
     s->user_ptr = prepared_data;
     s->user_is_device = is_dev;
-    s->user_mapped = attr.type == cudaMemoryTypeHost ? attr.devicePointer : nullptr;
     return TinyNN_SUCCESS;
 }
 

@@ -220,6 +220,47 @@ def test_an_input_that_is_an_output_comes_back_as_it_was_given(lite, oracle, dev
     net.close()
 
 
+def test_page_locked_inputs_of_odd_sizes_and_addresses(lite, oracle):
+    """Small page-locked inputs are fetched by a kernel: sizes and first bytes that are no multiple
+    of its 16-byte vectors, and a buffer that is unlocked between LITE_reset_tensor_memory and
+    the forwards, which it must not touch."""
+    import ctypes
+    from megcc_b200 import zoo
+    rt = ctypes.CDLL("/usr/local/cuda/lib64/libcudart.so")
+    r = cases.rng_for("pinned_odd")
+    for ic, hw in ((1, 3), (3, 7), (5, 13), (16, 12), (17, 97)):
+        spec = zoo.single_conv(ic=ic, oc=8, hw=hw, s_dst=0.4)
+        model = spec.to_graph().compile([1])
+        x = r.integers(-128, 128, (1, ic, hw, hw), dtype=np.int8)
+        want = netwalk.run(spec, x, oracle).reshape(-1)
+        room = torch.zeros(x.size + 64, dtype=torch.int8).pin_memory()
+        for at in (0, 1, 7, 16, 33):
+            room[at:at + x.size] = torch.from_numpy(x.reshape(-1))
+            net = lite.Network(model)
+            net.set_input_ptr("data", room.data_ptr() + at, x.nbytes)
+            for _ in range(3):
+                net.forward()
+                net.wait()
+                assert (net.output(net.output_names()[0]) == want).all(), (ic, hw, at)
+            net.close()
+    # (ic, hw) = (17, 97): 159953 bytes, 40 pages
+    page = 4096
+    raw = np.zeros(x.size + 2 * page, np.int8)
+    start = -raw.ctypes.data % page
+    buf = raw[start:start + x.size]
+    buf[:] = x.reshape(-1)
+    assert rt.cudaHostRegister(ctypes.c_void_p(buf.ctypes.data),
+                               ctypes.c_size_t(-(-x.size // page) * page), 0) == 0
+    net = lite.Network(model)
+    net.set_input_ptr("data", buf.ctypes.data, x.nbytes)
+    assert rt.cudaHostUnregister(ctypes.c_void_p(buf.ctypes.data)) == 0
+    for _ in range(3):
+        net.forward()
+        net.wait()
+        assert (net.output(net.output_names()[0]) == want).all()
+    net.close()
+
+
 def test_api_errors(lite):
     from megcc_b200 import zoo
     model = zoo.single_conv(hw=16).to_graph().compile([1])
