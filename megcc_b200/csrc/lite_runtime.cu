@@ -125,7 +125,7 @@ constexpr size_t kArenaSlack = 131072 + 4096;
 
 struct Arena {
     void* ptr = nullptr;
-    size_t bytes = 0;
+    size_t bytes = 0;  // what its networks need; once allocated, what it holds
     int device = 0;
     ~Arena() {
         if (ptr) {
@@ -1723,9 +1723,12 @@ int init_model_memory(Network* net) {
     if (e != cudaSuccess)
         return cuda_fail(e, "cudaSetDevice");
     Arena& a = *net->arena;
-    if (a.bytes < net->arena_need)
-        a.bytes = net->arena_need;
+    if (a.ptr && a.bytes < net->arena_need)
+        return fail(TinyNN_ERROR,
+                    "the shared runtime memory holds %zu bytes and this network needs %zu: load every "
+                    "network before it is shared", a.bytes, net->arena_need);
     if (!a.ptr) {
+        a.bytes = std::max(a.bytes, net->arena_need);
         // one allocation for every tensor and workspace of the model, with 128 KiB behind
         // the last tensor: the tensor-core ConvBias describes a small activation (batch 1 of a
         // late layer) to the TMA unit as 128 KiB starting at it, and the whole arena is
@@ -2416,9 +2419,10 @@ int LITE_share_runtime_memroy(LiteNetwork src_network, LiteNetwork dst_network) 
         return fail(TinyNN_ERROR, "shared runtime memory should be called before model run");
     if (src->device_id != dst->device_id)
         return fail(TinyNN_ERROR, "networks live on different devices");
-    // one arena sized for the larger of the two; both networks must then run on one
-    // stream's worth of ordering, which the caller gets by waiting between forwards
-    src->arena->bytes = src->arena_need > dst->arena_need ? src->arena_need : dst->arena_need;
+    // one arena sized for the largest of all that share it (either may have shared with others
+    // before); they must then run on one stream's worth of ordering, which the caller gets by
+    // waiting between forwards
+    src->arena->bytes = std::max({src->arena->bytes, dst->arena->bytes, src->arena_need, dst->arena_need});
     dst->arena = src->arena;
     return TinyNN_SUCCESS;
 }

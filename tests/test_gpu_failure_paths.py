@@ -117,3 +117,48 @@ def test_two_networks_share_one_runtime_arena(oracle):
     n_big.close()
     torch.cuda.synchronize()
     assert torch.cuda.mem_get_info()[0] >= before - (8 << 20)  # the arena went back
+
+
+def test_three_networks_share_an_arena_that_fits_each_of_them(oracle):
+    """a with b (the larger), then a with c (the smaller): b must still fit. A network that was
+    shared before its model was loaded, and needs more than the arena then holds, is refused."""
+    from megcc_b200 import lite, zoo
+    from megcc_b200.lite import LiteError
+    specs = [zoo.single_conv(ic=64, oc=64, hw=40, s_dst=0.9, seed=5), zoo.resnet18(hw=96, classes=64, seed=6),
+             zoo.single_conv(ic=64, oc=64, hw=16, s_dst=0.9, seed=7)]
+    shapes = [(2, 64, 40, 40), (8, 3, 96, 96), (1, 64, 16, 16)]
+    xs = [cases.rng_for(f"share3_{i}").integers(-128, 128, s, dtype=np.int8) for i, s in enumerate(shapes)]
+    wants = [netwalk.run(s, x, oracle).reshape(-1) for s, x in zip(specs, xs)]
+    nets = [lite.Network(s.to_graph().compile([x.shape[0]])) for s, x in zip(specs, xs)]
+    L = lite.lib()
+    lite.check(L.LITE_share_runtime_memroy(nets[0]._net, nets[1]._net))
+    lite.check(L.LITE_share_runtime_memroy(nets[0]._net, nets[2]._net))
+    for _ in range(3):
+        for net, x, want in zip(nets, xs, wants):
+            net.set_input("data", x)
+            net.forward()
+            net.wait()
+            assert (net.output(net.output_names()[0]) == want).all()
+    for net in nets:
+        net.close()
+    # shared while it held no model
+    first = lite.Network(specs[2].to_graph().compile([1]))
+    late = lite.Network(specs[2].to_graph().compile([1]))
+    empty, cfg, io = C.c_void_p(), lite.LiteConfig.from_buffer_copy(L.default_config().contents), lite.LiteNetworkIO()
+    lite.check(L.LITE_make_network(C.byref(empty), cfg, io))
+    lite.check(L.LITE_share_runtime_memroy(first._net, empty))
+    first.set_input("data", xs[2])
+    first.forward()
+    first.wait()
+    model = specs[1].to_graph().compile([8])
+    buf = C.create_string_buffer(model, len(model))
+    lite.check(L.LITE_load_model_from_mem(empty, buf, len(model)))
+    late.close()
+    late._net, late._model, late._tensors = empty, buf, {}
+    late.set_input("data", xs[1])
+    with pytest.raises(LiteError) as e:
+        late.forward()
+    assert "shared runtime memory" in str(e.value)
+    assert (first.output(first.output_names()[0]) == wants[2]).all()
+    late.close()
+    first.close()
