@@ -1084,6 +1084,17 @@ bool read_layout(const fb::Table& t, Layout* out) {
     return true;
 }
 
+// A tensor of the file holds its pixels one behind the other (its bytes are those of its extents):
+// a wider pitch in its strides would make pixel_pitch() lead kernels out of it. Only
+// join_concats sets wider ones.
+void dense_pixels(Layout* l) {
+    if (l->nr_dim != 4 || l->stride[3] <= (int)l->dims[1])
+        return;
+    const int c = (int)l->dims[1], h = (int)l->dims[2], w = (int)l->dims[3];
+    const int nhwc[4] = {h * w * c, 1, w * c, c}, nchw[4] = {c * h * w, h * w, w, 1};
+    memcpy(l->stride, l->stride[1] == 1 ? nhwc : nchw, sizeof(nhwc));
+}
+
 // Do the tensors share memory by intent (equal, or a slice and the whole)?
 bool same_memory(const DevModel& m, const Tensor* a, const Tensor* b) {
     auto whole = [&](const Tensor* t) -> const Tensor* {
@@ -1395,6 +1406,7 @@ int parse_model(Network* net, const void* mem, size_t size) {
                 return fail(TinyNN_ERROR_MODEL_PARSE,
                             "tensor %u at offset %lld (+%zu) lies outside the %zu byte arena", i,
                             (long long)off, t.size, m.tensor_memory);
+            dense_pixels(&t.layout);
             t.offset = (size_t)off;
             t.use_count = tt.scalar<int32_t>(fb::field::T_use_count, 0);
             if (!tt.str(fb::field::T_name, &m.names[i]) || m.names[i].empty())

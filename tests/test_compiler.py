@@ -287,3 +287,22 @@ def test_compile_side_builds_inside_the_reference_kernelgen(tmp_path):
     assert out.read_bytes() == mine
     syms = g.kernel_symbols()
     assert r.stdout.split()[:len(syms)] == syms and any("_z_QFUSE_ADD_RELU" in x for x in syms)
+
+
+def test_a_wider_pixel_pitch_in_the_file_is_not_believed():
+    """The fp32 kernels step from pixel to pixel by a pitch that the runtime sets for slices of a
+    concat. A file whose strides claim a wider one than its tensor holds must not lead them out
+    of it."""
+    from megcc_b200 import zoo
+    model = zoo.yolox_s(hw=64).to_graph().compile([2])
+    rc, text = describe(model)
+    assert rc == 0
+    m = next(m for m in re.finditer(r"tensor (\S+) .*format=1 .*dims=(\d+)x(\d+)x(\d+)x(\d+) "
+                                    r"stride=(\S+)", text) if int(m.group(3)) == 64 and int(m.group(5)) == 16)
+    strides = [int(v) for v in m.group(6).split("x")]
+    assert strides == [64 * 16 * 16, 1, 64 * 16, 64]
+    old = np.array(strides, dtype="<i4").tobytes()
+    assert model.count(old) >= 1
+    new = np.array([4 * 64 * 16 * 16, 1, 4 * 64 * 16, 4 * 64], dtype="<i4").tobytes()
+    rc, patched = describe(model.replace(old, new))
+    assert rc == 0 and patched == text
