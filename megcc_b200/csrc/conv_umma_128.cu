@@ -1,0 +1,13 @@
+// conv_umma_kernel with 128-column tiles
+#include "conv_umma_kernel.cuh"
+
+namespace mb200 {
+namespace umma_conv {
+template int launch_kernel<128, GEOM_WIDE>(
+        const CUtensorMap&, const CUtensorMap&, const UmmaConvParams&, cudaStream_t);
+template int launch_kernel<128, GEOM_WIDE128>(
+        const CUtensorMap&, const CUtensorMap&, const UmmaConvParams&, cudaStream_t);
+template int launch_form<128, GEOM_TAP16>(
+        const CUtensorMap&, const CUtensorMap&, const UmmaConvParams&, cudaStream_t);
+}  // namespace umma_conv
+}  // namespace mb200
