@@ -22,6 +22,10 @@
  * additionally want bias and channel scales 16-byte aligned and refuse them otherwise when
  * they were asked for by name (MB200_ALGO_UMMA / _PATCH); MB200_ALGO_AUTO falls back.
  *
+ * Order. Every operand, a filter, bias or scales among them, may be the result of earlier calls on
+ * the same stream, of this library or another: kernels are launched ahead of the end of the one
+ * in front of them, and read nothing that could still be written before that one has completed.
+ *
  * Scale range. Results are bit-identical to the reference's x86 kernels for every finite
  * positive scale triple. The vector and tensor-core kernels divide by dst_scale with a
  * three-instruction sequence that is exact for 2^-100 <= src_scale * flt_scale <= 2^69,

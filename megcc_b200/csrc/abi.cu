@@ -202,16 +202,40 @@ namespace mb200 {
 
 namespace {
 std::mutex g_ranges_mu;
-std::map<uintptr_t, size_t> g_ranges;  // base -> bytes
-}  // namespace
+typedef std::map<uintptr_t, size_t> Ranges;  // base -> bytes
+Ranges g_ranges, g_constant;
 
-bool readable_through(const void* p, size_t bytes) {
+bool within(const Ranges& ranges, const void* p, size_t bytes) {
     std::lock_guard<std::mutex> lock(g_ranges_mu);
-    auto it = g_ranges.upper_bound((uintptr_t)p);
-    if (it == g_ranges.begin())
+    auto it = ranges.upper_bound((uintptr_t)p);
+    if (it == ranges.begin())
         return false;
     --it;
     return (uintptr_t)p + bytes <= it->first + it->second;
+}
+
+// ConvArgs::params_early of operands that the caller handed in
+int params_early(const void* flt, const void* bias, const void* flt_scales) {
+    return (is_constant(flt) ? 1 : 0) | (is_constant(bias) && is_constant(flt_scales) ? 2 : 0);
+}
+}  // namespace
+
+bool readable_through(const void* p, size_t bytes) {
+    return within(g_ranges, p, bytes);
+}
+
+void register_constant_range(const void* base, size_t bytes) {
+    std::lock_guard<std::mutex> lock(g_ranges_mu);
+    g_constant[(uintptr_t)base] = bytes;
+}
+
+void unregister_constant_range(const void* base) {
+    std::lock_guard<std::mutex> lock(g_ranges_mu);
+    g_constant.erase((uintptr_t)base);
+}
+
+bool is_constant(const void* p) {
+    return !p || within(g_constant, p, 1);
 }
 
 int descriptor_images(const ConvArgs& a, const int8_t* src) {
@@ -360,6 +384,11 @@ int mb200_relayout_nhwc_to_nchw44_s8(
                                 (cudaStream_t)stream);
 }
 
+static int conv_bias_nhwc(
+        const mb200_conv_param* p, const int8_t* src, int src_is_nchw, const int8_t* flt_packed,
+        const int32_t* bias, const float* flt_scales, const mb200_conv_fuse* fuse, int8_t* dst,
+        int algo, int early, void* stream);
+
 int mb200_conv_bias_qs8_nhwc(
         const mb200_conv_param* p, const int8_t* src, int src_is_nchw, const int8_t* flt_packed,
         const int32_t* bias, const float* flt_scales, int8_t* dst, int algo, void* stream) {
@@ -371,10 +400,19 @@ int mb200_conv_bias_qs8_nhwc_fused(
         const mb200_conv_param* p, const int8_t* src, int src_is_nchw, const int8_t* flt_packed,
         const int32_t* bias, const float* flt_scales, const mb200_conv_fuse* fuse, int8_t* dst,
         int algo, void* stream) {
+    return conv_bias_nhwc(p, src, src_is_nchw, flt_packed, bias, flt_scales, fuse, dst, algo,
+                          params_early(flt_packed, bias, flt_scales), stream);
+}
+
+static int conv_bias_nhwc(
+        const mb200_conv_param* p, const int8_t* src, int src_is_nchw, const int8_t* flt_packed,
+        const int32_t* bias, const float* flt_scales, const mb200_conv_fuse* fuse, int8_t* dst,
+        int algo, int early, void* stream) {
     ConvArgs a{};
     int rc = make_args(p, src_is_nchw, &a);
     if (rc)
         return rc;
+    a.params_early = early;
     if (fuse) {
         if (!fuse->z)
             return set_error(ST_NULL_PTR, "fused operand z is NULL");
@@ -530,6 +568,7 @@ int mb200_conv_bias_qs8_s2d(
         return set_error(ST_OUT_OF_RANGE, "workspace of %zu bytes is too small", workspace_bytes);
     if (((uintptr_t)workspace | (uintptr_t)flt_s2d | (uintptr_t)dst) & 15)
         return set_error(ST_INVALID_LAYOUT, "workspace, filter and dst must be 16-byte aligned");
+    a.params_early = params_early(flt_s2d, bias, flt_scales);
     return launch_conv_s2d(a, src, flt_s2d, bias, flt_scales, dst, workspace, (cudaStream_t)stream);
 }
 
@@ -558,6 +597,7 @@ int mb200_conv_bias_pool_qs8_s2d(
     if (((uintptr_t)workspace | (uintptr_t)flt_s2d | (uintptr_t)dst) & 15)
         return set_error(ST_INVALID_LAYOUT, "workspace, filter and dst must be 16-byte aligned");
     a.pool = 1;
+    a.params_early = params_early(flt_s2d, bias, flt_scales);
     return launch_conv_s2d(a, src, flt_s2d, bias, flt_scales, dst, workspace, (cudaStream_t)stream);
 }
 
@@ -594,6 +634,7 @@ int mb200_conv_bias_qs8_nchw(
         int8_t* ws_flt = ws_dst + align_up((size_t)a.m * a.oc, 256);
         int8_t* ws_s2d = ws_flt + align_up(conv_s2d_filter_bytes(a), 256);
         a.src_is_nchw = 1;
+        a.params_early = 1;  // (the filter's packing does not release the kernels behind it early: see pdl.h)
         if ((rc = launch_conv_s2d_pack_filter(a, flt_oihw, ws_flt, st)))
             return rc;
         if ((rc = launch_conv_s2d(a, src, ws_flt, bias, flt_scales, ws_dst, ws_s2d, st)))
@@ -615,7 +656,9 @@ int mb200_conv_bias_qs8_nchw(
     // NCHW -> NHWC is a [C][HW] -> [HW][C] transpose per image
     if ((rc = launch_transpose_pack_s8(src, ws_src, a.n, a.ic, a.ih * a.iw, a, flt_oihw, ws_flt, st)))
         return rc;
-    if ((rc = mb200_conv_bias_qs8_nhwc(p, ws_src, 0, ws_flt, bias, flt_scales, ws_dst, algo, st)))
+    // (the filter's packing: likewise)
+    if ((rc = conv_bias_nhwc(p, ws_src, 0, ws_flt, bias, flt_scales, nullptr, ws_dst, algo,
+                             1 | params_early(nullptr, bias, flt_scales), st)))
         return rc;
     return launch_transpose_s8(ws_dst, dst, a.n, a.oh * a.ow, a.oc, st);
 }

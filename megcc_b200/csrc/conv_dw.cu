@@ -36,6 +36,7 @@ struct DwParams {
     // fast_ops == 1 -> trunc(fma((float)acc, fast_mul, +-fast_add)) saturated
     int fast_ops;
     float fast_mul, fast_add;
+    int early;  // quad kernel: filter, bias and scales may be fetched before the wait
 };
 
 // four words, byte i = channel i of taps a..d  ->  four words, byte j = tap j of one channel
@@ -168,8 +169,8 @@ __global__ void __launch_bounds__(256) conv_dw_kernel(
 // work is, and 16 or 32 outputs of a thread are some 600 dependent instructions on a few of the
 // SMs (4.5 to 6.4 us from its input being ready to the next kernel's for MobileNetV1's layers).
 // Here a thread has about 100, the filter (36 adjacent bytes per thread, straight into registers),
-// bias and scales are fetched before the wait for the previous kernel, and there is no shared
-// memory and no barrier. Bytes are loaded 4 at a time, so it is no match for the forms above once
+// bias and scales are fetched before the wait for the previous kernel where nothing in flight can
+// write them (a network's weights), and there is no shared memory and no barrier. Bytes are loaded 4 at a time, so it is no match for the forms above once
 // the GPU is full.
 __global__ void __launch_bounds__(128) conv_dw3x3_quad_kernel(
         const DwParams p, const uint32_t* __restrict__ src, const uint32_t* __restrict__ flt,
@@ -187,6 +188,8 @@ __global__ void __launch_bounds__(128) conv_dw3x3_quad_kernel(
     m /= a.ow;
     const int oy = (int)(m % a.oh);
     const int n = (int)(m / a.oh);
+    if (!p.early)
+        pdl_wait();
     uint32_t f[9];
 #pragma unroll
     for (int t = 0; t < 9; ++t)
@@ -199,7 +202,7 @@ __global__ void __launch_bounds__(128) conv_dw3x3_quad_kernel(
         s = __ldg(reinterpret_cast<const float4*>(flt_scales) + cq);
     const int iy0 = oy * a.sh - a.ph, ix0 = ox * a.sw - a.pw;
     const uint32_t* base = src + (size_t)((unsigned)n * a.ih) * a.iw * c4 + cq;
-    pdl_wait();  // (everything above is parameters)
+    pdl_wait();
     uint32_t v[9];
 #pragma unroll
     for (int t = 0; t < 9; ++t) {
@@ -399,6 +402,7 @@ int launch_conv_dw(
     DwParams p;
     p.a = a;
     p.c16 = a.ic / 16;
+    p.early = a.params_early == 3;
     p.inv_dst = 1.0f / a.s_dst;         // RN(1/d), as the division by a constant needs
     p.z_div = 1.0f / a.z_out_scale;     // the reference's scale_div = 1.f / scale_dst
     p.fast_ops = 0;

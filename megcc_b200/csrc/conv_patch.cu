@@ -78,6 +78,7 @@ struct PatchParams {
     // 1: the depthwise tensor has 32 channels and is seen as pixel PAIRS of 64 bytes
     // ([N][H][W/2][2][32]); column 32 h + c of a row is channel c of the pair's pixel h
     int dw_pairs;
+    int early_flt;  // the filter may be fetched before the previous kernel has completed
     EpilogueParams ep;
     int8_t* dst;
     int* status;
@@ -257,6 +258,8 @@ __global__ void __launch_bounds__(64 + 32 * EW, EW == 16 ? 1 : 2) conv_patch_ker
             // bytes are w[n0 + c][t] at (c, c). Written here in the layout the TMA would have
             // produced (rows of 64 bytes, 64-byte swizzle: 16-byte unit u of row r sits at
             // unit u ^ ((r >> 1) & 3)), then handed to the tensor core's (async) proxy.
+            if (!p.early_flt)
+                pdl_wait();
             uint4* b16 = reinterpret_cast<uint4*>(smem_b);
             for (int i = threadIdx.x; i < 9 * BN * 4; i += blockDim.x)
                 b16[i] = make_uint4(0, 0, 0, 0);
@@ -303,8 +306,10 @@ __global__ void __launch_bounds__(64 + 32 * EW, EW == 16 ? 1 : 2) conv_patch_ker
     if (warp == 0) {
         // ---------------- TMA producer ----------------
         if (lane == 0) {
-            // the filter slice, once: one [BN][16-byte] block per 16 bytes of K (weights: they
-            // do not depend on the kernel before this one, so they are fetched before the wait)
+            // the filter slice, once: one [BN][16-byte] block per 16 bytes of K; before the wait for
+            // the previous kernel where nothing in flight can write it
+            if (!p.early_flt)
+                pdl_wait();
             const int kchunks = p.kh * p.kw * p.chunks;
             if (ROWS && p.dw_flt) {
                 mbar_arrive(b_full);  // the operand was built in place before the roles split
@@ -946,6 +951,7 @@ int launch_conv_patch(
     p.ep.acc_out = a.acc_out;
     p.dw_flt = a.dw64 ? flt : nullptr;
     p.dw_pairs = a.dw64 == 2 ? 1 : 0;
+    p.early_flt = a.params_early & 1;
     p.dst = dst;
     p.status = device_status_word(st);
     if (!p.status)

@@ -48,6 +48,9 @@ struct ConvArgs {
     // 64 input channels and builds the block-diagonal filter tile from the raw [C][3][3] filter.
     // 2: 32 channels, a.iw / a.ow count pixel PAIRS (64-byte rows), a.oc == 64.
     int dw64;
+    // operands that may be fetched before the kernel has waited for the one in front of it (see
+    // pdl.h): bit 0 the filter, bit 1 bias and channel scales
+    int params_early;
     // general kernel only: divide by s_dst with the true division (scales outside the range
     // in which the three-instruction division by a constant is exact, see common.cuh)
     int true_division;
@@ -109,6 +112,11 @@ bool residual_fast_constants(
 // tensor is too small and nothing is known about the memory behind it.
 int descriptor_images(const ConvArgs& a, const int8_t* src);
 bool readable_through(const void* p, size_t bytes);
+// Device memory that no kernel writes as long as it is registered: a network's weights. Kernels may
+// fetch operands from it ahead of the kernels in front of them. Null counts as constant.
+void register_constant_range(const void* base, size_t bytes);
+void unregister_constant_range(const void* base);
+bool is_constant(const void* p);
 
 // tensor-core implicit GEMM; conv_umma_supported() says whether the shape qualifies
 bool conv_umma_supported(const ConvArgs& a, const int8_t* src, const int8_t* flt, const int8_t* dst);

@@ -1691,6 +1691,7 @@ int upload_weights(Network* net) {
         return cuda_fail(e, "weight upload");
     if (!mb200::device_status_word(net->stream))
         return fail(TinyNN_ERROR_MEMORY_MALLOC, "%s", mb200_last_error());
+    mb200::register_constant_range(net->weight_arena, total);  // nothing writes them from here on
     net->loaded = true;
     return TinyNN_SUCCESS;
 }
@@ -2459,8 +2460,10 @@ int LITE_destroy_network(LiteNetwork network) {
             if (o.host_stage)
                 cudaFreeHost(o.host_stage);
     }
-    if (net->weight_arena)
+    if (net->weight_arena) {
+        mb200::unregister_constant_range(net->weight_arena);
         cudaFree(net->weight_arena);
+    }
     for (int i = 0; i < Network::kCopyStreams; ++i) {
         if (net->copy_stream[i])
             cudaStreamDestroy(net->copy_stream[i]);

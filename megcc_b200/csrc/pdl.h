@@ -1,11 +1,15 @@
 // Programmatic dependent launch: a kernel launched with launch_pdl() may be scheduled while the
 // kernel before it on the stream is still running. Its CTAs take the SMs the predecessor's CTAs
 // leave, run their set-up (barrier initialisation, tensor-memory allocation, descriptor
-// prefetch) and then block in pdl_start() until the predecessor has completed and its writes
+// prefetch) and then block in pdl_wait() until the predecessor has completed and its writes
 // are visible. That hides the launch latency and the ramp of each of the 20-odd kernels of a
-// network behind the tail of the previous one. Every kernel launched this way calls
-// pdl_start() before it reads or writes global memory; a kernel launched without the
-// attribute executes the two instructions as no-ops.
+// network behind the tail of the previous one. A kernel launched this way reads and writes no
+// global memory before pdl_wait(), with one exception: operands that no kernel in flight writes.
+// Those are what the launch was told so of (ConvArgs::params_early): a network's weights, and a
+// filter that the call itself has packed with a kernel that does not release early. "The previous
+// kernel" is not enough: a kernel that releases its successor before its own wait lets the third
+// start while the first still runs. A kernel launched without the attribute executes the two
+// instructions as no-ops.
 #pragma once
 #include <cuda_runtime.h>
 

@@ -886,6 +886,49 @@ def test_split_tiles_match_oracle(ops, oracle, split, n, ic, oc, h, w, k, stride
         ops.set_option("conv_csplit", old)
 
 
+# parameters that the call before has computed: the kernels start before that one has ended, and the
+# last bytes of its result, which are written last, are the filter or the scales
+@pytest.mark.parametrize("kernel", ["quad_scales", "quad_filter", "patch_filter", "depthwise_tensor_filter",
+                                    "umma_filter"])
+def test_parameters_may_come_from_the_call_before(ops, oracle, kernel):
+    from megcc_b200._lib import check, lib
+    r = cases.rng_for("late_" + kernel)
+    n, c, hw, k, groups, algo = {"quad_scales": (1, 32, 20, 3, 32, "auto"),
+                                 "quad_filter": (1, 32, 20, 3, 32, "auto"),
+                                 "patch_filter": (2, 64, 40, 3, 1, "patch"),
+                                 "depthwise_tensor_filter": (2, 64, 40, 3, 64, "patch"),
+                                 "umma_filter": (2, 64, 40, 3, 1, "umma")}[kernel]
+    src = r.integers(-128, 128, (n, c, hw, hw)).astype(np.int8)
+    bias = r.integers(-1000, 1001, (c,)).astype(np.int32)
+    x = dev(src.transpose(0, 2, 3, 1))
+    s_dst = 0.3 if groups == 1 else 0.1
+    p = ops.conv_param(n, c, hw, hw, c, k, k, 1, 1, groups, "RELU", 0.05, 0.01, s_dst)
+    big = 1 << 25  # values of the call in front: some 50 us
+    values = torch.zeros(big, device="cuda")
+    late8 = torch.empty(big, dtype=torch.int8, device="cuda")
+    late32 = torch.empty(big, device="cuda")
+    for turn in range(4):
+        flt = r.integers(-127, 128, (c, c, k, k) if groups == 1 else (c, 1, 1, k, k)).astype(np.int8)
+        s_flt = r.uniform(0.005, 0.02, c).astype(np.float32) if kernel == "quad_scales" else np.float32(0.01)
+        packed = ops.pack_filter(p, dev(flt))
+        late8.fill_(77)
+        late32.fill_(1.0)
+        dev_bias, st = dev(bias), torch.cuda.current_stream().cuda_stream
+        if kernel == "quad_scales":
+            values[-c:] = dev(s_flt)
+            torch.cuda.synchronize()
+            check(lib().mb200_elemwise_f32(ops.ELEM["RELU"], values.data_ptr(), None, late32.data_ptr(), big, st))
+            out = ops.conv_bias_qs8_nhwc(p, x, packed, dev_bias, flt_scales=late32[-c:], algo=algo)
+        else:
+            values[-packed.numel():] = packed.float()
+            torch.cuda.synchronize()
+            check(lib().mb200_typecvt_f32_qs8(values.data_ptr(), late8.data_ptr(), big, 1.0, 1.0, st))
+            out = ops.conv_bias_qs8_nhwc(p, x, late8[-packed.numel():], dev_bias, algo=algo)
+        want = oracle.conv_bias_qs8(src, flt, bias, 1, 1, 0.05, s_flt, s_dst, "RELU", groups=groups)
+        assert (out.cpu().numpy().transpose(0, 3, 1, 2) == want).all(), turn
+    assert ops.device_status() == 0
+
+
 # transposes by words (64 x 64 tiles) and their neighbours that go byte by byte
 @pytest.mark.parametrize("n,c,h,w", [(1, 4, 2, 2), (2, 64, 8, 8), (3, 68, 7, 12), (1, 132, 9, 4), (2, 6, 8, 8),
                                      (2, 64, 7, 7)])
