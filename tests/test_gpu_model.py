@@ -381,16 +381,18 @@ def test_model_with_a_bare_metal_device_model_beside_the_cuda_one(lite, oracle):
     assert (out == want).all()
 
 
-def test_cycling_device_input_buffers_replays_captured_graphs(lite, oracle):
-    """A caller that alternates between a few device input buffers: each address gets its own
-    captured graph, kept (up to four) and replayed, and every forward is still bit-exact."""
+@pytest.mark.parametrize("buffers", [3, 7])
+def test_cycling_device_input_buffers_replays_captured_graphs(lite, oracle, buffers):
+    """A caller that alternates between device input buffers: each of a few addresses gets its own
+    captured graph, kept (up to four) and replayed; with more of them the inputs go through the
+    model's own memory; every forward is bit-exact. Then one buffer that stays."""
     from megcc_b200 import zoo
     spec = zoo.resnet18(hw=64, classes=64, seed=7)
     model = spec.to_graph().compile([8])
     net = lite.Network(model)
     name_in, name_out = net.input_names()[0], net.output_names()[0]
     r = cases.rng_for("cycle_inputs")
-    xs = [r.integers(-128, 128, (8, 3, 64, 64), dtype=np.int8) for _ in range(3)]
+    xs = [r.integers(-128, 128, (8, 3, 64, 64), dtype=np.int8) for _ in range(buffers)]
     wants = [netwalk.run(spec, x, oracle).reshape(-1) for x in xs]
     devs = [torch.from_numpy(x).cuda() for x in xs]
     for turn in range(4):  # eager pass, three captures, then replays only
@@ -399,4 +401,10 @@ def test_cycling_device_input_buffers_replays_captured_graphs(lite, oracle):
             net.forward()
             net.wait()
             assert (net.output(name_out) == want).all(), turn
+    for turn in range(70):
+        devs[-1].copy_(torch.from_numpy(xs[turn % buffers]))
+        torch.cuda.synchronize()
+        net.forward()
+        net.wait()
+        assert (net.output(name_out) == wants[turn % buffers]).all(), turn
     net.close()
