@@ -175,7 +175,17 @@ struct DevModel {
     // where tensors and workspaces really lie in the arena: as planned, or each on its own
     size_t arena_bytes = 0;
     std::vector<size_t> tensor_place, ws_place;
-    std::vector<cudaEvent_t> marks;  // one per instruction, for capture only
+    // the branches, worked out at load: in which lane (a stream of the capture) each instruction goes,
+    // what it waits for there, and the events that instructions of other lanes wait on
+    struct Step {
+        int instr, lane;
+        bool fork;  // the lane's first instruction
+        std::vector<int> waits;
+    };
+    std::vector<Step> steps;
+    std::vector<int> lane_ends;       // last instruction of each lane
+    std::vector<char> marked;         // per instruction: somebody waits for its event
+    std::vector<cudaEvent_t> marks;   // ... the events, and the fork behind them
 };
 
 struct Network;
@@ -218,8 +228,8 @@ struct Network {
 
 // The streams beside a network's own that branches of a small model are captured on. Nothing runs
 // on them (a graph is launched on the network's stream), so the networks of a device share one
-// set, the mutex held for a capture; it is created with the first capture that wants it (0.1 ms
-// per stream, which every network would pay) and given back with the last network that used it.
+// set, the mutex held for a capture; each is created with the first capture that wants it (0.07 ms
+// per stream; ResNet-18 wants one) and all are given back with the last network that used them.
 struct CaptureLanes {
     static constexpr int kLanes = 5;
     std::mutex mu;
@@ -230,11 +240,12 @@ struct CaptureLanes {
         static CaptureLanes lanes[64];
         return device >= 0 && device < 64 ? &lanes[device] : nullptr;
     }
-    // with mu held
-    bool ready(Network* net) {
-        for (auto& s : stream)
-            if (!s && cudaStreamCreateWithFlags(&s, cudaStreamNonBlocking) != cudaSuccess) {
-                s = nullptr;
+    // with mu held: the first `count` of them
+    bool ready(Network* net, int count) {
+        for (int i = 0; i < count; ++i)
+            if (!stream[i] &&
+                cudaStreamCreateWithFlags(&stream[i], cudaStreamNonBlocking) != cudaSuccess) {
+                stream[i] = nullptr;
                 return false;
             }
         users += !net->uses_lanes;
@@ -246,7 +257,8 @@ struct CaptureLanes {
         if (!net->uses_lanes || --users)
             return;
         for (auto& s : stream) {
-            cudaStreamDestroy(s);
+            if (s)
+                cudaStreamDestroy(s);
             s = nullptr;
         }
     }
@@ -1282,6 +1294,78 @@ void plan_memory(DevModel& m) {
     }
 }
 
+// Which branch of the captured graph each instruction goes to: the lane whose last instruction it
+// depends on, or one whose work it follows anyway, or a free one.
+void plan_lanes(DevModel& m) {
+    constexpr int kLanes = CaptureLanes::kLanes + 1;
+    const int n = (int)m.instrs.size();
+    std::vector<int> lane_of(n, 0);
+    int tail[kLanes];               // last instruction of each lane, -1: none
+    int seen[kLanes][kLanes];       // seen[a][b]: last instruction of lane b that lane a follows
+    for (int a = 0; a < kLanes; ++a) {
+        tail[a] = -1;
+        for (int b = 0; b < kLanes; ++b)
+            seen[a][b] = -1;
+    }
+    bool started[kLanes] = {true};
+    m.steps.clear();
+    m.marked.assign(n, 0);
+    for (int i = 0; i < n; ++i) {
+        if (m.instrs[i].in_place)
+            continue;
+        int need[kLanes];  // latest dependency on each lane
+        for (int l = 0; l < kLanes; ++l)
+            need[l] = -1;
+        for (int j = i - 1; j >= 0; --j)
+            if (!m.instrs[j].in_place && need[lane_of[j]] < 0 &&
+                conflicts(m, m.instrs[j], m.instrs[i]))
+                need[lane_of[j]] = j;
+        int best = -1, free_lane = -1, any = 0;
+        for (int l = 0; l < kLanes; ++l) {
+            if (tail[l] >= 0 && need[l] == tail[l] && (best < 0 || tail[l] > tail[best]))
+                best = l;  // continues this lane's chain
+            if (tail[l] < 0 && free_lane < 0)
+                free_lane = l;
+            if (tail[l] < tail[any])
+                any = l;
+        }
+        if (best < 0)
+            for (int l = 0; l < kLanes && best < 0; ++l) {
+                // a lane whose last instruction is an ancestor through the dependencies
+                bool behind = tail[l] >= 0;
+                bool follows = false;
+                for (int d = 0; d < kLanes && behind; ++d)
+                    if (need[d] >= 0 && d != l && need[d] == tail[d] && seen[d][l] >= tail[l])
+                        follows = true;
+                if (behind && follows)
+                    best = l;
+            }
+        if (best < 0)
+            best = free_lane >= 0 ? free_lane : any;
+        DevModel::Step step{i, best, !started[best], {}};
+        started[best] = true;
+        for (int d = 0; d < kLanes; ++d) {
+            if (d == best || need[d] <= seen[best][d])
+                continue;
+            step.waits.push_back(need[d]);
+            m.marked[need[d]] = 1;
+            seen[best][d] = need[d];
+            for (int b = 0; b < kLanes; ++b)  // (what the awaited lane follows now is no later
+                if (need[d] == tail[d] && seen[d][b] > seen[best][b])  // than what it had then)
+                    seen[best][b] = seen[d][b];
+        }
+        m.steps.push_back(std::move(step));
+        lane_of[i] = best;
+        tail[best] = i;
+        seen[best][best] = i;
+    }
+    m.lane_ends.clear();
+    for (int l = 0; l < kLanes && tail[l] >= 0; ++l)
+        m.lane_ends.push_back(tail[l]);
+    for (size_t l = 1; l < m.lane_ends.size(); ++l)
+        m.marked[m.lane_ends[l]] = 1;
+}
+
 // A small model (a batch of one) is bound by the latency of its instructions one after the
 // other, each of which leaves most SMs idle. Where it has branches (the heads of a detector,
 // the two arms of a residual block) and all its tensors fit the L2 together, every tensor gets
@@ -1318,6 +1402,7 @@ bool spread_small_model(DevModel& m) {
             off += place_up(m.instrs[i].op.ws.size);
         }
     m.arena_bytes = off;
+    plan_lanes(m);
     m.side_by_side = true;
     return true;
 }
@@ -1822,106 +1907,54 @@ int issue_instructions(Network* net, DevModel& m, bool timed) {
     return TinyNN_SUCCESS;
 }
 
-// The instructions as branches of the graph under capture: each goes to the lane whose last
-// instruction it depends on, or to one whose work it follows anyway, or to a free one.
+// The instructions as branches of the graph under capture.
 int issue_side_by_side(Network* net, DevModel& m) {
-    constexpr int kLanes = CaptureLanes::kLanes + 1;
-    cudaStream_t lanes[kLanes] = {net->stream};
-    for (int l = 1; l < kLanes; ++l)
+    cudaStream_t lanes[CaptureLanes::kLanes + 1] = {net->stream};
+    for (int l = 1; l <= CaptureLanes::kLanes; ++l)
         lanes[l] = CaptureLanes::of(net->device_id)->stream[l - 1];
     // every branch reports to the network's own status word
     struct Borrow {
         int* before;
         ~Borrow() { mb200::borrow_status_word(before); }
     } borrow{mb200::borrow_status_word(mb200::device_status_word(net->stream))};
-    const int n = (int)m.instrs.size();
-    std::vector<int> lane_of(n, 0);
-    int tail[kLanes];               // last instruction of each lane, -1: none
-    int seen[kLanes][kLanes];       // seen[a][b]: last instruction of lane b that lane a follows
-    for (int a = 0; a < kLanes; ++a) {
-        tail[a] = -1;
-        for (int b = 0; b < kLanes; ++b)
-            seen[a][b] = -1;
-    }
-    cudaEvent_t fork = m.marks[n];
+    cudaEvent_t fork = m.marks.back();
     cudaError_t e = cudaEventRecord(fork, net->stream);
-    bool started[kLanes] = {true};
-    for (int i = 0; i < n && e == cudaSuccess; ++i) {
-        if (m.instrs[i].in_place)
-            continue;
-        int need[kLanes];  // latest dependency on each lane
-        for (int l = 0; l < kLanes; ++l)
-            need[l] = -1;
-        for (int j = i - 1; j >= 0; --j)
-            if (!m.instrs[j].in_place && need[lane_of[j]] < 0 &&
-                conflicts(m, m.instrs[j], m.instrs[i]))
-                need[lane_of[j]] = j;
-        int best = -1, free_lane = -1, any = 0;
-        for (int l = 0; l < kLanes; ++l) {
-            if (tail[l] >= 0 && need[l] == tail[l] && (best < 0 || tail[l] > tail[best]))
-                best = l;  // continues this lane's chain
-            if (tail[l] < 0 && free_lane < 0)
-                free_lane = l;
-            if (tail[l] < tail[any])
-                any = l;
-        }
-        if (best < 0)
-            for (int l = 0; l < kLanes && best < 0; ++l) {
-                // a lane whose last instruction is an ancestor through the dependencies
-                bool behind = tail[l] >= 0;
-                bool follows = false;
-                for (int d = 0; d < kLanes && behind; ++d)
-                    if (need[d] >= 0 && d != l && need[d] == tail[d] && seen[d][l] >= tail[l])
-                        follows = true;
-                if (behind && follows)
-                    best = l;
-            }
-        if (best < 0)
-            best = free_lane >= 0 ? free_lane : any;
-        if (!started[best]) {
-            e = cudaStreamWaitEvent(lanes[best], fork, 0);
-            started[best] = true;
-        }
-        for (int d = 0; d < kLanes && e == cudaSuccess; ++d) {
-            if (d == best || need[d] <= seen[best][d])
-                continue;
-            e = cudaStreamWaitEvent(lanes[best], m.marks[need[d]], 0);
-            seen[best][d] = need[d];
-            for (int b = 0; b < kLanes; ++b)  // (what the awaited lane follows now is no later
-                if (need[d] == tail[d] && seen[d][b] > seen[best][b])  // than what it had then)
-                    seen[best][b] = seen[d][b];
-        }
+    for (const DevModel::Step& step : m.steps) {
+        cudaStream_t lane = lanes[step.lane];
+        if (e == cudaSuccess && step.fork)
+            e = cudaStreamWaitEvent(lane, fork, 0);
+        for (int w : step.waits)
+            if (e == cudaSuccess)
+                e = cudaStreamWaitEvent(lane, m.marks[w], 0);
         if (e != cudaSuccess)
             break;
+        OpPlan& op = m.instrs[step.instr].op;
         RuntimeOpt opt = net->opt;
-        opt.opr = &m.instrs[i].op;
-        opt.stream = lanes[best];
-        OpPlan& op = m.instrs[i].op;
+        opt.opr = &op;
+        opt.stream = lane;
         const int rc = op.kernel_fn(op.inputs.data(), (int)op.inputs.size(), op.outputs.data(),
                                     (int)op.outputs.size(), &op.ws, &opt);
         if (rc)
             return fail(rc, "kernel %s: %s", op.symbol.c_str(), mb200_last_error());
-        e = cudaEventRecord(m.marks[i], lanes[best]);
-        lane_of[i] = best;
-        tail[best] = i;
-        seen[best][best] = i;
+        if (m.marked[step.instr])
+            e = cudaEventRecord(m.marks[step.instr], lane);
     }
-    for (int l = 1; l < kLanes && e == cudaSuccess; ++l)
-        if (tail[l] >= 0)
-            e = cudaStreamWaitEvent(net->stream, m.marks[tail[l]], 0);
+    for (size_t l = 1; l < m.lane_ends.size() && e == cudaSuccess; ++l)
+        e = cudaStreamWaitEvent(net->stream, m.marks[m.lane_ends[l]], 0);
     return e == cudaSuccess ? TinyNN_SUCCESS : cuda_fail(e, "capturing parallel branches");
 }
 
 // What capturing side by side needs beforehand (nothing may be set up during a capture).
 bool ready_side_by_side(Network* net, DevModel& m, CaptureLanes* lanes) {
-    if (!lanes->ready(net))
+    if (!lanes->ready(net, (int)m.lane_ends.size() - 1))
         return false;
-    while (m.marks.size() < m.instrs.size() + 1) {
-        cudaEvent_t e;
-        if (cudaEventCreateWithFlags(&e, cudaEventDisableTiming) != cudaSuccess)
+    m.marks.resize(m.instrs.size() + 1, nullptr);
+    for (size_t i = 0; i < m.marks.size(); ++i)
+        if (!m.marks[i] && (i == m.instrs.size() || m.marked[i]) &&
+            cudaEventCreateWithFlags(&m.marks[i], cudaEventDisableTiming) != cudaSuccess) {
+            m.marks[i] = nullptr;
             return false;
-        m.marks.push_back(e);
-    }
+        }
     return true;
 }
 
@@ -2514,7 +2547,8 @@ int LITE_destroy_network(LiteNetwork network) {
         CaptureLanes::of(net->device_id)->leave(net);
     for (auto& m : net->models)
         for (cudaEvent_t e : m.marks)
-            cudaEventDestroy(e);
+            if (e)
+                cudaEventDestroy(e);
     if (net->stream)
         cudaStreamDestroy(net->stream);
     delete net;
