@@ -140,8 +140,9 @@ LITE_API int LITE_get_all_input_name(const LiteNetwork network, size_t* size, co
 LITE_API int LITE_get_all_output_name(const LiteNetwork network, size_t* size, const char** name);
 /* runtime/src/lite/network.c:285-303 (spelling of the symbol is the reference's). Both networks
  * load their models first and share before either has run. The arena is as large as the largest
- * network that shares it asks for; a network that has independent instructions, and at most 96 MB of
- * tensors in all, asks for the sum of its tensors instead of the model file's plan. */
+ * network that shares it asks for; a network that has independent instructions, and at most 48 MB of
+ * tensors in all (96 MB where a fifth of its instructions are off the longest chain), asks for the sum
+ * of its tensors instead of the model file's plan. */
 LITE_API int LITE_share_runtime_memroy(LiteNetwork src_network, LiteNetwork dst_network);
 /* runtime/src/lite/network.c:305-368 */
 LITE_API int LITE_destroy_network(LiteNetwork network);

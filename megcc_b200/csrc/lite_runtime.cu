@@ -1366,15 +1366,39 @@ void plan_lanes(DevModel& m) {
         m.marked[m.lane_ends[l]] = 1;
 }
 
+// Instructions on the longest chain of dependencies.
+int longest_chain(const DevModel& m) {
+    std::vector<int> depth(m.instrs.size(), 0);
+    int longest = 0;
+    for (size_t i = 0; i < m.instrs.size(); ++i) {
+        if (m.instrs[i].in_place)
+            continue;
+        for (size_t j = 0; j < i; ++j)
+            if (depth[j] > depth[i] && conflicts(m, m.instrs[j], m.instrs[i]))
+                depth[i] = depth[j];
+        longest = std::max(longest, ++depth[i]);
+    }
+    return longest;
+}
+
 // A small model (a batch of one) is bound by the latency of its instructions one after the
 // other, each of which leaves most SMs idle. Where it has branches (the heads of a detector,
-// the two arms of a residual block) and all its tensors fit the L2 together, every tensor gets
-// memory of its own instead of the planned reuse, so that nothing but data ties two
-// instructions, and independent instructions are captured on parallel branches of the graph.
-// Only where every instruction is the library's own: a registered KernelFunc is promised one
-// stream and one instruction after the other, and may have scratch or state of its own.
+// the two arms of a residual block), every tensor gets memory of its own instead of the planned
+// reuse, so that nothing but data ties two instructions, and independent instructions are captured on
+// parallel branches of the graph. Only where every instruction is the library's own: a registered
+// KernelFunc is promised one stream and one instruction after the other, and may have scratch or
+// state of its own.
+//
+// Up to which size of its tensors together: what branches save is the time of the instructions off
+// the longest chain, what they cost is the planned reuse of memory in the L2 and kernels that
+// share SMs which the larger batch would have filled. Measured per forward in one build, planned
+// and in order against spread and on branches: ResNet-18 (3 of its 23 instructions off the chain) 127
+// and 113 us with one image (2.7 MB), 185 and 179 with 16 (43 MB), 203 and 215 with 24 (65 MB), 226
+// and 237 with 32 (87 MB), 269 and 275 with 48 (130 MB): 48 MB. The detector (34 of 108 off the chain)
+// 561 and 448 at 416 x 416 (72 MB), 568 and 470 at 448 (84 MB), 581 and 500 at 480 (96 MB), and still
+// 701 and 594 at 640 (171 MB): there 96 MB bound the memory that a network takes for its speed, not
+// the gain.
 bool spread_small_model(DevModel& m) {
-    constexpr size_t kMost = 96u << 20;
     size_t total = 0;
     for (size_t i = 0; i < m.tensors.size(); ++i)
         total += m.view_of[i] ? 0 : place_up(m.tensors[i].size);
@@ -1387,7 +1411,14 @@ bool spread_small_model(DevModel& m) {
         total += place_up(m.instrs[i].op.ws.size);
         branches |= i > 0 && !conflicts(m, m.instrs[i - 1], m.instrs[i]);
     }
-    if (!branches || total > kMost)
+    if (!branches)
+        return false;
+    // (a fifth of the instructions lies between the two models above)
+    int launched = 0;
+    for (auto& ins : m.instrs)
+        launched += !ins.in_place;
+    const bool many = (launched - longest_chain(m)) * 5 >= launched;
+    if (total > (many ? 96u << 20 : 48u << 20))
         return false;
     size_t off = 0;
     for (size_t i = 0; i < m.tensors.size(); ++i) {
