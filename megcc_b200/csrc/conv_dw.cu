@@ -27,6 +27,7 @@ namespace mb200 {
 namespace {
 
 constexpr int kTapWords = 3;  // 12 taps at most
+constexpr int kMostSmem = 96 * 1024;  // (one value, whatever layer another thread launches meanwhile)
 
 struct DwParams {
     ConvArgs a;
@@ -386,7 +387,7 @@ bool conv_dw_supported(
     if ((size_t)a.m * (a.ic / 16) >= (1ull << 31) ||
         (size_t)a.n * a.ih * a.iw * (a.ic / 16) >= (1ull << 31))
         return false;
-    if ((size_t)a.ic * kTapWords * 4 > 96 * 1024)
+    if ((size_t)a.ic * kTapWords * 4 > (size_t)kMostSmem)
         return false;
     if (((uintptr_t)src | (uintptr_t)dst) & 15)
         return false;
@@ -450,7 +451,7 @@ int launch_conv_dw(
         auto kernel = outs == 4 ? (a.sh == 1 ? conv_dw3x3_row_kernel<1, 4> : conv_dw3x3_row_kernel<2, 4>)
                                 : (a.sh == 1 ? conv_dw3x3_row_kernel<1, 2> : conv_dw3x3_row_kernel<2, 2>);
         if (smem > 48 * 1024 &&
-            cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) !=
+            cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kMostSmem) !=
                     cudaSuccess)
             return check_launch("conv_dw smem attribute");
         launch_pdl(kernel, dim3((unsigned)blocks), dim3(128), (size_t)smem, st, p, (const uint4*)src,
@@ -459,7 +460,7 @@ int launch_conv_dw(
     }
     if (smem > 48 * 1024 &&
         cudaFuncSetAttribute(conv_dw_kernel<3, 3>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             smem) != cudaSuccess)
+                             kMostSmem) != cudaSuccess)
         return check_launch("conv_dw smem attribute");
     launch_pdl(conv_dw_kernel<3, 3>, dim3((unsigned)grid), dim3(256), (size_t)smem, st, p,
                (const uint4*)src, flt, bias, flt_scales, (uint4*)dst);

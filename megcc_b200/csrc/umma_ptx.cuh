@@ -7,6 +7,7 @@
 #include <stdint.h>
 
 #include <atomic>
+#include <mutex>
 
 #ifndef MB200_TRY_WAIT_HINT_NS
 #define MB200_TRY_WAIT_HINT_NS 2000
@@ -437,15 +438,20 @@ inline int sm_count() {
 }
 
 // Remembers, per device, that a kernel was allowed `bytes` of dynamic shared memory: the
-// attribute call costs a launch about a microsecond and never changes. One static object per
-// kernel instantiation; concurrent first calls both set the same value.
+// attribute call costs a launch about a microsecond. One static object per kernel instantiation.
+// A kernel may ask for different sizes, from several threads: the attribute only ever grows,
+// and what is remembered is never more than what is set.
 struct KernelReady {
     std::atomic<int> bytes_set[64] = {};
+    std::mutex mu;
     template <class Kernel>
     bool smem(Kernel kernel, int bytes) {
         int dev = 0;
         if (cudaGetDevice(&dev) != cudaSuccess)
             return false;
+        if (dev >= 0 && dev < 64 && bytes_set[dev].load(std::memory_order_relaxed) >= bytes)
+            return true;
+        std::lock_guard<std::mutex> lock(mu);
         if (dev >= 0 && dev < 64 && bytes_set[dev].load(std::memory_order_relaxed) >= bytes)
             return true;
         if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes) !=

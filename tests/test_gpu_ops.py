@@ -1,5 +1,7 @@
 """Parity of the CUDA operators, called through the C ABI, with the CPU oracle and with the
 golden vectors produced by the reference's own x86 kernels. Bit-exact everywhere."""
+import os
+
 import numpy as np
 import pytest
 
@@ -927,6 +929,62 @@ def test_parameters_may_come_from_the_call_before(ops, oracle, kernel):
         want = oracle.conv_bias_qs8(src, flt, bias, 1, 1, 0.05, s_flt, s_dst, "RELU", groups=groups)
         assert (out.cpu().numpy().transpose(0, 3, 1, 2) == want).all(), turn
     assert ops.device_status() == 0
+
+
+FIRST_LAUNCHES = """
+import threading, numpy as np, torch
+from megcc_b200 import ops
+# one kernel instantiation, shared-memory sizes from 30 to 200 KB: the first launches of a process, at
+# the same time
+shapes = [(16, 64, 4, 1), (32, 64, 3, 1), (32, 64, 5, 2), (64, 64, 1, 0), (96, 64, 3, 1), (32, 64, 7, 3),
+          (96, 64, 2, 0), (128, 64, 2, 0)]
+rng = np.random.default_rng(3)
+jobs = []
+for ic, oc, k, pad in shapes:
+    p = ops.conv_param(8, ic, 40, 40, oc, k, k, 1, pad, 1, "RELU", 0.05, 0.01, 0.5)
+    x = torch.from_numpy(rng.integers(-128, 128, (8, 40, 40, ic), dtype=np.int8)).cuda()
+    f = torch.from_numpy(rng.integers(-127, 128, (oc, k, k, ic), dtype=np.int8).reshape(-1)).cuda()
+    jobs.append((p, x, f))
+wide = [(p, x, f) for p, x, f in ((ops.conv_param(1, c, 9, 9, c, 3, 3, 1, 1, c, "RELU", 0.05, 0.01, 0.1),
+        torch.from_numpy(rng.integers(-128, 128, (1, 9, 9, c), dtype=np.int8)).cuda(),
+        torch.from_numpy(rng.integers(-127, 128, c * 9, dtype=np.int8)).cuda()) for c in (4112, 6000, 8192))]
+torch.cuda.synchronize()
+gate, got = threading.Barrier(len(jobs) + len(wide)), {}
+
+def work(i, algo, p, x, f):
+    try:
+        torch.cuda.set_device(0)
+        with torch.cuda.stream(torch.cuda.Stream()):
+            gate.wait()
+            outs = [ops.conv_bias_qs8_nhwc(p, x, f, None, algo=algo) for _ in range(20)]
+            torch.cuda.current_stream().synchronize()
+        got[i] = outs
+    except Exception as e:
+        got[i] = e
+
+old = ops.set_option("dw_one_output", 1)
+threads = [threading.Thread(target=work, args=(i, "patch" if i < len(jobs) else "auto") + j)
+           for i, j in enumerate(jobs + wide)]
+for t in threads:
+    t.start()
+for t in threads:
+    t.join()
+ops.set_option("dw_one_output", old)
+for i, (p, x, f) in enumerate(jobs + wide):
+    assert not isinstance(got[i], Exception), (i, got[i])
+    want = ops.conv_bias_qs8_nhwc(p, x, f, None, algo="direct")
+    assert all(torch.equal(o, want) for o in got[i]), i
+assert ops.device_status() == 0
+print("same")
+"""
+
+
+def test_first_launches_of_a_process_from_several_threads():
+    import subprocess
+    import sys
+    out = subprocess.run([sys.executable, "-c", FIRST_LAUNCHES], capture_output=True, text=True,
+                         timeout=300, cwd=os.path.dirname(os.path.dirname(os.path.abspath(__file__))))
+    assert out.returncode == 0 and out.stdout.strip().endswith("same"), out.stderr[-2000:]
 
 
 # transposes by words (64 x 64 tiles) and their neighbours that go byte by byte
