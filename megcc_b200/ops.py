@@ -63,7 +63,7 @@ def conv_bias_qs8_nhwc(p, src, flt_packed, bias, dst=None, flt_scales=None, algo
                        src_is_nchw=False):
     f, at = fast(), _at(p)
     if dst is None:
-        dst = src.new_empty(f.conv_shape(at))
+        dst = src.new_empty(f.conv_shape(at), dtype=torch.int8)
     check(f.mb200_conv_bias_qs8_nhwc(
         at, _ptr(src), int(src_is_nchw), _ptr(flt_packed), _ptr(bias), _ptr(flt_scales),
         dst.data_ptr(), ALGO[algo], _stream()))
@@ -74,7 +74,7 @@ def conv_bias_qs8_nhwc_fused(p, src, flt_packed, bias, z, mode, z_scale, out_sca
     """ConvBias (p.nonline must be IDENTITY) followed by QADD / QFUSE_ADD_RELU with the int8
     tensor z of the output's NHWC shape, in one kernel."""
     f, at = fast(), _at(p)
-    dst = src.new_empty(f.conv_shape(at))
+    dst = src.new_empty(f.conv_shape(at), dtype=torch.int8)
     fuse = ConvFuse(z.data_ptr(), QELEM[mode], z_scale, out_scale)
     check(f.mb200_conv_bias_qs8_nhwc_fused(
         at, _ptr(src), 0, _ptr(flt_packed), _ptr(bias), None, C.addressof(fuse),
@@ -94,9 +94,9 @@ def conv_bias_qs8_nchw(p, src, flt_oihw, bias, flt_scales=None, algo="auto"):
     """ConvBias in the reference's own layouts (NCHW activations, OIHW filter)."""
     f, at = fast(), _at(p)
     n, oh, ow, oc = f.conv_shape(at)
-    dst = src.new_empty((n, oc, oh, ow))
+    dst = src.new_empty((n, oc, oh, ow), dtype=torch.int8)
     nbytes = f.mb200_conv_bias_qs8_nchw_workspace(at)
-    ws = src.new_empty(nbytes + 256)
+    ws = src.new_empty(nbytes + 256, dtype=torch.int8)
     base = ws.data_ptr()
     check(f.mb200_conv_bias_qs8_nchw(
         at, _ptr(src), _ptr(flt_oihw), _ptr(bias), _ptr(flt_scales), dst.data_ptr(),
@@ -123,7 +123,7 @@ def matmul_s8_s32(a, b_packed):
 def matmul_s8_qs8(a, b_packed, acc_scale, dst_scale):
     m, k = a.shape
     n = b_packed.shape[0]
-    c = a.new_empty((m, n))
+    c = a.new_empty((m, n), dtype=torch.int8)
     check(fast().mb200_matmul_s8_qs8(m, n, k, _ptr(a), _ptr(b_packed), _ptr(c), acc_scale,
                                      dst_scale, _stream()))
     return c
@@ -243,7 +243,7 @@ def matmul_f32(a, b):
     f, st = fast(), _stream()
     packed = a.new_empty(f.mb200_matmul_f32_packed_b_bytes(k, n) // 4, dtype=torch.float32)
     check(f.mb200_matmul_f32_pack_b(k, n, _ptr(b), _ptr(packed), st))
-    c = a.new_empty((m, n))
+    c = a.new_empty((m, n), dtype=torch.float32)
     nbytes = f.mb200_matmul_f32_workspace_bytes(m, k)
     keep, ws = _scratch(nbytes, a.device)
     check(f.mb200_matmul_f32(m, n, k, _ptr(a), _ptr(packed), _ptr(c), ws, nbytes, st))
@@ -332,7 +332,7 @@ def conv_bias_qs8_s2d(p, src, flt_packed, bias, flt_scales=None, src_is_nchw=Tru
     """First-layer ConvBias (few input channels) through the space-to-depth form; flt_packed
     from mb200_conv_s2d_pack_filter or pack_filter_nchw44."""
     oh, ow = out_hw(p)
-    dst = src.new_empty((p.n, oh, ow, p.oc))
+    dst = src.new_empty((p.n, oh, ow, p.oc), dtype=torch.int8)
     nbytes = lib().mb200_conv_s2d_workspace_bytes(C.byref(p))
     keep, ws = _scratch(nbytes, src.device)
     check(lib().mb200_conv_bias_qs8_s2d(

@@ -797,6 +797,27 @@ def test_typecvt_between_fp32_and_qsi8_follows_the_gi_rule(ops, oracle):
         assert (got == oracle.typecvt_qs8_f32(q, 0.3, 0.7)).all()
 
 
+def test_results_are_int8_whatever_the_inputs_bytes_are_called(ops):
+    """Inputs that hold int8 values as torch.uint8 (bytes from a file or a decoder)."""
+    r = cases.rng_for("uint8_inputs")
+    x = dev(r.integers(-128, 128, (2, 40, 40, 64), dtype=np.int8))
+    f = dev(r.integers(-127, 128, (64, 64, 3, 3), dtype=np.int8))
+    p = ops.conv_param(2, 64, 40, 40, 64, 3, 3, 1, 1, 1, "IDENTITY", 0.05, 0.01, 0.5)
+    packed = ops.pack_filter(p, f)
+    first = ops.conv_param(8, 3, 64, 64, 64, 7, 7, 2, 3, 1, "RELU", 0.05, 0.01, 0.5)
+    stem = dev(r.integers(-127, 128, (64, 3, 7, 7), dtype=np.int8))
+    img = dev(r.integers(-128, 128, (8, 3, 64, 64), dtype=np.int8))
+    a, b = x.reshape(-1, 64), dev(r.integers(-127, 128, (64, 96), dtype=np.int8))
+    calls = [lambda v: ops.conv_bias_qs8_nhwc(p, v(x), packed, None),
+             lambda v: ops.conv_bias_qs8_nhwc_fused(p, v(x), packed, None, v(x), "QADD", 0.5, 0.7),
+             lambda v: ops.conv_bias_qs8_nchw(p, v(x.permute(0, 3, 1, 2).contiguous()), v(f), None),
+             lambda v: ops.conv_bias_qs8_s2d(first, v(img), ops.pack_filter_s2d(first, stem), None),
+             lambda v: ops.matmul_s8_qs8(v(a), ops.matmul_pack_b(b), 0.001, 0.5)]
+    for i, call in enumerate(calls):
+        want, got = call(lambda t: t), call(lambda t: t.view(torch.uint8))
+        assert got.dtype == torch.int8 and torch.equal(got, want), i
+
+
 def test_qrelu_matches_oracle(ops, oracle):
     a = cases.rng_for("qrelu").integers(-128, 128, (3, 5, 7, 11), dtype=np.int8)
     out = ops.qelemwise_qs8("QRELU", dev(a), None, 0.3, 1.0, 0.7).cpu().numpy()
