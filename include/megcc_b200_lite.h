@@ -191,7 +191,9 @@ LITE_API int mb200_lite_set_kernel_tables(
         int nr_init);
 /* Per-network switches. "use_graph" (default 1): replay the instruction list as one CUDA
  * graph; 0 issues the kernels one by one on every forward. "profile": as
- * mb200_lite_set_profile. New networks take their defaults from the environment once per
+ * mb200_lite_set_profile. "selftest_fail_branches": 1 lets the network's next capture of
+ * parallel branches (of a small model) fail half way, after which it captures its instructions in
+ * order, as it does after a failure of any other cause. New networks take their defaults from the environment once per
  * process (MB200_NO_GRAPH=1, MB200_PROFILE=1); nothing reads the environment afterwards. */
 LITE_API int mb200_lite_set_option(LiteNetwork network, const char* name, int value);
 /* Per-instruction timing (the reference's compile-time TINYNN_PROFILE_KERNEL,

@@ -217,6 +217,7 @@ struct Network {
     std::shared_ptr<Arena> arena = std::make_shared<Arena>();
     size_t arena_need = 0;
     bool loaded = false, pending = false, use_graph = true, profile = false;
+    bool fail_branches = false;  // self-test: the next capture of branches gives up half way
     std::vector<std::unique_ptr<IoHandle>> handles;
     // Large host inputs are copied in as several pieces on side streams: one copy stream
     // measured 40 GB/s over PCIe gen5 x16, four concurrent pieces 54 GB/s.
@@ -1951,6 +1952,10 @@ int issue_side_by_side(Network* net, DevModel& m) {
     cudaEvent_t fork = m.marks.back();
     cudaError_t e = cudaEventRecord(fork, net->stream);
     for (const DevModel::Step& step : m.steps) {
+        if (net->fail_branches && &step == &m.steps[m.steps.size() / 2]) {
+            net->fail_branches = false;
+            return fail(TinyNN_ERROR, "self-test: capturing parallel branches given up");
+        }
         cudaStream_t lane = lanes[step.lane];
         if (e == cudaSuccess && step.fork)
             e = cudaStreamWaitEvent(lane, fork, 0);
@@ -2621,6 +2626,10 @@ int mb200_lite_set_option(LiteNetwork network, const char* name, int value) {
     }
     if (strcmp(name, "profile") == 0) {
         net->profile = value != 0;
+        return TinyNN_SUCCESS;
+    }
+    if (strcmp(name, "selftest_fail_branches") == 0) {
+        net->fail_branches = value != 0;
         return TinyNN_SUCCESS;
     }
     return fail(TinyNN_ERROR_OUT_OF_RANGE, "unknown option '%s'", name);

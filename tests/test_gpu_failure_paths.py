@@ -85,6 +85,64 @@ def test_lite_wait_reports_a_kernel_that_gave_up_and_only_on_its_own_network(ora
     b.close()
 
 
+def test_a_capture_of_branches_that_fails_falls_back_to_the_instructions_in_order(oracle):
+    """ResNet-18 and one image is captured on parallel branches. Where that fails half way, with a
+    lane forked off and not joined, the forward goes on in order, and the lanes, which the
+    device's networks share, serve the next network's branches."""
+    from megcc_b200 import lite, zoo
+    spec = zoo.resnet18(hw=64, classes=64, seed=11)
+    model = spec.to_graph().compile([1])
+    r = cases.rng_for("failed_branches")
+    a, b = lite.Network(model), lite.Network(model)
+    a.set_option("selftest_fail_branches", 1)
+    for turn in range(4):
+        for net in (a, b):
+            x = r.integers(-128, 128, (1, 3, 64, 64), dtype=np.int8)
+            net.set_input("data", x)
+            net.forward()
+            net.wait()
+            assert (net.output(net.output_names()[0]) == netwalk.run(spec, x, oracle).reshape(-1)).all(), turn
+    with pytest.raises(lite.LiteError):
+        a.set_option("no_such_option", 1)
+    a.close()
+    b.close()
+
+
+def test_networks_of_two_threads_capture_on_shared_lanes(oracle):
+    """Each thread makes, runs and closes its own networks: captures on the device's lanes, and the
+    lanes' end with the last network that used them, come in any order."""
+    import threading
+    from megcc_b200 import lite, zoo
+    spec = zoo.resnet18(hw=64, classes=64, seed=12)
+    model = spec.to_graph().compile([1])
+    r = cases.rng_for("two_threads")
+    xs = [r.integers(-128, 128, (1, 3, 64, 64), dtype=np.int8) for _ in range(2)]
+    wants = [netwalk.run(spec, x, oracle).reshape(-1) for x in xs]
+    gate, wrong = threading.Barrier(2), []
+
+    def work(i):
+        try:
+            gate.wait()
+            for turn in range(6):
+                net = lite.Network(model)
+                net.set_input("data", xs[i])
+                for _ in range(5):
+                    net.forward()
+                    net.wait()
+                    if not (net.output(net.output_names()[0]) == wants[i]).all():
+                        wrong.append((i, turn))
+                net.close()
+        except Exception as e:  # (an assertion in a thread would go unseen)
+            wrong.append((i, repr(e)))
+
+    threads = [threading.Thread(target=work, args=(i,)) for i in range(2)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert not wrong
+
+
 def test_two_networks_share_one_runtime_arena(oracle):
     """LITE_share_runtime_memroy (runtime/src/lite/network.c:285-303 in the reference): both
     networks lay their tensors into one arena sized for the larger; used one after the other
