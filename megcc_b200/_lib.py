@@ -124,9 +124,8 @@ def lib():
 # the functions behind the operator calls of a program's inner loop
 FAST = ("mb200_conv_bias_qs8_nhwc", "mb200_conv_bias_qs8_nhwc_fused", "mb200_conv_bias_qs8_nchw",
         "mb200_matmul_s8_qs8", "mb200_qelemwise_qs8", "mb200_conv_bias_f32_nhwc",
-        "mb200_conv_bias_qs8_nchw_workspace", "mb200_conv_f32_workspace_bytes",
-        "mb200_matmul_f32_packed_b_bytes", "mb200_matmul_f32_pack_b",
-        "mb200_matmul_f32_workspace_bytes", "mb200_matmul_f32", "mb200_elemwise_f32")
+        "mb200_conv_bias_qs8_nchw_workspace", "mb200_matmul_f32_packed_b_bytes",
+        "mb200_matmul_f32_pack_b", "mb200_matmul_f32", "mb200_elemwise_f32")
 _fast = None
 
 

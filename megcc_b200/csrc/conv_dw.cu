@@ -21,6 +21,7 @@
 #include "internal.h"
 #include "pdl.h"
 #include "tuning.h"
+#include "umma_ptx.cuh"
 
 namespace mb200 {
 
@@ -418,14 +419,14 @@ int launch_conv_dw(
     const size_t work = (size_t)a.m * p.c16;
     // While a thread per 4 outputs still fits the GPU at once (2048 threads on each SM), the
     // shortest thread wins; beyond that the instructions per output decide.
-    if (tuning().dw_out == 0 && !tuning().dw_one_output && work * 4 <= (size_t)148 * 2048 &&
+    if (tuning().dw_out == 0 && !tuning().dw_one_output && work * 4 <= (size_t)umma::sm_count() * 2048 &&
         ((uintptr_t)flt & 3) == 0) {
         launch_pdl(conv_dw3x3_quad_kernel, dim3((unsigned)((work * 4 + 127) / 128)), dim3(128), 0, st,
                    p, (const uint32_t*)src, (const uint32_t*)flt, bias, flt_scales, (uint32_t*)dst);
         return check_launch("conv_dw_quad");
     }
     size_t grid = (work + 255) / 256;
-    const size_t cap = (size_t)148 * 8;
+    const size_t cap = (size_t)umma::sm_count() * 8;
     if (grid > cap)
         grid = cap;
     if (grid < 1)
@@ -443,7 +444,7 @@ int launch_conv_dw(
         const int outs = forced == 4 ? 4 : 2;
         const size_t items = (size_t)a.n * a.oh * ((a.ow + outs - 1) / outs) * p.c16;
         size_t blocks = (items + 127) / 128;
-        const size_t most = (size_t)148 * 16;
+        const size_t most = (size_t)umma::sm_count() * 16;
         if (blocks > most)
             blocks = most;
         if (blocks < 1)

@@ -1121,11 +1121,6 @@ bool conv_f32_umma_supported(const ConvF32Args& a, const float* src, const float
     return plain_matrix(a) || f32_descriptor_images(a, src) != 0;
 }
 
-size_t conv_f32_workspace_bytes(const ConvF32Args& a) {
-    (void)a;  // the activation is split into its tf32 planes in shared memory
-    return 0;
-}
-
 int launch_conv_f32_pack_filter_split(
         const ConvF32Args& a, const float* flt_oihw, float* out, cudaStream_t st) {
     const int icp = conv_f32_padded_ic(a.ic);
@@ -1167,11 +1162,10 @@ int launch_conv_f32_direct(
 
 int launch_conv_f32_umma(
         const ConvF32Args& a, const float* src, const float* flt_split, const float* bias,
-        const float* z, float* dst, void* workspace, cudaStream_t st) {
+        const float* z, float* dst, cudaStream_t st) {
     const DriverApi& api = driver_api();
     if (!api.ok)
         return set_error(ST_RUNTIME, "cuTensorMapEncode* entry points not found in the driver");
-    (void)workspace;  // the operands are split in shared memory: no scratch tensor
     if ((uintptr_t)flt_split & 15)
         return set_error(ST_INVALID_LAYOUT, "the filter must be 16-byte aligned");
 

@@ -232,7 +232,6 @@ __global__ void __launch_bounds__(64 + 32 * EW, EW == 16 ? 1 : 2) conv_patch_ker
     const int m_first = blockIdx.x / p.n_tiles;
     const int m_step = gridDim.x / p.n_tiles;
     const int n0 = tile_n * BN;
-    const int plane = p.plane_stride;
 
     if (threadIdx.x == 0) {
         for (int s = 0; s < kMaxStages; ++s) {

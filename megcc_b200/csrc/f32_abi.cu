@@ -62,7 +62,7 @@ namespace mb200 {
 int conv_bias_f32_pitched(
         const mb200_conv_f32_param* p, const float* src, long long src_pitch,
         const float* flt_packed, const float* bias, const float* z, long long z_pitch, float* dst,
-        long long dst_pitch, void* workspace, size_t workspace_bytes, int algo, cudaStream_t st) {
+        long long dst_pitch, int algo, cudaStream_t st) {
     ConvF32Args a{};
     int rc = make_f32_args(p, dst_pitch, &a);
     if (rc)
@@ -77,16 +77,14 @@ int conv_bias_f32_pitched(
          (uintptr_t)z) & 3)
         return set_error(ST_INVALID_LAYOUT, "fp32 operands must be 4-byte aligned");
     const bool umma_ok = conv_f32_umma_supported(a, src, dst) &&
-                         workspace_bytes >= conv_f32_workspace_bytes(a) &&
-                         (((uintptr_t)workspace | (uintptr_t)flt_packed | (uintptr_t)bias |
-                           (uintptr_t)z) & 15) == 0;
+                         (((uintptr_t)flt_packed | (uintptr_t)bias | (uintptr_t)z) & 15) == 0;
     if (algo == MB200_ALGO_UMMA && !umma_ok)
         return set_error(ST_NO_IMPLEMENT,
                          "tensor-core fp32 ConvBias needs a dense filter, ic %% 4 == 0 (with a spatial "
                          "filter ic == 16 or ic >= 32), 16-byte aligned operands and, with a spatial "
                          "filter, >= 128 KiB of readable memory from the input on");
     if (algo == MB200_ALGO_UMMA || (algo == MB200_ALGO_AUTO && umma_ok))
-        return launch_conv_f32_umma(a, src, flt_packed, bias, z, dst, workspace, st);
+        return launch_conv_f32_umma(a, src, flt_packed, bias, z, dst, st);
     if (algo != MB200_ALGO_AUTO && algo != MB200_ALGO_DIRECT)
         return set_error(ST_OUT_OF_RANGE, "unknown algo %d", algo);
     return launch_conv_f32_direct(a, src, flt_packed, bias, z, dst, st);
@@ -119,19 +117,18 @@ int mb200_conv_f32_pack_filter(
                                       : launch_conv_f32_pack_filter_plain(a, flt_oihw, flt_packed, st);
 }
 
-size_t mb200_conv_f32_workspace_bytes(const mb200_conv_f32_param* p) {
-    ConvF32Args a{};
-    if (make_f32_args(p, 0, &a))
-        return 0;
-    return conv_f32_split_eligible(a) ? up256(conv_f32_workspace_bytes(a)) : 0;
+// (kept, like the workspace arguments, for callers of earlier versions: the operands are split on
+// chip, no scratch is used)
+size_t mb200_conv_f32_workspace_bytes(const mb200_conv_f32_param*) {
+    return 0;
 }
 
 int mb200_conv_bias_f32_nhwc(
         const mb200_conv_f32_param* p, const float* src, const float* flt_packed,
-        const float* bias, const float* z, float* dst, long long dst_pitch, void* workspace,
-        size_t workspace_bytes, int algo, void* stream) {
-    return conv_bias_f32_pitched(p, src, 0, flt_packed, bias, z, 0, dst, dst_pitch, workspace,
-                                 workspace_bytes, algo, (cudaStream_t)stream);
+        const float* bias, const float* z, float* dst, long long dst_pitch, void*, size_t, int algo,
+        void* stream) {
+    return conv_bias_f32_pitched(p, src, 0, flt_packed, bias, z, 0, dst, dst_pitch, algo,
+                                 (cudaStream_t)stream);
 }
 
 // ---- fp32 matrix product: a 1x1 ConvBias over M "pixels" with K channels ----
@@ -175,24 +172,21 @@ int mb200_matmul_f32_pack_b(int k, int n, const float* b, float* b_packed, void*
                                       : launch_transpose_f32(b, b_packed, 1, k, n, st);
 }
 
-size_t mb200_matmul_f32_workspace_bytes(int m, int k) {
-    mb200_conv_f32_param p;
-    if (matmul_f32_param(m, 1, k, &p))
-        return 0;
-    return mb200_conv_f32_workspace_bytes(&p);
+size_t mb200_matmul_f32_workspace_bytes(int, int) {
+    return 0;
 }
 
 int mb200_matmul_f32(
-        int m, int n, int k, const float* a, const float* b_packed, float* c, void* workspace,
-        size_t workspace_bytes, void* stream) {
+        int m, int n, int k, const float* a, const float* b_packed, float* c, void*, size_t,
+        void* stream) {
     mb200_conv_f32_param p;
     int rc = matmul_f32_param(m, n, k, &p);
     if (rc)
         return rc;
     if (!a || !b_packed || !c)
         return set_error(ST_NULL_PTR, "matmul operand pointer is NULL");
-    return mb200_conv_bias_f32_nhwc(&p, a, b_packed, nullptr, nullptr, c, 0, workspace,
-                                    workspace_bytes, MB200_ALGO_AUTO, stream);
+    return mb200_conv_bias_f32_nhwc(&p, a, b_packed, nullptr, nullptr, c, 0, nullptr, 0,
+                                    MB200_ALGO_AUTO, stream);
 }
 
 int mb200_elemwise_f32(

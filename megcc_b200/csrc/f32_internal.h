@@ -26,7 +26,6 @@ int conv_f32_padded_ic(int ic);
 bool conv_f32_split_eligible(const ConvF32Args& a);
 size_t conv_f32_split_filter_floats(const ConvF32Args& a);
 bool conv_f32_umma_supported(const ConvF32Args& a, const float* src, const float* dst);
-size_t conv_f32_workspace_bytes(const ConvF32Args& a);
 int launch_conv_f32_pack_filter_split(
         const ConvF32Args& a, const float* flt_oihw, float* out, cudaStream_t st);
 int launch_conv_f32_pack_filter_plain(
@@ -38,7 +37,7 @@ int launch_conv_f32_direct(
         const float* z, float* dst, cudaStream_t st);
 int launch_conv_f32_umma(
         const ConvF32Args& a, const float* src, const float* flt_split, const float* bias,
-        const float* z, float* dst, void* workspace, cudaStream_t st);
+        const float* z, float* dst, cudaStream_t st);
 
 int launch_elemwise_f32(
         int mode, const float* a, const float* b, float* dst, size_t nr_elem, cudaStream_t st);
@@ -57,7 +56,7 @@ int launch_pooling_f32(
 int conv_bias_f32_pitched(
         const mb200_conv_f32_param* p, const float* src, long long src_pitch,
         const float* flt_packed, const float* bias, const float* z, long long z_pitch, float* dst,
-        long long dst_pitch, void* workspace, size_t workspace_bytes, int algo, cudaStream_t st);
+        long long dst_pitch, int algo, cudaStream_t st);
 int launch_focus_f32(
         const float* src_nchw, float* dst_nhwc, int n, int c, int h, int w, int c_out,
         cudaStream_t st);

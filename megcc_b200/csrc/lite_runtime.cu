@@ -739,7 +739,7 @@ TinyNNStatus builtin_kernel(
                     &p, (const float*)inputs[0]->ptr, pixel_pitch(inputs[0]),
                     (const float*)inputs[1]->ptr, bias, z,
                     z ? pixel_pitch(inputs[nr_input - 1]) : 0, (float*)dst->ptr, pixel_pitch(dst),
-                    ws->ptr, ws->size, MB200_ALGO_AUTO, (cudaStream_t)st);
+                    MB200_ALGO_AUTO, (cudaStream_t)st);
         }
         case OP_MATMUL_F32: {
             const Tensor* a = inputs[0];

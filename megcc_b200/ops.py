@@ -228,10 +228,8 @@ def conv_bias_f32_nhwc(p, src, flt_packed, bias=None, z=None, dst=None, dst_pitc
         oh = (p.ih + 2 * p.pad_h - p.kh) // p.stride_h + 1
         ow = (p.iw + 2 * p.pad_w - p.kw) // p.stride_w + 1
         dst = src.new_empty((p.n, oh, ow, p.oc), dtype=torch.float32)
-    nbytes = f.mb200_conv_f32_workspace_bytes(at)
-    keep, ws = _scratch(nbytes, src.device)
     check(f.mb200_conv_bias_f32_nhwc(
-        at, _ptr(src), _ptr(flt_packed), _ptr(bias), _ptr(z), _ptr(dst), dst_pitch, ws, nbytes,
+        at, _ptr(src), _ptr(flt_packed), _ptr(bias), _ptr(z), _ptr(dst), dst_pitch, None, 0,
         ALGO[algo], _stream()))
     return dst
 
@@ -244,9 +242,7 @@ def matmul_f32(a, b):
     packed = a.new_empty(f.mb200_matmul_f32_packed_b_bytes(k, n) // 4, dtype=torch.float32)
     check(f.mb200_matmul_f32_pack_b(k, n, _ptr(b), _ptr(packed), st))
     c = a.new_empty((m, n), dtype=torch.float32)
-    nbytes = f.mb200_matmul_f32_workspace_bytes(m, k)
-    keep, ws = _scratch(nbytes, a.device)
-    check(f.mb200_matmul_f32(m, n, k, _ptr(a), _ptr(packed), _ptr(c), ws, nbytes, st))
+    check(f.mb200_matmul_f32(m, n, k, _ptr(a), _ptr(packed), _ptr(c), None, 0, st))
     return c
 
 
