@@ -87,13 +87,15 @@ MB200_API const char* mb200_version(void);
 /* text of the last error raised on the calling thread ("" if none) */
 MB200_API const char* mb200_last_error(void);
 /* Kernel-selection switches for experiments and tests (the library's own choices are the
- * defaults): "conv_bn" 0|128|256, "conv_pair" 0|1, "conv_splitk" 0|2..4, "wide128" 1|0,
- * "patch_ctas" 0|1..3, "patch_alone" 0|1, "patch_plain" 0|1, "dw_out" 0|2|4,
- * "dw_one_output" 0|1, "fast_requant" 1|0, "debug" 0|1, "pdl" 1|0 (programmatic dependent
- * launch of consecutive kernels). Their initial values come from the
- * environment variables of the same meaning (MB200_CONV_BN, ...), read ONCE per process; no
- * launch consults the environment. Every setting yields bit-identical results. Process-wide,
- * not thread-safe against concurrent launches. */
+ * defaults): "conv_bn" 0|64|128|256, "conv_pair" 0|1, "conv_splitk" 0|2..4, "conv_csplit" 0|1|2|4|8
+ * (CTAs of a cluster that share a tile's K loop), "wide128" 1|0, "patch_ctas" 0|1..3,
+ * "patch_alone" 0|1, "patch_plain" 0|1, "epilogue_forms" 1|0, "dw_tensor" 1|0, "dw_out" 0|2|4,
+ * "dw_one_output" 0|1, "fast_requant" 1|0, "f32_bn" 0|32|64|128, "f32_split" 0|1|2|4|8, "debug" 0|1,
+ * "pdl" 1|0 (programmatic dependent launch of consecutive kernels). Their initial values come from
+ * the environment variables of the same meaning (MB200_CONV_BN, ...), read ONCE per process; no
+ * launch consults the environment. Every setting yields bit-identical int8 results; the two of the
+ * fp32 kernel change the order of its sums. Process-wide, not thread-safe against concurrent
+ * launches. */
 MB200_API int mb200_set_option(const char* name, int value);
 MB200_API int mb200_get_option(const char* name, int* value);
 /* Reads and clears the status word that kernels launched on `stream` set when a bounded wait
@@ -253,7 +255,7 @@ MB200_API int mb200_requant_fast_constants(
  * and none for x86 (BareMetal/MatrixMul.cpp:13-23 admits f32/f16), so the arithmetic follows
  * the exact integer definition. B is re-laid once to K-major rows (k*n bytes) by
  * mb200_matmul_pack_b, as a weight's Init step would. Runs on the tensor cores when
- * k % 64 == 0 and A holds at least 128 KiB. ---- */
+ * k % 64 == 0 and the operands are 16-byte aligned, whatever m and n; on the CUDA cores otherwise. ---- */
 MB200_API int mb200_matmul_pack_b(int k, int n, const int8_t* b, int8_t* b_packed, void* stream);
 MB200_API int mb200_matmul_s8_s32(
         int m, int n, int k, const int8_t* a, const int8_t* b_packed, int32_t* c, void* stream);
@@ -313,7 +315,9 @@ MB200_API int mb200_relayout_nhwc_to_nchw_s8(
  * fp32 path (the detector configuration and the fp32 MatrixMul sweep). NHWC fp32 tensors,
  * 4-byte aligned at least; the vector and tensor-core paths want 16 bytes and fall back to
  * scalar kernels otherwise. Results agree with the reference's x86 kernels within 1e-4
- * relative / 1e-5 absolute (fp32 sums in a different order), not bit for bit.
+ * relative / 1e-5 absolute (fp32 sums in a different order), not bit for bit, for finite operands:
+ * the tensor-core path multiplies the two halves of a split value, and an infinity, whose second
+ * half is a NaN, gives NaN there.
  * ====================================================================================== */
 
 /* nonlineMode of an fp32 ConvBias. The reference's fp32 ConvBias kernels take IDENTITY / RELU /
@@ -338,10 +342,10 @@ typedef struct mb200_conv_f32_param {
 /* ---- ConvBias fp32 (replaces GI_kernel_conv2d_im2col_<k>x<k>_NCHW_DENSE_..._f32,
  * compiler/lib/KernelGen/GeneralIntrinsic/ConvKernel/Fp32Im2col.cpp:88-120, body :198-217).
  * The Init step (mb200_conv_f32_pack_filter) turns the OIHW filter into the K-major form
- * [OC][KH][KW][ICpg] followed, for dense filters whose channel count fills whole TMA rows (16
- * or a multiple of 32), by its two tf32 planes for the tensor cores. The activation is split
- * into its planes in shared memory, so the ConvBias needs no scratch:
- * mb200_conv_f32_workspace_bytes(p) answers 0 and `workspace` may be NULL (both are kept so
+ * [OC][KH][KW][ICpg], or, for dense filters with ic % 4 == 0 (with a spatial filter ic == 16 or
+ * ic >= 32), to its two tf32 planes for the tensor cores, channels padded to whole rows. The
+ * activation is split into its planes on chip, so the ConvBias needs no scratch:
+ * mb200_conv_f32_workspace_bytes(p) answers 0 and `workspace` is not looked at (both are kept so
  * that callers written against earlier versions keep working).
  *   bias   [OC] floats or NULL
  *   z      optional NHWC tensor of the output's shape added AFTER the activation (the shortcut
@@ -362,8 +366,8 @@ MB200_API int mb200_conv_bias_f32_nhwc(
  * GI_kernel_fp32_matmul_4x12_nn, compiler/lib/KernelGen/GeneralIntrinsic/MatMulKernel/
  * Fp32MatMulM4N12.cpp:8-160). B is prepared once by mb200_matmul_f32_pack_b into
  * mb200_matmul_f32_packed_b_bytes(k, n) bytes; the product needs no scratch
- * (mb200_matmul_f32_workspace_bytes answers 0). Tensor cores (three tf32 passes)
- * when k % 32 == 0 (or k == 16) and A holds at least 128 KiB. */
+ * (mb200_matmul_f32_workspace_bytes answers 0). Tensor cores (three tf32 passes) when k % 4 == 0 and
+ * the operands are 16-byte aligned, whatever m and n; CUDA cores otherwise. */
 MB200_API size_t mb200_matmul_f32_packed_b_bytes(int k, int n);
 MB200_API int mb200_matmul_f32_pack_b(int k, int n, const float* b, float* b_packed, void* stream);
 MB200_API size_t mb200_matmul_f32_workspace_bytes(int m, int k);

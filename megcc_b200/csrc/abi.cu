@@ -223,7 +223,9 @@ bool within(const Ranges& ranges, const void* p, size_t bytes) {
 
 // ConvArgs::params_early of operands that the caller handed in
 int params_early(const void* flt, const void* bias, const void* flt_scales) {
-    return (is_constant(flt) ? 1 : 0) | (is_constant(bias) && is_constant(flt_scales) ? 2 : 0);
+    if (!is_constant(flt))
+        return 0;
+    return is_constant(bias) && is_constant(flt_scales) ? 3 : 1;
 }
 }  // namespace
 
@@ -468,8 +470,9 @@ static int conv_bias_nhwc(
         return launch_conv_patch(a, src, flt_packed, bias, flt_scales, dst, st);
     if (algo == MB200_ALGO_UMMA && !umma_ok)
         return set_error(ST_NO_IMPLEMENT,
-                         "tensor-core ConvBias needs dense, NHWC, ic %% 64 == 0, oc %% 8 == 0, "
-                         "16-byte aligned tensors and >= 128 KiB of input");
+                         "tensor-core ConvBias needs dense, NHWC, ic %% 64 == 0, 16-byte aligned "
+                         "tensors and, with a spatial filter or a stride, >= 128 KiB of readable "
+                         "memory from the input on");
     if (algo == MB200_ALGO_UMMA || (algo == MB200_ALGO_AUTO && umma_ok))
         return launch_conv_umma(a, src, flt_packed, bias, flt_scales, dst, st);
     if (algo != MB200_ALGO_AUTO && algo != MB200_ALGO_DIRECT)

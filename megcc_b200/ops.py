@@ -12,6 +12,7 @@ from ._lib import ConvF32Param, ConvFuse, ConvParam, check, fast, lib
 ACT = {"IDENTITY": 0, "RELU": 1, "H_SWISH": 2}
 POOL = {"MAX": 0, "AVERAGE": 1, "AVERAGE_COUNT_EXCLUDE_PADDING": 2}
 QELEM = {"QADD": 0, "QFUSE_ADD_RELU": 1, "QMUL": 2, "QRELU": 3}
+_S8 = torch.int8  # (a look-up less per call)
 ALGO = {"auto": 0, "direct": 1, "umma": 2, "patch": 3}
 
 
@@ -63,7 +64,7 @@ def conv_bias_qs8_nhwc(p, src, flt_packed, bias, dst=None, flt_scales=None, algo
                        src_is_nchw=False):
     f, at = fast(), _at(p)
     if dst is None:
-        dst = src.new_empty(f.conv_shape(at), dtype=torch.int8)
+        dst = src.new_empty(f.conv_shape(at), dtype=_S8)
     check(f.mb200_conv_bias_qs8_nhwc(
         at, _ptr(src), int(src_is_nchw), _ptr(flt_packed), _ptr(bias), _ptr(flt_scales),
         dst.data_ptr(), ALGO[algo], _stream()))
@@ -74,7 +75,7 @@ def conv_bias_qs8_nhwc_fused(p, src, flt_packed, bias, z, mode, z_scale, out_sca
     """ConvBias (p.nonline must be IDENTITY) followed by QADD / QFUSE_ADD_RELU with the int8
     tensor z of the output's NHWC shape, in one kernel."""
     f, at = fast(), _at(p)
-    dst = src.new_empty(f.conv_shape(at), dtype=torch.int8)
+    dst = src.new_empty(f.conv_shape(at), dtype=_S8)
     fuse = ConvFuse(z.data_ptr(), QELEM[mode], z_scale, out_scale)
     check(f.mb200_conv_bias_qs8_nhwc_fused(
         at, _ptr(src), 0, _ptr(flt_packed), _ptr(bias), None, C.addressof(fuse),
@@ -94,9 +95,9 @@ def conv_bias_qs8_nchw(p, src, flt_oihw, bias, flt_scales=None, algo="auto"):
     """ConvBias in the reference's own layouts (NCHW activations, OIHW filter)."""
     f, at = fast(), _at(p)
     n, oh, ow, oc = f.conv_shape(at)
-    dst = src.new_empty((n, oc, oh, ow), dtype=torch.int8)
+    dst = src.new_empty((n, oc, oh, ow), dtype=_S8)
     nbytes = f.mb200_conv_bias_qs8_nchw_workspace(at)
-    ws = src.new_empty(nbytes + 256, dtype=torch.int8)
+    ws = src.new_empty(nbytes + 256)
     base = ws.data_ptr()
     check(f.mb200_conv_bias_qs8_nchw(
         at, _ptr(src), _ptr(flt_oihw), _ptr(bias), _ptr(flt_scales), dst.data_ptr(),
@@ -123,7 +124,7 @@ def matmul_s8_s32(a, b_packed):
 def matmul_s8_qs8(a, b_packed, acc_scale, dst_scale):
     m, k = a.shape
     n = b_packed.shape[0]
-    c = a.new_empty((m, n), dtype=torch.int8)
+    c = a.new_empty((m, n), dtype=_S8)
     check(fast().mb200_matmul_s8_qs8(m, n, k, _ptr(a), _ptr(b_packed), _ptr(c), acc_scale,
                                      dst_scale, _stream()))
     return c
