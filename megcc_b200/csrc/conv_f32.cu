@@ -611,12 +611,20 @@ __global__ void __launch_bounds__(f32_threads(BN), 1) conv_f32_umma_kernel(
         // 16-byte unit u of row r sits at unit u ^ swz of its row
         const int swz = ROWB == 128 ? (row & 7) : ((row >> 1) & 3);
         const int total_iters = my_tiles * (ke - kb);
+        // With two groups and an odd number of stages a stage passes from group to group, and a
+        // group has not seen the fill before the one it waits for. Where that one is late (its load
+        // overtaken by those behind it), its parity is the one that the wait takes for done, and
+        // the stage's old tile would be converted. So the wait for the MMAs of step g - kT comes
+        // first there: they were issued after every step before them, the fill of step g - stages
+        // among those (five stages or more, kT of at most four).
+        const bool passed_on = kGroups > 1 && (p.stages & 1) != 0;
         int s = group, t = group;
         uint32_t phase = 0, t_phase = 0;
         // ring slot of the step whose MMAs the next t_empty wait is for (g - kT)
         int s_done = group;
         for (int g = group; g < total_iters; g += kGroups) {
-            bool ok = mbar_wait(&full_bar[s], phase, abort_flag, p.wait_cycles);
+            bool ok = !passed_on || mbar_wait(&t_empty[t], t_phase ^ 1u, abort_flag, p.wait_cycles);
+            ok = ok && mbar_wait(&full_bar[s], phase, abort_flag, p.wait_cycles);
             ok = __all_sync(0xffffffffu, ok);
             if (!ok) {
                 give_up(ERR_PRODUCER_WAIT);

@@ -165,6 +165,31 @@ def test_conv_f32_tile_forms_match_oracle(ops, oracle, case):
     assert ops.device_status() == 0
 
 
+@pytest.mark.parametrize("ic,oc,stride", [(32, 64, 2), (64, 32, 1)])
+def test_conv_f32_of_a_whole_batch_is_the_same_every_time(ops, ic, oc, stride):
+    """Layers whose resident filter leaves an odd number of ring stages to two groups of converter
+    warps, on an input far beyond the L2, where a load may be overtaken by those behind it: two
+    thousand launches give the same bits, and they are the general kernel's within the bar."""
+    n, hw = 16, 320
+    g = torch.Generator(device="cuda")
+    g.manual_seed(17)
+    x = torch.randn((n, hw, hw, ic), device="cuda", generator=g)
+    flt = torch.randn((oc, ic, 3, 3), device="cuda", generator=g) / (ic * 9) ** 0.5
+    bias = torch.randn(oc, device="cuda", generator=g)
+    p = ops.conv_f32_param(n, ic, hw, hw, oc, 3, 3, stride, 1, 1, "SILU")
+    packed = ops.pack_filter_f32(p, flt)
+    want = ops.conv_bias_f32_nhwc(p, x, packed, bias, algo="direct")
+    first = ops.conv_bias_f32_nhwc(p, x, packed, bias, algo="umma")
+    assert ((first - want).abs() <= ATOL + RTOL * want.abs()).all()
+    out = torch.empty_like(first)
+    wrong = torch.zeros((), dtype=torch.int64, device="cuda")
+    for _ in range(2000):
+        ops.conv_bias_f32_nhwc(p, x, packed, bias, dst=out, algo="umma")
+        wrong += (out != first).any()
+    assert int(wrong) == 0
+    assert ops.device_status() == 0
+
+
 @pytest.mark.parametrize("shape", [(1000, 1000, 1000), (129, 65, 4100), (77, 31, 999)],
                          ids=["k1000", "k4100_split", "k999_odd"])
 def test_matmul_f32_partial_rows_match_oracle(ops, oracle, shape):
