@@ -616,8 +616,10 @@ __global__ void __launch_bounds__(f32_threads(BN), 1) conv_f32_umma_kernel(
         // overtaken by those behind it), its parity is the one that the wait takes for done, and
         // the stage's old tile would be converted. So the wait for the MMAs of step g - kT comes
         // first there: they were issued after every step before them, the fill of step g - stages
-        // among those (five stages or more, kT of at most four).
-        const bool passed_on = kGroups > 1 && (p.stages & 1) != 0;
+        // among those (kT is at most four, and no launch has three stages). With seven stages the
+        // group's step before this one has waited for as much.
+        const bool passed_on =
+                kGroups > 1 && (p.stages & 1) != 0 && p.stages < C::kTStages + kGroups;
         int s = group, t = group;
         uint32_t phase = 0, t_phase = 0;
         // ring slot of the step whose MMAs the next t_empty wait is for (g - kT)
