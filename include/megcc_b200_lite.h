@@ -185,7 +185,8 @@ LITE_API int mb200_lite_stream(const LiteNetwork network, void** stream);
  * A registered KernelFunc is called for one instruction after the other, in the model's order,
  * with the network's own stream (mb200_lite_stream) and with outputs in device memory: a model
  * that holds one is not captured on parallel branches, and what a registered kernel writes
- * is copied to the host behind it. */
+ * is copied to the host behind it. Weights are constant once the model is loaded: a registered
+ * KernelFunc does not write to them (the library's kernels fetch them ahead of their turn). */
 LITE_API int mb200_lite_set_kernel_tables(
         LiteNetwork network, const void* kernels, int nr_kernels, const void* init_kernels,
         int nr_init);

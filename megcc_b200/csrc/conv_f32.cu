@@ -1054,7 +1054,10 @@ int f32_cluster_capacity(int bn, int rowb, int size) {
 // cost. A tile that is its CTA's only one has nothing to hide its end behind: wide tiles cost
 // more there (128 -> 128 1x1 over 52 x 52: 4.6 us with 32 columns, 5.3 with 64, 7.8 with 128). A
 // split adds the exchange of the partial tiles; it is taken only where the clusters all run at
-// once. (512 -> 128 1x1 over 26 x 26: 5.8 us as 24 tiles split in four, 6.8 as 12 in eight.)
+// once. (512 -> 128 1x1 over 26 x 26: 5.8 us as 24 tiles split in four, 6.8 as 12 in eight.) Over 160
+// layers that are in no network here (16 to 512 channels to 16 to 512, 25 to 20000 pixels) the choice is 2 %
+// on average behind the best of all widths and splits; one layer (16 -> 85 3x3 over 2 x 13 x 13, unsplit 6.9 us,
+// split 4.5) is 52 % off, all others at most 15 %.
 void choose_f32_tile(int m_tiles, int oc, int k_iters, int rowb, int* bn, int* splits) {
     const int sms = sm_count();
     long long best = -1;
