@@ -23,8 +23,10 @@
  * they were asked for by name (MB200_ALGO_UMMA / _PATCH); MB200_ALGO_AUTO falls back.
  *
  * Order. Every operand, a filter, bias or scales among them, may be the result of earlier calls on
- * the same stream, of this library or another: kernels are launched ahead of the end of the one
- * in front of them, and read nothing that could still be written before that one has completed.
+ * the same stream: kernels are launched ahead of the end of the one in front of them, and read
+ * nothing that it writes before it has completed. That holds for this library's calls and for
+ * kernels launched in the ordinary way; one of another library that releases its successors early
+ * (programmatic dependent launch) must not be the last on the stream to write a filter, bias or scales.
  *
  * Scale range. Results are bit-identical to the reference's x86 kernels for every finite
  * positive scale triple. The vector and tensor-core kernels divide by dst_scale with a

@@ -9,6 +9,7 @@
 #include <mutex>
 
 #include "internal.h"
+#include "pdl.h"
 #include "tuning.h"
 
 namespace mb200 {
@@ -221,13 +222,61 @@ bool within(const Ranges& ranges, const void* p, size_t bytes) {
     return (uintptr_t)p + bytes <= it->first + it->second;
 }
 
-// ConvArgs::params_early of operands that the caller handed in
-int params_early(const void* flt, const void* bias, const void* flt_scales) {
-    if (!is_constant(flt))
-        return 0;
-    return is_constant(bias) && is_constant(flt_scales) ? 3 : 1;
+// One stream's last launch. A slot belongs to the stream that used it last; a stream that finds
+// another's there knows nothing of its own. (A default stream stands for one stream per device or
+// thread: the per-thread one is never known, the legacy one is told apart by its device.)
+struct LastLaunch {
+    std::mutex mu;
+    uintptr_t key = 1;
+    uintptr_t lo = 0, hi = 0;
+};
+LastLaunch g_last_launch[256];
+
+LastLaunch& last_launch_of(cudaStream_t st, uintptr_t* key) {
+    uintptr_t k = (uintptr_t)st;
+    if (!st || st == cudaStreamLegacy) {
+        int dev = 0;
+        cudaGetDevice(&dev);
+        k = ((uintptr_t)dev << 4) | 8;  // (no address of a stream)
+    }
+    *key = k;
+    return g_last_launch[(k * 0x9E3779B97F4A7C15ull) >> 56];
+}
+
+// ConvArgs::params_early of operands that the caller handed in: what is constant, or not written by the
+// last launch, may be fetched ahead of that one's end
+int params_early(
+        const ConvArgs& a, const void* flt, const void* bias, const void* flt_scales, cudaStream_t st) {
+    const size_t flt_bytes = (size_t)a.oc * (a.ic / a.groups) * a.kh * a.kw;
+    const bool flt_early = is_constant(flt) || !last_launch_writes(st, flt, flt_bytes);
+    auto side_early = [&](const void* p) {
+        return is_constant(p) || !last_launch_writes(st, p, (size_t)a.oc * 4);
+    };
+    return (flt_early ? 1 : 0) | (side_early(bias) && side_early(flt_scales) ? 2 : 0);
 }
 }  // namespace
+
+LaunchRecord::LaunchRecord(cudaStream_t st, const Writes& writes) {
+    uintptr_t key;
+    LastLaunch& slot = last_launch_of(st, &key);
+    slot.mu.lock();
+    slot.key = key;
+    slot.lo = (uintptr_t)writes.first;
+    slot.hi = slot.lo + writes.bytes;
+    slot_ = &slot;
+}
+LaunchRecord::~LaunchRecord() {
+    ((LastLaunch*)slot_)->mu.unlock();
+}
+
+bool last_launch_writes(cudaStream_t st, const void* p, size_t bytes) {
+    if (st == cudaStreamPerThread)
+        return true;
+    uintptr_t key;
+    LastLaunch& slot = last_launch_of(st, &key);
+    std::lock_guard<std::mutex> lock(slot.mu);
+    return slot.key != key || ((uintptr_t)p < slot.hi && slot.lo < (uintptr_t)p + bytes);
+}
 
 bool readable_through(const void* p, size_t bytes) {
     return within(g_ranges, p, bytes);
@@ -410,18 +459,22 @@ int mb200_conv_bias_qs8_nhwc_fused(
         const int32_t* bias, const float* flt_scales, const mb200_conv_fuse* fuse, int8_t* dst,
         int algo, void* stream) {
     return conv_bias_nhwc(p, src, src_is_nchw, flt_packed, bias, flt_scales, fuse, dst, algo,
-                          params_early(flt_packed, bias, flt_scales), stream);
+                          -1, stream);
 }
 
 static int conv_bias_nhwc(
         const mb200_conv_param* p, const int8_t* src, int src_is_nchw, const int8_t* flt_packed,
         const int32_t* bias, const float* flt_scales, const mb200_conv_fuse* fuse, int8_t* dst,
-        int algo, int early, void* stream) {
+        int algo, int early, void* stream) {  // early: ConvArgs::params_early, -1: not known
     ConvArgs a{};
     int rc = make_args(p, src_is_nchw, &a);
     if (rc)
         return rc;
-    a.params_early = early;
+    // (asked only for the kernels that make use of it)
+    auto ask_early = [&] {
+        a.params_early = early >= 0 ? early
+                                    : params_early(a, flt_packed, bias, flt_scales, (cudaStream_t)stream);
+    };
     if (fuse) {
         if (!fuse->z)
             return set_error(ST_NULL_PTR, "fused operand z is NULL");
@@ -453,6 +506,7 @@ static int conv_bias_nhwc(
                              "halo-patch depthwise ConvBias needs 3x3, stride 1, channels %% 64 "
                              "== 0 (or 32 channels, even width, padding 1), NHWC, 16-byte aligned "
                              "tensors and >= 128 KiB of input");
+        ask_early();
         return launch_conv_patch_dw(a, src, flt_packed, bias, flt_scales, dst, st);
     }
     const bool patch_ok = side_ok && conv_patch_supported(a, src, flt_packed, dst);
@@ -466,8 +520,10 @@ static int conv_bias_nhwc(
     // kernel measured equal or up to 18 % faster (128 -> 256 channels at 28 x 28, batch 256)
     const bool pointwise = a.kh == 1 && a.kw == 1 && umma_ok;
     if (algo == MB200_ALGO_PATCH ||
-        (algo == MB200_ALGO_AUTO && patch_ok && !pointwise && conv_patch_efficiency(a) >= 0.75f))
+        (algo == MB200_ALGO_AUTO && patch_ok && !pointwise && conv_patch_efficiency(a) >= 0.75f)) {
+        ask_early();
         return launch_conv_patch(a, src, flt_packed, bias, flt_scales, dst, st);
+    }
     if (algo == MB200_ALGO_UMMA && !umma_ok)
         return set_error(ST_NO_IMPLEMENT,
                          "tensor-core ConvBias needs dense, NHWC, ic %% 64 == 0, 16-byte aligned "
@@ -481,11 +537,15 @@ static int conv_bias_nhwc(
     // with a block-diagonal filter (63 of 64 MACs multiply zeros, and it is still the faster
     // form: the CUDA-core kernel below is bound by instruction issue)
     if (algo == MB200_ALGO_AUTO && side_ok && tuning().dw_tensor &&
-        conv_patch_dw_supported(a, src, flt_packed, dst))
+        conv_patch_dw_supported(a, src, flt_packed, dst)) {
+        ask_early();
         return launch_conv_patch_dw(a, src, flt_packed, bias, flt_scales, dst, st);
+    }
     // depthwise 3x3: vector loads and dp4a over taps
-    if (algo == MB200_ALGO_AUTO && side_ok && conv_dw_supported(a, src, flt_packed, dst))
+    if (algo == MB200_ALGO_AUTO && side_ok && conv_dw_supported(a, src, flt_packed, dst)) {
+        ask_early();
         return launch_conv_dw(a, src, flt_packed, bias, flt_scales, dst, st);
+    }
     return launch_conv_direct(a, src, flt_packed, bias, flt_scales, dst, nullptr, st);
 }
 
@@ -578,7 +638,8 @@ int mb200_conv_bias_qs8_s2d(
         return set_error(ST_OUT_OF_RANGE, "workspace of %zu bytes is too small", workspace_bytes);
     if (((uintptr_t)workspace | (uintptr_t)flt_s2d | (uintptr_t)dst) & 15)
         return set_error(ST_INVALID_LAYOUT, "workspace, filter and dst must be 16-byte aligned");
-    a.params_early = params_early(flt_s2d, bias, flt_scales);
+    // (the space-to-depth pass lies between the kernel that fetches it and the last launch: complete)
+    a.params_early = 1;
     return launch_conv_s2d(a, src, flt_s2d, bias, flt_scales, dst, workspace, (cudaStream_t)stream);
 }
 
@@ -607,7 +668,7 @@ int mb200_conv_bias_pool_qs8_s2d(
     if (((uintptr_t)workspace | (uintptr_t)flt_s2d | (uintptr_t)dst) & 15)
         return set_error(ST_INVALID_LAYOUT, "workspace, filter and dst must be 16-byte aligned");
     a.pool = 1;
-    a.params_early = params_early(flt_s2d, bias, flt_scales);
+    a.params_early = 1;  // (likewise)
     return launch_conv_s2d(a, src, flt_s2d, bias, flt_scales, dst, workspace, (cudaStream_t)stream);
 }
 
@@ -644,7 +705,7 @@ int mb200_conv_bias_qs8_nchw(
         int8_t* ws_flt = ws_dst + align_up((size_t)a.m * a.oc, 256);
         int8_t* ws_s2d = ws_flt + align_up(conv_s2d_filter_bytes(a), 256);
         a.src_is_nchw = 1;
-        a.params_early = 1;  // (the filter's packing does not release the kernels behind it early: see pdl.h)
+        a.params_early = 1;
         if ((rc = launch_conv_s2d_pack_filter(a, flt_oihw, ws_flt, st)))
             return rc;
         if ((rc = launch_conv_s2d(a, src, ws_flt, bias, flt_scales, ws_dst, ws_s2d, st)))
@@ -666,9 +727,8 @@ int mb200_conv_bias_qs8_nchw(
     // NCHW -> NHWC is a [C][HW] -> [HW][C] transpose per image
     if ((rc = launch_transpose_pack_s8(src, ws_src, a.n, a.ic, a.ih * a.iw, a, flt_oihw, ws_flt, st)))
         return rc;
-    // (the filter's packing: likewise)
-    if ((rc = conv_bias_nhwc(p, ws_src, 0, ws_flt, bias, flt_scales, nullptr, ws_dst, algo,
-                             1 | params_early(nullptr, bias, flt_scales), st)))
+    // (the kernel that packs the filter does not release the ConvBias: all is complete by then)
+    if ((rc = conv_bias_nhwc(p, ws_src, 0, ws_flt, bias, flt_scales, nullptr, ws_dst, algo, 3, st)))
         return rc;
     return launch_transpose_s8(ws_dst, dst, a.n, a.oh * a.ow, a.oc, st);
 }

@@ -181,7 +181,6 @@ __global__ void __launch_bounds__(128) conv_dw3x3_quad_kernel(
     const ConvArgs& a = p.a;
     const unsigned c4 = (unsigned)p.c16 * 4;
     const unsigned idx = blockIdx.x * blockDim.x + threadIdx.x;
-    pdl_release();
     if (idx >= (unsigned)a.m * c4)
         return;
     const unsigned cq = idx % c4;
@@ -205,6 +204,7 @@ __global__ void __launch_bounds__(128) conv_dw3x3_quad_kernel(
     const int iy0 = oy * a.sh - a.ph, ix0 = ox * a.sw - a.pw;
     const uint32_t* base = src + (size_t)((unsigned)n * a.ih) * a.iw * c4 + cq;
     pdl_wait();
+    pdl_release();
     uint32_t v[9];
 #pragma unroll
     for (int t = 0; t < 9; ++t) {
@@ -417,11 +417,12 @@ int launch_conv_dw(
             p.fast_ops = 0;
     }
     const size_t work = (size_t)a.m * p.c16;
+    const Writes writes{dst, work * 16};
     // While a thread per 4 outputs still fits the GPU at once (2048 threads on each SM), the
     // shortest thread wins; beyond that the instructions per output decide.
     if (tuning().dw_out == 0 && !tuning().dw_one_output && work * 4 <= (size_t)umma::sm_count() * 2048 &&
         ((uintptr_t)flt & 3) == 0) {
-        launch_pdl(conv_dw3x3_quad_kernel, dim3((unsigned)((work * 4 + 127) / 128)), dim3(128), 0, st,
+        launch_pdl(writes, conv_dw3x3_quad_kernel, dim3((unsigned)((work * 4 + 127) / 128)), dim3(128), 0, st,
                    p, (const uint32_t*)src, (const uint32_t*)flt, bias, flt_scales, (uint32_t*)dst);
         return check_launch("conv_dw_quad");
     }
@@ -455,7 +456,7 @@ int launch_conv_dw(
             cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kMostSmem) !=
                     cudaSuccess)
             return check_launch("conv_dw smem attribute");
-        launch_pdl(kernel, dim3((unsigned)blocks), dim3(128), (size_t)smem, st, p, (const uint4*)src,
+        launch_pdl(writes, kernel, dim3((unsigned)blocks), dim3(128), (size_t)smem, st, p, (const uint4*)src,
                    flt, bias, flt_scales, (uint4*)dst);
         return check_launch("conv_dw_row");
     }
@@ -463,7 +464,7 @@ int launch_conv_dw(
         cudaFuncSetAttribute(conv_dw_kernel<3, 3>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                              kMostSmem) != cudaSuccess)
         return check_launch("conv_dw smem attribute");
-    launch_pdl(conv_dw_kernel<3, 3>, dim3((unsigned)grid), dim3(256), (size_t)smem, st, p,
+    launch_pdl(writes, conv_dw_kernel<3, 3>, dim3((unsigned)grid), dim3(256), (size_t)smem, st, p,
                (const uint4*)src, flt, bias, flt_scales, (uint4*)dst);
     return check_launch("conv_dw");
 }

@@ -413,7 +413,6 @@ __global__ void __launch_bounds__(f32_threads(BN), 1) conv_f32_umma_kernel(
     __syncthreads();
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     const uint32_t tmem_base = *tmem_slot;
-    pdl_release();
 
     auto give_up = [&](int code) {
         if (!*abort_flag) {
@@ -441,6 +440,7 @@ __global__ void __launch_bounds__(f32_threads(BN), 1) conv_f32_umma_kernel(
             fx = tap - fy * p.taps_w;
         }
         pdl_wait();  // from here on the kernel touches global memory
+        pdl_release();
         if (p.b_resident) {
             const uint32_t bar = smem_u32(b_full), b0 = smem_u32(tiles_b);
             mbar_expect_tx_if(leader, bar, (uint32_t)(p.k_iters * C::kBBytes));
@@ -1033,7 +1033,7 @@ int launch_f32_kernel(
     if (tuning().debug)
         fprintf(stderr, "conv_f32_umma<%d,%d>: grid %d tiles %d k_iters %d stages %d resident %d "
                 "splits %d\n", BN, ROWB, grid, total, p.k_iters, p.stages, p.b_resident, p.splits);
-    launch_pdl_cluster(conv_f32_umma_kernel<BN, ROWB>, dim3(grid), dim3(f32_threads(BN)),
+    launch_pdl_cluster(Writes{p.ep.dst, (size_t)p.m_total * p.ep.dst_pitch * 4}, conv_f32_umma_kernel<BN, ROWB>, dim3(grid), dim3(f32_threads(BN)),
                        (size_t)C::kDynamic, p.splits, st, ma, mb, p);
     return check_launch("conv_f32_umma");
 }
@@ -1168,7 +1168,7 @@ int launch_conv_f32_direct(
     const bool split = conv_f32_split_eligible(a);
     const int icp = split ? conv_f32_padded_ic(a.ic) : a.ic / a.groups;
     const float* lo = split ? flt_packed + (size_t)a.oc * a.kh * a.kw * icp : nullptr;
-    launch_pdl(conv_f32_direct_kernel, dim3(grid_1d((size_t)a.m * a.oc, 256)), dim3(256), 0, st, a,
+    launch_pdl(Writes{dst, (size_t)a.m * a.dst_pitch * 4}, conv_f32_direct_kernel, dim3(grid_1d((size_t)a.m * a.oc, 256)), dim3(256), 0, st, a,
                src, flt_packed, lo, icp, bias, z, dst);
     return check_launch("conv_f32_direct");
 }

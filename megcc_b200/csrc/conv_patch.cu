@@ -300,7 +300,6 @@ __global__ void __launch_bounds__(64 + 32 * EW, EW == 16 ? 1 : 2) conv_patch_ker
     __syncthreads();
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     const uint32_t tmem_base = *tmem_slot;
-    pdl_release();  // the next kernel may be scheduled onto SMs this one leaves
 
     if (warp == 0) {
         // ---------------- TMA producer ----------------
@@ -327,6 +326,7 @@ __global__ void __launch_bounds__(64 + 32 * EW, EW == 16 ? 1 : 2) conv_patch_ker
                     tma_load_2d(smem_b + kc * (BN * 16), &map_b, b_full, kc * 16, n0);
             }
             pdl_wait();  // activations: only once the previous kernel has completed
+            pdl_release();  // the next kernel may be scheduled onto SMs this one leaves
             int s = 0;
             uint32_t phase = 0;
             PatchWalker at(m_first, p);
@@ -715,7 +715,9 @@ int launch_patch_form(
         fprintf(stderr, "conv_patch<%d,%d,%d,%d,%d,%d,%d,%d>: per_sm %d grid %d m_tiles %d n_tiles %d "
                 "smem %d stages %d b_single_load %d\n", BN, KH, KW, CHUNKS, EW, ROWS, POOL, FORM, per_sm,
                 grid, p.m_tiles, p.n_tiles, smem, p.stages, p.b_single_load);
-    launch_pdl(conv_patch_kernel<BN, KH, KW, CHUNKS, EW, ROWS, POOL, FORM>, dim3(grid), dim3(kThreads),
+    const size_t outputs = (size_t)p.n * p.oh * p.ow * p.oc;
+    const Writes writes = p.ep.acc_out ? Writes{p.ep.acc_out, outputs * 4} : Writes{p.dst, outputs};
+    launch_pdl(writes, conv_patch_kernel<BN, KH, KW, CHUNKS, EW, ROWS, POOL, FORM>, dim3(grid), dim3(kThreads),
                (size_t)smem, st, ma, mb, p);
     return check_launch("conv_patch");
 }

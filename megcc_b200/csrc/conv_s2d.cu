@@ -232,16 +232,17 @@ int launch_conv_s2d(
         sy = (long long)a.iw * a.ic;
         sn = sy * a.ih;
     }
+    const Writes writes{workspace, (size_t)a.n * g.h2 * g.w2 * 16};
     if (a.src_is_nchw && a.ic == 3 && a.iw % 8 == 0 && ((uintptr_t)src & 7) == 0 &&
         g.w2 == a.iw / 2 && (size_t)a.n * g.h2 * g.w2 < (1u << 31)) {
-        launch_pdl(space_to_depth_nchw3_x4_kernel, dim3(grid_for((size_t)a.n * g.h2 * (a.iw / 8))),
+        launch_pdl(writes, space_to_depth_nchw3_x4_kernel, dim3(grid_for((size_t)a.n * g.h2 * (a.iw / 8))),
                    dim3(256), 0, st, src, (uint4*)workspace, a.n, a.ih, a.iw, g.h2);
     } else if (a.src_is_nchw && a.iw % 2 == 0 && ((uintptr_t)src & 1) == 0 && g.w2 == a.iw / 2 &&
                (size_t)a.n * g.h2 * g.w2 < (1u << 31)) {
-        launch_pdl(space_to_depth_nchw2_kernel, dim3(grid_for((size_t)a.n * g.h2 * g.w2)), dim3(256),
+        launch_pdl(writes, space_to_depth_nchw2_kernel, dim3(grid_for((size_t)a.n * g.h2 * g.w2)), dim3(256),
                    0, st, src, (uint4*)workspace, a.n, a.ic, a.ih, a.iw, g.h2, g.w2);
     } else {
-        launch_pdl(space_to_depth_kernel, dim3(grid_for((size_t)a.n * g.h2 * g.w2)), dim3(256), 0, st,
+        launch_pdl(writes, space_to_depth_kernel, dim3(grid_for((size_t)a.n * g.h2 * g.w2)), dim3(256), 0, st,
                    src, (uint4*)workspace, a.n, a.ic, a.ih, a.iw, g.h2, g.w2, sn, sc, sy, sx);
     }
     int rc = check_launch("space_to_depth");

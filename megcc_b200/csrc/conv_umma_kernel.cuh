@@ -172,7 +172,6 @@ __global__ void __launch_bounds__(Shape<BN>::kThreads, Shape<BN>::kMinCtas) conv
     __syncthreads();
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     const uint32_t tmem_base = *tmem_slot;
-    pdl_release();  // set-up done: the next kernel may take the SMs this one leaves free
 
     if (warp == 0) {
         // ---------------- TMA producer ----------------
@@ -199,8 +198,10 @@ __global__ void __launch_bounds__(Shape<BN>::kThreads, Shape<BN>::kMinCtas) conv
                     fy = tap / p.taps_w;
                     fx = tap - fy * p.taps_w;
                 }
-                if (item == first_item)
-                    pdl_wait();  // (the first tile is worked out before the wait)
+                if (item == first_item) {
+                    pdl_wait();     // (the first tile is worked out before the wait)
+                    pdl_release();  // the next kernel may take the SMs this one leaves free
+                }
                 for (int it = w.k0; it < w.k1; ++it) {
                     if (!mbar_wait(&empty_bar[s], phase ^ 1u, abort_flag, p.wait_cycles)) {
                         if (!*abort_flag) {
@@ -603,7 +604,9 @@ int launch_form(
         fprintf(stderr, "conv_umma<%d,%d,%d,%d>: csplit %d per_sm %d grid %d items %d (whole tiles %d, split %d) smem %d\n",
                 BN, GEOM, (int)SPLITK, FORM, p.csplit, per_sm, grid, total, SPLITK ? p.full_tiles : total,
                 SPLITK ? p.split : 1, SmemLayout<BN, GEOM>::kDynamic);
-    launch_pdl_cluster(conv_umma_kernel<BN, GEOM, SPLITK, FORM>, dim3(grid), dim3(kThreads),
+    const size_t outputs = (size_t)p.m_total * p.oc;
+    const Writes writes = p.ep.acc_out ? Writes{p.ep.acc_out, outputs * 4} : Writes{p.dst, outputs};
+    launch_pdl_cluster(writes, conv_umma_kernel<BN, GEOM, SPLITK, FORM>, dim3(grid), dim3(kThreads),
                        (size_t)SmemLayout<BN, GEOM>::kDynamic, p.csplit, st, ma, mb, p);
     return check_launch("conv_umma");
 }

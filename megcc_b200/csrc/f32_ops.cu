@@ -345,7 +345,7 @@ __global__ void __launch_bounds__(256) transpose_f32_kernel(
 int launch_elemwise_f32(
         int mode, const float* a, const float* b, float* dst, size_t nr_elem, cudaStream_t st) {
     const int vec_ok = ((((uintptr_t)a | (uintptr_t)b | (uintptr_t)dst) & 15) == 0) ? 1 : 0;
-    launch_pdl(elemwise_f32_kernel, dim3(grid_for_f32(nr_elem / 4 + 1, 256)), dim3(256), 0, st, mode,
+    launch_pdl(Writes{dst, nr_elem * 4}, elemwise_f32_kernel, dim3(grid_for_f32(nr_elem / 4 + 1, 256)), dim3(256), 0, st, mode,
                a, b, dst, nr_elem, vec_ok);
     return check_launch("elemwise_f32");
 }
@@ -375,7 +375,7 @@ int launch_concat_f32(
     for (int i = 0; i < nr; ++i)
         a.skip[i] = a.skip[i] && a.pitch[i] == a.c_out && nr > 1;
     const size_t work = pixels * (size_t)(a.c_out / (a.vec ? 4 : 1));
-    launch_pdl(concat_f32_kernel, dim3(grid_for_f32(work, 256)), dim3(256), 0, st, a, dst, pixels);
+    launch_pdl(Writes{dst, pixels * a.c_out * 4}, concat_f32_kernel, dim3(grid_for_f32(work, 256)), dim3(256), 0, st, a, dst, pixels);
     return check_launch("concat_f32");
 }
 
@@ -386,7 +386,7 @@ int launch_resize_nearest_f32(
     // scale = (float)out / in, the reference's own float expression
     const float scale_h = (float)oh / ih, scale_w = (float)ow / iw;
     const size_t work = (size_t)n * oh * ow * (c / (vec ? 4 : 1));
-    launch_pdl(resize_nearest_f32_kernel, dim3(grid_for_f32(work, 256)), dim3(256), 0, st, src, dst,
+    launch_pdl(Writes{dst, (size_t)n * oh * ow * dst_pitch * 4}, resize_nearest_f32_kernel, dim3(grid_for_f32(work, 256)), dim3(256), 0, st, src, dst,
                n, c, ih, iw, oh, ow, scale_h, scale_w, vec, (int)src_pitch, (int)dst_pitch);
     return check_launch("resize_nearest_f32");
 }
@@ -397,6 +397,7 @@ int launch_pooling_f32(
     const int oh = (ih + 2 * ph - wh) / sh + 1, ow = (iw + 2 * pw - ww) / sw + 1;
     const int vec = ((c | src_pitch | dst_pitch) % 4 == 0 &&
                      ((((uintptr_t)src | (uintptr_t)dst) & 15) == 0)) ? 1 : 0;
+    const Writes writes{dst, (size_t)n * oh * ow * dst_pitch * 4};
     // Row maxima pay from about a 3 x 3 window on; the image's channels of a CTA, raw and reduced,
     // have to fit shared memory. 32 channels per CTA (128-byte rows) while that gives every SM
     // one, else 8 (a sector).
@@ -411,14 +412,14 @@ int launch_pooling_f32(
             static umma::KernelReady ready;
             if (!ready.smem(maxpool_rows_f32_kernel, (int)kMost))
                 return check_launch("maxpool_rows_f32 smem attribute");
-            launch_pdl(maxpool_rows_f32_kernel, dim3(c / 4 / cv, n), dim3(256), per_cv * cv, st,
+            launch_pdl(writes, maxpool_rows_f32_kernel, dim3(c / 4 / cv, n), dim3(256), per_cv * cv, st,
                        reinterpret_cast<const float4*>(src), reinterpret_cast<float4*>(dst),
                        (int)(src_pitch / 4), (int)(dst_pitch / 4), cv, ih, iw, oh, ow, wh, ww, ph, pw);
             return check_launch("maxpool_rows_f32");
         }
     }
     const size_t work = (size_t)n * oh * ow * (c / (vec ? 4 : 1));
-    launch_pdl(pooling_f32_kernel, dim3(grid_for_f32(work, 256)), dim3(256), 0, st, src, dst, mode, n,
+    launch_pdl(writes, pooling_f32_kernel, dim3(grid_for_f32(work, 256)), dim3(256), 0, st, src, dst, mode, n,
                c, ih, iw, oh, ow, wh, ww, sh, sw, ph, pw, vec, (int)src_pitch, (int)dst_pitch);
     return check_launch("pooling_f32");
 }
@@ -430,11 +431,11 @@ int launch_focus_f32(
     // whole columns of two: an even width and planes that start on 8 bytes; rows of two sectors
     if (c == 3 && c_out == 16 && w % 2 == 0 && h % 2 == 0 && ((uintptr_t)src_nchw & 7) == 0 &&
         ((uintptr_t)dst_nhwc & 31) == 0) {
-        launch_pdl(focus_rgb_f32_kernel, dim3(grid_for_f32(work, 256)), dim3(256), 0, st, src_nchw,
+        launch_pdl(Writes{dst_nhwc, work * 64}, focus_rgb_f32_kernel, dim3(grid_for_f32(work, 256)), dim3(256), 0, st, src_nchw,
                    dst_nhwc, n, h, w);
         return check_launch("focus_rgb_f32");
     }
-    launch_pdl(focus_f32_kernel, dim3(grid_for_f32(work, 256)), dim3(256), 0, st, src_nchw, dst_nhwc,
+    launch_pdl(Writes{dst_nhwc, work * c_out * 4}, focus_f32_kernel, dim3(grid_for_f32(work, 256)), dim3(256), 0, st, src_nchw, dst_nhwc,
                n, c, h, w, c_out);
     return check_launch("focus_f32");
 }
@@ -446,7 +447,7 @@ int launch_transpose_f32(
     if (batch > 65535)
         return set_error(ST_OUT_OF_RANGE, "transpose: batch %d exceeds the grid z limit", batch);
     dim3 grid((cols + 31) / 32, (rows + 31) / 32, batch), block(32, 8);
-    launch_pdl(transpose_f32_kernel, grid, block, 0, st, src, dst, rows, cols);
+    launch_pdl(Writes{dst, (size_t)batch * rows * cols * 4}, transpose_f32_kernel, grid, block, 0, st, src, dst, rows, cols);
     return check_launch("transpose_f32");
 }
 

@@ -561,9 +561,9 @@ __global__ void __launch_bounds__(256) transpose4_s8_kernel(
         int tiles_r, int tiles, const int8_t* __restrict__ flt, int8_t* __restrict__ packed, int oc,
         int icpg, int kh, int kw) {
     __shared__ uint32_t turned[64][17];  // [column][four rows]
+    pdl_wait();
     if (!flt)
         pdl_release();
-    pdl_wait();
     const int t = threadIdx.x;
     if ((int)blockIdx.x >= tiles) {
         const size_t total = (size_t)oc * icpg * kh * kw;
@@ -649,7 +649,7 @@ int launch_pooling(
         (size_t)n * ih * iw * (c / 16) < (1u << 30) && oh > 0 && ow > 0) {
         // a window with no valid element cannot occur: padding is below the window size
         const size_t pairs = (size_t)n * oh * ((ow + 1) / 2) * (c / 16);
-        launch_pdl(pooling_max_3x3s2_vec16_kernel, dim3(grid_for(pairs, 256)), dim3(256), 0, st,
+        launch_pdl(Writes{dst, total}, pooling_max_3x3s2_vec16_kernel, dim3(grid_for(pairs, 256)), dim3(256), 0, st,
                    (const uint4*)src, (uint4*)dst, n, c / 16, ih, iw, oh, ow, ph, pw);
         return check_launch("pooling_max_3x3s2_vec16");
     }
@@ -659,20 +659,20 @@ int launch_pooling(
         const size_t work = (size_t)n * (c / 16);
         const int per_image = (c / 16 + 31) / 32;
         if (ih * iw >= 8 && (size_t)n * per_image < (1u << 30)) {
-            launch_pdl(pooling_global_avg_split_kernel, dim3(n * per_image), dim3(128), 0, st,
+            launch_pdl(Writes{dst, total}, pooling_global_avg_split_kernel, dim3(n * per_image), dim3(128), 0, st,
                        (const uint4*)src, (uint32_t*)dst, c / 16, ih * iw, per_image);
             return check_launch("pooling_global_avg_split");
         }
-        launch_pdl(pooling_global_avg_vec16_kernel, dim3(grid_for(work, 64)), dim3(64), 0, st,
+        launch_pdl(Writes{dst, total}, pooling_global_avg_vec16_kernel, dim3(grid_for(work, 64)), dim3(64), 0, st,
                    (const uint4*)src, (uint4*)dst, n, c / 16, ih * iw);
         return check_launch("pooling_global_avg_vec16");
     }
     if (vec16) {
-        launch_pdl(pooling_max_vec16_kernel, dim3(grid_for(total / 16, 256)), dim3(256), 0, st,
+        launch_pdl(Writes{dst, total}, pooling_max_vec16_kernel, dim3(grid_for(total / 16, 256)), dim3(256), 0, st,
                    (const uint4*)src, (uint4*)dst, n, c / 16, ih, iw, oh, ow, wh, ww, sh, sw, ph, pw);
         return check_launch("pooling_max_vec16");
     }
-    launch_pdl(pooling_kernel, dim3(grid_for(total, 256)), dim3(256), 0, st, src, dst, mode, n, c, ih,
+    launch_pdl(Writes{dst, total}, pooling_kernel, dim3(grid_for(total, 256)), dim3(256), 0, st, src, dst, mode, n, c, ih,
                iw, oh, ow, wh, ww, sh, sw, ph, pw);
     return check_launch("pooling");
 }
@@ -687,7 +687,7 @@ int launch_qelemwise(
     volatile float scale_mul = t * scale_div;
     const int vec_ok = (((uintptr_t)a | (uintptr_t)b | (uintptr_t)dst) & 15) == 0;
     const size_t work = nr_elem / 16 + 1;
-    launch_pdl(qelemwise_kernel, dim3(grid_for(work, 256)), dim3(256), 0, st,
+    launch_pdl(Writes{dst, nr_elem}, qelemwise_kernel, dim3(grid_for(work, 256)), dim3(256), 0, st,
                a, b, dst, mode, nr_elem, s0, s1, scale_div, scale_mul, vec_ok);
     return check_launch("qelemwise");
 }
@@ -698,7 +698,7 @@ int launch_qelemwise_bcast(
     volatile float scale_div = 1.f / s_dst;
     volatile float t = s0 * s1;
     volatile float scale_mul = t * scale_div;
-    launch_pdl(qelemwise_bcast_kernel, dim3(grid_for(nr_elem, 256)), dim3(256), 0, st, a, b, dst,
+    launch_pdl(Writes{dst, nr_elem}, qelemwise_bcast_kernel, dim3(grid_for(nr_elem, 256)), dim3(256), 0, st, a, b, dst,
                mode, nr_elem, channels, inner ? inner : 1u, s0, s1, (float)scale_div,
                (float)scale_mul);
     return check_launch("qelemwise_bcast");
@@ -708,7 +708,7 @@ int launch_typecvt_f32_qs8(
         const float* src, int8_t* dst, size_t nr_elem, float s_src, float s_dst, cudaStream_t st) {
     (void)s_src;  // a float tensor's scale counts as 1 (GeneralIntrinsic/Typecvt.cpp:56-69)
     volatile float scale = 1.f / s_dst;
-    launch_pdl(typecvt_f32_qs8_kernel, dim3(grid_for(nr_elem, 256)), dim3(256), 0, st, src, dst,
+    launch_pdl(Writes{dst, nr_elem}, typecvt_f32_qs8_kernel, dim3(grid_for(nr_elem, 256)), dim3(256), 0, st, src, dst,
                nr_elem, (float)scale);
     return check_launch("typecvt_f32_qs8");
 }
@@ -717,7 +717,7 @@ int launch_typecvt_qs8_f32(
         const int8_t* src, float* dst, size_t nr_elem, float s_src, float s_dst, cudaStream_t st) {
     (void)s_dst;  // a float tensor's scale counts as 1
     volatile float scale = s_src / 1.f;
-    launch_pdl(typecvt_qs8_f32_kernel, dim3(grid_for(nr_elem, 256)), dim3(256), 0, st, src, dst,
+    launch_pdl(Writes{dst, nr_elem * 4}, typecvt_qs8_f32_kernel, dim3(grid_for(nr_elem, 256)), dim3(256), 0, st, src, dst,
                nr_elem, (float)scale);
     return check_launch("typecvt_qs8_f32");
 }
@@ -734,7 +734,7 @@ int launch_copy_bytes(const void* src, void* dst, size_t bytes, cudaStream_t st)
     if (bytes == 0)
         return 0;
     const int vec_ok = ((((uintptr_t)src | (uintptr_t)dst) & 15) == 0) ? 1 : 0;
-    launch_pdl(copy_bytes_kernel, dim3(grid_for(vec_ok ? bytes / 16 + 15 : bytes, 256)), dim3(256), 0,
+    launch_pdl(Writes{dst, bytes}, copy_bytes_kernel, dim3(grid_for(vec_ok ? bytes / 16 + 15 : bytes, 256)), dim3(256), 0,
                st, (const uint8_t*)src, (uint8_t*)dst, bytes, vec_ok);
     return check_launch("copy_bytes");
 }
@@ -757,7 +757,8 @@ int launch_transpose_pack_s8(
     const int tc = (cols + 63) / 64, tr = (rows + 63) / 64, tiles = tc * tr * batch;
     const int icpg = a.ic / a.groups;
     const int packers = grid_for((size_t)a.oc * icpg * a.kh * a.kw, 256);
-    launch_pdl(transpose4_s8_kernel, dim3(tiles + packers), dim3(256), 0, st, src, dst, rows, cols, tc,
+    // (it packs the filter as well, but does not release its successor)
+    launch_pdl(Writes{dst, (size_t)batch * rows * cols}, transpose4_s8_kernel, dim3(tiles + packers), dim3(256), 0, st, src, dst, rows, cols, tc,
                tr, tiles, flt, packed, a.oc, icpg, a.kh, a.kw);
     return check_launch("transpose_pack_s8");
 }
@@ -770,12 +771,12 @@ int launch_transpose_s8(
         return set_error(4, "transpose: batch %d exceeds the grid z limit", batch);
     if (transpose_by_words(src, dst, batch, rows, cols)) {
         const int tc = (cols + 63) / 64, tr = (rows + 63) / 64, tiles = tc * tr * batch;
-        launch_pdl(transpose4_s8_kernel, dim3(tiles), dim3(256), 0, st, src, dst, rows, cols, tc, tr,
+        launch_pdl(Writes{dst, (size_t)batch * rows * cols}, transpose4_s8_kernel, dim3(tiles), dim3(256), 0, st, src, dst, rows, cols, tc, tr,
                    tiles, (const int8_t*)nullptr, (int8_t*)nullptr, 0, 1, 1, 1);
         return check_launch("transpose4_s8");
     }
     dim3 grid((cols + 31) / 32, (rows + 31) / 32, batch), block(32, 8);
-    launch_pdl(transpose_s8_kernel, grid, block, 0, st, src, dst, rows, cols);
+    launch_pdl(Writes{dst, (size_t)batch * rows * cols}, transpose_s8_kernel, grid, block, 0, st, src, dst, rows, cols);
     return check_launch("transpose_s8");
 }
 

@@ -4,12 +4,12 @@
 // prefetch) and then block in pdl_wait() until the predecessor has completed and its writes
 // are visible. That hides the launch latency and the ramp of each of the 20-odd kernels of a
 // network behind the tail of the previous one. A kernel launched this way reads and writes no
-// global memory before pdl_wait(), with one exception: operands that no kernel in flight writes.
-// Those are what the launch was told so of (ConvArgs::params_early): a network's weights, and a
-// filter that the call itself has packed with a kernel that does not release early. "The previous
-// kernel" is not enough: a kernel that releases its successor before its own wait lets the third
-// start while the first still runs. A kernel launched without the attribute executes the two
-// instructions as no-ops.
+// global memory before pdl_wait(), with one exception: operands that no kernel in flight writes, as
+// the launch was told (ConvArgs::params_early). And it releases its successor only behind its own
+// pdl_wait(): so when a kernel starts, all but the one in front of it have completed, and what
+// that one writes is what its launch recorded (last_launch_writes). A kernel launched without the
+// attribute executes the two instructions as no-ops, and one that never releases is complete when
+// its successor starts.
 #pragma once
 #include <cuda_runtime.h>
 
@@ -21,7 +21,7 @@ namespace mb200 {
 
 #if defined(__CUDACC__)
 // Releases the NEXT kernel for scheduling (it still waits for this one to complete before it
-// touches memory), then waits for the PREVIOUS kernel's completion.
+// touches memory); only behind a pdl_wait().
 __device__ __forceinline__ void pdl_release() {
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
 }
@@ -29,14 +29,33 @@ __device__ __forceinline__ void pdl_wait() {
     asm volatile("griddepcontrol.wait;" ::: "memory");
 }
 __device__ __forceinline__ void pdl_start() {
-    pdl_release();
     pdl_wait();
+    pdl_release();
 }
 #endif
 
+// the memory that a launch writes
+struct Writes {
+    const void* first;
+    size_t bytes;
+};
+
+// What the library's last launch on a stream writes, kept per stream (abi.cu). Held for the launch,
+// so that records come in the order of the launches.
+class LaunchRecord {
+public:
+    LaunchRecord(cudaStream_t st, const Writes& writes);
+    ~LaunchRecord();
+
+private:
+    void* slot_;
+};
+// May the last launch on the stream write any of these bytes? (true where it is not known)
+bool last_launch_writes(cudaStream_t st, const void* p, size_t bytes);
+
 template <class... KArgs, class... Args>
 inline cudaError_t launch_pdl(
-        void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t st,
+        const Writes& writes, void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t st,
         Args&&... args) {
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = grid;
@@ -48,13 +67,14 @@ inline cudaError_t launch_pdl(
     attr[0].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
     cfg.numAttrs = tuning().pdl ? 1 : 0;
+    LaunchRecord record(st, writes);
     return cudaLaunchKernelEx(&cfg, kernel, std::forward<Args>(args)...);
 }
 
 // The same with `cluster` consecutive CTAs of the grid as one thread-block cluster (1: none).
 template <class... KArgs, class... Args>
 inline cudaError_t launch_pdl_cluster(
-        void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, int cluster, cudaStream_t st,
+        const Writes& writes, void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, int cluster, cudaStream_t st,
         Args&&... args) {
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = grid;
@@ -76,6 +96,7 @@ inline cudaError_t launch_pdl_cluster(
     }
     cfg.attrs = attr;
     cfg.numAttrs = n;
+    LaunchRecord record(st, writes);
     return cudaLaunchKernelEx(&cfg, kernel, std::forward<Args>(args)...);
 }
 
