@@ -12,7 +12,7 @@ from ._lib import ConvF32Param, ConvFuse, ConvParam, check, fast, lib
 ACT = {"IDENTITY": 0, "RELU": 1, "H_SWISH": 2}
 POOL = {"MAX": 0, "AVERAGE": 1, "AVERAGE_COUNT_EXCLUDE_PADDING": 2}
 QELEM = {"QADD": 0, "QFUSE_ADD_RELU": 1, "QMUL": 2, "QRELU": 3}
-_S8 = torch.int8  # (a look-up less per call)
+_S8 = torch.int8
 ALGO = {"auto": 0, "direct": 1, "umma": 2, "patch": 3}
 
 
@@ -24,6 +24,11 @@ def _stream():
 
 def _ptr(t):
     return None if t is None else t.data_ptr()
+
+
+def _empty_s8(like, shape):
+    """An int8 tensor on the device of `like`. (Naming the type costs a call 0.1 us.)"""
+    return like.new_empty(shape) if like.dtype is _S8 else like.new_empty(shape, dtype=_S8)
 
 
 def _at(p, kind=ConvParam):
@@ -64,7 +69,7 @@ def conv_bias_qs8_nhwc(p, src, flt_packed, bias, dst=None, flt_scales=None, algo
                        src_is_nchw=False):
     f, at = fast(), _at(p)
     if dst is None:
-        dst = src.new_empty(f.conv_shape(at), dtype=_S8)
+        dst = _empty_s8(src, f.conv_shape(at))
     check(f.mb200_conv_bias_qs8_nhwc(
         at, _ptr(src), int(src_is_nchw), _ptr(flt_packed), _ptr(bias), _ptr(flt_scales),
         dst.data_ptr(), ALGO[algo], _stream()))
@@ -75,7 +80,7 @@ def conv_bias_qs8_nhwc_fused(p, src, flt_packed, bias, z, mode, z_scale, out_sca
     """ConvBias (p.nonline must be IDENTITY) followed by QADD / QFUSE_ADD_RELU with the int8
     tensor z of the output's NHWC shape, in one kernel."""
     f, at = fast(), _at(p)
-    dst = src.new_empty(f.conv_shape(at), dtype=_S8)
+    dst = _empty_s8(src, f.conv_shape(at))
     fuse = ConvFuse(z.data_ptr(), QELEM[mode], z_scale, out_scale)
     check(f.mb200_conv_bias_qs8_nhwc_fused(
         at, _ptr(src), 0, _ptr(flt_packed), _ptr(bias), None, C.addressof(fuse),
@@ -95,7 +100,7 @@ def conv_bias_qs8_nchw(p, src, flt_oihw, bias, flt_scales=None, algo="auto"):
     """ConvBias in the reference's own layouts (NCHW activations, OIHW filter)."""
     f, at = fast(), _at(p)
     n, oh, ow, oc = f.conv_shape(at)
-    dst = src.new_empty((n, oc, oh, ow), dtype=_S8)
+    dst = _empty_s8(src, (n, oc, oh, ow))
     nbytes = f.mb200_conv_bias_qs8_nchw_workspace(at)
     ws = src.new_empty(nbytes + 256)
     base = ws.data_ptr()
@@ -124,7 +129,7 @@ def matmul_s8_s32(a, b_packed):
 def matmul_s8_qs8(a, b_packed, acc_scale, dst_scale):
     m, k = a.shape
     n = b_packed.shape[0]
-    c = a.new_empty((m, n), dtype=_S8)
+    c = _empty_s8(a, (m, n))
     check(fast().mb200_matmul_s8_qs8(m, n, k, _ptr(a), _ptr(b_packed), _ptr(c), acc_scale,
                                      dst_scale, _stream()))
     return c
