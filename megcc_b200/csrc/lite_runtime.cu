@@ -1393,11 +1393,11 @@ int longest_chain(const DevModel& m) {
 // Up to which size of its tensors together: what branches save is the time of the instructions off
 // the longest chain, what they cost is the planned reuse of memory in the L2 and kernels that
 // share SMs which the larger batch would have filled. Measured per forward in one build, planned
-// and in order against spread and on branches: ResNet-18 (3 of its 23 instructions off the chain) 127
-// and 113 us with one image (2.7 MB), 185 and 179 with 16 (43 MB), 203 and 215 with 24 (65 MB), 226
-// and 237 with 32 (87 MB), 269 and 275 with 48 (130 MB): 48 MB. The detector (34 of 108 off the chain)
-// 561 and 448 at 416 x 416 (72 MB), 568 and 470 at 448 (84 MB), 581 and 500 at 480 (96 MB), and still
-// 701 and 594 at 640 (171 MB): there 96 MB bound the memory that a network takes for its speed, not
+// and in order against spread and on branches: ResNet-18 (3 of its 23 instructions off the chain) 109
+// and 100 us with one image (2.7 MB), 172 and 169 with 16 (43 MB), 195 and 213 with 24 (65 MB), 214
+// and 232 with 32 (87 MB), 264 and 270 with 48 (130 MB): 48 MB. The detector (34 of 108 off the chain)
+// 561 and 448 at 416 x 416 (72 MB), 568 and 468 at 448 (84 MB), 579 and 500 at 480 (96 MB), and still
+// 693 and 593 at 640 (171 MB): there 96 MB bound the memory that a network takes for its speed, not
 // the gain.
 bool spread_small_model(DevModel& m) {
     size_t total = 0;

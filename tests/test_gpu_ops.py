@@ -913,7 +913,9 @@ def test_split_tiles_match_oracle(ops, oracle, split, n, ic, oc, h, w, k, stride
 # last bytes of its result, which are written last, are the filter or the scales
 @pytest.mark.parametrize("kernel", ["quad_scales", "quad_filter", "patch_filter", "depthwise_tensor_filter",
                                     "umma_filter"])
-def test_parameters_may_come_from_the_call_before(ops, oracle, kernel):
+@pytest.mark.parametrize("between", [0, 1, 3])
+def test_parameters_may_come_from_the_call_before(ops, oracle, kernel, between):
+    """... or from one further back: `between` small launches stand between the two."""
     from megcc_b200._lib import check, lib
     r = cases.rng_for("late_" + kernel)
     n, c, hw, k, groups, algo = {"quad_scales": (1, 32, 20, 3, 32, "auto"),
@@ -930,6 +932,7 @@ def test_parameters_may_come_from_the_call_before(ops, oracle, kernel):
     values = torch.zeros(big, device="cuda")
     late8 = torch.empty(big, dtype=torch.int8, device="cuda")
     late32 = torch.empty(big, device="cuda")
+    small = torch.zeros(64, dtype=torch.int8, device="cuda")
     for turn in range(4):
         flt = r.integers(-127, 128, (c, c, k, k) if groups == 1 else (c, 1, 1, k, k)).astype(np.int8)
         s_flt = r.uniform(0.005, 0.02, c).astype(np.float32) if kernel == "quad_scales" else np.float32(0.01)
@@ -941,11 +944,15 @@ def test_parameters_may_come_from_the_call_before(ops, oracle, kernel):
             values[-c:] = dev(s_flt)
             torch.cuda.synchronize()
             check(lib().mb200_elemwise_f32(ops.ELEM["RELU"], values.data_ptr(), None, late32.data_ptr(), big, st))
+            for _ in range(between):
+                ops.qelemwise_qs8("QADD", small, small, 0.1, 0.1, 0.2)
             out = ops.conv_bias_qs8_nhwc(p, x, packed, dev_bias, flt_scales=late32[-c:], algo=algo)
         else:
             values[-packed.numel():] = packed.float()
             torch.cuda.synchronize()
             check(lib().mb200_typecvt_f32_qs8(values.data_ptr(), late8.data_ptr(), big, 1.0, 1.0, st))
+            for _ in range(between):
+                ops.qelemwise_qs8("QADD", small, small, 0.1, 0.1, 0.2)
             out = ops.conv_bias_qs8_nhwc(p, x, late8[-packed.numel():], dev_bias, algo=algo)
         want = oracle.conv_bias_qs8(src, flt, bias, 1, 1, 0.05, s_flt, s_dst, "RELU", groups=groups)
         assert (out.cpu().numpy().transpose(0, 3, 1, 2) == want).all(), turn
