@@ -161,8 +161,8 @@ struct DevModel {
     };
     static constexpr size_t kMaxGraphs = 4;
     std::vector<CapturedGraph> graphs;
-    // with parallel branches: the addresses of the last forward that found no graph, and how often
-    // in a row it was them (see copy_displaced_inputs)
+    // the addresses of the last forward that found no graph, and how often in a row it was them (see
+    // copy_displaced_inputs)
     std::vector<void*> missed;
     int missed_times = 0;
     bool memory_ready = false;
@@ -2021,14 +2021,21 @@ size_t find_graph(const DevModel& m, const std::vector<void*>& inputs) {
 
 // A caller with more device buffers than graphs are kept (a pool of frames): its inputs are copied
 // into the model's own place and the graph that reads them there serves all of them. Capturing and
-// instantiating a graph of parallel branches, and giving back the one that it displaces, takes
-// longer than a small model's forward: ResNet-18, one image, five buffers in turn: 565 us a
-// forward, 118 with four; a detector's frame of 416 x 416: 2270 and 459. Addresses that come many
-// times in a row are a new buffer that stays, and get a graph.
+// instantiating a graph, and giving back the one that it displaces, takes longer than a small model's
+// forward, parallel branches above all: ResNet-18, one image, five buffers in turn: 565 us a
+// forward, 118 with four; a detector's frame of 416 x 416: 2270 and 459; MobileNetV1, one image,
+// without branches: 216 and 96. Behind forwards of larger batches a capture is hidden (from about
+// 4 MB of input, 0.2 ms of kernels) and the copy would not be. Addresses that come many times in a
+// row are a new buffer that stays, and get a graph.
 int copy_displaced_inputs(Network* net, DevModel& m, std::vector<void*>* ptrs) {
     constexpr int kStays = 64;
-    if (!m.side_by_side || m.graphs.size() < DevModel::kMaxGraphs ||
-        find_graph(m, *ptrs) < m.graphs.size())
+    constexpr size_t kSmall = 4u << 20;
+    if (m.graphs.size() < DevModel::kMaxGraphs || find_graph(m, *ptrs) < m.graphs.size())
+        return TinyNN_SUCCESS;
+    size_t bytes = 0;
+    for (auto& s : m.inputs)
+        bytes += s.user_is_device ? s.bytes : 0;
+    if (!m.side_by_side && bytes > kSmall)
         return TinyNN_SUCCESS;
     m.missed_times = m.missed == *ptrs ? m.missed_times + 1 : 1;
     m.missed = *ptrs;

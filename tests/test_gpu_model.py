@@ -381,13 +381,14 @@ def test_model_with_a_bare_metal_device_model_beside_the_cuda_one(lite, oracle):
     assert (out == want).all()
 
 
+@pytest.mark.parametrize("model_name", ["resnet18", "mobilenet_v1"])
 @pytest.mark.parametrize("buffers", [3, 7])
-def test_cycling_device_input_buffers_replays_captured_graphs(lite, oracle, buffers):
+def test_cycling_device_input_buffers_replays_captured_graphs(lite, oracle, buffers, model_name):
     """A caller that alternates between device input buffers: each of a few addresses gets its own
     captured graph, kept (up to four) and replayed; with more of them the inputs go through the
     model's own memory; every forward is bit-exact. Then one buffer that stays."""
     from megcc_b200 import zoo
-    spec = zoo.resnet18(hw=64, classes=64, seed=7)
+    spec = getattr(zoo, model_name)(hw=64, classes=64, seed=7)
     model = spec.to_graph().compile([8])
     net = lite.Network(model)
     name_in, name_out = net.input_names()[0], net.output_names()[0]
