@@ -265,6 +265,10 @@ LaunchRecord::LaunchRecord(cudaStream_t st, const Writes& writes) {
     slot.hi = slot.lo + writes.bytes;
     slot_ = &slot;
 }
+void LaunchRecord::forget() {
+    ((LastLaunch*)slot_)->lo = 0;
+    ((LastLaunch*)slot_)->hi = UINTPTR_MAX;
+}
 LaunchRecord::~LaunchRecord() {
     ((LastLaunch*)slot_)->mu.unlock();
 }

@@ -46,8 +46,15 @@ class LaunchRecord {
 public:
     LaunchRecord(cudaStream_t st, const Writes& writes);
     ~LaunchRecord();
+    // (a launch that failed leaves the one before it the last, of which nothing is known any more)
+    cudaError_t result(cudaError_t e) {
+        if (e != cudaSuccess)
+            forget();
+        return e;
+    }
 
 private:
+    void forget();
     void* slot_;
 };
 // May the last launch on the stream write any of these bytes? (true where it is not known)
@@ -68,7 +75,7 @@ inline cudaError_t launch_pdl(
     cfg.attrs = attr;
     cfg.numAttrs = tuning().pdl ? 1 : 0;
     LaunchRecord record(st, writes);
-    return cudaLaunchKernelEx(&cfg, kernel, std::forward<Args>(args)...);
+    return record.result(cudaLaunchKernelEx(&cfg, kernel, std::forward<Args>(args)...));
 }
 
 // The same with `cluster` consecutive CTAs of the grid as one thread-block cluster (1: none).
@@ -97,7 +104,7 @@ inline cudaError_t launch_pdl_cluster(
     cfg.attrs = attr;
     cfg.numAttrs = n;
     LaunchRecord record(st, writes);
-    return cudaLaunchKernelEx(&cfg, kernel, std::forward<Args>(args)...);
+    return record.result(cudaLaunchKernelEx(&cfg, kernel, std::forward<Args>(args)...));
 }
 
 }  // namespace mb200
