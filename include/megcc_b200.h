@@ -257,7 +257,7 @@ MB200_API int mb200_requant_fast_constants(
  * and none for x86 (BareMetal/MatrixMul.cpp:13-23 admits f32/f16), so the arithmetic follows
  * the exact integer definition. B is re-laid once to K-major rows (k*n bytes) by
  * mb200_matmul_pack_b, as a weight's Init step would. Runs on the tensor cores when
- * k % 64 == 0 and the operands are 16-byte aligned, whatever m and n; on the CUDA cores otherwise. ---- */
+ * k % 16 == 0 and the operands are 16-byte aligned, whatever m and n; on the CUDA cores otherwise. ---- */
 MB200_API int mb200_matmul_pack_b(int k, int n, const int8_t* b, int8_t* b_packed, void* stream);
 MB200_API int mb200_matmul_s8_s32(
         int m, int n, int k, const int8_t* a, const int8_t* b_packed, int32_t* c, void* stream);

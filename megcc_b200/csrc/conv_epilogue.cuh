@@ -507,9 +507,14 @@ __device__ __forceinline__ uint32_t ask_for_params(
 // its register budget of 96 is a matter of luck: 20 bytes spilled in the tile loop cost a first
 // layer 25 %.
 //   FMA    per-tensor scales in the verified one-FMA form
-//   CHAIN  the reference's operations, two values per instruction: one scale per output channel
-//          (or per-tensor scales that have no one-FMA form)
+//   CHAIN  the reference's operations, two values per instruction: one scale per output channel.
+//          (Per-tensor scales without a one-FMA form stay with FORM_ANY, whose two- and
+//          three-operation forms are shorter: a 4096 x 1024 x 2048 product 12.1 us with CHAIN, 10.6 so.)
 // each with RELU, without activation, or with a QFUSE_ADD_RELU step in its verified short form.
+//   RAGGED FMA or CHAIN, with or without RELU, where the channels are a multiple of 4 and not of
+//          32 (a 1000-class classifier): the stores are narrower and the last chunk is cut. CHAIN also
+//          without channel scales where a pixel starts on no 8-byte boundary, which FORM_ANY
+//          stores byte by byte (a 3000 x 1500 x 1024 product: 48.6 us so, 12.9 here)
 enum EpilogueForm : int {
     FORM_ANY = -1,
     FORM_FMA_RELU = 0,
@@ -518,12 +523,24 @@ enum EpilogueForm : int {
     FORM_CHAIN_RELU = 3,
     FORM_CHAIN_NONE = 4,
     FORM_CHAIN_ADD_RELU = 5,
+    FORM_FMA_RAGGED = 6,
+    FORM_CHAIN_RAGGED = 7,
 };
+__host__ __device__ constexpr bool form_is_chain(int form) {
+    return (form >= FORM_CHAIN_RELU && form <= FORM_CHAIN_ADD_RELU) || form == FORM_CHAIN_RAGGED;
+}
 
 // host: the form a launch may use
 inline int epilogue_form(const EpilogueParams& e, const int8_t* dst) {
-    if (e.acc_out || (e.oc & 31) || ((uintptr_t)dst & 31) || e.act == ACT_H_SWISH)
+    if (e.acc_out || e.act == ACT_H_SWISH)
         return FORM_ANY;
+    if ((e.oc & 31) || ((uintptr_t)dst & 31)) {
+        if ((e.oc & 3) || ((uintptr_t)dst & 15) || e.z_mode != 0)
+            return FORM_ANY;
+        if (e.fast_ops == 1 && !e.flt_scales)
+            return FORM_FMA_RAGGED;
+        return e.flt_scales || (e.bounded && (e.oc & 7)) ? FORM_CHAIN_RAGGED : FORM_ANY;
+    }
     int mode = e.act == ACT_RELU ? 0 : 1;
     if (e.z_mode != 0) {
         if (e.z_mode != 2 || e.z_fast_a == 0.f || ((uintptr_t)e.z & 31))
@@ -532,7 +549,7 @@ inline int epilogue_form(const EpilogueParams& e, const int8_t* dst) {
     }
     if (e.fast_ops == 1 && !e.flt_scales)
         return FORM_FMA_RELU + mode;
-    return e.flt_scales || e.bounded ? FORM_CHAIN_RELU + mode : FORM_ANY;
+    return e.flt_scales ? FORM_CHAIN_RELU + mode : FORM_ANY;
 }
 
 // Per-channel scales are on the device only: can any of the layer's results leave the range in
@@ -561,8 +578,11 @@ template <int FORM>
 __device__ __forceinline__ void epilogue_form_chunk(
         uint32_t taddr, const EpilogueParams& e, int8_t* dst, size_t off, int ch0, bool valid,
         bool unbounded, uint64_t* release_bar) {
-    constexpr bool kChain = FORM >= FORM_CHAIN_RELU;
-    constexpr int kMode = FORM % 3;
+    constexpr bool kChain = form_is_chain(FORM);
+    constexpr bool kRagged = FORM >= FORM_FMA_RAGGED;
+    // (RAGGED: without activation, then negative bytes are cleared where the layer has a RELU; a value
+    // below zero rounds to something <= 0 in either form)
+    constexpr int kMode = kRagged ? 1 : FORM % 3;
     constexpr int kAct = kMode == 0 ? ACT_RELU : ACT_IDENTITY;
     uint32_t lo[16], hi[16], packed[8], zw[8];
     umma::tmem_ld16_nowait(taddr, lo);
@@ -577,6 +597,8 @@ __device__ __forceinline__ void epilogue_form_chunk(
     auto half = [&](const uint32_t (&v)[16], int base) {
 #pragma unroll
         for (int j = 0; j < 4; ++j) {
+            if (kRagged && ch0 + 4 * (base + j) >= e.oc)
+                break;  // (the channels are a multiple of 4)
             const int4 b = __ldg(bias4 + base + j);
             const int a0 = (int)v[4 * j] + b.x, a1 = (int)v[4 * j + 1] + b.y,
                       a2 = (int)v[4 * j + 2] + b.z, a3 = (int)v[4 * j + 3] + b.w;
@@ -586,7 +608,7 @@ __device__ __forceinline__ void epilogue_form_chunk(
                 requant_pair_fast<kAct, 1>(a2, a3, e, r2, r3);
             } else {
                 float4 s = make_float4(e.s_flt, e.s_flt, e.s_flt, e.s_flt);
-                if (e.flt_scales)
+                if (!kRagged || e.flt_scales)
                     s = __ldg(reinterpret_cast<const float4*>(e.flt_scales + ch0) + base + j);
                 if (unbounded) {
                     r0 = requant_one<kAct, false>(a0, e.s_src, s.x, e.s_dst, e.inv_dst);
@@ -607,7 +629,10 @@ __device__ __forceinline__ void epilogue_form_chunk(
             }
             const uint32_t pk = umma::pack4_prmt(r0, r1, r2, r3);
             // RELU of the ConvBias, or of the fused sum, on packed bytes
-            packed[base + j] = kMode == 1 ? pk : relu_s8x4(pk);
+            if (kRagged)
+                packed[base + j] = e.act == ACT_RELU ? relu_s8x4(pk) : pk;
+            else
+                packed[base + j] = kMode == 1 ? pk : relu_s8x4(pk);
         }
     };
     half(lo, 0);
@@ -618,6 +643,23 @@ __device__ __forceinline__ void epilogue_form_chunk(
         umma::mbar_arrive(release_bar);
     }
     half(hi, 4);
+    if constexpr (kRagged) {
+        if (valid) {
+            int8_t* out = dst + off;
+            if ((e.oc & 7) == 0) {  // every pixel starts on an 8-byte boundary, dst on a 16-byte one
+#pragma unroll
+                for (int h = 0; h < 4; ++h)
+                    if (ch0 + 8 * h < e.oc)
+                        reinterpret_cast<uint2*>(out)[h] = make_uint2(packed[2 * h], packed[2 * h + 1]);
+            } else {
+#pragma unroll
+                for (int j = 0; j < 8; ++j)
+                    if (ch0 + 4 * j < e.oc)
+                        reinterpret_cast<uint32_t*>(out)[j] = packed[j];
+            }
+        }
+        return;
+    }
     if (valid)
         asm volatile("st.global.v8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"l"(dst + off),
                      "r"(packed[0]), "r"(packed[1]), "r"(packed[2]), "r"(packed[3]),

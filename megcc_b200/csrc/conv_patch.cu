@@ -424,7 +424,7 @@ __global__ void __launch_bounds__(64 + 32 * EW, EW == 16 ? 1 : 2) conv_patch_ker
             if (p.ep.flt_scales)
                 pool_scales = __ldg(reinterpret_cast<const float4*>(p.ep.flt_scales + pool_ch));
         }
-        const bool unbounded = FORM >= FORM_CHAIN_RELU && chain_unbounded(p.ep);
+        const bool unbounded = form_is_chain(FORM) && chain_unbounded(p.ep);
         PatchWalker at(m_first, p);
         uint32_t asked = 0;
         if (POOL == 0 && m_first < p.m_tiles) {
@@ -560,8 +560,7 @@ __global__ void __launch_bounds__(64 + 32 * EW, EW == 16 ? 1 : 2) conv_patch_ker
             // load, requantisation, store
             auto do_chunk = [&](int c, bool last) {
                 if constexpr (FORM != FORM_ANY) {
-                    // (the channel count is a multiple of 32: a chunk exists as a whole or not;
-                    // pixel pairs: bias and channel scales are those of channel column % 32)
+                    // (pixel pairs: bias and channel scales are those of channel column % 32)
                     const int ch0 = n0 + c * 32;
                     uint64_t* release = last ? &acc_empty[buf] : nullptr;
                     if (ch0 < p.oc)
@@ -737,6 +736,8 @@ int launch_patch(
         MB200_PATCH_FORM(FORM_CHAIN_RELU)
         MB200_PATCH_FORM(FORM_CHAIN_NONE)
         MB200_PATCH_FORM(FORM_CHAIN_ADD_RELU)
+        MB200_PATCH_FORM(FORM_FMA_RAGGED)
+        MB200_PATCH_FORM(FORM_CHAIN_RAGGED)
         default:
             return launch_patch_form<BN, KH, KW, CHUNKS, EW, ROWS>(ma, mb, p, smem, grid, st);
     }

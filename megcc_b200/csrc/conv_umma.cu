@@ -15,7 +15,8 @@
 //   word, drains what it started, frees its TMEM and returns.
 //
 // Two operand geometries:
-//   WIDE  one tap x 64 channels per pipeline stage, 64-byte swizzle (input channels % 64 == 0)
+//   WIDE  one tap x 64 or 128 channels per pipeline stage, 64- / 128-byte swizzle (input channels
+//         % 16 == 0, at least 64 with a spatial filter or a stride)
 //   TAP16 four taps x 16 channels per stage, no swizzle: the form a stride-2 convolution with
 //         at most 4 input channels takes after a 2x2 space-to-depth step (see conv_s2d.cu)
 //
@@ -199,7 +200,8 @@ bool conv_umma_supported(
         const ConvArgs& a, const int8_t* src, const int8_t* flt, const int8_t* dst) {
     if (a.groups != 1 || a.src_is_nchw)
         return false;
-    if (a.ic % kBK != 0)
+    // rows start on 16-byte boundaries; an im2col map asks for boxes no wider than the tensor
+    if (a.ic % 16 != 0 || (a.ic < kBK && !conv_is_plain_matrix(a)))
         return false;
     if (a.kh * a.kw > 49 || a.dh != 1 || a.dw != 1)
         return false;
@@ -215,7 +217,10 @@ bool conv_umma_supported(
     return true;
 }
 
-// geom: 0 = WIDE (src NHWC with ic % 64 == 0, filter [OC][KH][KW][IC]);
+// geom: 0 = WIDE (src NHWC with ic % 16 == 0, filter [OC][KH][KW][IC]). Where the channels are no whole
+//           number of a stage's rows, the load fills the rest of the last row with zeros: a
+//           704 x 5920 x 7328 product takes 27 us that way, 12577 on one CUDA thread per output;
+
 //       1 = TAP16 (src NHWC with exactly 16 channels, stride 1, filter [OC][taps][16] with the
 //           tap count a multiple of 4; `a` then describes that transformed convolution, with
 //           a.ph/a.pw the LOW padding and a.oh/a.ow the output extent)
@@ -232,8 +237,12 @@ int launch_conv_umma_geom(
     if (((uintptr_t)bias & 15) || ((uintptr_t)flt_scales & 15))
         return set_error(ST_INVALID_LAYOUT, "bias and channel scales must be 16-byte aligned");
 
-    // 128-channel rows whenever the channel count allows: fewer, larger TMA requests
-    if (geom == GEOM_WIDE && a.ic % 128 == 0 && tuning().wide128)
+    // 128-channel rows (fewer, larger TMA requests) wherever they do not hold more padding than
+    // 64-channel ones, and from 512 channels on, where another half row of zeros is at most an eighth
+    // of the K loop
+    const int half_rows = (a.ic + kBK - 1) / kBK;
+    if (geom == GEOM_WIDE && (half_rows % 2 == 0 || a.ic >= 512) &&
+        (a.ic >= 128 || conv_is_plain_matrix(a)) && tuning().wide128)
         geom = GEOM_WIDE128;
     // MB200_CONV_PAIR=1: one 256 x 256 tile per pair of SMs (conv_pair.cu) wherever it applies.
     // Off by default: both kernels are bound by shared-memory bandwidth (operand reads of
@@ -247,11 +256,19 @@ int launch_conv_umma_geom(
     int bn = a.oc <= 64 ? 64 : 128, csplit = 1;
     {
         // 256 output channels per tile when the K loop is long enough to hide the epilogue
-        // of a single CTA per SM and there are tiles for every SM
+        // of a single CTA per SM and the busiest SM is done earlier: a step of 128 bytes takes 745
+        // clocks with 256 columns and 512 with 128 (operand reads and TMA writes share the SM's
+        // shared-memory port). Measured: 4096 x 1000 x 2048 (128 tiles of 256 columns, 256 of 128) 12.3
+        // against 13.3 us, 704 x 5920 x 7328 (144, 282) 29.7 against 34.2; 1696 x 1088 x 3040 (70, 126)
+        // 14.9 against 12.0.
         const long long k_bytes = (long long)taps * a.ic;
-        const long long tiles256 = (long long)((a.m + kBM - 1) / kBM) * ((a.oc + 255) / 256);
+        const long long m_tiles = (a.m + kBM - 1) / kBM;
+        const long long sms = sm_count();
+        const long long busiest256 = (m_tiles * ((a.oc + 255) / 256) + sms - 1) / sms;
+        const long long busiest128 = (m_tiles * ((a.oc + 127) / 128) + sms - 1) / sms;
         const int force = tuning().conv_bn;
-        if (geom == GEOM_WIDE128 && a.oc > 128 && k_bytes >= 1024 && tiles256 >= sm_count())
+        if (geom == GEOM_WIDE128 && a.oc > 128 && k_bytes >= 1024 &&
+            busiest256 * 745 < busiest128 * 512)
             bn = 256;
         if (force == 256 && geom == GEOM_WIDE128 && a.oc > 128)
             bn = 256;
@@ -328,7 +345,8 @@ int launch_conv_umma_geom(
     p.oc = a.oc;
     p.oh = a.oh;
     p.ow = a.ow;
-    p.cblocks = geom == GEOM_TAP16 ? 1 : a.ic / chans;
+    p.cblocks = geom == GEOM_TAP16 ? 1 : (a.ic + chans - 1) / chans;
+    p.tap_step = a.ic - (p.cblocks - 1) * chans;
     p.taps_w = a.kw;
     p.k_iters = geom == GEOM_TAP16 ? taps / 4 : taps * p.cblocks;
     p.sh = a.sh;

@@ -46,7 +46,8 @@ struct Geom {
 
 struct UmmaConvParams {
     int m_total, oc, oh, ow;
-    int cblocks;        // WIDE: 64-channel blocks per tap
+    int cblocks;        // channel blocks per tap; the last may reach past the tap's channels
+    int tap_step;       // filter bytes from a tap's last block to the next tap's first (kBKg, less the overhang)
     int taps_w;         // filter taps along W (TAP16: taps of the space-to-depth filter)
     int k_iters;        // pipeline stages per tile
     int sh, sw;         // output -> base pixel scaling
@@ -190,13 +191,14 @@ __global__ void __launch_bounds__(Shape<BN>::kThreads, Shape<BN>::kMinCtas) conv
                 const int rem = m0 - img * (p.oh * p.ow);
                 const int oy = rem / p.ow, ox = rem - oy * p.ow;
                 const int base_w = ox * p.sw + p.base_w, base_h = oy * p.sh + p.base_h;
-                int cb = 0, fx = 0, fy = 0;
+                int cb = 0, fx = 0, fy = 0, bx = 0;
                 if (w.k0 != 0) {
                     // a later part of a split tile starts in the middle of the filter
                     cb = w.k0 % p.cblocks;
                     const int tap = w.k0 / p.cblocks;
                     fy = tap / p.taps_w;
                     fx = tap - fy * p.taps_w;
+                    bx = tap * ((p.cblocks - 1) * kBKc + p.tap_step) + cb * kBKc;
                 }
                 if (item == first_item) {
                     pdl_wait();     // (the first tile is worked out before the wait)
@@ -230,9 +232,13 @@ __global__ void __launch_bounds__(Shape<BN>::kThreads, Shape<BN>::kMinCtas) conv
                         else
                             tma_load_im2col_4d(sa, &map_a, &full_bar[s], cb * kBKc, base_w, base_h,
                                                img, (uint16_t)(fx * p.dw), (uint16_t)(fy * p.dh));
-                        tma_load_2d(sb, &map_b, &full_bar[s], it * kBKc, n0);
+                        // (an overhanging block reads the next tap's filter bytes, or zeros behind the
+                        // last: its activation bytes are zeros)
+                        tma_load_2d(sb, &map_b, &full_bar[s], bx, n0);
+                        bx += kBKc;
                         if (++cb == p.cblocks) {
                             cb = 0;
+                            bx += p.tap_step - kBKc;
                             if (++fx == p.taps_w) {
                                 fx = 0;
                                 ++fy;
@@ -335,7 +341,7 @@ __global__ void __launch_bounds__(Shape<BN>::kThreads, Shape<BN>::kMinCtas) conv
         bool ok = true;
         uint32_t ep_phase = 0;  // parity of the epilogue's own rendezvous (split-K)
         pdl_wait();  // before the first read of z and the first store
-        const bool unbounded = FORM >= FORM_CHAIN_RELU && chain_unbounded(p.ep);
+        const bool unbounded = form_is_chain(FORM) && chain_unbounded(p.ep);
         uint32_t asked = 0;
         if (!SPLITK && p.csplit <= 1 && first_item < total_tiles) {
             // the first tile's parameters and residual come while its MMAs run
@@ -458,7 +464,6 @@ __global__ void __launch_bounds__(Shape<BN>::kThreads, Shape<BN>::kMinCtas) conv
 #pragma unroll 1
             for (int c = half * kChunksPerWarp; c < (half + 1) * kChunksPerWarp; ++c) {
                 if constexpr (FORM != FORM_ANY) {
-                    // (the channel count is a multiple of 32: a chunk exists as a whole or not)
                     const int ch0 = n0 + c * 32;
                     uint64_t* release =
                             c + 1 == (half + 1) * kChunksPerWarp ? &acc_empty[buf] : nullptr;
@@ -623,6 +628,8 @@ int launch_kernel(
         case FORM_CHAIN_NONE: return launch_form<BN, GEOM, false, FORM_CHAIN_NONE>(ma, mb, p, st);
         case FORM_CHAIN_ADD_RELU:
             return launch_form<BN, GEOM, false, FORM_CHAIN_ADD_RELU>(ma, mb, p, st);
+        case FORM_FMA_RAGGED: return launch_form<BN, GEOM, false, FORM_FMA_RAGGED>(ma, mb, p, st);
+        case FORM_CHAIN_RAGGED: return launch_form<BN, GEOM, false, FORM_CHAIN_RAGGED>(ma, mb, p, st);
         default: return launch_form<BN, GEOM>(ma, mb, p, st);
     }
 }

@@ -1023,3 +1023,31 @@ def test_relayout_by_words_is_exact(ops, n, c, h, w):
     y = ops.nchw_to_nhwc(torch.from_numpy(x).cuda())
     assert (y.cpu().numpy() == x.transpose(0, 2, 3, 1)).all()
     assert (ops.nhwc_to_nchw(y).cpu().numpy() == x).all()
+
+
+# channel counts that leave the last row of a pipeline stage partly zeros, behind a spatial filter, a
+# stride and neither; 64- and 128-channel rows, shared K loops, 128- and 256-column tiles
+@pytest.mark.parametrize("n,ic,oc,h,w,k,stride", [(1, 80, 64, 13, 9, 3, 1), (2, 96, 128, 12, 11, 3, 2),
+                                                  (1, 144, 64, 7, 6, 1, 2), (1, 16, 64, 9, 9, 1, 1),
+                                                  (1, 592, 160, 6, 7, 3, 1), (40, 176, 32, 28, 28, 3, 2),
+                                                  (3, 240, 320, 14, 14, 3, 1), (9, 48, 96, 56, 56, 1, 1)])
+@pytest.mark.parametrize("form", ["fast", "channel", "residual"])
+@pytest.mark.parametrize("bn", [0, 256])
+def test_channels_beside_the_stage_rows_match_oracle(ops, oracle, n, ic, oc, h, w, k, stride, form, bn, tune):
+    tune("conv_bn", bn)
+    check_small_conv(ops, oracle, n, ic, oc, h, w, k, stride, k // 2, 1, form)
+
+
+@pytest.mark.parametrize("shape", [(130, 100, 80), (5, 64, 16), (257, 300, 208), (1, 8, 528), (128, 1000, 48),
+                                   (300, 520, 1040)])
+def test_matmul_int8_of_ragged_depth(ops, oracle, shape):
+    test_matmul_int8_matches_oracle(ops, oracle, shape)
+
+
+# channels that are a multiple of 4 and not of 32: the last chunk is cut after each of its quads, the
+# stores are of 8 and of 4 bytes; tiles of the implicit product (64, 128, 256 columns) and of the patches
+@pytest.mark.parametrize("oc", [4, 36, 72, 100, 124, 1000])
+@pytest.mark.parametrize("n,ic,h,k", [(2, 64, 17, 3), (3, 64, 40, 1), (33, 128, 28, 1), (2, 32, 33, 3)])
+@pytest.mark.parametrize("form", ["fast", "channel"])
+def test_ragged_channels_match_oracle(ops, oracle, oc, n, ic, h, k, form):
+    check_small_conv(ops, oracle, n, ic, oc, h, h + 1, k, 1, k // 2, 1, form)
