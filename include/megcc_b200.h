@@ -91,7 +91,8 @@ MB200_API const char* mb200_last_error(void);
 /* Kernel-selection switches for experiments and tests (the library's own choices are the
  * defaults): "conv_bn" 0|64|128|256, "conv_pair" 0|1, "conv_splitk" 0|2..4, "conv_csplit" 0|1|2|4|8
  * (CTAs of a cluster that share a tile's K loop), "wide128" 1|0, "patch_ctas" 0|1..3,
- * "patch_alone" 0|1, "patch_plain" 0|1, "epilogue_forms" 1|0, "dw_tensor" 1|0, "dw_out" 0|2|4,
+ * "patch_alone" 0|1, "patch_plain" 0|1, "epilogue_forms" 1|0, "gather" 0|1|2, "nchw_store" 0|1|2,
+ * "dw_tensor" 1|0, "dw_out" 0|2|4,
  * "dw_one_output" 0|1, "fast_requant" 1|0, "f32_bn" 0|32|64|128, "f32_split" 0|1|2|4|8, "debug" 0|1,
  * "pdl" 1|0 (programmatic dependent launch of consecutive kernels). Their initial values come from
  * the environment variables of the same meaning (MB200_CONV_BN, ...), read ONCE per process; no
@@ -213,6 +214,12 @@ MB200_API int mb200_conv_bias_qs8_nchw(
         const mb200_conv_param* p, const int8_t* src, const int8_t* flt_oihw,
         const int32_t* bias, const float* flt_scales, int8_t* dst, void* workspace,
         size_t workspace_bytes, int algo, void* stream);
+/* A small ConvBias of that kind needs no scratch: mb200_conv_nchw_in_place(p) answers 1 and the second
+ * call reads and writes the NCHW tensors and the OIHW filter as they lie, in one kernel. */
+MB200_API int mb200_conv_nchw_in_place(const mb200_conv_param* p);
+MB200_API int mb200_conv_bias_qs8_nchw_in_place(
+        const mb200_conv_param* p, const int8_t* src, const int8_t* flt_oihw, const int32_t* bias,
+        const float* flt_scales, int8_t* dst, void* stream);
 /* The same operator for callers that cannot allocate device memory (a process whose own
  * pool already owns the whole device, or a loop that cannot afford the device-wide
  * synchronisation of cudaMalloc): this entry point has no counterpart in the reference.
@@ -257,7 +264,8 @@ MB200_API int mb200_requant_fast_constants(
  * and none for x86 (BareMetal/MatrixMul.cpp:13-23 admits f32/f16), so the arithmetic follows
  * the exact integer definition. B is re-laid once to K-major rows (k*n bytes) by
  * mb200_matmul_pack_b, as a weight's Init step would. Runs on the tensor cores when
- * k % 16 == 0 and the operands are 16-byte aligned, whatever m and n; on the CUDA cores otherwise. ---- */
+ * k % 16 == 0 and the operands are 16-byte aligned, and by ordinary loads otherwise (products of less than
+ * 2^20 terms: on the CUDA cores). ---- */
 MB200_API int mb200_matmul_pack_b(int k, int n, const int8_t* b, int8_t* b_packed, void* stream);
 MB200_API int mb200_matmul_s8_s32(
         int m, int n, int k, const int8_t* a, const int8_t* b_packed, int32_t* c, void* stream);

@@ -65,6 +65,8 @@ SIGNATURES = {
     "mb200_conv_bias_qs8_nchw_workspace": (C.c_size_t, [C.POINTER(ConvParam)]),
     "mb200_conv_bias_qs8_nchw": (C.c_int, [C.POINTER(ConvParam), _P, _P, _P, _P, _P, _P,
                                            C.c_size_t, C.c_int, _P]),
+    "mb200_conv_nchw_in_place": (C.c_int, [C.POINTER(ConvParam)]),
+    "mb200_conv_bias_qs8_nchw_in_place": (C.c_int, [C.POINTER(ConvParam), _P, _P, _P, _P, _P, _P]),
     "mb200_conv_bias_qs8_nchw_noalloc_max_scratch": (C.c_size_t, []),
     "mb200_conv_bias_qs8_nchw_noalloc": (C.c_int, [C.POINTER(ConvParam), _P, _P, _P, _P, _P, _P]),
     "mb200_conv_acc_qs8_nhwc": (C.c_int, [C.POINTER(ConvParam), _P, _P, _P, _P, _P]),
@@ -124,7 +126,8 @@ def lib():
 # the functions behind the operator calls of a program's inner loop
 FAST = ("mb200_conv_bias_qs8_nhwc", "mb200_conv_bias_qs8_nhwc_fused", "mb200_conv_bias_qs8_nchw",
         "mb200_matmul_s8_qs8", "mb200_qelemwise_qs8", "mb200_conv_bias_f32_nhwc",
-        "mb200_conv_bias_qs8_nchw_workspace", "mb200_matmul_f32_packed_b_bytes",
+        "mb200_conv_bias_qs8_nchw_workspace", "mb200_conv_nchw_in_place",
+        "mb200_conv_bias_qs8_nchw_in_place", "mb200_matmul_f32_packed_b_bytes",
         "mb200_matmul_f32_pack_b", "mb200_matmul_f32", "mb200_elemwise_f32")
 _fast = None
 

@@ -121,6 +121,8 @@ const TuningField kTuningFields[] = {
         {"conv_csplit", "MB200_CONV_CSPLIT", &Tuning::conv_csplit, false},
         {"f32_bn", "MB200_F32_BN", &Tuning::f32_bn, false},
         {"f32_split", "MB200_F32_SPLIT", &Tuning::f32_split, false},
+        {"gather", "MB200_GATHER", &Tuning::gather, false},
+        {"nchw_store", "MB200_NCHW_STORE", &Tuning::nchw_store, false},
         {"dw_tensor", "MB200_DW_TENSOR", &Tuning::dw_tensor, false},
         {"dw_out", "MB200_DW_OUT", &Tuning::dw_out, false},
         {"dw_one_output", "MB200_DW_ONE_OUTPUT", &Tuning::dw_one_output, false},
@@ -449,7 +451,7 @@ int mb200_relayout_nhwc_to_nchw44_s8(
 static int conv_bias_nhwc(
         const mb200_conv_param* p, const int8_t* src, int src_is_nchw, const int8_t* flt_packed,
         const int32_t* bias, const float* flt_scales, const mb200_conv_fuse* fuse, int8_t* dst,
-        int algo, int early, void* stream);
+        int algo, int early, void* stream, int8_t** nchw = nullptr);
 
 int mb200_conv_bias_qs8_nhwc(
         const mb200_conv_param* p, const int8_t* src, int src_is_nchw, const int8_t* flt_packed,
@@ -466,10 +468,23 @@ int mb200_conv_bias_qs8_nhwc_fused(
                           -1, stream);
 }
 
+// Does the ConvBias kernel store an NCHW result itself, a byte per lane, or does a transposing kernel
+// follow it? One launch less is 2.6 us of a call (64 -> 64 3x3 over 56 x 56: 13.3 us,
+// 11.2 so); byte stores cost large
+// results more than that (m x oc: 87808 x 256 over K = 288 33 -> 55 us, 10800 x 512 over 192 16.4 -> 18.8;
+// 28125 x 128 over 864 31.4 -> 29.1, 2312 x 16 over 576 16.2 -> 13.3).
+static bool nchw_store_pays(const ConvArgs& a) {
+    if (tuning().nchw_store != 1)
+        return tuning().nchw_store == 2;
+    return (long long)a.m * a.oc <= 4ll << 20;
+}
+
 static int conv_bias_nhwc(
         const mb200_conv_param* p, const int8_t* src, int src_is_nchw, const int8_t* flt_packed,
         const int32_t* bias, const float* flt_scales, const mb200_conv_fuse* fuse, int8_t* dst,
-        int algo, int early, void* stream) {  // early: ConvArgs::params_early, -1: not known
+        int algo, int early, void* stream, int8_t** nchw) {
+    // early: ConvArgs::params_early, -1: not known. nchw: where an NCHW result is wanted in the end; a
+    // kernel that can write it there does so in place of `dst`, and the pointer is cleared.
     ConvArgs a{};
     int rc = make_args(p, src_is_nchw, &a);
     if (rc)
@@ -525,18 +540,31 @@ static int conv_bias_nhwc(
     // (where its rows are whole 64-byte ones: MobileNetV1 at batch 64, whose first pointwise layer has 32
     // channels, took 458 us with that layer padded to them and 435 with it here)
     const bool pointwise = a.kh == 1 && a.kw == 1 && umma_ok && a.ic % 64 == 0;
+    // (the kernels that the switches named here select store NHWC only)
+    auto result = [&]() {
+        if (!nchw || !nchw_store_pays(a) || algo != MB200_ALGO_AUTO || tuning().conv_pair ||
+            tuning().conv_splitk || tuning().patch_alone || tuning().patch_plain)
+            return dst;
+        a.dst_nchw = 1;
+        int8_t* out = *nchw;
+        *nchw = nullptr;
+        return out;
+    };
     if (algo == MB200_ALGO_PATCH ||
         (algo == MB200_ALGO_AUTO && patch_ok && !pointwise && conv_patch_efficiency(a) >= 0.75f)) {
         ask_early();
-        return launch_conv_patch(a, src, flt_packed, bias, flt_scales, dst, st);
+        int8_t* out = result();
+        return launch_conv_patch(a, src, flt_packed, bias, flt_scales, out, st);
     }
     if (algo == MB200_ALGO_UMMA && !(umma_ok && a.ic % 64 == 0))
         return set_error(ST_NO_IMPLEMENT,
                          "tensor-core ConvBias needs dense, NHWC, ic %% 64 == 0, 16-byte aligned "
                          "tensors and, with a spatial filter or a stride, >= 128 KiB of readable "
                          "memory from the input on");
-    if (algo == MB200_ALGO_UMMA || (algo == MB200_ALGO_AUTO && umma_ok))
-        return launch_conv_umma(a, src, flt_packed, bias, flt_scales, dst, st);
+    if (algo == MB200_ALGO_UMMA || (algo == MB200_ALGO_AUTO && umma_ok)) {
+        int8_t* out = result();
+        return launch_conv_umma(a, src, flt_packed, bias, flt_scales, out, st);
+    }
     if (algo != MB200_ALGO_AUTO && algo != MB200_ALGO_DIRECT)
         return set_error(ST_OUT_OF_RANGE, "unknown algo %d", algo);
     // depthwise 3x3 / stride 1 over whole 64-channel slices: the halo-patch tensor-core kernel
@@ -551,6 +579,10 @@ static int conv_bias_nhwc(
     if (algo == MB200_ALGO_AUTO && side_ok && conv_dw_supported(a, src, flt_packed, dst)) {
         ask_early();
         return launch_conv_dw(a, src, flt_packed, bias, flt_scales, dst, st);
+    }
+    if (algo == MB200_ALGO_AUTO && conv_gather_supported(a, src, false) && conv_gather_pays(a, false)) {
+        int8_t* out = result();
+        return launch_conv_gather(a, false, src, flt_packed, bias, flt_scales, out, st);
     }
     return launch_conv_direct(a, src, flt_packed, bias, flt_scales, dst, nullptr, st);
 }
@@ -691,6 +723,11 @@ size_t mb200_conv_bias_qs8_nchw_workspace(const mb200_conv_param* p) {
     return src + dst + flt;
 }
 
+// AUTO: does this ConvBias read and write the reference's layouts as they lie?
+static bool nchw_in_place(const ConvArgs& a) {
+    return !conv_s2d_supported(a) && conv_gather_supported(a, nullptr, true) && conv_gather_pays(a, true);
+}
+
 int mb200_conv_bias_qs8_nchw(
         const mb200_conv_param* p, const int8_t* src, const int8_t* flt_oihw,
         const int32_t* bias, const float* flt_scales, int8_t* dst, void* workspace,
@@ -728,6 +765,8 @@ int mb200_conv_bias_qs8_nchw(
             return set_error(ST_OUT_OF_RANGE, "workspace of %zu bytes is too small",
                              workspace_bytes);
     }
+    if (algo == MB200_ALGO_AUTO && nchw_in_place(a) && !(((uintptr_t)bias | (uintptr_t)flt_scales) & 3))
+        return launch_conv_gather(a, true, src, flt_oihw, bias, flt_scales, dst, st);
     int8_t* ws_src = (int8_t*)workspace;
     int8_t* ws_dst = ws_src + align_up((size_t)a.n * a.ih * a.iw * a.ic, 256);
     int8_t* ws_flt = ws_dst + align_up((size_t)a.m * a.oc, 256);
@@ -735,9 +774,33 @@ int mb200_conv_bias_qs8_nchw(
     if ((rc = launch_transpose_pack_s8(src, ws_src, a.n, a.ic, a.ih * a.iw, a, flt_oihw, ws_flt, st)))
         return rc;
     // (the kernel that packs the filter does not release the ConvBias: all is complete by then)
-    if ((rc = conv_bias_nhwc(p, ws_src, 0, ws_flt, bias, flt_scales, nullptr, ws_dst, algo, 3, st)))
+    int8_t* nchw = dst;
+    if ((rc = conv_bias_nhwc(p, ws_src, 0, ws_flt, bias, flt_scales, nullptr, ws_dst, algo, 3, st, &nchw)))
         return rc;
+    if (!nchw)
+        return ST_SUCCESS;
     return launch_transpose_s8(ws_dst, dst, a.n, a.oh * a.ow, a.oc, st);
+}
+
+int mb200_conv_nchw_in_place(const mb200_conv_param* p) {
+    ConvArgs a{};
+    return make_args(p, 0, &a) == ST_SUCCESS && nchw_in_place(a) ? 1 : 0;
+}
+
+int mb200_conv_bias_qs8_nchw_in_place(
+        const mb200_conv_param* p, const int8_t* src, const int8_t* flt_oihw,
+        const int32_t* bias, const float* flt_scales, int8_t* dst, void* stream) {
+    ConvArgs a{};
+    int rc = make_args(p, 0, &a);
+    if (rc)
+        return rc;
+    if (!src || !flt_oihw || !dst)
+        return set_error(ST_NULL_PTR, "conv tensor pointer is NULL");
+    if (((uintptr_t)bias | (uintptr_t)flt_scales) & 3)
+        return set_error(ST_INVALID_LAYOUT, "bias and channel scales must be 4-byte aligned");
+    if (!nchw_in_place(a))
+        return set_error(ST_NO_IMPLEMENT, "this ConvBias needs re-laid tensors: mb200_conv_bias_qs8_nchw");
+    return launch_conv_gather(a, true, src, flt_oihw, bias, flt_scales, dst, (cudaStream_t)stream);
 }
 
 int mb200_requant_fast_constants(
@@ -793,6 +856,10 @@ int mb200_matmul_s8_s32(
         args.acc_out = c;
         return launch_conv_umma(args, a, b_packed, nullptr, nullptr, (int8_t*)c, st);
     }
+    if (conv_gather_supported(args, a, false) && conv_gather_pays(args, false)) {
+        args.acc_out = c;
+        return launch_conv_gather(args, false, a, b_packed, nullptr, nullptr, (int8_t*)c, st);
+    }
     return launch_conv_direct(args, a, b_packed, nullptr, nullptr, nullptr, c, st);
 }
 
@@ -815,6 +882,8 @@ int mb200_matmul_s8_qs8(
     cudaStream_t st = (cudaStream_t)stream;
     if (!args.true_division && conv_umma_supported(args, a, b_packed, c))
         return launch_conv_umma(args, a, b_packed, nullptr, nullptr, c, st);
+    if (conv_gather_supported(args, a, false) && conv_gather_pays(args, false))
+        return launch_conv_gather(args, false, a, b_packed, nullptr, nullptr, c, st);
     return launch_conv_direct(args, a, b_packed, nullptr, nullptr, c, nullptr, st);
 }
 

@@ -3,6 +3,7 @@
 // (compiler/lib/KernelGen/BareMetal/Activation.cpp:105-113) -> activation -> int8 -> store.
 #pragma once
 #include "common.cuh"
+#include "internal.h"
 #include "umma_ptx.cuh"
 
 namespace mb200 {
@@ -41,12 +42,44 @@ struct EpilogueParams {
     // when set, the int32 accumulators (+ bias) are stored here instead of the int8 result
     // (same [pixel][channel] indexing); used by the int8 -> int32 matrix product
     int32_t* acc_out;
+    int nchw_plane;  // non-zero: the result is NCHW with this many pixels per plane (FORM_NCHW)
 };
 
 // host: is |(float)acc * s_src * s_flt / s_dst| < 2^30 for every int32 acc?
 inline bool requant_is_bounded(float s_src, float s_flt, float s_dst) {
     const double m = 2147483648.0 * (double)fabsf(s_src) * (double)fabsf(s_flt) / (double)fabsf(s_dst);
     return m == m && m < 1073741824.0;
+}
+
+// host: the epilogue of a ConvBias
+inline void fill_epilogue(
+        const ConvArgs& a, const int32_t* bias, const float* flt_scales, EpilogueParams* e) {
+    e->oc = a.oc;
+    e->act = a.act;
+    e->bounded = requant_is_bounded(a.s_src, a.s_flt, a.s_dst) ? 1 : 0;
+    e->s_src = a.s_src;
+    e->s_flt = a.s_flt;
+    e->s_dst = a.s_dst;
+    e->inv_dst = 1.0f / a.s_dst;  // correctly rounded on the host
+    // a fused step follows a ConvBias without activation
+    e->fast_mul = e->fast_add = 0.f;
+    e->fast_ops = 0;
+    if (e->bounded && !flt_scales)
+        e->fast_ops = requant_fast_constants(a.s_src, a.s_flt, a.s_dst,
+                                             (a.z && a.z_mode) ? ACT_IDENTITY : a.act, &e->fast_mul,
+                                             &e->fast_add);
+    e->bias = bias;
+    e->flt_scales = flt_scales;
+    e->z = a.z;
+    e->z_mode = a.z ? a.z_mode : 0;
+    e->z_scale = a.z_scale;
+    e->z_div = 1.0f / a.z_out_scale;  // the reference's scale_div = 1.f / scale_dst
+    e->z_fast_a = e->z_fast_b = 0.f;
+    if (e->z_mode != 0)
+        residual_fast_constants(a.s_dst, a.z_scale, a.z_out_scale, e->z_mode, &e->z_fast_a,
+                                &e->z_fast_b);
+    e->acc_out = a.acc_out;
+    e->nchw_plane = a.dst_nchw ? a.oh * a.ow : 0;
 }
 
 template <int ACT, bool BOUNDED>
@@ -452,34 +485,54 @@ __device__ __forceinline__ uint32_t quad_z(const EpilogueParams& e, size_t off, 
             w |= (uint32_t)(uint8_t)e.z[off + i] << (8 * i);
     return w;
 }
-__device__ __forceinline__ void epilogue_quad(
-        const int (&acc)[4], const EpilogueParams& e, const QuadParams& q, uint32_t zw, int8_t* dst,
-        size_t off, int ch0) {
+// NCHW result: where the value of channel ch0 lies whose place in NHWC would be `off`
+__device__ __forceinline__ size_t nchw_offset(const EpilogueParams& e, size_t off, int ch0) {
+    const uint32_t pixel = (uint32_t)((off - ch0) / (uint32_t)e.oc);
+    const uint32_t img = pixel / (uint32_t)e.nchw_plane;
+    return ((size_t)img * e.oc + ch0) * e.nchw_plane + (pixel - img * (uint32_t)e.nchw_plane);
+}
+// the four results, a byte each
+__device__ __forceinline__ uint32_t quad_values(
+        const int (&acc)[4], const EpilogueParams& e, const QuadParams& q, uint32_t zw) {
     int r[4];
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
-        const int a = acc[i] + q.bias[i];
-        if (e.acc_out) {
-            if (ch0 + i < e.oc)
-                e.acc_out[off + i] = a;
-            continue;
-        }
-        const float t = __fmul_rn(__fmul_rn(__int2float_rn(a), e.s_src), q.scale[i]);
+        const float t = __fmul_rn(__fmul_rn(__int2float_rn(acc[i] + q.bias[i]), e.s_src), q.scale[i]);
         r[i] = round_clamp_s8(apply_act(e.act, div_rn_by_const(t, e.s_dst, e.inv_dst)));
         if (e.z_mode != 0) {
             const int zv = (int)(int8_t)(zw >> (8 * i));
             r[i] = e.z_mode == 1 ? fuse_z<1>(r[i], zv, e) : fuse_z<2>(r[i], zv, e);
         }
     }
-    if (e.acc_out)
+    return umma::pack4_prmt(r[0], r[1], r[2], r[3]);
+}
+__device__ __forceinline__ void nchw_quad(
+        const int (&acc)[4], const EpilogueParams& e, const QuadParams& q, int8_t* dst, size_t off, int ch0) {
+    const uint32_t word = quad_values(acc, e, q, 0);
+    int8_t* out = dst + nchw_offset(e, off, ch0);
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+        if (ch0 + i < e.oc)
+            out[(size_t)i * e.nchw_plane] = (int8_t)(word >> (8 * i));
+}
+__device__ __forceinline__ void epilogue_quad(
+        const int (&acc)[4], const EpilogueParams& e, const QuadParams& q, uint32_t zw, int8_t* dst,
+        size_t off, int ch0) {
+    if (e.acc_out) {
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+            if (ch0 + i < e.oc)
+                e.acc_out[off + i] = acc[i] + q.bias[i];
         return;
+    }
+    const uint32_t word = quad_values(acc, e, q, zw);
     if ((e.oc & 3) == 0 && ((uintptr_t)dst & 3) == 0) {
-        *reinterpret_cast<uint32_t*>(dst + off) = umma::pack4_prmt(r[0], r[1], r[2], r[3]);
+        *reinterpret_cast<uint32_t*>(dst + off) = word;
     } else {
 #pragma unroll
         for (int i = 0; i < 4; ++i)
             if (ch0 + i < e.oc)
-                dst[off + i] = (int8_t)r[i];
+                dst[off + i] = (int8_t)(word >> (8 * i));
     }
 }
 
@@ -525,6 +578,7 @@ enum EpilogueForm : int {
     FORM_CHAIN_ADD_RELU = 5,
     FORM_FMA_RAGGED = 6,
     FORM_CHAIN_RAGGED = 7,
+    FORM_NCHW = 8,
 };
 __host__ __device__ constexpr bool form_is_chain(int form) {
     return (form >= FORM_CHAIN_RELU && form <= FORM_CHAIN_ADD_RELU) || form == FORM_CHAIN_RAGGED;
@@ -532,6 +586,8 @@ __host__ __device__ constexpr bool form_is_chain(int form) {
 
 // host: the form a launch may use
 inline int epilogue_form(const EpilogueParams& e, const int8_t* dst) {
+    if (e.nchw_plane)
+        return FORM_NCHW;
     if (e.acc_out || e.act == ACT_H_SWISH)
         return FORM_ANY;
     if ((e.oc & 31) || ((uintptr_t)dst & 31)) {
@@ -568,6 +624,43 @@ __device__ __forceinline__ bool chain_unbounded(const EpilogueParams& e) {
     return !(fabsf(e.s_src) * most * fabsf(e.inv_dst) < 0.49f);
 }
 
+// NCHW result: sixteen channels of one pixel, every epilogue without a fused step
+__device__ __forceinline__ void nchw_store16(
+        const uint32_t (&v)[16], const EpilogueParams& e, int8_t* dst, size_t off, int ch0) {
+    int8_t* out = dst + nchw_offset(e, off, ch0);
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+        const int c = ch0 + 4 * j;
+        if (c >= e.oc)
+            break;
+        const int acc[4] = {(int)v[4 * j], (int)v[4 * j + 1], (int)v[4 * j + 2], (int)v[4 * j + 3]};
+        // (bias and channel scales start on 16-byte boundaries here)
+        QuadParams qp;
+        if (c + 4 <= e.oc) {
+            const int4 b = e.bias ? __ldg(reinterpret_cast<const int4*>(e.bias + c)) : make_int4(0, 0, 0, 0);
+            const float4 f = e.flt_scales ? __ldg(reinterpret_cast<const float4*>(e.flt_scales + c))
+                                          : make_float4(e.s_flt, e.s_flt, e.s_flt, e.s_flt);
+            qp = QuadParams{{b.x, b.y, b.z, b.w}, {f.x, f.y, f.z, f.w}};
+        } else {
+            qp = quad_params(e, c);
+        }
+        uint32_t word;
+        if (e.fast_ops == 1) {
+            int r0, r1, r2, r3;
+            requant_pair_fast<ACT_IDENTITY, 1>(acc[0] + qp.bias[0], acc[1] + qp.bias[1], e, r0, r1);
+            requant_pair_fast<ACT_IDENTITY, 1>(acc[2] + qp.bias[2], acc[3] + qp.bias[3], e, r2, r3);
+            word = umma::pack4_prmt(r0, r1, r2, r3);
+            word = e.act == ACT_RELU ? relu_s8x4(word) : word;
+        } else {
+            word = quad_values(acc, e, qp, 0);
+        }
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+            if (c + i < e.oc)
+                out[(size_t)(4 * j + i) * e.nchw_plane] = (int8_t)(word >> (8 * i));
+    }
+}
+
 // One 32-column chunk: registers <- TMEM, requantisation, one 32-byte store. The chunk's
 // accumulators come as two 16-column loads of which the second is in flight while the first
 // half is requantised: the warps are bound by the latency of this chain. `release_bar` (or null):
@@ -579,11 +672,27 @@ __device__ __forceinline__ void epilogue_form_chunk(
         uint32_t taddr, const EpilogueParams& e, int8_t* dst, size_t off, int ch0, bool valid,
         bool unbounded, uint64_t* release_bar) {
     constexpr bool kChain = form_is_chain(FORM);
-    constexpr bool kRagged = FORM >= FORM_FMA_RAGGED;
+    constexpr bool kRagged = FORM == FORM_FMA_RAGGED || FORM == FORM_CHAIN_RAGGED;
     // (RAGGED: without activation, then negative bytes are cleared where the layer has a RELU; a value
     // below zero rounds to something <= 0 in either form)
     constexpr int kMode = kRagged ? 1 : FORM % 3;
     constexpr int kAct = kMode == 0 ? ACT_RELU : ACT_IDENTITY;
+    if constexpr (FORM == FORM_NCHW) {
+        // sixteen columns at a time: few registers, and a warp's byte stores are runs of adjacent
+        // pixels
+#pragma unroll 1
+        for (int h = 0; h < 32; h += 16) {
+            uint32_t v[16];
+            umma::tmem_ld16(taddr + (uint32_t)h, v);
+            if (h != 0 && release_bar) {
+                asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+                umma::mbar_arrive(release_bar);
+            }
+            if (valid)
+                nchw_store16(v, e, dst, off + h, ch0 + h);
+        }
+        return;
+    }
     uint32_t lo[16], hi[16], packed[8], zw[8];
     umma::tmem_ld16_nowait(taddr, lo);
     if (kMode == 2 && valid)

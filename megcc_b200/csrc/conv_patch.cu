@@ -729,7 +729,7 @@ int launch_patch(
 #define MB200_PATCH_FORM(F)                                                                    \
     case F:                                                                                    \
         return launch_patch_form<BN, KH, KW, CHUNKS, EW, ROWS, 0, F>(ma, mb, p, smem, grid, st);
-    switch (tuning().epilogue_forms ? epilogue_form(p.ep, p.dst) : FORM_ANY) {
+    switch (tuning().epilogue_forms || p.ep.nchw_plane ? epilogue_form(p.ep, p.dst) : FORM_ANY) {
         MB200_PATCH_FORM(FORM_FMA_RELU)
         MB200_PATCH_FORM(FORM_FMA_NONE)
         MB200_PATCH_FORM(FORM_FMA_ADD_RELU)
@@ -738,6 +738,7 @@ int launch_patch(
         MB200_PATCH_FORM(FORM_CHAIN_ADD_RELU)
         MB200_PATCH_FORM(FORM_FMA_RAGGED)
         MB200_PATCH_FORM(FORM_CHAIN_RAGGED)
+        MB200_PATCH_FORM(FORM_NCHW)
         default:
             return launch_patch_form<BN, KH, KW, CHUNKS, EW, ROWS>(ma, mb, p, smem, grid, st);
     }
@@ -921,36 +922,12 @@ int launch_conv_patch(
     p.a_flat16 = (!pl.rows64 && a.ic == 16) ? 1 : 0;
     p.mma_per_tap = a.ic == 16 ? 0 : a.ic / 32;
     p.a_lbo = a.ic == 16 ? 16 : p.plane_stride;
-    p.ep.oc = a.oc;
-    p.ep.act = a.act;
-    p.ep.bounded = requant_is_bounded(a.s_src, a.s_flt, a.s_dst) ? 1 : 0;
-    p.ep.s_src = a.s_src;
-    p.ep.s_flt = a.s_flt;
-    p.ep.s_dst = a.s_dst;
-    p.ep.inv_dst = 1.0f / a.s_dst;  // correctly rounded on the host
-    // a fused step follows a ConvBias without activation
-    p.ep.fast_mul = p.ep.fast_add = 0.f;
-    p.ep.fast_ops = 0;
-    if (p.ep.bounded && !flt_scales)
-        p.ep.fast_ops = requant_fast_constants(a.s_src, a.s_flt, a.s_dst,
-                                               (a.z && a.z_mode) ? ACT_IDENTITY : a.act,
-                                               &p.ep.fast_mul, &p.ep.fast_add);
-    p.ep.bias = bias;
-    p.ep.flt_scales = flt_scales;
-    p.ep.z = a.z;
-    p.ep.z_mode = a.z ? a.z_mode : 0;
-    p.ep.z_scale = a.z_scale;
-    p.ep.z_div = 1.0f / a.z_out_scale;  // the reference's scale_div = 1.f / scale_dst
-    p.ep.z_fast_a = p.ep.z_fast_b = 0.f;
-    if (p.ep.z_mode != 0)
-        residual_fast_constants(a.s_dst, a.z_scale, a.z_out_scale, p.ep.z_mode, &p.ep.z_fast_a,
-                                &p.ep.z_fast_b);
+    fill_epilogue(a, bias, flt_scales, &p.ep);
     if (tuning().debug)
         fprintf(stderr, "%s: scales %g %g %g act %d z_mode %d verified requant: %d ops, %g + %.9g, short residual %g %g\n", "conv_patch",
                 a.s_src, a.s_flt, a.s_dst, a.act, p.ep.z_mode, p.ep.fast_ops, p.ep.fast_mul, p.ep.fast_add,
                 p.ep.z_fast_a,
                 p.ep.z_fast_b);
-    p.ep.acc_out = a.acc_out;
     p.dw_flt = a.dw64 ? flt : nullptr;
     p.dw_pairs = a.dw64 == 2 ? 1 : 0;
     p.early_flt = a.params_early & 1;

@@ -73,7 +73,7 @@ namespace {
 // off are 3x3 layers over 320 channels (64-byte rows are priced at half of 128-byte ones and cost
 // more) and 1x1 layers with 20 to 50 row tiles, where 64 columns unsplit would be up to 34 % faster
 // than the 128 taken.
-void choose_split(int m_tiles, int oc, int k_iters, bool wide128, int* bn, int* csplit) {
+void choose_split(int m_tiles, int oc, int k_iters, bool wide128, int sms, int* bn, int* csplit) {
     long long best = -1;
     const int bn_first = *bn;
     for (int b = 64; b <= 128; b *= 2) {
@@ -87,10 +87,10 @@ void choose_split(int m_tiles, int oc, int k_iters, bool wide128, int* bn, int* 
                     break;
                 const int fit = wide128 ? umma_clusters<64, GEOM_WIDE128>(s)
                                         : umma_clusters<64, GEOM_WIDE>(s);
-                if (k_iters / s < 2 || tiles > fit || tiles * s > sm_count())
+                if (k_iters / s < 2 || tiles > fit || tiles * s > sms)
                     break;
             }
-            const long long waves = (tiles * s + sm_count() - 1) / sm_count();
+            const long long waves = (tiles * s + sms - 1) / sms;
             const long long steps = (long long)((k_iters + s - 1) / s) * step;
             const int quads = b / (8 * s) > 1 ? b / (8 * s) : 1;
             const int end = (b == 128 ? 1800 : 1200) + (oc % 32 ? 3000 : 0);
@@ -282,8 +282,9 @@ int launch_conv_umma_geom(
         const long long tiles = (long long)((a.m + kBM - 1) / kBM) * ((a.oc + bn - 1) / bn);
         const int k_iters = geom == GEOM_TAP16 ? taps / 4 : taps * ((a.ic + chans - 1) / chans);
         if (geom != GEOM_TAP16 && bn <= 128 && force == 0 && a.test_wait_cycles == 0 &&
-            tiles <= sm_count())
-            choose_split((a.m + kBM - 1) / kBM, a.oc, k_iters, geom == GEOM_WIDE128, &bn, &csplit);
+            tiles <= sms)
+            choose_split((a.m + kBM - 1) / kBM, a.oc, k_iters, geom == GEOM_WIDE128,
+                         (int)sms, &bn, &csplit);
         const int fs = tuning().conv_csplit;
         if ((fs == 1 || fs == 2 || fs == 4 || fs == 8) && geom != GEOM_TAP16 && bn <= 128)
             csplit = k_iters >= fs ? fs : 1;
@@ -358,36 +359,12 @@ int launch_conv_umma_geom(
     p.m_tiles = (a.m + kBM - 1) / kBM;
     p.n_tiles = (a.oc + bn - 1) / bn;
     p.a_tiled = a_tiled ? 1 : 0;
-    p.ep.oc = a.oc;
-    p.ep.act = a.act;
-    p.ep.bounded = requant_is_bounded(a.s_src, a.s_flt, a.s_dst) ? 1 : 0;
-    p.ep.s_src = a.s_src;
-    p.ep.s_flt = a.s_flt;
-    p.ep.s_dst = a.s_dst;
-    p.ep.inv_dst = 1.0f / a.s_dst;  // correctly rounded on the host
-    // a fused step follows a ConvBias without activation
-    p.ep.fast_mul = p.ep.fast_add = 0.f;
-    p.ep.fast_ops = 0;
-    if (p.ep.bounded && !flt_scales)
-        p.ep.fast_ops = requant_fast_constants(a.s_src, a.s_flt, a.s_dst,
-                                               (a.z && a.z_mode) ? ACT_IDENTITY : a.act,
-                                               &p.ep.fast_mul, &p.ep.fast_add);
-    p.ep.bias = bias;
-    p.ep.flt_scales = flt_scales;
-    p.ep.z = a.z;
-    p.ep.z_mode = a.z ? a.z_mode : 0;
-    p.ep.z_scale = a.z_scale;
-    p.ep.z_div = 1.0f / a.z_out_scale;  // the reference's scale_div = 1.f / scale_dst
-    p.ep.z_fast_a = p.ep.z_fast_b = 0.f;
-    if (p.ep.z_mode != 0)
-        residual_fast_constants(a.s_dst, a.z_scale, a.z_out_scale, p.ep.z_mode, &p.ep.z_fast_a,
-                                &p.ep.z_fast_b);
+    fill_epilogue(a, bias, flt_scales, &p.ep);
     if (tuning().debug)
         fprintf(stderr, "%s: scales %g %g %g act %d z_mode %d verified requant: %d ops, %g + %.9g, short residual %g %g\n", "conv_umma",
                 a.s_src, a.s_flt, a.s_dst, a.act, p.ep.z_mode, p.ep.fast_ops, p.ep.fast_mul, p.ep.fast_add,
                 p.ep.z_fast_a,
                 p.ep.z_fast_b);
-    p.ep.acc_out = a.acc_out;
     p.dst = dst;
     p.status = device_status_word(st);
     p.wait_cycles = a.test_wait_cycles > 0 ? a.test_wait_cycles : kWaitCycles;

@@ -548,9 +548,13 @@ __global__ void __launch_bounds__(Shape<BN>::kThreads, Shape<BN>::kMinCtas) conv
         cluster_arrive();  // (a release: the loads above are done)
 #pragma unroll
         for (int k = 0; k < kItems; ++k)
-            if (k < items)
-                epilogue_quad(v[k], p.ep, qp, zw[k], p.dst, (size_t)(m0 + k * kRowStep) * p.oc + ch,
-                              ch);
+            if (k < items) {
+                const size_t off = (size_t)(m0 + k * kRowStep) * p.oc + ch;
+                if constexpr (FORM == FORM_NCHW)
+                    nchw_quad(v[k], p.ep, qp, p.dst, off, ch);
+                else
+                    epilogue_quad(v[k], p.ep, qp, zw[k], p.dst, off, ch);
+            }
         __syncwarp();
         cluster_wait();  // nobody leaves while its share may still be read
     }
@@ -620,7 +624,9 @@ int launch_form(
 template <int BN, int GEOM>
 int launch_kernel(
         const CUtensorMap& ma, const CUtensorMap& mb, const UmmaConvParams& p, cudaStream_t st) {
-    switch (p.csplit > 1 || !tuning().epilogue_forms ? FORM_ANY : epilogue_form(p.ep, p.dst)) {
+    switch (p.ep.nchw_plane                              ? FORM_NCHW
+            : p.csplit > 1 || !tuning().epilogue_forms ? FORM_ANY
+                                                       : epilogue_form(p.ep, p.dst)) {
         case FORM_FMA_RELU: return launch_form<BN, GEOM, false, FORM_FMA_RELU>(ma, mb, p, st);
         case FORM_FMA_NONE: return launch_form<BN, GEOM, false, FORM_FMA_NONE>(ma, mb, p, st);
         case FORM_FMA_ADD_RELU: return launch_form<BN, GEOM, false, FORM_FMA_ADD_RELU>(ma, mb, p, st);
@@ -630,6 +636,7 @@ int launch_kernel(
             return launch_form<BN, GEOM, false, FORM_CHAIN_ADD_RELU>(ma, mb, p, st);
         case FORM_FMA_RAGGED: return launch_form<BN, GEOM, false, FORM_FMA_RAGGED>(ma, mb, p, st);
         case FORM_CHAIN_RAGGED: return launch_form<BN, GEOM, false, FORM_CHAIN_RAGGED>(ma, mb, p, st);
+        case FORM_NCHW: return launch_form<BN, GEOM, false, FORM_NCHW>(ma, mb, p, st);
         default: return launch_form<BN, GEOM>(ma, mb, p, st);
     }
 }

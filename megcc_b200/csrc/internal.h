@@ -39,6 +39,8 @@ struct ConvArgs {
     float z_scale, z_out_scale;
     // tensor-core kernels only: store the int32 accumulators here instead of int8 results
     int32_t* acc_out;
+    // tensor-core kernels of dense layers, without a fused step: the result is NCHW
+    int dst_nchw;
     // halo-patch kernel only (reached through the space-to-depth path): 1 = the MAX pooling
     // 3x3 / stride 2 / pad 1 that follows the ConvBias is taken in its epilogue and dst is the
     // pooled tensor [n][(oh-1)/2+1][(ow-1)/2+1][oc]
@@ -130,6 +132,14 @@ int launch_conv_pair(
         const float* flt_scales, int8_t* dst, cudaStream_t st);
 int launch_conv_umma(
         const ConvArgs& a, const int8_t* src, const int8_t* flt, const int32_t* bias,
+        const float* flt_scales, int8_t* dst, cudaStream_t st);
+// tensor-core ConvBias whose operands are fetched by ordinary loads, any alignment (conv_gather.cu);
+// nchw: source, filter and result in the reference's own layouts
+bool conv_gather_supported(const ConvArgs& a, const int8_t* src, bool nchw);
+// ... where it is the faster one as well (against a CUDA thread per output, or against re-laid tensors)
+bool conv_gather_pays(const ConvArgs& a, bool nchw);
+int launch_conv_gather(
+        const ConvArgs& a, bool nchw, const int8_t* src, const int8_t* flt, const int32_t* bias,
         const float* flt_scales, int8_t* dst, cudaStream_t st);
 // stride-1 tensor-core ConvBias with halo-patch tiles and a resident filter (conv_patch.cu)
 bool conv_patch_supported(const ConvArgs& a, const int8_t* src, const int8_t* flt, const int8_t* dst);

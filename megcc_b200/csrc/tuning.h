@@ -17,6 +17,8 @@ struct Tuning {
     int conv_csplit = 0;    // MB200_CONV_CSPLIT    0 = by shape, 1 | 2 | 4 | 8 = CTAs of a cluster per tile's K loop
     int f32_bn = 0;         // MB200_F32_BN         0 = by shape, 32 | 64 | 128 = that fp32 tile width
     int f32_split = 0;      // MB200_F32_SPLIT      0 = by shape, 1 | 2 | 4 | 8 = CTAs per tile's K loop
+    int gather = 1;         // MB200_GATHER         0 = never operands by ordinary loads, 2 = wherever they can be
+    int nchw_store = 1;     // MB200_NCHW_STORE     0 = NCHW results by a transposing kernel, 2 = never by one
     int dw_tensor = 1;      // MB200_DW_TENSOR      0 = depthwise 3x3/1 on the CUDA cores only
     int dw_out = 0;         // MB200_DW_OUT         2 | 4 = outputs per thread of the depthwise kernel
     int dw_one_output = 0;  // MB200_DW_ONE_OUTPUT  1 = one output per thread

@@ -101,6 +101,10 @@ def conv_bias_qs8_nchw(p, src, flt_oihw, bias, flt_scales=None, algo="auto"):
     f, at = fast(), _at(p)
     n, oh, ow, oc = f.conv_shape(at)
     dst = _empty_s8(src, (n, oc, oh, ow))
+    if algo == "auto" and f.mb200_conv_nchw_in_place(at):
+        check(f.mb200_conv_bias_qs8_nchw_in_place(
+            at, _ptr(src), _ptr(flt_oihw), _ptr(bias), _ptr(flt_scales), dst.data_ptr(), _stream()))
+        return dst
     nbytes = f.mb200_conv_bias_qs8_nchw_workspace(at)
     ws = src.new_empty(nbytes + 256)
     base = ws.data_ptr()

@@ -1051,3 +1051,53 @@ def test_matmul_int8_of_ragged_depth(ops, oracle, shape):
 @pytest.mark.parametrize("form", ["fast", "channel"])
 def test_ragged_channels_match_oracle(ops, oracle, oc, n, ic, h, k, form):
     check_small_conv(ops, oracle, n, ic, oc, h, h + 1, k, 1, k // 2, 1, form)
+
+
+# operands that no tensor map describes, on the tensor cores all the same: rows of any length at any
+# byte, filters over channel counts beside 16, strides and dilation-free taps, tile and step edges
+@pytest.mark.parametrize("shape", [(1, 1, 1), (129, 65, 63), (128, 64, 64), (3, 300, 17), (200, 7, 129), (131, 130, 503),
+                                   (64, 1001, 66)])
+@pytest.mark.parametrize("offset", [0, 1, 6])
+def test_matmul_int8_of_rows_at_any_byte(ops, oracle, shape, offset, tune):
+    tune("gather", 2)
+    m, n, k = shape
+    r = cases.rng_for(f"gather_rows_{shape}_{offset}")
+    a, b = (r.integers(-128, 128, s).astype(np.int8) for s in ((m, k), (k, n)))
+    room = torch.empty(m * k + offset, dtype=torch.int8, device="cuda")
+    ad = room[offset:].view(m, k)
+    ad.copy_(dev(a))
+    bp = ops.matmul_pack_b(dev(b))
+    want = oracle.matmul_s8_s32(a, b)
+    assert (ops.matmul_s8_s32(ad, bp).cpu().numpy() == want).all()
+    got = ops.matmul_s8_qs8(ad, bp, 0.002, 1.0).cpu().numpy()
+    assert (got == oracle.typecvt_qs32_qs8(want, 0.002, 1.0)).all()
+    assert ops.device_status() == 0
+
+
+@pytest.mark.parametrize("n,ic,oc,h,w,k,stride,pad", [(2, 4, 5, 7, 9, 3, 1, 1), (1, 20, 70, 13, 12, 3, 2, 0),
+                                                      (3, 24, 64, 9, 8, 5, 1, 2), (1, 48, 33, 16, 8, 3, 2, 1),
+                                                      (2, 32, 130, 10, 13, 1, 2, 0), (1, 64, 64, 12, 11, 3, 1, 1),
+                                                      (1, 12, 8, 130, 1, 1, 1, 0)])
+@pytest.mark.parametrize("form", ["fast", "channel", "residual"])
+def test_gathered_operands_match_oracle(ops, oracle, n, ic, oc, h, w, k, stride, pad, form, tune):
+    tune("gather", 2)
+    check_small_conv(ops, oracle, n, ic, oc, h, w, k, stride, pad, 1, form)
+
+
+# the reference's layouts: read and written in place, or the result only, or neither; every activation,
+# channels beside 4, 16 and 32, whole and partial tiles, several images in a warp
+@pytest.mark.parametrize("gather,store", [(2, 1), (1, 2), (1, 0)])
+@pytest.mark.parametrize("n,ic,oc,h,w,k,stride", [(2, 3, 5, 9, 7, 3, 1), (5, 64, 64, 7, 5, 3, 1), (1, 64, 72, 40, 40, 3, 1),
+                                                  (2, 128, 130, 12, 30, 1, 1), (1, 20, 33, 6, 6, 7, 2),
+                                                  (3, 64, 100, 33, 31, 3, 2), (2, 16, 40, 96, 80, 3, 1)])
+@pytest.mark.parametrize("act,channel", [("RELU", False), ("H_SWISH", True), ("IDENTITY", True), ("IDENTITY", False)])
+def test_conv_in_the_reference_layouts(ops, oracle, gather, store, n, ic, oc, h, w, k, stride, act, channel, tune):
+    tune("gather", gather)
+    tune("nchw_store", store)
+    c = dict(name=f"nchw_{n}_{ic}_{oc}_{k}", n=n, ic=ic, oc=oc, h=h, w=w, k=k, stride=stride, pad=k // 2, groups=1,
+             act=act, range=(-128, 127), bias_range=(-1000, 1000), scales=(0.05, 0.01, 0.4 * (ic * k * k / 576) ** 0.5))
+    sf = np.linspace(0.004, 0.02, oc).astype(np.float32) if channel else None
+    out, (src, flt, bias) = run_conv_nchw(ops, c, flt_scales=sf)
+    want = oracle.conv_bias_qs8(src, flt, bias, stride, k // 2, 0.05, sf if channel else 0.01, c["scales"][2], act)
+    assert (out == want).all()
+    assert ops.device_status() == 0
