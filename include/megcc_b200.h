@@ -93,11 +93,12 @@ MB200_API const char* mb200_last_error(void);
  * (CTAs of a cluster that share a tile's K loop), "wide128" 1|0, "patch_ctas" 0|1..3,
  * "patch_alone" 0|1, "patch_plain" 0|1, "epilogue_forms" 1|0, "gather" 0|1|2, "nchw_store" 0|1|2,
  * "dw_tensor" 1|0, "dw_out" 0|2|4,
- * "dw_one_output" 0|1, "fast_requant" 1|0, "f32_bn" 0|32|64|128, "f32_split" 0|1|2|4|8, "debug" 0|1,
+ * "dw_one_output" 0|1, "fast_requant" 1|0, "f32_bn" 0|32|64|128, "f32_split" 0|1|2|4|8,
+ * "f32_half" 0|1|2, "debug" 0|1,
  * "pdl" 1|0 (programmatic dependent launch of consecutive kernels). Their initial values come from
  * the environment variables of the same meaning (MB200_CONV_BN, ...), read ONCE per process; no
- * launch consults the environment. Every setting yields bit-identical int8 results; the two of the
- * fp32 kernel change the order of its sums. Process-wide, not thread-safe against concurrent
+ * launch consults the environment. Every setting yields bit-identical int8 results; the three of the
+ * fp32 kernels change the order of its sums. Process-wide, not thread-safe against concurrent
  * launches. */
 MB200_API int mb200_set_option(const char* name, int value);
 MB200_API int mb200_get_option(const char* name, int* value);
@@ -384,6 +385,13 @@ MB200_API size_t mb200_matmul_f32_workspace_bytes(int m, int k);
 MB200_API int mb200_matmul_f32(
         int m, int n, int k, const float* a, const float* b_packed, float* c, void* workspace,
         size_t workspace_bytes, void* stream);
+/* The same with B as it is, [K][N]: preparation and product in one call, with the planes of B that suit the
+ * product's sizes, over mb200_matmul_f32_scratch_bytes(m, n, k) bytes of device scratch (16-byte
+ * aligned). Tensor cores for every m, n, k where C is 16-byte aligned. */
+MB200_API size_t mb200_matmul_f32_scratch_bytes(int m, int n, int k);
+MB200_API int mb200_matmul_f32_product(
+        int m, int n, int k, const float* a, const float* b, float* c, void* scratch,
+        size_t scratch_bytes, void* stream);
 
 /* ---- Elemwise fp32, same-shape operands (b ignored for unary modes) ---- */
 MB200_API int mb200_elemwise_f32(

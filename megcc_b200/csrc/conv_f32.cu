@@ -64,8 +64,7 @@
 #include <stdio.h>
 #include <stdlib.h>
 
-#include <type_traits>
-
+#include "conv_f32_epilogue.cuh"
 #include "f32_internal.h"
 #include "pdl.h"
 #include "tuning.h"
@@ -170,110 +169,6 @@ __global__ void __launch_bounds__(256) pack_matrix_f32_kernel(
             const float h = round_tf32(v);
             dst[(size_t)c * kp + r] = h;
             dst[plane + (size_t)c * kp + r] = __fsub_rn(v, h);
-        }
-    }
-}
-
-// ------------------------------------------------------------------------------------------
-// epilogue
-// ------------------------------------------------------------------------------------------
-struct F32Epilogue {
-    int oc, act;
-    const float* bias;
-    const float* z;  // optional tensor added after the activation (residual), or nullptr
-    long long z_pitch;
-    float* dst;
-    long long dst_pitch;  // floats between consecutive pixels of dst (>= oc)
-};
-
-// 1 / (1 + 2^(-x log2 e)) from the hardware's two approximations (2 and 1 ulp), without the range
-// handling that the general exponential and quotient put around them: a subnormal power is lost
-// beside the 1 anyway, and an infinite one gives the right 0. 5 instructions instead of some 25.
-__device__ __forceinline__ float sigmoid_f32(float x) {
-    float e, r;
-    asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(e) : "f"(x * -1.442695041f));
-    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(1.f + e));
-    return r;
-}
-
-template <int ACT>
-__device__ __forceinline__ float act_f32(float x) {
-    if (ACT == MB200_F32_RELU)
-        return x > 0.f ? x : 0.f;
-    if (ACT == MB200_F32_SIGMOID)
-        return sigmoid_f32(x);
-    if (ACT == MB200_F32_SILU)
-        return x * sigmoid_f32(x);
-    if (ACT == MB200_F32_H_SWISH) {
-        float t = x + 3.f;
-        t = t > 0.f ? t : 0.f;
-        t = t > 6.f ? 6.f : t;
-        return x * t * (1.f / 6.f);
-    }
-    return x;
-}
-
-// Calls f with the activation as a compile-time constant. The choice is made once per tile and
-// warp: made per element (a run-time switch inside the unrolled loops) it serialised the
-// elements, 250 clocks each, and the epilogue was the kernel's longest chain.
-template <class F>
-__device__ __forceinline__ void with_act(int act, F&& f) {
-    switch (act) {
-        case MB200_F32_RELU: f(std::integral_constant<int, MB200_F32_RELU>()); break;
-        case MB200_F32_SIGMOID: f(std::integral_constant<int, MB200_F32_SIGMOID>()); break;
-        case MB200_F32_SILU: f(std::integral_constant<int, MB200_F32_SILU>()); break;
-        case MB200_F32_H_SWISH: f(std::integral_constant<int, MB200_F32_H_SWISH>()); break;
-        default: f(std::integral_constant<int, MB200_F32_IDENTITY>()); break;
-    }
-}
-
-// One pixel's channels of a finished tile (a row per lane): bias, activation, residual, stores.
-// With a short K loop (1x1 filters) this is the kernel's longest chain. So the bias lies in
-// shared memory (fetched once per tile column: from global memory each eight channels waited
-// for their load behind the stores before them), the residual is brought into the L2 while the
-// tile is computed, and stores are whole 32-byte sectors. 32 x 80 x 80 pixels of 128 channels to
-// 80: 96 us before, 48 now (floor 26 by its bytes); 128 to 128: 66 -> 54. (Turning the tile round
-// in shared memory, so that a warp stores 64-byte pieces of 16 rows instead of sectors of 32,
-// measured the same within 3 % either way and costs 16 KB of the ring.)
-template <int COLS, int ACT>
-__device__ __forceinline__ void store_f32_row(
-        const float (&sum)[COLS], const F32Epilogue& e, const float4* bias, size_t m, int ch0,
-        bool vec4, bool vec8) {
-    float* out = e.dst + m * e.dst_pitch + ch0;
-    const float* zin = e.z ? e.z + m * e.z_pitch + ch0 : nullptr;
-#pragma unroll
-    for (int c = 0; c < COLS / 8; ++c) {
-        if (ch0 + 8 * c >= e.oc)
-            break;  // (also keeps the steps apart: run together they need too many registers)
-        const bool whole = vec4 && ch0 + 8 * c + 8 <= e.oc;
-        const float4 b0 = bias[2 * c], b1 = bias[2 * c + 1];
-        const float b[8] = {b0.x, b0.y, b0.z, b0.w, b1.x, b1.y, b1.z, b1.w};
-        float v[8];
-#pragma unroll
-        for (int j = 0; j < 8; ++j)
-            v[j] = act_f32<ACT>(sum[8 * c + j] + b[j]);
-        if (whole) {
-            if (zin) {
-                const float4 z0 = *(reinterpret_cast<const float4*>(zin) + 2 * c);
-                const float4 z1 = *(reinterpret_cast<const float4*>(zin) + 2 * c + 1);
-                v[0] += z0.x, v[1] += z0.y, v[2] += z0.z, v[3] += z0.w;
-                v[4] += z1.x, v[5] += z1.y, v[6] += z1.z, v[7] += z1.w;
-            }
-            if (vec8) {
-                asm volatile("st.global.v8.f32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"l"(
-                                     out + 8 * c),
-                             "f"(v[0]), "f"(v[1]), "f"(v[2]), "f"(v[3]), "f"(v[4]), "f"(v[5]),
-                             "f"(v[6]), "f"(v[7])
-                             : "memory");
-            } else {
-                reinterpret_cast<float4*>(out)[2 * c] = make_float4(v[0], v[1], v[2], v[3]);
-                reinterpret_cast<float4*>(out)[2 * c + 1] = make_float4(v[4], v[5], v[6], v[7]);
-            }
-        } else {
-#pragma unroll
-            for (int j = 0; j < 8; ++j)
-                if (ch0 + 8 * c + j < e.oc)
-                    out[8 * c + j] = zin ? v[j] + zin[8 * c + j] : v[j];
         }
     }
 }
@@ -988,6 +883,20 @@ __global__ void __launch_bounds__(256) pack_filter_f32_plain_kernel(
     }
 }
 
+// [rows][k] -> [rows][4 k4], zeros behind the k values. Bound by HBM: 8 bytes per element.
+__global__ void __launch_bounds__(256) pad_rows_f32_kernel(
+        const float* __restrict__ src, float4* __restrict__ dst, long long rows, int k, int k4) {
+    pdl_start();
+    const long long total = rows * k4;
+    for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < total;
+         i += (long long)gridDim.x * blockDim.x) {
+        const long long r = i / k4;
+        const int c = (int)(i - r * k4) * 4;
+        const float* s = src + r * k + c;
+        dst[i] = make_float4(s[0], c + 1 < k ? s[1] : 0.f, c + 2 < k ? s[2] : 0.f, c + 3 < k ? s[3] : 0.f);
+    }
+}
+
 int grid_1d(size_t work, int block) {
     size_t g = (work + block - 1) / block;
     const size_t most = (size_t)sm_count() * 16;
@@ -1058,7 +967,15 @@ int f32_cluster_capacity(int bn, int rowb, int size) {
 // layers that are in no network here (16 to 512 channels to 16 to 512, 25 to 20000 pixels) the choice is 2 %
 // on average behind the best of all widths and splits; one layer (16 -> 85 3x3 over 2 x 13 x 13, unsplit 6.9 us,
 // split 4.5) is 52 % off, all others at most 15 %.
-void choose_f32_tile(int m_tiles, int oc, int k_iters, int rowb, int* bn, int* splits) {
+struct F32Choice {
+    int bn, splits;
+    bool half;  // 128 columns, from fp16 planes
+};
+F32Choice choose_f32_tile(const ConvF32Args& a, bool planes) {
+    const int rowb = a.ic <= 16 ? 64 : 128, oc = a.oc;
+    const int m_tiles = (a.m + kBM - 1) / kBM;
+    const int k_iters = a.kh * a.kw * (conv_f32_padded_ic(a.ic) * 4 / rowb);
+    F32Choice c{128, 1, false};
     const int sms = sm_count();
     long long best = -1;
     for (int b = 128; b >= 32; b /= 2) {
@@ -1077,11 +994,23 @@ void choose_f32_tile(int m_tiles, int oc, int k_iters, int rowb, int* bn, int* s
                     (s > 1 ? 2500 : 0);
             if (best < 0 || clocks < best) {
                 best = clocks;
-                *bn = b;
-                *splits = s;
+                c.bn = b;
+                c.splits = s;
             }
         }
     }
+    // 128 columns from fp16 planes (conv_f32_half.cu): two rows of A in the time of 1.64 here (32 x 80 x 80
+    // pixels, 128 -> 128 3x3: 251 us and 206; 32 x 20 x 20, 256 -> 256: 100 as 64 columns, 82)
+    const long long waves = ((long long)m_tiles * ((oc + 127) / 128) + sms - 1) / sms;
+    c.half = planes && waves * ((long long)((k_iters + 1) / 2) * 1395 + 2500 + (waves > 1 ? 0 : 3000)) < best;
+    if (tuning().f32_bn == 32 || tuning().f32_bn == 64 || tuning().f32_bn == 128)
+        c.bn = tuning().f32_bn;
+    if (tuning().f32_split == 1 || tuning().f32_split == 2 || tuning().f32_split == 4 ||
+        tuning().f32_split == 8)
+        c.splits = k_iters >= tuning().f32_split ? tuning().f32_split : 1;
+    if (tuning().f32_bn || tuning().f32_split || tuning().f32_half != 1)
+        c.half = planes && tuning().f32_half == 2;
+    return c;
 }
 
 bool plain_matrix(const ConvF32Args& a) {
@@ -1096,7 +1025,15 @@ int conv_f32_padded_ic(int ic) {
 }
 
 size_t conv_f32_split_filter_floats(const ConvF32Args& a) {
-    return 2 * (size_t)a.oc * a.kh * a.kw * conv_f32_padded_ic(a.ic);
+    return 2 * (size_t)a.oc * a.kh * a.kw * conv_f32_padded_ic(a.ic) +
+           (conv_f32_half_planes(a) ? conv_f32_half_filter_floats(a) : 0);
+}
+// Filters that 128-channel tiles can be taken for (rows of 128 bytes, more than 64 channels) hold the fp16
+// planes as well: which kernel runs is known only with the batch. (Not the second operand of a matrix
+// product packed by itself: its callers pack anew with every product, and the planes cost another read.)
+bool conv_f32_half_planes(const ConvF32Args& a) {
+    const bool product = a.kh == 1 && a.kw == 1 && a.ih == 1 && a.iw == 1;
+    return conv_f32_split_eligible(a) && a.ic > 16 && a.oc > 64 && !product;
 }
 
 // Channel counts the tensor-core kernel takes: rows the TMA can address (16-byte multiples).
@@ -1140,7 +1077,9 @@ int launch_conv_f32_pack_filter_split(
     const size_t plane = (size_t)a.oc * a.kh * a.kw * icp;
     pack_filter_f32_kernel<<<grid_1d(plane, 256), 256, 0, st>>>(flt_oihw, out, a.oc, a.ic, icp,
                                                                  a.kh, a.kw);
-    return check_launch("pack_filter_f32");
+    const int rc = check_launch("pack_filter_f32");
+    return rc || !conv_f32_half_planes(a) ? rc
+                                          : launch_conv_f32_pack_filter_half(a, flt_oihw, out + 2 * plane, st);
 }
 
 int launch_conv_f32_pack_filter_plain(
@@ -1173,9 +1112,10 @@ int launch_conv_f32_direct(
     return check_launch("conv_f32_direct");
 }
 
-int launch_conv_f32_umma(
-        const ConvF32Args& a, const float* src, const float* flt_split, const float* bias,
-        const float* z, float* dst, cudaStream_t st) {
+// `planes`: the fp16 planes of the filter, null: there are none, or the choice has fallen on the tf32 ones
+static int launch_f32_tensor(
+        const ConvF32Args& a, const float* src, const float* flt_split, const float* planes,
+        const F32Choice& choice, const float* bias, const float* z, float* dst, cudaStream_t st) {
     const DriverApi& api = driver_api();
     if (!api.ok)
         return set_error(ST_RUNTIME, "cuTensorMapEncode* entry points not found in the driver");
@@ -1193,13 +1133,8 @@ int launch_conv_f32_umma(
     p.m_tiles = (a.m + kBM - 1) / kBM;
     p.cblocks = icp / chans;
     p.k_iters = taps * p.cblocks;
-    int bn = 128;
-    choose_f32_tile(p.m_tiles, a.oc, p.k_iters, rowb, &bn, &p.splits);
-    if (tuning().f32_bn == 32 || tuning().f32_bn == 64 || tuning().f32_bn == 128)
-        bn = tuning().f32_bn;
-    if (tuning().f32_split == 1 || tuning().f32_split == 2 || tuning().f32_split == 4 ||
-        tuning().f32_split == 8)
-        p.splits = p.k_iters >= tuning().f32_split ? tuning().f32_split : 1;
+    const int bn = choice.bn;
+    p.splits = choice.splits;
     CUtensorMap map_a, map_b;
     if (a_tiled) {
         cuuint64_t dims[2] = {(cuuint64_t)a.ic, (cuuint64_t)a.m};
@@ -1230,6 +1165,8 @@ int launch_conv_f32_umma(
         if (r != CUDA_SUCCESS)
             return set_error(ST_RUNTIME, "cuTensorMapEncodeIm2col(f32) failed: %d", (int)r);
     }
+    if (choice.half)
+        return launch_conv_f32_half(a, map_a, a_tiled, planes, bias, z, dst, st);
     {
         const cuuint64_t k_total = (cuuint64_t)taps * icp;
         cuuint64_t dims[2] = {k_total, (cuuint64_t)2 * a.oc};
@@ -1273,6 +1210,50 @@ int launch_conv_f32_umma(
     return bn == 32   ? launch_f32_kernel<32, 64>(map_a, map_b, p, st)
            : bn == 64 ? launch_f32_kernel<64, 64>(map_a, map_b, p, st)
                       : launch_f32_kernel<128, 64>(map_a, map_b, p, st);
+}
+
+int launch_conv_f32_umma(
+        const ConvF32Args& a, const float* src, const float* flt_split, const float* bias,
+        const float* z, float* dst, cudaStream_t st) {
+    const bool has = conv_f32_half_planes(a);
+    const size_t split = 2 * (size_t)a.oc * a.kh * a.kw * conv_f32_padded_ic(a.ic);
+    return launch_f32_tensor(a, src, flt_split, has ? flt_split + split : nullptr, choose_f32_tile(a, has),
+                             bias, z, dst, st);
+}
+
+// ---- a matrix product with both operands as the caller has them ----
+static bool product_pads(int k, const float* a) {
+    return k % 4 != 0 || ((uintptr_t)a & 15) != 0;
+}
+
+size_t matmul_f32_scratch_floats(const ConvF32Args& a) {
+    const int kp = conv_f32_padded_ic(a.ic);
+    const size_t b = 2 * (size_t)a.oc * kp + (size_t)(a.oc + 3) / 4 * 4;
+    // (an aligned A of whole vectors needs none: the pointer decides at the call)
+    return b + (size_t)a.m * ((a.ic + 3) / 4 * 4);
+}
+
+// Which planes of B are made is decided with the sizes of the product. Rows of A that the TMA cannot
+// address are copied to a pitch that it can: a 230 x 617 x 1974 product takes 22.5 us, 556 on the CUDA cores.
+int launch_matmul_f32(
+        ConvF32Args a, const float* src, const float* b, float* c, float* scratch, cudaStream_t st) {
+    const F32Choice choice = choose_f32_tile(a, a.ic > 16 && a.oc > 64);
+    const int kp = conv_f32_padded_ic(a.ic);
+    float* packed = scratch;
+    if (product_pads(a.ic, src)) {
+        float* rows = scratch + 2 * (size_t)a.oc * kp + (size_t)(a.oc + 3) / 4 * 4;
+        a.src_pitch = (a.ic + 3) / 4 * 4;
+        const size_t total = (size_t)a.m * a.src_pitch;
+        launch_pdl(Writes{rows, total * 4}, pad_rows_f32_kernel, dim3(grid_1d(total / 4, 256)), dim3(256), 0,
+                   st, src, reinterpret_cast<float4*>(rows), (long long)a.m, a.ic, (int)a.src_pitch / 4);
+        const int rc = check_launch("pad_rows_f32");
+        if (rc)
+            return rc;
+        src = rows;
+    }
+    const int rc = choice.half ? launch_matmul_f32_pack_half(a.ic, a.oc, b, packed, st)
+                               : launch_matmul_f32_pack_split(a.ic, a.oc, b, packed, st);
+    return rc ? rc : launch_f32_tensor(a, src, packed, packed, choice, nullptr, nullptr, c, st);
 }
 
 }  // namespace mb200

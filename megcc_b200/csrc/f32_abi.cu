@@ -189,6 +189,40 @@ int mb200_matmul_f32(
                                     MB200_ALGO_AUTO, stream);
 }
 
+static int product_args(int m, int n, int k, ConvF32Args* a) {
+    mb200_conv_f32_param p;
+    const int rc = matmul_f32_param(m, n, k, &p);
+    return rc ? rc : make_f32_args(&p, 0, a);
+}
+
+size_t mb200_matmul_f32_scratch_bytes(int m, int n, int k) {
+    ConvF32Args a{};
+    return product_args(m, n, k, &a) ? 0 : up256(matmul_f32_scratch_floats(a) * sizeof(float));
+}
+
+int mb200_matmul_f32_product(
+        int m, int n, int k, const float* a, const float* b, float* c, void* scratch,
+        size_t scratch_bytes, void* stream) {
+    ConvF32Args args{};
+    const int rc = product_args(m, n, k, &args);
+    if (rc)
+        return rc;
+    if (!a || !b || !c || !scratch)
+        return set_error(ST_NULL_PTR, "matmul operand or scratch pointer is NULL");
+    if (((uintptr_t)a | (uintptr_t)b | (uintptr_t)c) & 3)
+        return set_error(ST_INVALID_LAYOUT, "fp32 operands must be 4-byte aligned");
+    if ((uintptr_t)scratch & 15)
+        return set_error(ST_INVALID_LAYOUT, "scratch must be 16-byte aligned");
+    if (scratch_bytes < mb200_matmul_f32_scratch_bytes(m, n, k))
+        return set_error(ST_OUT_OF_RANGE, "scratch of %zu bytes is too small", scratch_bytes);
+    cudaStream_t st = (cudaStream_t)stream;
+    if (((uintptr_t)c & 15) == 0)
+        return launch_matmul_f32(args, a, b, c, (float*)scratch, st);
+    // (a result that no vector store reaches: the general kernel)
+    const int pack = mb200_matmul_f32_pack_b(k, n, b, (float*)scratch, stream);
+    return pack ? pack : mb200_matmul_f32(m, n, k, a, (const float*)scratch, c, nullptr, 0, stream);
+}
+
 int mb200_elemwise_f32(
         int mode, const float* a, const float* b, float* dst, size_t nr_elem, void* stream) {
     const bool unary = mode >= MB200_ELEM_RELU && mode <= MB200_ELEM_EXP;

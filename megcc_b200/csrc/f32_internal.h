@@ -5,6 +5,8 @@
 #include <stdint.h>
 #include <string.h>
 
+#include <cuda.h>
+
 #include "../../include/megcc_b200.h"
 #include "internal.h"
 
@@ -25,6 +27,18 @@ int conv_f32_padded_ic(int ic);
 // does the packed filter of this shape consist of the two tf32 planes (else: plain K-major)?
 bool conv_f32_split_eligible(const ConvF32Args& a);
 size_t conv_f32_split_filter_floats(const ConvF32Args& a);
+// fp16 planes for the wide layers (conv_f32_half.cu), behind the tf32 planes of the filters that have them
+bool conv_f32_half_planes(const ConvF32Args& a);
+size_t conv_f32_half_filter_floats(const ConvF32Args& a);
+int launch_conv_f32_pack_filter_half(
+        const ConvF32Args& a, const float* flt_oihw, float* out, cudaStream_t st);
+int launch_matmul_f32_pack_half(int k, int n, const float* b, float* out, cudaStream_t st);
+size_t matmul_f32_scratch_floats(const ConvF32Args& a);
+int launch_matmul_f32(
+        ConvF32Args a, const float* src, const float* b, float* c, float* scratch, cudaStream_t st);
+int launch_conv_f32_half(
+        const ConvF32Args& a, const CUtensorMap& map_a, bool a_tiled, const float* planes,
+        const float* bias, const float* z, float* dst, cudaStream_t st);
 bool conv_f32_umma_supported(const ConvF32Args& a, const float* src, const float* dst);
 int launch_conv_f32_pack_filter_split(
         const ConvF32Args& a, const float* flt_oihw, float* out, cudaStream_t st);

@@ -245,14 +245,14 @@ def conv_bias_f32_nhwc(p, src, flt_packed, bias=None, z=None, dst=None, dst_pitc
 
 
 def matmul_f32(a, b):
-    """C = A[M, K] @ B[K, N] (fp32 device tensors) through pack + product."""
+    """C = A[M, K] @ B[K, N] (fp32 device tensors)."""
     m, k = a.shape
     n = b.shape[1]
-    f, st = fast(), _stream()
-    packed = a.new_empty(f.mb200_matmul_f32_packed_b_bytes(k, n) // 4, dtype=torch.float32)
-    check(f.mb200_matmul_f32_pack_b(k, n, _ptr(b), _ptr(packed), st))
+    f = fast()
+    nbytes = f.mb200_matmul_f32_scratch_bytes(m, n, k)
+    scratch = a.new_empty(nbytes // 4, dtype=torch.float32)
     c = a.new_empty((m, n), dtype=torch.float32)
-    check(f.mb200_matmul_f32(m, n, k, _ptr(a), _ptr(packed), _ptr(c), None, 0, st))
+    check(f.mb200_matmul_f32_product(m, n, k, _ptr(a), _ptr(b), _ptr(c), scratch.data_ptr(), nbytes, _stream()))
     return c
 
 

@@ -350,3 +350,70 @@ def test_concat_slices_in_place_match_oracle(ops, oracle, batch, form):
         for n, w in zip(net.output_names(), want):
             close(net.output(n, dtype=np.float32).reshape(w.shape), w)
     net.close()
+
+
+# the kernel on fp16 planes (128-column tiles): a last segment of half the elements, channels beside 32, one
+# and several tile columns, a resident filter, strides, residual step, pitches; and pixels whose magnitudes
+# lie far apart, which share a filter but not a scale
+@pytest.mark.parametrize("case", [(9, 32, 128, 12, 11, 3, 1), (2, 36, 72, 30, 30, 1, 1), (2, 96, 200, 17, 19, 3, 2),
+                                  (9, 64, 129, 9, 7, 3, 1), (160, 128, 128, 13, 13, 1, 1), (1, 256, 256, 14, 13, 3, 1)],
+                         ids=lambda c: "x".join(map(str, c)))
+@pytest.mark.parametrize("form", ["SILU", "residual", "far apart"])
+def test_fp16_planes_match_64_bits(ops, oracle, case, form):
+    n, ic, oc, h, w, k, stride = case
+    r = cases.rng_for(f"f32_half_{case}_{form}")
+    src = r.standard_normal((n, ic, h, w)).astype(np.float32)
+    flt = (r.standard_normal((oc, ic, k, k)) / np.sqrt(ic * k * k)).astype(np.float32)
+    if form == "far apart":
+        src *= np.exp2(r.integers(-60, 60, (n, 1, h, w))).astype(np.float32)
+        flt *= np.exp2(r.integers(-40, 40, (oc, 1, 1, 1))).astype(np.float32)
+        flt[0] = 0
+    act = "SILU" if form == "SILU" else "IDENTITY"
+    bias = None if form == "far apart" else r.standard_normal(oc).astype(np.float32)
+    p = ops.conv_f32_param(n, ic, h, w, oc, k, k, stride, k // 2, 1, act)
+    x64, f64 = torch.from_numpy(src).double(), torch.from_numpy(flt).double()
+    want = torch.nn.functional.conv2d(x64, f64, None if bias is None else torch.from_numpy(bias).double(),
+                                      stride=stride, padding=k // 2)
+    z = None
+    if form == "SILU":
+        want = want * torch.sigmoid(want)
+    elif form == "residual":
+        z = r.standard_normal(tuple(want.permute(0, 2, 3, 1).shape)).astype(np.float32)
+        want = want + torch.from_numpy(z).double().permute(0, 3, 1, 2)
+    # the terms of one output, in magnitude: every rounding is relative to them. 2^-22 for the split, 2^-24 for
+    # each of at most 36 segment sums and the truncations of a segment's chain; in all below 2^-19
+    terms = torch.nn.functional.conv2d(x64.abs(), f64.abs(), stride=stride, padding=k // 2)
+    old = ops.set_option("f32_half", 2)
+    try:
+        got = ops.conv_bias_f32_nhwc(p, ops.nchw_to_nhwc_f32(dev(src)), ops.pack_filter_f32(p, dev(flt)),
+                                     None if bias is None else dev(bias), z=None if z is None else dev(z),
+                                     algo="umma")
+    finally:
+        ops.set_option("f32_half", old)
+    err = (got.cpu().double().permute(0, 3, 1, 2) - want).abs()
+    slack = 0 if form == "far apart" else 1e-5 * (1 + want.abs())  # bias, activation and residual in fp32
+    assert bool((err <= terms * 2.0 ** -19 + slack).all())
+    assert ops.device_status() == 0
+
+
+# products whose rows the TMA cannot address are copied to a pitch that it can; a result off the vector
+# boundary, every remainder of k, both planes' choices
+@pytest.mark.parametrize("shape", [(130, 65, 63), (1, 7, 5), (128, 64, 1), (257, 300, 1026), (2100, 260, 130)],
+                         ids=lambda c: "x".join(map(str, c)))
+@pytest.mark.parametrize("half", [0, 1, 2])
+@pytest.mark.parametrize("offset", [0, 1])
+def test_fp32_products_of_any_depth(ops, shape, half, offset):
+    m, n, k = shape
+    r = cases.rng_for(f"f32_any_depth_{shape}")
+    room = torch.zeros(m * k + offset, device="cuda")
+    a = room[offset:].view(m, k)
+    a.copy_(dev(r.standard_normal((m, k)).astype(np.float32)))
+    b = dev(r.standard_normal((k, n)).astype(np.float32))
+    old = ops.set_option("f32_half", half)
+    try:
+        got = ops.matmul_f32(a, b)
+    finally:
+        ops.set_option("f32_half", old)
+    want, terms = a.double() @ b.double(), a.double().abs() @ b.double().abs()
+    assert bool(((got.double() - want).abs() <= terms * 2.0 ** -19).all())
+    assert ops.device_status() == 0
