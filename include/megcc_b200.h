@@ -94,7 +94,7 @@ MB200_API const char* mb200_last_error(void);
  * "patch_alone" 0|1, "patch_plain" 0|1, "epilogue_forms" 1|0, "gather" 0|1|2, "nchw_store" 0|1|2,
  * "dw_tensor" 1|0, "dw_out" 0|2|4,
  * "dw_one_output" 0|1, "fast_requant" 1|0, "f32_bn" 0|32|64|128, "f32_split" 0|1|2|4|8,
- * "f32_half" 0|1|2, "debug" 0|1,
+ * "f32_half" 0|1|2, "f32_patch" 0|1|2, "debug" 0|1,
  * "pdl" 1|0 (programmatic dependent launch of consecutive kernels). Their initial values come from
  * the environment variables of the same meaning (MB200_CONV_BN, ...), read ONCE per process; no
  * launch consults the environment. Every setting yields bit-identical int8 results; the three of the

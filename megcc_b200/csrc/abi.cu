@@ -121,6 +121,7 @@ const TuningField kTuningFields[] = {
         {"conv_csplit", "MB200_CONV_CSPLIT", &Tuning::conv_csplit, false},
         {"f32_bn", "MB200_F32_BN", &Tuning::f32_bn, false},
         {"f32_half", "MB200_F32_HALF", &Tuning::f32_half, false},
+        {"f32_patch", "MB200_F32_PATCH", &Tuning::f32_patch, false},
         {"f32_split", "MB200_F32_SPLIT", &Tuning::f32_split, false},
         {"gather", "MB200_GATHER", &Tuning::gather, false},
         {"nchw_store", "MB200_NCHW_STORE", &Tuning::nchw_store, false},

@@ -1026,7 +1026,8 @@ int conv_f32_padded_ic(int ic) {
 
 size_t conv_f32_split_filter_floats(const ConvF32Args& a) {
     return 2 * (size_t)a.oc * a.kh * a.kw * conv_f32_padded_ic(a.ic) +
-           (conv_f32_half_planes(a) ? conv_f32_half_filter_floats(a) : 0);
+           (conv_f32_half_planes(a) ? conv_f32_half_filter_floats(a) : 0) +
+           (conv_f32_patch_shape(a) ? conv_f32_patch_filter_floats(a) : 0);
 }
 // Filters that 128-channel tiles can be taken for (rows of 128 bytes, more than 64 channels) hold the fp16
 // planes as well: which kernel runs is known only with the batch. (Not the second operand of a matrix
@@ -1077,9 +1078,13 @@ int launch_conv_f32_pack_filter_split(
     const size_t plane = (size_t)a.oc * a.kh * a.kw * icp;
     pack_filter_f32_kernel<<<grid_1d(plane, 256), 256, 0, st>>>(flt_oihw, out, a.oc, a.ic, icp,
                                                                  a.kh, a.kw);
-    const int rc = check_launch("pack_filter_f32");
-    return rc || !conv_f32_half_planes(a) ? rc
-                                          : launch_conv_f32_pack_filter_half(a, flt_oihw, out + 2 * plane, st);
+    int rc = check_launch("pack_filter_f32");
+    out += 2 * plane;
+    if (!rc && conv_f32_half_planes(a)) {
+        rc = launch_conv_f32_pack_filter_half(a, flt_oihw, out, st);
+        out += conv_f32_half_filter_floats(a);
+    }
+    return rc || !conv_f32_patch_shape(a) ? rc : launch_conv_f32_pack_filter_patch(a, flt_oihw, out, st);
 }
 
 int launch_conv_f32_pack_filter_plain(
@@ -1216,9 +1221,11 @@ int launch_conv_f32_umma(
         const ConvF32Args& a, const float* src, const float* flt_split, const float* bias,
         const float* z, float* dst, cudaStream_t st) {
     const bool has = conv_f32_half_planes(a);
-    const size_t split = 2 * (size_t)a.oc * a.kh * a.kw * conv_f32_padded_ic(a.ic);
-    return launch_f32_tensor(a, src, flt_split, has ? flt_split + split : nullptr, choose_f32_tile(a, has),
-                             bias, z, dst, st);
+    const float* planes = flt_split + 2 * (size_t)a.oc * a.kh * a.kw * conv_f32_padded_ic(a.ic);
+    if (conv_f32_patch_shape(a) && !tuning().f32_bn && !tuning().f32_split && conv_f32_patch_pays(a) &&
+        ((uintptr_t)flt_split & 15) == 0)
+        return launch_conv_f32_patch(a, src, planes + (has ? conv_f32_half_filter_floats(a) : 0), bias, z, dst, st);
+    return launch_f32_tensor(a, src, flt_split, has ? planes : nullptr, choose_f32_tile(a, has), bias, z, dst, st);
 }
 
 // ---- a matrix product with both operands as the caller has them ----

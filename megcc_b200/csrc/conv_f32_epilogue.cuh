@@ -1,4 +1,4 @@
-// The epilogue that the fp32 tensor-core kernels share (conv_f32.cu, conv_f32_half.cu).
+// The epilogue that the fp32 tensor-core kernels share (conv_f32.cu, conv_f32_half.cu, conv_f32_patch.cu).
 #pragma once
 #include <stdint.h>
 

@@ -33,6 +33,15 @@ size_t conv_f32_half_filter_floats(const ConvF32Args& a);
 int launch_conv_f32_pack_filter_half(
         const ConvF32Args& a, const float* flt_oihw, float* out, cudaStream_t st);
 int launch_matmul_f32_pack_half(int k, int n, const float* b, float* out, cudaStream_t st);
+// 3x3, stride 1, padding 1 from halo patches (conv_f32_patch.cu)
+bool conv_f32_patch_shape(const ConvF32Args& a);
+bool conv_f32_patch_pays(const ConvF32Args& a);
+size_t conv_f32_patch_filter_floats(const ConvF32Args& a);
+int launch_conv_f32_pack_filter_patch(
+        const ConvF32Args& a, const float* flt_oihw, float* out, cudaStream_t st);
+int launch_conv_f32_patch(
+        const ConvF32Args& a, const float* src, const float* planes, const float* bias,
+        const float* z, float* dst, cudaStream_t st);
 size_t matmul_f32_scratch_floats(const ConvF32Args& a);
 int launch_matmul_f32(
         ConvF32Args a, const float* src, const float* b, float* c, float* scratch, cudaStream_t st);

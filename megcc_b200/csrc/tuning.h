@@ -17,6 +17,7 @@ struct Tuning {
     int conv_csplit = 0;    // MB200_CONV_CSPLIT    0 = by shape, 1 | 2 | 4 | 8 = CTAs of a cluster per tile's K loop
     int f32_bn = 0;         // MB200_F32_BN         0 = by shape, 32 | 64 | 128 = that fp32 tile width
     int f32_half = 1;       // MB200_F32_HALF       0 = never the kernel on fp16 planes, 2 = wherever its filter is there
+    int f32_patch = 1;      // MB200_F32_PATCH      0 = no halo patches for fp32 3x3 layers, 2 = wherever they can be
     int f32_split = 0;      // MB200_F32_SPLIT      0 = by shape, 1 | 2 | 4 | 8 = CTAs per tile's K loop
     int gather = 1;         // MB200_GATHER         0 = never operands by ordinary loads, 2 = wherever they can be
     int nchw_store = 1;     // MB200_NCHW_STORE     0 = NCHW results by a transposing kernel, 2 = never by one

@@ -417,3 +417,45 @@ def test_fp32_products_of_any_depth(ops, shape, half, offset):
     want, terms = a.double() @ b.double(), a.double().abs() @ b.double().abs()
     assert bool(((got.double() - want).abs() <= terms * 2.0 ** -19).all())
     assert ops.device_status() == 0
+
+
+# fp32 3x3 layers from halo patches: images below, at and beside one patch (16 x 8), channels that fill a part of
+# a 64-channel block, a 16- and a 32-channel step, one and several tile columns and blocks, results off the
+# vector boundary; pixels whose magnitudes lie far apart share a filter but not a scale
+@pytest.mark.parametrize("case", [(16, 16, 8, 16, 8), (7, 32, 32, 17, 9), (61, 36, 33, 5, 3), (2, 64, 64, 33, 23),
+                                  (2, 132, 72, 15, 16), (300, 128, 128, 1, 1), (1, 196, 257, 20, 20),
+                                  (40, 32, 30, 32, 40)], ids=lambda c: "x".join(map(str, c)))
+@pytest.mark.parametrize("form", ["SILU", "residual", "far apart"])
+def test_fp32_halo_patches_match_64_bits(ops, case, form):
+    n, ic, oc, h, w = case
+    r = cases.rng_for(f"f32_patch_{case}_{form}")
+    src = r.standard_normal((n, ic, h, w)).astype(np.float32)
+    flt = (r.standard_normal((oc, ic, 3, 3)) / np.sqrt(ic * 9)).astype(np.float32)
+    if form == "far apart":
+        src *= np.exp2(r.integers(-60, 60, (n, 1, h, w))).astype(np.float32)
+        flt *= np.exp2(r.integers(-40, 40, (oc, 1, 1, 1))).astype(np.float32)
+        flt[0] = 0
+    bias = None if form == "far apart" else r.standard_normal(oc).astype(np.float32)
+    p = ops.conv_f32_param(n, ic, h, w, oc, 3, 3, 1, 1, 1, "SILU" if form == "SILU" else "IDENTITY")
+    x64, f64 = torch.from_numpy(src).double(), torch.from_numpy(flt).double()
+    want = torch.nn.functional.conv2d(x64, f64, None if bias is None else torch.from_numpy(bias).double(), padding=1)
+    z = None
+    if form == "SILU":
+        want = want * torch.sigmoid(want)
+    elif form == "residual":
+        z = r.standard_normal(tuple(want.permute(0, 2, 3, 1).shape)).astype(np.float32)
+        want = want + torch.from_numpy(z).double().permute(0, 3, 1, 2)
+    # as above: 2^-22 for the split, 2^-24 for each of at most 36 segment sums, the truncations of a chain
+    terms = torch.nn.functional.conv2d(x64.abs(), f64.abs(), padding=1)
+    slack = 0 if form == "far apart" else 1e-5 * (1 + want.abs())  # bias, activation and residual in fp32
+    x, f = ops.nchw_to_nhwc_f32(dev(src)), ops.pack_filter_f32(p, dev(flt))
+    for mode in (0, 1, 2):
+        old = ops.set_option("f32_patch", mode)
+        try:
+            got = ops.conv_bias_f32_nhwc(p, x, f, None if bias is None else dev(bias),
+                                         z=None if z is None else dev(z), algo="umma")
+        finally:
+            ops.set_option("f32_patch", old)
+        err = (got.cpu().double().permute(0, 3, 1, 2) - want).abs()
+        assert bool((err <= terms * 2.0 ** -19 + slack).all()), (mode, float((err / terms).max()))
+    assert ops.device_status() == 0
