@@ -68,7 +68,9 @@ constexpr int kThreads = 64 + 32 * (kEpilogueWarps + kConverterWarps);
 // converters' largest values (two segments, two halves); each epilogue warp's bias and channel factors
 constexpr int kFactorOff = 1024, kMostOff = kFactorOff + 8 * kBM * 4;
 constexpr int kBiasOff = kMostOff + 4 * kBM * 4;
-constexpr int kFrontBytes = (kBiasOff + kEpilogueWarps * kBN / 2 * 8 + 1023) / 1024 * 1024;
+constexpr int kTurn = 16;     // columns of a result turned round at a time
+constexpr int kTurnOff = kBiasOff + kEpilogueWarps * kBN / 2 * 8;
+constexpr int kFrontBytes = (kTurnOff + kEpilogueWarps * 32 * kTurn * 4 + 1023) / 1024 * 1024;
 constexpr int kTileBudget = 227 * 1024 - 1024 - kFrontBytes;  // (1024: alignment)
 constexpr int kDynamic = 227 * 1024;
 
@@ -530,11 +532,7 @@ __global__ void __launch_bounds__(kThreads, 1) conv_f32_half_kernel(
         constexpr int kCols = kBN / 2;       // columns of this warp
         float* bias_row = reinterpret_cast<float*>(smem + kBiasOff) + (warp - 2) * 2 * kCols;
         float* factor_row = bias_row + kCols;
-        const float4* bias = reinterpret_cast<const float4*>(bias_row);
-        // 16- and 32-byte accesses: every row starts on such a boundary when the first does
-        const bool vec4 = ((p.ep.dst_pitch | (p.ep.z ? p.ep.z_pitch : 0)) & 3) == 0 &&
-                          (((uintptr_t)p.ep.dst | (uintptr_t)p.ep.z) & 15) == 0;
-        const bool vec8 = vec4 && (p.ep.dst_pitch & 7) == 0 && ((uintptr_t)p.ep.dst & 31) == 0;
+        const uint32_t turned_w = smem_u32(smem + kTurnOff) + (warp - 2) * (32 * kTurn * 4);
         uint32_t turn = 0;
         bool ok = true;
         if (lane == 0) {  // the accumulators of the first two segments are free
@@ -597,14 +595,10 @@ __global__ void __launch_bounds__(kThreads, 1) conv_f32_half_kernel(
             }
             if (!ok)
                 break;
-            if (m < p.m_total && n0 + half * kCols < p.oc) {
-#pragma unroll
-                for (int j = 0; j < kCols; ++j)  // (a power of two: exact)
-                    sum[j] = __fmul_rn(sum[j], factor_row[j]);
-                with_act(p.ep.act, [&](auto a) {
-                    store_f32_row<kCols, decltype(a)::value>(sum, p.ep, bias, (size_t)m,
-                                                             n0 + half * kCols, vec4, vec8);
-                });
+            if (n0 + half * kCols < p.oc) {
+                const F32RowsInLine rows{(size_t)(m - lane), (size_t)p.m_total};
+                store_f32_rows<kCols, kTurn, true>(sum, p.ep, turned_w, factor_row, bias_row, rows,
+                                                   n0 + half * kCols);
             }
         }
     }

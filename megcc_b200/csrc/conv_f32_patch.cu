@@ -162,92 +162,16 @@ struct TilePos {
     }
 };
 
-// A warp's rows (four rows of eight pixels, one pixel per lane), TURN columns at a time, turned round in shared
-// memory, so that a warp's accesses to the result (and to z) are whole rows of the tile: a lane per row
-// stored 32-byte sectors at the same place of 32 lines, which took the shared-memory pipe, that the MMAs read
-// their operands by, three clocks each. 320 x 320, 16 -> 32:
-// 430 us with a row of the turned tile at a time, 370 with four.
-// FORM 0: whole 16-byte units, no z; 1: whole units and z; 2: any
-template <int COLS, int TURN, int ACT, int FORM>
-__device__ __forceinline__ void store_turned(
-        const float (&sum)[COLS], const PatchF32Params& p, uint32_t buffer, const float* scales, const float* biases,
-        const TilePos& at, int q, int ch0) {
-    constexpr int kUnits = TURN / 4;         // 16-byte units of a row
-    constexpr int kRows = 32 / kUnits;       // rows of an access
-    const int lane = threadIdx.x & 31;
-    const int unit = lane % kUnits;
-    // unit u of row r sits at unit u ^ swizzle(r): every eight lanes' accesses take all banks
-    auto swizzle = [](int r) { return TURN == 32 ? r & 7 : r >> 1 & 3; };
-    const int y0 = at.y0 + q * 4, x0 = at.x0 + lane / kUnits;
-    const size_t m0 = ((size_t)at.img * p.oh + y0) * p.ow + x0;
-    float* out0 = p.ep.dst + m0 * p.ep.dst_pitch + ch0 + unit * 4;
-    const float* z0 = FORM != 0 && p.ep.z ? p.ep.z + m0 * p.ep.z_pitch + ch0 + unit * 4 : nullptr;
-#pragma unroll
-    for (int c = 0; c < COLS / TURN; ++c) {
-        const int ch = ch0 + c * TURN + unit * 4;
-        if (ch0 + c * TURN >= p.oc)
-            break;
-        __syncwarp();
-#pragma unroll
-        for (int u = 0; u < kUnits; ++u)
-            asm volatile("st.shared.v4.f32 [%0], {%1, %2, %3, %4};" ::"r"(
-                                 buffer + (lane * kUnits + (u ^ swizzle(lane))) * 16),
-                         "f"(sum[c * TURN + 4 * u]), "f"(sum[c * TURN + 4 * u + 1]),
-                         "f"(sum[c * TURN + 4 * u + 2]), "f"(sum[c * TURN + 4 * u + 3])
-                         : "memory");
-        __syncwarp();
-        const float4 scale = *reinterpret_cast<const float4*>(scales + c * TURN + unit * 4);
-        const float4 bias = *reinterpret_cast<const float4*>(biases + c * TURN + unit * 4);
-        // (several rows at a time: one by one they are a chain of 400 clocks each)
-        constexpr int kAtOnce = FORM == 0 ? 4 : FORM == 1 ? 2 : 1;
-#pragma unroll
-        for (int h = 0; h < kUnits; h += kAtOnce) {
-            float4 v[kAtOnce], add[kAtOnce];
-#pragma unroll
-            for (int i = 0; i < kAtOnce; ++i) {
-                const int r = (h + i) * kRows + lane / kUnits;
-                asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];"
-                             : "=f"(v[i].x), "=f"(v[i].y), "=f"(v[i].z), "=f"(v[i].w)
-                             : "r"(buffer + (r * kUnits + (unit ^ swizzle(r))) * 16));
-                if (FORM == 1) {
-                    const int dy = (h + i) * kRows >> 3, dx = (h + i) * kRows & 7;
-                    add[i] = make_float4(0.f, 0.f, 0.f, 0.f);
-                    if (y0 + dy < p.oh && x0 + dx < p.ow && ch < p.oc)
-                        add[i] = *reinterpret_cast<const float4*>(z0 + (dy * p.ow + dx) * p.ep.z_pitch + c * TURN);
-                }
-            }
-#pragma unroll
-            for (int i = 0; i < kAtOnce; ++i) {
-                // (the scale is a power of two: exact)
-                v[i].x = act_f32<ACT>(__fmul_rn(v[i].x, scale.x) + bias.x);
-                v[i].y = act_f32<ACT>(__fmul_rn(v[i].y, scale.y) + bias.y);
-                v[i].z = act_f32<ACT>(__fmul_rn(v[i].z, scale.z) + bias.z);
-                v[i].w = act_f32<ACT>(__fmul_rn(v[i].w, scale.w) + bias.w);
-                if (FORM == 1)
-                    v[i].x += add[i].x, v[i].y += add[i].y, v[i].z += add[i].z, v[i].w += add[i].w;
-            }
-#pragma unroll
-            for (int i = 0; i < kAtOnce; ++i) {
-                const int dy = (h + i) * kRows >> 3, dx = (h + i) * kRows & 7;
-                if (!(y0 + dy < p.oh && x0 + dx < p.ow && ch < p.oc))
-                    continue;
-                float* out = out0 + (dy * p.ow + dx) * p.ep.dst_pitch + c * TURN;
-                if (FORM != 2) {
-                    *reinterpret_cast<float4*>(out) = v[i];
-                } else {
-                    const float* z = z0 ? z0 + (dy * p.ow + dx) * p.ep.z_pitch + c * TURN : nullptr;
-                    out[0] = z ? v[i].x + z[0] : v[i].x;
-                    if (ch + 1 < p.oc)
-                        out[1] = z ? v[i].y + z[1] : v[i].y;
-                    if (ch + 2 < p.oc)
-                        out[2] = z ? v[i].z + z[2] : v[i].z;
-                    if (ch + 3 < p.oc)
-                        out[3] = z ? v[i].w + z[3] : v[i].w;
-                }
-            }
-        }
+// A warp's rows: four of the patch, eight pixels each (a lane's own first row lies in the first of them)
+struct PatchRows {
+    const PatchF32Params& p;
+    size_t first;
+    int y0, x0;
+    __device__ __forceinline__ bool there(int row0, int row) const {
+        return y0 + (row >> 3) < p.oh && x0 + row0 + (row & 7) < p.ow;
     }
-}
+    __device__ __forceinline__ int step(int row) const { return (row >> 3) * p.ow + (row & 7); }
+};
 
 // OIHW fp32 -> the filter's planes and factors, a block per channel of the (padded) tile columns
 __global__ void __launch_bounds__(256) pack_filter_patch_kernel(
@@ -544,9 +468,6 @@ __global__ void __launch_bounds__(Cfg<BN>::kThreads, 1) conv_f32_patch_kernel(
         constexpr int kCols = C::kCols;
         const int col0 = (warp - 2) / 4 * kCols;  // this warp's columns
         const uint32_t turned_w = smem_u32(turned) + (warp - 2) * C::kTurnBytes;
-        // 16-byte accesses: every row starts on such a boundary when the first does
-        const bool vec4 = ((p.ep.dst_pitch | (p.ep.z ? p.ep.z_pitch : 0)) & 3) == 0 &&
-                          (((uintptr_t)p.ep.dst | (uintptr_t)p.ep.z) & 15) == 0 && (p.oc & 3) == 0;
         float* channels = reinterpret_cast<float*>(smem + C::kChannelOff) + col0;  // [2][factor, bias][BN]
         uint32_t turn = 0, plane_turn = 0;
         int set = 1;
@@ -634,19 +555,10 @@ __global__ void __launch_bounds__(Cfg<BN>::kThreads, 1) conv_f32_patch_kernel(
                 break;
             if (at.n0 + col0 < p.oc) {
                 const float* channel = channels + set * 2 * BN;
-                with_act(p.ep.act, [&](auto a) {
-                    constexpr int kAct = decltype(a)::value;
-                    auto store = [&](auto form) {
-                        store_turned<kCols, C::kTurn, kAct, decltype(form)::value>(
-                                sum, p, turned_w, channel, channel + BN, at, q, at.n0 + col0);
-                    };
-                    if (!vec4)
-                        store(Number<2>());
-                    else if (p.ep.z)
-                        store(Number<1>());
-                    else
-                        store(Number<0>());
-                });
+                const int y0 = at.y0 + q * 4;
+                const PatchRows rows{p, ((size_t)at.img * p.oh + y0) * p.ow + at.x0, y0, at.x0};
+                store_f32_rows<kCols, C::kTurn, true>(sum, p.ep, turned_w, channel, channel + BN, rows,
+                                                      at.n0 + col0);
             }
         }
     }
