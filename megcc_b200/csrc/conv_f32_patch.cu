@@ -317,6 +317,8 @@ __global__ void __launch_bounds__(Cfg<BN>::kThreads, 1) conv_f32_patch_kernel(
                 const uint32_t buf = plane_turn & 1;
                 ok = __all_sync(0xffffffffu,
                                 mbar_wait_u32(plane_full_a + 8 * buf, (plane_turn >> 1) & 1u, abort_flag));
+                if (!ok)
+                    break;  // (the next wait may well succeed: filter and accumulators know nothing of the planes)
                 const uint32_t a_block = a_first + buf * 2 * kAPlane;
                 const int left = p.ic - block * kBlock;
                 const int steps = left >= kBlock ? kBlock / 16 : (left + 15) / 16;
