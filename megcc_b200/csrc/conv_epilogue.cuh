@@ -683,6 +683,7 @@ __device__ __forceinline__ void epilogue_form_chunk(
 #pragma unroll 1
         for (int h = 0; h < 32; h += 16) {
             uint32_t v[16];
+            __syncwarp();
             umma::tmem_ld16(taddr + (uint32_t)h, v);
             if (h != 0 && release_bar) {
                 asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
@@ -694,6 +695,7 @@ __device__ __forceinline__ void epilogue_form_chunk(
         return;
     }
     uint32_t lo[16], hi[16], packed[8], zw[8];
+    __syncwarp();
     umma::tmem_ld16_nowait(taddr, lo);
     if (kMode == 2 && valid)
         asm volatile("ld.global.nc.v8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"

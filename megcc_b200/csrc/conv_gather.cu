@@ -377,33 +377,34 @@ __global__ void __launch_bounds__(kThreads, 3) conv_gather_kernel(const GatherPa
             for (int c = 0; c < 2; ++c) {
                 const int col = half * 32 + c * 16;
                 uint32_t v[16];
+                __syncwarp();
                 tmem_ld16(tmem_base + ((uint32_t)(q * 32) << 16) + (uint32_t)col, v);
-                if (mo >= p.m_total)
-                    continue;
+                if (mo < p.m_total) {
 #pragma unroll
-                for (int j = 0; j < 4; ++j) {
-                    const int c0 = n0 + col + 4 * j;
-                    if (c0 >= p.oc)
-                        break;
-                    const int acc[4] = {(int)v[4 * j], (int)v[4 * j + 1], (int)v[4 * j + 2],
-                                        (int)v[4 * j + 3]};
-                    const QuadParams qp = side[(col >> 2) + j];
-                    if constexpr (MODE == GATHER_NCHW) {
-                        const uint32_t word = quad_values(acc, p.ep, qp, 0);
-                        int8_t* out = p.dst + ((size_t)oimg * p.oc + c0) * pixels + opix;
+                    for (int j = 0; j < 4; ++j) {
+                        const int c0 = n0 + col + 4 * j;
+                        if (c0 >= p.oc)
+                            break;
+                        const int acc[4] = {(int)v[4 * j], (int)v[4 * j + 1], (int)v[4 * j + 2],
+                                            (int)v[4 * j + 3]};
+                        const QuadParams qp = side[(col >> 2) + j];
+                        if constexpr (MODE == GATHER_NCHW) {
+                            const uint32_t word = quad_values(acc, p.ep, qp, 0);
+                            int8_t* out = p.dst + ((size_t)oimg * p.oc + c0) * pixels + opix;
 #pragma unroll
-                        for (int i = 0; i < 4; ++i)
-                            if (c0 + i < p.oc)
-                                out[(size_t)i * pixels] = (int8_t)(word >> (8 * i));
-                    } else {
-                        const size_t off = (size_t)mo * p.oc + c0;
-                        if (turned)
-                            *reinterpret_cast<uint32_t*>(turn + lane * kPitch + c * 16 + 4 * j) =
-                                    quad_values(acc, p.ep, qp, quad_z(p.ep, off, c0));
-                        else if (p.ep.nchw_plane)
-                            nchw_quad(acc, p.ep, qp, p.dst, off, c0);
-                        else
-                            epilogue_quad(acc, p.ep, qp, quad_z(p.ep, off, c0), p.dst, off, c0);
+                            for (int i = 0; i < 4; ++i)
+                                if (c0 + i < p.oc)
+                                    out[(size_t)i * pixels] = (int8_t)(word >> (8 * i));
+                        } else {
+                            const size_t off = (size_t)mo * p.oc + c0;
+                            if (turned)
+                                *reinterpret_cast<uint32_t*>(turn + lane * kPitch + c * 16 + 4 * j) =
+                                        quad_values(acc, p.ep, qp, quad_z(p.ep, off, c0));
+                            else if (p.ep.nchw_plane)
+                                nchw_quad(acc, p.ep, qp, p.dst, off, c0);
+                            else
+                                epilogue_quad(acc, p.ep, qp, quad_z(p.ep, off, c0), p.dst, off, c0);
+                        }
                     }
                 }
             }

@@ -327,6 +327,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1) conv_pa
 #pragma unroll 1
             for (int c = first * kChunksPerWarp; c < (first + 1) * kChunksPerWarp; ++c) {
                 uint32_t v[32];
+                __syncwarp();
                 tmem_ld32(taddr + (uint32_t)(c * 32), v);
                 if (c + 1 == (first + 1) * kChunksPerWarp) {
                     // this warp's accumulators are in registers: release the buffer (one

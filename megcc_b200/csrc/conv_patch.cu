@@ -572,6 +572,7 @@ __global__ void __launch_bounds__(64 + 32 * EW, EW == 16 ? 1 : 2) conv_patch_ker
                         mbar_arrive(release);
                 } else {
                     uint32_t v[32];
+                    __syncwarp();
                     tmem_ld32(taddr + (uint32_t)(c * 32), v);
                     if (last) {
                         asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");

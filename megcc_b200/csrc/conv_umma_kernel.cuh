@@ -476,6 +476,7 @@ __global__ void __launch_bounds__(Shape<BN>::kThreads, Shape<BN>::kMinCtas) conv
                     }
                 } else {
                     uint32_t v[32];
+                    __syncwarp();
                     tmem_ld32(taddr + (uint32_t)(c * 32), v);
                     if (c + 1 == (half + 1) * kChunksPerWarp) {
                         // all of this thread's accumulators are in registers: hand the buffer back

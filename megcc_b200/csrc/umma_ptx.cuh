@@ -321,6 +321,8 @@ __device__ __forceinline__ void umma_commit_if(uint32_t leader, uint32_t bar) {
             : "memory");
 }
 
+// Loads of tensor memory are the whole warp's (.aligned). Where its lanes part between two of them (pixels
+// beyond the result store nothing), nothing but a __syncwarp() in front of the second brings them together.
 __device__ __forceinline__ void tmem_ld32(uint32_t taddr, uint32_t (&v)[32]) {
     asm volatile(
             "tcgen05.ld.sync.aligned.32x32b.x32.b32 "
