@@ -564,7 +564,7 @@ int launch_conv_gather(
     p.status = device_status_word(st);
     if (!p.status)
         return ST_MALLOC;
-    const int grid = (a.m + kBM - 1) / kBM * p.n_tiles;
+    const int grid = ((a.m - 1) / kBM + 1) * p.n_tiles;  // (a.m may be as large as an int holds)
     switch (gather_mode(a, src, nchw)) {
         case GATHER_VEC16: return launch_mode<GATHER_VEC16>(p, grid, st);
         case GATHER_WORDS: return launch_mode<GATHER_WORDS>(p, grid, st);

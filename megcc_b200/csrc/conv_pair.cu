@@ -470,7 +470,7 @@ int launch_conv_pair(
     p.base_w = -a.pw;
     p.dh = a.dh;
     p.dw = a.dw;
-    p.m_tiles = (a.m + 2 * kBM - 1) / (2 * kBM);
+    p.m_tiles = (a.m - 1) / (2 * kBM) + 1;
     p.n_tiles = (a.oc + kBN - 1) / kBN;
     p.ep.oc = a.oc;
     p.ep.act = a.act;

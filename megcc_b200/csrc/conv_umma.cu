@@ -262,7 +262,7 @@ int launch_conv_umma_geom(
         // against 13.3 us, 704 x 5920 x 7328 (144, 282) 29.7 against 34.2; 1696 x 1088 x 3040 (70, 126)
         // 14.9 against 12.0.
         const long long k_bytes = (long long)taps * a.ic;
-        const long long m_tiles = (a.m + kBM - 1) / kBM;
+        const long long m_tiles = (a.m - 1) / kBM + 1;
         const long long sms = sm_count();
         const long long busiest256 = (m_tiles * ((a.oc + 255) / 256) + sms - 1) / sms;
         const long long busiest128 = (m_tiles * ((a.oc + 127) / 128) + sms - 1) / sms;
@@ -279,11 +279,11 @@ int launch_conv_umma_geom(
         if (force == 64 || (force == 0 && k_bytes <= 256 && bn == 128))
             bn = 64;
         // fewer tiles than SMs: narrower tiles, K split over clusters
-        const long long tiles = (long long)((a.m + kBM - 1) / kBM) * ((a.oc + bn - 1) / bn);
+        const long long tiles = (long long)((a.m - 1) / kBM + 1) * ((a.oc + bn - 1) / bn);
         const int k_iters = geom == GEOM_TAP16 ? taps / 4 : taps * ((a.ic + chans - 1) / chans);
         if (geom != GEOM_TAP16 && bn <= 128 && force == 0 && a.test_wait_cycles == 0 &&
             tiles <= sms)
-            choose_split((a.m + kBM - 1) / kBM, a.oc, k_iters, geom == GEOM_WIDE128,
+            choose_split((a.m - 1) / kBM + 1, a.oc, k_iters, geom == GEOM_WIDE128,
                          (int)sms, &bn, &csplit);
         const int fs = tuning().conv_csplit;
         if ((fs == 1 || fs == 2 || fs == 4 || fs == 8) && geom != GEOM_TAP16 && bn <= 128)
@@ -356,7 +356,7 @@ int launch_conv_umma_geom(
     p.base_w = -a.pw;
     p.dh = a.dh;
     p.dw = a.dw;
-    p.m_tiles = (a.m + kBM - 1) / kBM;
+    p.m_tiles = (a.m - 1) / kBM + 1;
     p.n_tiles = (a.oc + bn - 1) / bn;
     p.a_tiled = a_tiled ? 1 : 0;
     fill_epilogue(a, bias, flt_scales, &p.ep);

@@ -21,3 +21,11 @@ def test_the_outcome_of_a_bounded_wait_is_looked_at(path):
         if after and after.group(1) and not re.search(r"\bok\b", after.group(2)):
             forgotten.append(text[:wait.start()].count("\n") + 1)
     assert not forgotten, f"{os.path.basename(path)}: waits at lines {forgotten}"
+
+
+# An int8 ConvBias may have as many pixels as an int counts: rounding them up to tiles must not pass that.
+# (fp32: 2^30 at most.)
+@pytest.mark.parametrize("path", [p for p in SOURCES if "f32" not in os.path.basename(p)], ids=os.path.basename)
+def test_pixels_are_rounded_up_without_overflow(path):
+    text = re.sub(r"//[^\n]*", "", open(path).read())
+    assert not re.search(r"(?<!\(long long\))\ba\.m \+ ", text)
