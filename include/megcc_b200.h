@@ -354,7 +354,10 @@ typedef struct mb200_conv_f32_param {
  * compiler/lib/KernelGen/GeneralIntrinsic/ConvKernel/Fp32Im2col.cpp:88-120, body :198-217).
  * The Init step (mb200_conv_f32_pack_filter) turns the OIHW filter into the K-major form
  * [OC][KH][KW][ICpg], or, for dense filters with ic % 4 == 0 (with a spatial filter ic == 16 or
- * ic >= 32), to its two tf32 planes for the tensor cores, channels padded to whole rows. The
+ * ic >= 32), to its planes for the tensor cores, channels padded to whole rows: two tf32 ones, two fp16
+ * ones behind them with more than 64 output and 16 input channels, and two more in the order of the
+ * halo-patch kernel for 3x3 filters. What is packed follows from the filter's groups, channels and
+ * extent only, so a packed filter serves every input size, stride and padding. The
  * activation is split into its planes on chip, so the ConvBias needs no scratch:
  * mb200_conv_f32_workspace_bytes(p) answers 0 and `workspace` is not looked at (both are kept so
  * that callers written against earlier versions keep working).
@@ -377,8 +380,9 @@ MB200_API int mb200_conv_bias_f32_nhwc(
  * GI_kernel_fp32_matmul_4x12_nn, compiler/lib/KernelGen/GeneralIntrinsic/MatMulKernel/
  * Fp32MatMulM4N12.cpp:8-160). B is prepared once by mb200_matmul_f32_pack_b into
  * mb200_matmul_f32_packed_b_bytes(k, n) bytes; the product needs no scratch
- * (mb200_matmul_f32_workspace_bytes answers 0). Tensor cores (three tf32 passes) when k % 4 == 0 and
- * the operands are 16-byte aligned, whatever m and n; CUDA cores otherwise. */
+ * (mb200_matmul_f32_workspace_bytes answers 0). The packed B is the packed filter of a 1x1 ConvBias.
+ * Tensor cores when k % 4 == 0 and the operands are 16-byte aligned, whatever m and n; CUDA cores
+ * otherwise. */
 MB200_API size_t mb200_matmul_f32_packed_b_bytes(int k, int n);
 MB200_API int mb200_matmul_f32_pack_b(int k, int n, const float* b, float* b_packed, void* stream);
 MB200_API size_t mb200_matmul_f32_workspace_bytes(int m, int k);

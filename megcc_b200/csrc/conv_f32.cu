@@ -1027,23 +1027,25 @@ int conv_f32_padded_ic(int ic) {
 size_t conv_f32_split_filter_floats(const ConvF32Args& a) {
     return 2 * (size_t)a.oc * a.kh * a.kw * conv_f32_padded_ic(a.ic) +
            (conv_f32_half_planes(a) ? conv_f32_half_filter_floats(a) : 0) +
-           (conv_f32_patch_shape(a) ? conv_f32_patch_filter_floats(a) : 0);
-}
-// Filters that 128-channel tiles can be taken for (rows of 128 bytes, more than 64 channels) hold the fp16
-// planes as well: which kernel runs is known only with the batch. (Not the second operand of a matrix
-// product packed by itself: its callers pack anew with every product, and the planes cost another read.)
-bool conv_f32_half_planes(const ConvF32Args& a) {
-    const bool product = a.kh == 1 && a.kw == 1 && a.ih == 1 && a.iw == 1;
-    return conv_f32_split_eligible(a) && a.ic > 16 && a.oc > 64 && !product;
+           (conv_f32_patch_planes(a) ? conv_f32_patch_filter_floats(a) : 0);
 }
 
-// Channel counts the tensor-core kernel takes: rows the TMA can address (16-byte multiples).
+// What a packed filter holds follows from the filter's own groups, channels and extent and from nothing else:
+// a filter packed under one input, stride and padding may be used under another, and so may the second
+// operand of a matrix product as a 1x1 filter.
+//
+// The two planes: channel counts the tensor-core kernel takes, rows the TMA can address (16-byte multiples).
 // A last, partial row of 32 channels is filled with zeros by the load; the im2col form asks
 // for whole rows of a tensor at least that wide.
-bool conv_f32_split_eligible(const ConvF32Args& a) {
+bool conv_f32_split_planes(const ConvF32Args& a) {
     if (a.groups != 1 || a.ic % 4 != 0)
         return false;
-    return plain_matrix(a) || a.ic == 16 || a.ic >= 32;
+    return (a.kh == 1 && a.kw == 1) || a.ic == 16 || a.ic >= 32;
+}
+// Filters that 128-channel tiles can be taken for (rows of 128 bytes, more than 64 channels) hold the fp16
+// planes as well: which kernel runs is known only with the batch.
+bool conv_f32_half_planes(const ConvF32Args& a) {
+    return conv_f32_split_planes(a) && a.ic > 16 && a.oc > 64;
 }
 
 // Images of `src` the activation's im2col map describes (see descriptor_images in internal.h)
@@ -1059,7 +1061,7 @@ static int f32_descriptor_images(const ConvF32Args& a, const float* src) {
 // Tensor-core path: dense, an eligible channel count, 16-byte aligned operands and pitches,
 // and, with a spatial filter, 128 KiB of readable memory behind `src` for the TMA map.
 bool conv_f32_umma_supported(const ConvF32Args& a, const float* src, const float* dst) {
-    if (!conv_f32_split_eligible(a))
+    if (!conv_f32_split_planes(a) || !(plain_matrix(a) || a.ic == 16 || a.ic >= 32))
         return false;
     if (a.kh * a.kw > 49 || a.ph > 64 || a.pw > 64 || a.sh > 8 || a.sw > 8)
         return false;
@@ -1084,7 +1086,7 @@ int launch_conv_f32_pack_filter_split(
         rc = launch_conv_f32_pack_filter_half(a, flt_oihw, out, st);
         out += conv_f32_half_filter_floats(a);
     }
-    return rc || !conv_f32_patch_shape(a) ? rc : launch_conv_f32_pack_filter_patch(a, flt_oihw, out, st);
+    return rc || !conv_f32_patch_planes(a) ? rc : launch_conv_f32_pack_filter_patch(a, flt_oihw, out, st);
 }
 
 int launch_conv_f32_pack_filter_plain(
@@ -1106,10 +1108,16 @@ int launch_matmul_f32_pack_split(
     return check_launch("pack_matrix_f32");
 }
 
+int launch_matmul_f32_pack_b(const ConvF32Args& a, const float* b, float* out, cudaStream_t st) {
+    const int rc = launch_matmul_f32_pack_split(a.ic, a.oc, b, out, st);
+    out += 2 * (size_t)a.oc * conv_f32_padded_ic(a.ic);
+    return rc || !conv_f32_half_planes(a) ? rc : launch_matmul_f32_pack_half(a.ic, a.oc, b, out, st);
+}
+
 int launch_conv_f32_direct(
         const ConvF32Args& a, const float* src, const float* flt_packed, const float* bias,
         const float* z, float* dst, cudaStream_t st) {
-    const bool split = conv_f32_split_eligible(a);
+    const bool split = conv_f32_split_planes(a);
     const int icp = split ? conv_f32_padded_ic(a.ic) : a.ic / a.groups;
     const float* lo = split ? flt_packed + (size_t)a.oc * a.kh * a.kw * icp : nullptr;
     launch_pdl(Writes{dst, (size_t)a.m * a.dst_pitch * 4}, conv_f32_direct_kernel, dim3(grid_1d((size_t)a.m * a.oc, 256)), dim3(256), 0, st, a,

@@ -627,13 +627,16 @@ int launch_conv_f32_pack_filter_patch(
     return check_launch("pack_filter_f32_patch");
 }
 
-// May this ConvBias take the patch kernel? (By shape: its filter then holds the fp16 planes.)
+// Does a packed filter hold the planes of this kernel? (By the filter alone, see conv_f32_split_planes.)
+bool conv_f32_patch_planes(const ConvF32Args& a) {
+    return conv_f32_split_planes(a) && a.kh == 3 && a.kw == 3;
+}
+// ... and may the ConvBias take it?
 bool conv_f32_patch_shape(const ConvF32Args& a) {
-    return conv_f32_split_eligible(a) && a.kh == 3 && a.kw == 3 && a.sh == 1 && a.sw == 1 && a.ph == 1 &&
-           a.pw == 1;
+    return conv_f32_patch_planes(a) && a.sh == 1 && a.sw == 1 && a.ph == 1 && a.pw == 1;
 }
 
-// ... and is it the faster one? Both kernels' time goes with the tiles of the busiest SM; a patch that is not
+// ... and is it the faster one then? Both kernels' time goes with the tiles of the busiest SM; a patch that is not
 // full is paid for in full. What a patch takes beside an im2col tile of the same columns and channels, in
 // percent, was measured with full patches and 1600 to 25600 of them (us, im2col -> patches; 32 images of
 // 80 x 80 where nothing else is said):

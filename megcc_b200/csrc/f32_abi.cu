@@ -98,7 +98,7 @@ size_t mb200_conv_f32_packed_filter_bytes(const mb200_conv_f32_param* p) {
     ConvF32Args a{};
     if (make_f32_args(p, 0, &a))
         return 0;
-    return conv_f32_split_eligible(a) ? up256(conv_f32_split_filter_floats(a) * sizeof(float))
+    return conv_f32_split_planes(a) ? up256(conv_f32_split_filter_floats(a) * sizeof(float))
                                       : plain_filter_bytes(a);
 }
 
@@ -113,7 +113,7 @@ int mb200_conv_f32_pack_filter(
     if (((uintptr_t)flt_oihw & 3) || ((uintptr_t)flt_packed & 15))
         return set_error(ST_INVALID_LAYOUT, "filter must be 4-byte, packed filter 16-byte aligned");
     cudaStream_t st = (cudaStream_t)stream;
-    return conv_f32_split_eligible(a) ? launch_conv_f32_pack_filter_split(a, flt_oihw, flt_packed, st)
+    return conv_f32_split_planes(a) ? launch_conv_f32_pack_filter_split(a, flt_oihw, flt_packed, st)
                                       : launch_conv_f32_pack_filter_plain(a, flt_oihw, flt_packed, st);
 }
 
@@ -167,9 +167,9 @@ int mb200_matmul_f32_pack_b(int k, int n, const float* b, float* b_packed, void*
     ConvF32Args a{};
     if ((rc = make_f32_args(&p, 0, &a)))
         return rc;
-    // [K][N] row-major -> [N][K], the K-major filter of a 1x1 conv (or its two planes)
-    return conv_f32_split_eligible(a) ? launch_matmul_f32_pack_split(k, n, b, b_packed, st)
-                                      : launch_transpose_f32(b, b_packed, 1, k, n, st);
+    // [K][N] row-major -> [N][K], the K-major filter of a 1x1 conv (or its planes)
+    return conv_f32_split_planes(a) ? launch_matmul_f32_pack_b(a, b, b_packed, st)
+                                    : launch_transpose_f32(b, b_packed, 1, k, n, st);
 }
 
 size_t mb200_matmul_f32_workspace_bytes(int, int) {
@@ -218,9 +218,12 @@ int mb200_matmul_f32_product(
     cudaStream_t st = (cudaStream_t)stream;
     if (((uintptr_t)c & 15) == 0)
         return launch_matmul_f32(args, a, b, c, (float*)scratch, st);
-    // (a result that no vector store reaches: the general kernel)
-    const int pack = mb200_matmul_f32_pack_b(k, n, b, (float*)scratch, stream);
-    return pack ? pack : mb200_matmul_f32(m, n, k, a, (const float*)scratch, c, nullptr, 0, stream);
+    // (a result that no vector store reaches: the general kernel, which reads the first planes only)
+    const int pack = conv_f32_split_planes(args)
+                             ? launch_matmul_f32_pack_split(k, n, b, (float*)scratch, st)
+                             : launch_transpose_f32(b, (float*)scratch, 1, k, n, st);
+    return pack ? pack
+                : launch_conv_f32_direct(args, a, (const float*)scratch, nullptr, nullptr, c, st);
 }
 
 int mb200_elemwise_f32(

@@ -24,8 +24,8 @@ struct ConvF32Args {
 };
 
 int conv_f32_padded_ic(int ic);
-// does the packed filter of this shape consist of the two tf32 planes (else: plain K-major)?
-bool conv_f32_split_eligible(const ConvF32Args& a);
+// does the packed filter begin with the two tf32 planes (else: plain K-major)?
+bool conv_f32_split_planes(const ConvF32Args& a);
 size_t conv_f32_split_filter_floats(const ConvF32Args& a);
 // fp16 planes for the wide layers (conv_f32_half.cu), behind the tf32 planes of the filters that have them
 bool conv_f32_half_planes(const ConvF32Args& a);
@@ -34,6 +34,7 @@ int launch_conv_f32_pack_filter_half(
         const ConvF32Args& a, const float* flt_oihw, float* out, cudaStream_t st);
 int launch_matmul_f32_pack_half(int k, int n, const float* b, float* out, cudaStream_t st);
 // 3x3, stride 1, padding 1 from halo patches (conv_f32_patch.cu)
+bool conv_f32_patch_planes(const ConvF32Args& a);
 bool conv_f32_patch_shape(const ConvF32Args& a);
 bool conv_f32_patch_pays(const ConvF32Args& a);
 size_t conv_f32_patch_filter_floats(const ConvF32Args& a);
@@ -49,6 +50,8 @@ int launch_conv_f32_half(
         const ConvF32Args& a, const CUtensorMap& map_a, bool a_tiled, const float* planes,
         const float* bias, const float* z, float* dst, cudaStream_t st);
 bool conv_f32_umma_supported(const ConvF32Args& a, const float* src, const float* dst);
+// the packed filter of a 1x1 ConvBias from [K][N]
+int launch_matmul_f32_pack_b(const ConvF32Args& a, const float* b, float* out, cudaStream_t st);
 int launch_conv_f32_pack_filter_split(
         const ConvF32Args& a, const float* flt_oihw, float* out, cudaStream_t st);
 int launch_conv_f32_pack_filter_plain(

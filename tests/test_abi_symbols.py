@@ -113,3 +113,19 @@ def test_verified_requant_constants_agree_with_the_reference_chain():
     # no licence without positive scales, nor for H_SWISH
     assert constants(0.05, -0.01, 2.0, 1)[0] == 0
     assert constants(0.05, 0.01, 2.0, 2)[0] == 0
+
+
+# What a packed fp32 filter holds depends on the filter alone: it may be used under another input, stride or
+# padding than it was packed under, and a product's packed B as a 1x1 filter.
+@pytest.mark.parametrize("ic", [4, 16, 20, 24, 32, 64, 68])
+@pytest.mark.parametrize("oc", [8, 64, 65, 256])
+@pytest.mark.parametrize("k", [1, 3, 5])
+def test_packed_f32_filter_size_follows_the_filter(ic, oc, k):
+    from megcc_b200 import _lib, ops
+    size = _lib.lib().mb200_conv_f32_packed_filter_bytes
+    sizes = {size(ctypes.byref(ops.conv_f32_param(n, ic, h, w, oc, k, k, stride, pad)))
+             for n, h, w in ((1, 5, 5), (32, 20, 20), (1, 1, 1)) for stride in (1, 2) for pad in (0, k // 2)
+             if min(h, w) + 2 * pad >= k}
+    if k == 1:
+        sizes.add(_lib.lib().mb200_matmul_f32_packed_b_bytes(ic, oc))
+    assert len(sizes) == 1 and sizes.pop() > 0

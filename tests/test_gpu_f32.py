@@ -459,3 +459,39 @@ def test_fp32_halo_patches_match_64_bits(ops, case, form):
         err = (got.cpu().double().permute(0, 3, 1, 2) - want).abs()
         assert bool((err <= terms * 2.0 ** -19 + slack).all()), (mode, float((err / terms).max()))
     assert ops.device_status() == 0
+
+
+# a filter packed under one input, stride and padding and used under another, in every kernel it holds planes for
+@pytest.mark.parametrize("case", [(256, 256, 1), (64, 128, 1), (20, 72, 1), (64, 64, 3), (32, 128, 3)],
+                         ids=lambda c: "x".join(map(str, c)))
+@pytest.mark.parametrize("packed_as", ["point", "stride 2", "no padding", "product"])
+def test_packed_filters_serve_every_input(ops, case, packed_as):
+    import ctypes as C
+    from megcc_b200._lib import check, lib
+    ic, oc, k = case
+    if packed_as == "product" and k != 1:
+        pytest.skip("a product's B is a 1x1 filter")
+    r = cases.rng_for(f"f32_packed_{case}")
+    flt = dev((r.standard_normal((oc, ic, k, k)) / np.sqrt(ic * k * k)).astype(np.float32))
+    if packed_as == "product":
+        b = flt.view(oc, ic).t().contiguous()
+        packed = torch.empty(lib().mb200_matmul_f32_packed_b_bytes(ic, oc) // 4, device="cuda")
+        check(lib().mb200_matmul_f32_pack_b(ic, oc, C.c_void_p(b.data_ptr()), C.c_void_p(packed.data_ptr()),
+                                            C.c_void_p(torch.cuda.current_stream().cuda_stream)))
+    else:
+        e, stride, pad = (1, 1, k // 2) if packed_as == "point" else (9, 2, k // 2) if packed_as == "stride 2" else (9, 1, 0)
+        packed = ops.pack_filter_f32(ops.conv_f32_param(1, ic, e, e, oc, k, k, stride, pad), flt)
+    for n, h, stride, pad in ((1, 6, 1, k // 2), (32, 20, 1, k // 2), (32, 20, 2, k // 2), (8, 20, 1, 0)):
+        x = dev(r.standard_normal((n, ic, h, h)).astype(np.float32))
+        p = ops.conv_f32_param(n, ic, h, h, oc, k, k, stride, pad)
+        want = torch.nn.functional.conv2d(x.double(), flt.double(), stride=stride, padding=pad)
+        terms = torch.nn.functional.conv2d(x.double().abs(), flt.double().abs(), stride=stride, padding=pad)
+        for half, patch in ((1, 1), (2, 0), (0, 2), (0, 0)):
+            old = ops.set_option("f32_half", half), ops.set_option("f32_patch", patch)
+            try:
+                got = ops.conv_bias_f32_nhwc(p, ops.nchw_to_nhwc_f32(x), packed)
+            finally:
+                ops.set_option("f32_half", old[0]), ops.set_option("f32_patch", old[1])
+            # (2^-22 for the split, 2^-24 for each of at most 36 segment sums, the truncations of a chain)
+            assert bool(((got.double().permute(0, 3, 1, 2) - want).abs() <= terms * 2.0 ** -19).all()), (n, h, stride, pad, half, patch)
+    assert ops.device_status() == 0
