@@ -65,6 +65,7 @@
 #include <stdlib.h>
 
 #include "conv_f32_epilogue.cuh"
+#include "conv_f32_exact.cuh"
 #include "f32_internal.h"
 #include "pdl.h"
 #include "tuning.h"
@@ -1002,14 +1003,15 @@ F32Choice choose_f32_tile(const ConvF32Args& a, bool planes) {
     // 128 columns from fp16 planes (conv_f32_half.cu): two rows of A in the time of 1.64 here (32 x 80 x 80
     // pixels, 128 -> 128 3x3: 251 us and 206; 32 x 20 x 20, 256 -> 256: 100 as 64 columns, 82)
     const long long waves = ((long long)m_tiles * ((oc + 127) / 128) + sms - 1) / sms;
-    c.half = planes && waves * ((long long)((k_iters + 1) / 2) * 1395 + 2500 + (waves > 1 ? 0 : 3000)) < best;
+    const bool fits = planes && waves <= kExactTiles;
+    c.half = fits && waves * ((long long)((k_iters + 1) / 2) * 1395 + 2500 + (waves > 1 ? 0 : 3000)) < best;
     if (tuning().f32_bn == 32 || tuning().f32_bn == 64 || tuning().f32_bn == 128)
         c.bn = tuning().f32_bn;
     if (tuning().f32_split == 1 || tuning().f32_split == 2 || tuning().f32_split == 4 ||
         tuning().f32_split == 8)
         c.splits = k_iters >= tuning().f32_split ? tuning().f32_split : 1;
     if (tuning().f32_bn || tuning().f32_split || tuning().f32_half != 1)
-        c.half = planes && tuning().f32_half == 2;
+        c.half = fits && tuning().f32_half == 2;
     return c;
 }
 
@@ -1125,9 +1127,10 @@ int launch_conv_f32_direct(
     return check_launch("conv_f32_direct");
 }
 
-// `planes`: the fp16 planes of the filter, null: there are none, or the choice has fallen on the tf32 ones
+// `planes`: the fp16 planes of the filter, where the choice may fall on them. `raw`: the second operand of a
+// matrix product, of which these planes alone were made then, or null
 static int launch_f32_tensor(
-        const ConvF32Args& a, const float* src, const float* flt_split, const float* planes,
+        const ConvF32Args& a, const float* src, const float* flt_split, const float* planes, const float* raw,
         const F32Choice& choice, const float* bias, const float* z, float* dst, cudaStream_t st) {
     const DriverApi& api = driver_api();
     if (!api.ok)
@@ -1179,7 +1182,8 @@ static int launch_f32_tensor(
             return set_error(ST_RUNTIME, "cuTensorMapEncodeIm2col(f32) failed: %d", (int)r);
     }
     if (choice.half)
-        return launch_conv_f32_half(a, map_a, a_tiled, planes, bias, z, dst, st);
+        return launch_conv_f32_half(a, map_a, a_tiled, src, planes, raw ? raw : flt_split, raw != nullptr, bias, z,
+                                    dst, st);
     {
         const cuuint64_t k_total = (cuuint64_t)taps * icp;
         cuuint64_t dims[2] = {k_total, (cuuint64_t)2 * a.oc};
@@ -1228,12 +1232,16 @@ static int launch_f32_tensor(
 int launch_conv_f32_umma(
         const ConvF32Args& a, const float* src, const float* flt_split, const float* bias,
         const float* z, float* dst, cudaStream_t st) {
+    // (a residual in the result's own place: the kernels on fp16 planes may store a tile twice)
+    const bool in_place = z == dst;
     const bool has = conv_f32_half_planes(a);
     const float* planes = flt_split + 2 * (size_t)a.oc * a.kh * a.kw * conv_f32_padded_ic(a.ic);
-    if (conv_f32_patch_shape(a) && !tuning().f32_bn && !tuning().f32_split && conv_f32_patch_pays(a) &&
+    if (!in_place && conv_f32_patch_shape(a) && !tuning().f32_bn && !tuning().f32_split && conv_f32_patch_pays(a) &&
         ((uintptr_t)flt_split & 15) == 0)
-        return launch_conv_f32_patch(a, src, planes + (has ? conv_f32_half_filter_floats(a) : 0), bias, z, dst, st);
-    return launch_f32_tensor(a, src, flt_split, has ? planes : nullptr, choose_f32_tile(a, has), bias, z, dst, st);
+        return launch_conv_f32_patch(a, src, planes + (has ? conv_f32_half_filter_floats(a) : 0), flt_split, bias,
+                                     z, dst, st);
+    return launch_f32_tensor(a, src, flt_split, planes, nullptr, choose_f32_tile(a, has && !in_place), bias,
+                             z, dst, st);
 }
 
 // ---- a matrix product with both operands as the caller has them ----
@@ -1268,7 +1276,7 @@ int launch_matmul_f32(
     }
     const int rc = choice.half ? launch_matmul_f32_pack_half(a.ic, a.oc, b, packed, st)
                                : launch_matmul_f32_pack_split(a.ic, a.oc, b, packed, st);
-    return rc ? rc : launch_f32_tensor(a, src, packed, packed, choice, nullptr, nullptr, c, st);
+    return rc ? rc : launch_f32_tensor(a, src, packed, packed, b, choice, nullptr, nullptr, c, st);
 }
 
 }  // namespace mb200

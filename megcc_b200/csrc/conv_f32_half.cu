@@ -2,20 +2,19 @@
 // 128 pixels x 128 channels, operands split into two fp16 values. (conv_f32.cu splits into two tf32 values
 // and has everything else: narrow tiles, tiles split over a cluster, rows of 64 bytes.)
 //
-// Every operand is scaled by a power of two and split,
-//     v s = hi + lo,   hi = RN_f16(v s),   lo = RN_f16(v s - hi)          (v s - hi is exact)
-// and a product is three passes of tcgen05.mma kind::f16,
-//     lo*hi + hi*lo + hi*hi                                            (lo*lo is < 2^-22)
+// Every operand is scaled by a power of two and split, v s = hi + 2^-12 lo (conv_f32_split.cuh), and a product
+// is three passes of tcgen05.mma kind::f16,
+//     2^-12 (lo*hi + hi*lo) + hi*hi                                    (lo*lo is < 2^-22)
 // which leaves a relative error of a few 2^-23 per product, the order of fp32 itself: the same 11 + 11
 // bits as with tf32 at half the tensor time and half the filter's bytes. fp16 has few exponents, so the
 // scale follows the data: one per pixel and 64 elements of K for the activation, from the largest of them,
-// one per output channel for the filter. The largest element then lies in [2^14, 2^15); one 2^29 times
-// smaller still keeps its 22 bits, below that they go one by one (an absolute error of 2^-40 of the
-// largest). A K segment of 64 elements has accumulators of its own, whose sum is multiplied by the
+// one per output channel for the filter. Elements down to 2^-30 of the largest keep their bits; tiles whose
+// operands lie further apart are put off and taken from tf32 planes at the kernel's end
+// (conv_f32_exact.cuh). A K segment of 64 elements has accumulators of its own, whose sum is multiplied by the
 // pixel's factor when it is added up.
 //
 // The tensor core adds into its accumulator with truncation (see conv_f32.cu), so chains are kept short
-// here too: a segment's eight small products come first (their sum is 2^-11 of the main one, so its
+// here too: a segment's eight small products come first (their sum goes into the main one 2^-12 times, so its
 // truncation does not matter), then four K = 16 steps of hi*hi; the epilogue warps add finished segments
 // into fp32 registers with round-to-nearest.
 //
@@ -39,6 +38,7 @@
 #include <stdio.h>
 
 #include "conv_f32_epilogue.cuh"
+#include "conv_f32_exact.cuh"
 #include "conv_f32_split.cuh"
 #include "f32_internal.h"
 #include "pdl.h"
@@ -64,9 +64,11 @@ constexpr int kABytes = kBM * kChans * 4;
 constexpr int kBBytes = 2 * kBN * kSegK * 2;  // both planes of a filter segment
 constexpr int kEpilogueWarps = 8, kConverterWarps = 8;
 constexpr int kThreads = 64 + 32 * (kEpilogueWarps + kConverterWarps);
-// shared memory in front of the tiles: barriers; the pixels' factors of the last eight segments; the
+// shared memory in front of the tiles: barriers and which tile columns are wide or loose; a bit for each tile that
+// is put off; the pixels' factors of the last eight segments; the
 // converters' largest values (two segments, two halves); each epilogue warp's bias and channel factors
-constexpr int kFactorOff = 1024, kMostOff = kFactorOff + 8 * kBM * 4;
+constexpr int kLateOff = 448, kFactorOff = 1024, kMostOff = kFactorOff + 8 * kBM * 4;
+static_assert(kLateOff + sizeof(LateTiles) <= kFactorOff, "the list of tiles");
 constexpr int kBiasOff = kMostOff + 4 * kBM * 4;
 constexpr int kTurn = 16;     // columns of a result turned round at a time
 constexpr int kTurnOff = kBiasOff + kEpilogueWarps * kBN / 2 * 8;
@@ -75,7 +77,8 @@ constexpr int kTileBudget = 227 * 1024 - 1024 - kFrontBytes;  // (1024: alignmen
 constexpr int kDynamic = 227 * 1024;
 
 // A operand (two fp16 per column) in tensor memory, B in shared memory (descriptor as its two words);
-// issued by the lane whose `leader` is non-zero
+// issued by the lane whose `leader` is non-zero. SHIFT: what is in the accumulator counts 2^-SHIFT times
+template <int SHIFT = 0>
 __device__ __forceinline__ void umma_f16_ta(
         uint32_t leader, uint32_t tmem_d, uint32_t tmem_a, uint32_t b_lo, uint32_t b_hi,
         uint32_t idesc, uint32_t accumulate) {
@@ -83,8 +86,8 @@ __device__ __forceinline__ void umma_f16_ta(
             "{\n\t.reg .pred p, q;\n\t.reg .b64 d;\n\t"
             "mov.b64 d, {%2, %3};\n\t"
             "setp.ne.b32 p, %5, 0;\n\tsetp.ne.b32 q, %6, 0;\n\t"
-            "@q tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], d, %4, p;\n\t}" ::"r"(tmem_d),
-            "r"(tmem_a), "r"(b_lo), "r"(b_hi), "r"(idesc), "r"(accumulate), "r"(leader)
+            "@q tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], d, %4, p, %7;\n\t}" ::"r"(tmem_d),
+            "r"(tmem_a), "r"(b_lo), "r"(b_hi), "r"(idesc), "r"(accumulate), "r"(leader), "n"(SHIFT)
             : "memory");
 }
 
@@ -99,34 +102,35 @@ __device__ __forceinline__ void tmem_st8(uint32_t taddr, const uint32_t (&v)[8])
 // ------------------------------------------------------------------------------------------
 // filter packing (load time)
 // ------------------------------------------------------------------------------------------
-// fp16 planes [2][OC][KH][KW][ICp] (hi, lo), zero-filled beyond IC, then a factor per OC
+// fp16 planes [2][OC][KH][KW][ICp] (hi, lo), zero-filled beyond IC, then a word per OC (channel_word)
 struct Planes {
     uint16_t *hi, *lo;
-    float* factor;
+    uint32_t* word;
 };
 __device__ __forceinline__ Planes planes_at(float* out, size_t plane) {
     uint16_t* hi = reinterpret_cast<uint16_t*>(out);
-    return Planes{hi, hi + plane, out + plane};
+    return Planes{hi, hi + plane, reinterpret_cast<uint32_t*>(out + plane)};
 }
 
 // OIHW fp32 -> the planes, a block per output channel
 __global__ void __launch_bounds__(256) pack_filter_half_kernel(
         const float* __restrict__ src, float* __restrict__ out, int oc, int ic, int icp, int kh,
         int kw) {
-    __shared__ float shared[8];
+    __shared__ Magnitudes shared[8];
     const int taps = kh * kw, o = blockIdx.x;
     const float* w = src + (size_t)o * ic * taps;
-    float most = 0.f;
+    Magnitudes of = Magnitudes::none();
     for (int i = threadIdx.x; i < ic * taps; i += 256)
-        most = fmaxf(most, fabsf(w[i]));
-    const uint32_t field = scale_field(block_largest(most, shared));
+        of.take(w[i]);
+    of = block_magnitudes(of, shared);
+    const uint32_t field = scale_field(of.largest);
     const Planes d = planes_at(out, (size_t)oc * taps * icp);
     if (threadIdx.x == 0)
-        d.factor[o] = field_to_float(channel_factor_field(field));
+        d.word[o] = of.word();
     for (int i = threadIdx.x; i < taps * icp; i += 256) {
         const int tap = i / icp, c = i - tap * icp;
         uint32_t h, l;
-        split_f16(c < ic ? w[(size_t)c * taps + tap] : 0.f, 0.f, field_to_float(field), h, l);
+        split_f16(c < ic ? w[(size_t)c * taps + tap] : 0.f, 0.f, SplitScale<false>(field), h, l);
         d.hi[(size_t)o * taps * icp + i] = (uint16_t)h;
         d.lo[(size_t)o * taps * icp + i] = (uint16_t)l;
     }
@@ -139,8 +143,9 @@ __global__ void __launch_bounds__(256) pack_filter_half_kernel(
 constexpr int kPackParts = 8;
 __global__ void __launch_bounds__(256) pack_matrix_half_kernel(
         const float* __restrict__ src, float* __restrict__ out, int k, int n, int kp) {
-    __shared__ __align__(16) float most[32];
-    __shared__ float part[8][33];
+    // (a column's magnitudes, 16 bytes each: other blocks of the cluster read them)
+    __shared__ __align__(16) float found[32][4];
+    __shared__ Magnitudes part[8][33];
     __shared__ float tile[64][33];
     const int lane = threadIdx.x & 31, row = threadIdx.x >> 5;
     const int n0 = (int)(blockIdx.x / kPackParts) * 32;
@@ -148,15 +153,18 @@ __global__ void __launch_bounds__(256) pack_matrix_half_kernel(
     const int blocks = (kp + 63) / 64;
     const int c = n0 + lane;
     // rows of this block: every kPackParts-th 64
-    float v = 0.f;
+    Magnitudes v = Magnitudes::none();
     if (c < n) {
         for (int b = rank; b < blocks; b += kPackParts) {
+            float x[8];
 #pragma unroll
             for (int j = 0; j < 8; ++j) {
                 const int r = b * 64 + row + 8 * j;
-                if (r < k)
-                    v = fmaxf(v, fabsf(__ldg(src + (size_t)r * n + c)));
+                x[j] = __ldg(src + (size_t)(r < k ? r : 0) * n + c);  // (a value twice does not matter)
             }
+#pragma unroll
+            for (int j = 0; j < 8; ++j)
+                v.take(x[j]);
         }
     }
     part[row][lane] = v;
@@ -164,27 +172,28 @@ __global__ void __launch_bounds__(256) pack_matrix_half_kernel(
     if (row == 0) {
 #pragma unroll
         for (int j = 1; j < 8; ++j)
-            v = fmaxf(v, part[j][lane]);
-        most[lane] = v;
+            v.take(part[j][lane]);
+        found[lane][0] = v.largest;
+        found[lane][1] = v.least;
+        found[lane][2] = v.least_nonzero;
     }
     __syncthreads();
     cluster_arrive();
     cluster_wait();
     // (a thread's column for the writes: four threads of a column's row)
     const int col = threadIdx.x >> 3, kq = (threadIdx.x & 7) * 8;
-    float largest = 0.f;
+    v = Magnitudes::none();
     for (int i = 0; i < kPackParts; ++i) {
-        const uint4 w = ld_cluster_v4(smem_u32(most + (col & ~3)), i);
-        const uint32_t u = (col & 3) == 0 ? w.x : (col & 3) == 1 ? w.y : (col & 3) == 2 ? w.z : w.w;
-        largest = fmaxf(largest, __uint_as_float(u));
+        const uint4 w = ld_cluster_v4(smem_u32(found[col]), i);
+        v.take(Magnitudes{__uint_as_float(w.x), __uint_as_float(w.y), __uint_as_float(w.z)});
     }
     cluster_arrive();
-    const uint32_t field = scale_field(largest);
-    const float scale = field_to_float(field);
+    const uint32_t field = scale_field(v.largest);
+    const SplitScale<true> scale(field);
     const Planes d = planes_at(out, (size_t)n * kp);
     const int cw = n0 + col;
     if (rank == 0 && cw < n && kq == 0)
-        d.factor[cw] = field_to_float(channel_factor_field(field));
+        d.word[cw] = v.word();
     for (int b = rank; b < blocks; b += kPackParts) {
 #pragma unroll
         for (int j = 0; j < 8; ++j) {
@@ -214,6 +223,15 @@ __global__ void __launch_bounds__(256) pack_matrix_half_kernel(
 // ------------------------------------------------------------------------------------------
 // the kernel
 // ------------------------------------------------------------------------------------------
+// rows that follow one another
+struct RowPixel {
+    int m0, m_total, oh, ow;
+    __device__ __forceinline__ ExactPixel operator()(int row) const {
+        const int m = m0 + row, img = m / (oh * ow), rem = m - img * (oh * ow), y = rem / ow;
+        return ExactPixel{img, y, rem - y * ow, m < m_total};
+    }
+};
+
 struct HalfConvParams {
     int m_total, oc, oh, ow;
     int cblocks;      // 32-channel rows per tap
@@ -226,13 +244,17 @@ struct HalfConvParams {
     int a_stages, b_stages;  // depth of the rings: rows of A (even), segments of B (at most kTStages)
     int b_resident;   // 1: the whole filter sits in shared memory
     F32Epilogue ep;
-    const float* factor;  // per output channel: what a unit of the accumulated sums stands for
+    const float* factor;  // per output channel: what a unit of the accumulated sums stands for (channel_word)
+    ExactOperands exact;
     int* status;
+    __device__ __forceinline__ RowPixel pixel(int tile) const {
+        return RowPixel{tile / n_tiles * kBM, m_total, oh, ow};
+    }
 };
 
 __global__ void __launch_bounds__(kThreads, 1) conv_f32_half_kernel(
         const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b,
-        const HalfConvParams p) {
+        const __grid_constant__ HalfConvParams p) {
     extern __shared__ uint8_t smem_raw[];
     uint8_t* smem = (uint8_t*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
     uint64_t* a_full = (uint64_t*)smem;            // [kMaxAStages] TMA -> converters
@@ -245,8 +267,12 @@ __global__ void __launch_bounds__(kThreads, 1) conv_f32_half_kernel(
     uint64_t* done = ready + kTStages;             // [kTStages]
     uint64_t* b_full = done + kTStages;            // a resident filter
     uint64_t* drain_bar = b_full + 1;
-    uint32_t* tmem_slot = (uint32_t*)(drain_bar + 1);
+    uint64_t* exact_bars = drain_bar + 1;          // [2]
+    uint32_t* tmem_slot = (uint32_t*)(exact_bars + 2);
     volatile int* abort_flag = (volatile int*)(tmem_slot + 1);
+    ColumnStates* columns = (ColumnStates*)(tmem_slot + 2);
+    LateTiles* late = reinterpret_cast<LateTiles*>(smem + kLateOff);
+    const uint32_t late_a = smem_u32(late);
     float* pixel_factor = reinterpret_cast<float*>(smem + kFactorOff);  // [8][kBM]
     float* half_most = reinterpret_cast<float*>(smem + kMostOff);       // [2][2][kBM]
     uint8_t* tiles_b = smem + kFrontBytes;  // resident filter or ring of segments
@@ -269,12 +295,17 @@ __global__ void __launch_bounds__(kThreads, 1) conv_f32_half_kernel(
         }
         mbar_init(b_full, 1);
         mbar_init(drain_bar, 1);
+        mbar_init(&exact_bars[0], 1);
+        mbar_init(&exact_bars[1], 1);
         *abort_flag = 0;
+        columns->reset();
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     } else if (threadIdx.x == 32 * 2) {
         tma_prefetch_map(&map_a);
         tma_prefetch_map(&map_b);
     }
+    if (threadIdx.x < sizeof(LateTiles) / 4)
+        late->bits[threadIdx.x] = 0;
     if (warp == 1) {
         asm volatile(
                 "tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(
@@ -408,15 +439,17 @@ __global__ void __launch_bounds__(kThreads, 1) conv_f32_half_kernel(
                         umma_f16_ta(leader, d, a_lo + 8 * k, b_hi + 2 * k, kDescHi, idesc, k != 0);
                         umma_f16_ta(leader, d, a_hi + 8 * k, b_lo + 2 * k, kDescHi, idesc, 1);
                     }
+                    umma_f16_ta<kLoShift>(leader, d, a_hi, b_hi, kDescHi, idesc, 1);
 #pragma unroll
-                    for (int k = 0; k < kSegK / 16; ++k)
+                    for (int k = 1; k < kSegK / 16; ++k)
                         umma_f16_ta(leader, d, a_hi + 8 * k, b_hi + 2 * k, kDescHi, idesc, 1);
                 } else {
                     for (int k = 0; k < steps; ++k) {
                         umma_f16_ta(leader, d, a_lo + 8 * k, b_hi + 2 * k, kDescHi, idesc, k != 0);
                         umma_f16_ta(leader, d, a_hi + 8 * k, b_lo + 2 * k, kDescHi, idesc, 1);
                     }
-                    for (int k = 0; k < steps; ++k)
+                    umma_f16_ta<kLoShift>(leader, d, a_hi, b_hi, kDescHi, idesc, 1);
+                    for (int k = 1; k < steps; ++k)
                         umma_f16_ta(leader, d, a_hi + 8 * k, b_hi + 2 * k, kDescHi, idesc, 1);
                 }
                 umma_commit_if(leader, done_a + 8 * t);
@@ -449,6 +482,21 @@ __global__ void __launch_bounds__(kThreads, 1) conv_f32_half_kernel(
         int s = half, t = 0, g = 0;
         uint32_t a_phase = 0, t_phase = 1;
         bool ok = true;
+        // Operands that the planes do not hold put the tile off
+        uint32_t ordinal = 0;
+        int m = 0, column = 0;
+        bool strict = false, fits = true;
+        LargestValues values;
+        auto begin_tile = [&] {
+            const int tile = first_tile + (int)ordinal * tile_step;
+            const int tile_m = p.n_tiles == 1 ? tile : tile / p.n_tiles;
+            m = tile_m * kBM + row;
+            column = tile - tile_m * p.n_tiles;
+            strict = __any_sync(0xffffffffu, columns->is_strict(column));
+            fits = true;
+            values.reset();
+        };
+        begin_tile();
         // (after a wait that ran out a warp goes on without waits and work: the two warps of a pixel quarter
         // meet at a barrier in every segment)
         for (int turn = 0; turn < total; ++turn) {
@@ -481,7 +529,8 @@ __global__ void __launch_bounds__(kThreads, 1) conv_f32_half_kernel(
             asm volatile("bar.sync %0, 64;" ::"r"(1 + q) : "memory");
             most = fmaxf(most, exchange[(half ^ 1) * kBM]);
             const uint32_t field = scale_field(most);
-            const float scale = field_to_float(field);
+            const SplitScale<true> scale(field);
+            values.take(most);
             if (ok) {
                 // (the sums of eight segments ago have been taken: the accumulators of six ago
                 // were free before the MMAs of four ago, which have retired)
@@ -499,6 +548,21 @@ __global__ void __launch_bounds__(kThreads, 1) conv_f32_half_kernel(
                     tmem_st8(ta + 8 * h, hi);
                     tmem_st8(ta + kTCols / 2 + 8 * h, lo);
                 }
+                if (strict && there) {
+                    // (read again: kept for this, the values slowed the loop down for everyone, 2048^3 71 -> 78 us)
+                    uint32_t least = 0xffffffffu;
+#pragma unroll
+                    for (int u = 0; u < kChans / 4; ++u) {
+                        const float4 v = src[u ^ swz];
+                        least = min(min(least, min(magnitude_0_last(v.x), magnitude_0_last(v.y))),
+                                    min(magnitude_0_last(v.z), magnitude_0_last(v.w)));
+                    }
+                    fits = fits && least >= least_magnitude(field);
+                    strict = __any_sync(0xffffffffu, columns->is_strict(column));  // (it may just have been found out)
+                }
+                // (a row behind the last pixel may hold whatever lies behind the input)
+                if (g + 1 == p.segs)
+                    put_tile_off_if(!(fits && values.fit()) && m < p.m_total, late_a, ordinal);
                 asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
                 asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
                 __syncwarp();
@@ -509,8 +573,11 @@ __global__ void __launch_bounds__(kThreads, 1) conv_f32_half_kernel(
                     mbar_arrive_u32(a_empty_a + 8 * s);
                 }
             }
-            if (++g == p.segs)
+            if (++g == p.segs) {
                 g = 0;
+                ++ordinal;
+                begin_tile();
+            }
             s += 2;
             if (s >= p.a_stages) {
                 s -= p.a_stages;
@@ -540,6 +607,7 @@ __global__ void __launch_bounds__(kThreads, 1) conv_f32_half_kernel(
             mbar_arrive(&ready[1]);
         }
         pdl_wait();  // before the first read of z and the first store
+        find_column_states<32 * kEpilogueWarps, 5>(p.factor, p.oc, kBN, (int)threadIdx.x - 64, columns, &late->any);
         for (int tile = first_tile; tile < total_tiles && ok; tile += tile_step) {
             const int tile_n = tile % p.n_tiles, tile_m = tile / p.n_tiles;
             const int m = tile_m * kBM + row, n0 = tile_n * kBN;
@@ -549,7 +617,7 @@ __global__ void __launch_bounds__(kThreads, 1) conv_f32_half_kernel(
                 for (int j = lane; j < kCols; j += 32) {
                     const int ch = n0 + half * kCols + j;
                     bias_row[j] = p.ep.bias && ch < p.oc ? __ldg(p.ep.bias + ch) : 0.f;
-                    factor_row[j] = ch < p.oc ? __ldg(p.factor + ch) : 0.f;
+                    factor_row[j] = ch < p.oc ? channel_factor(__float_as_uint(__ldg(p.factor + ch))) : 0.f;
                 }
                 __syncwarp();
             }
@@ -603,9 +671,14 @@ __global__ void __launch_bounds__(kThreads, 1) conv_f32_half_kernel(
         }
     }
 
-    // ---------------- teardown ----------------
+    // ---------------- the tiles put off, teardown ----------------
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
+    if (*(volatile uint32_t*)&late->any != 0 && !*abort_flag) {
+        exact_tiles<kBN>(p, late, columns, tiles_b, tmem_base, exact_bars, abort_flag);
+        asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+        __syncthreads();
+    }
     if (*abort_flag) {
         if (warp == 1 && lane == 0) {
             umma_commit(drain_bar);
@@ -658,10 +731,11 @@ int launch_matmul_f32_pack_half(int k, int n, const float* b, float* out, cudaSt
     return check_launch("pack_matrix_half");
 }
 
-// map_a: rows of 32 channels and 128 pixels, as for conv_f32.cu
+// map_a: rows of 32 channels and 128 pixels, as for conv_f32.cu. `weights`: the filter's tf32 planes, or the
+// second operand of a matrix product as it is ([K][N])
 int launch_conv_f32_half(
-        const ConvF32Args& a, const CUtensorMap& map_a, bool a_tiled, const float* planes,
-        const float* bias, const float* z, float* dst, cudaStream_t st) {
+        const ConvF32Args& a, const CUtensorMap& map_a, bool a_tiled, const float* src, const float* planes,
+        const float* weights, bool weights_raw, const float* bias, const float* z, float* dst, cudaStream_t st) {
     static KernelReady ready;
     if (!ready.smem(conv_f32_half_kernel, kDynamic))
         return check_launch("conv_f32_half smem attribute");
@@ -710,6 +784,7 @@ int launch_conv_f32_half(
     p.ep.dst = dst;
     p.ep.dst_pitch = a.dst_pitch;
     p.factor = planes + (size_t)a.oc * k_total;
+    p.exact = conv_f32_exact_operands(a, src, weights, weights_raw);
     p.status = device_status_word(st);
     if (!p.status)
         return ST_MALLOC;

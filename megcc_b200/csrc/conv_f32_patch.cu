@@ -8,8 +8,9 @@
 // shared-memory address, so a shifted start needs nothing else), rows of eight pixels, 10 pixels apart.
 //
 // Arithmetic as in conv_f32_half.cu: each pixel's 64 channels share a power of two, a channel's filter another;
-// lo*hi + hi*lo + hi*hi, a segment (one tap x 64 channels) in accumulators of its own, whose sum is taken
-// into fp32 registers times the pixel's factor, which is the tap's pixel here.
+// 2^-12 (lo*hi + hi*lo) + hi*hi, a segment (one tap x 64 channels) in accumulators of its own, whose sum is taken
+// into fp32 registers times the pixel's factor, which is the tap's pixel here. Tiles whose operands lie too far
+// apart for that are put off and taken from tf32 planes at the kernel's end (conv_f32_exact.cuh).
 //
 // What bounds it: the MMAs' operands from shared memory (A 4 KB, B 1 to 4 KB each, 128 bytes a clock: 40, 48,
 // 64 clocks for 32, 64, 128 columns; issued one in 60 to 75) and whatever else takes that memory's time;
@@ -28,6 +29,7 @@
 #include <stdio.h>
 
 #include "conv_f32_epilogue.cuh"
+#include "conv_f32_exact.cuh"
 #include "conv_f32_split.cuh"
 #include "f32_internal.h"
 #include "pdl.h"
@@ -66,7 +68,8 @@ struct Cfg {
     static constexpr int kTurn = kCols < 32 ? kCols : 32;      // ... turned round at a time
     static constexpr int kTurnBytes = 32 * kTurn * 4;
     static constexpr int kThreads = 64 + 32 * (kEpilogueWarps + kConverterWarps);
-    static constexpr int kFactorOff = 256;
+    static constexpr int kLateOff = 240;  // LateTiles
+    static constexpr int kFactorOff = (kLateOff + (int)sizeof(LateTiles) + 15) / 16 * 16;
     // Pixel factors: the converters write those of block n + 2 when the MMAs of block n have retired, and the
     // epilogue is at most kBars groups behind these.
     static constexpr int kFactorSets = kBars * kGroup < kTaps ? 3 : 4;
@@ -82,6 +85,16 @@ struct Cfg {
     static_assert(kBars * kGroup * BN <= 512, "tensor memory");
     static_assert(kDynamic <= 227 * 1024, "shared memory");
     static_assert(kBars * kGroup < 2 * kTaps, "factor sets");
+    static_assert((64 + BN / 2) * 1024 <= kPlaneBytes + kBStages * kBBytes, "a tile from tf32 planes");
+};
+
+// A tile's rows for the general form: patch rows of eight pixels
+struct PatchPixel {
+    int img, y0, x0, oh, ow;
+    __device__ __forceinline__ ExactPixel operator()(int row) const {
+        const int y = y0 + (row >> 3), x = x0 + (row & 7);
+        return ExactPixel{img, y, x, y < oh && x < ow};
+    }
 };
 
 struct PatchF32Params {
@@ -92,12 +105,18 @@ struct PatchF32Params {
     int tiles_y, tiles_x, m_tiles, n_tiles;
     F32Epilogue ep;
     const uint8_t* filter;   // [tile column][block][tap][plane][BN][64 channels], rows swizzled as in shared memory
-    const float* factor;     // per output channel: what a unit of the accumulated sums stands for
+    const float* factor;     // per output channel: what a unit of the accumulated sums stands for (channel_word)
+    ExactOperands exact;
     int* status;
+    __device__ __forceinline__ PatchPixel pixel(int tile) const {
+        const int m = tile / n_tiles, per_image = tiles_y * tiles_x, img = m / per_image, r = m - img * per_image;
+        return PatchPixel{img, r / tiles_x * kTH, r % tiles_x * kTW, oh, ow};
+    }
 };
 
 // both operands in shared memory (descriptors as their two words); issued by the lane whose `leader` is
-// non-zero
+// non-zero. SHIFT: what is in the accumulator counts 2^-SHIFT times
+template <int SHIFT = 0>
 __device__ __forceinline__ void umma_f16_ss(
         uint32_t leader, uint32_t tmem_d, uint32_t a_lo, uint32_t b_lo, uint32_t a_hi, uint32_t b_hi,
         uint32_t idesc, uint32_t accumulate) {
@@ -105,8 +124,8 @@ __device__ __forceinline__ void umma_f16_ss(
             "{\n\t.reg .pred p, q;\n\t.reg .b64 a, b;\n\t"
             "mov.b64 a, {%1, %2};\n\tmov.b64 b, {%3, %4};\n\t"
             "setp.ne.b32 p, %6, 0;\n\tsetp.ne.b32 q, %7, 0;\n\t"
-            "@q tcgen05.mma.cta_group::1.kind::f16 [%0], a, b, %5, p;\n\t}" ::"r"(tmem_d),
-            "r"(a_lo), "r"(a_hi), "r"(b_lo), "r"(b_hi), "r"(idesc), "r"(accumulate), "r"(leader)
+            "@q tcgen05.mma.cta_group::1.kind::f16 [%0], a, b, %5, p, %8;\n\t}" ::"r"(tmem_d),
+            "r"(a_lo), "r"(a_hi), "r"(b_lo), "r"(b_hi), "r"(idesc), "r"(accumulate), "r"(leader), "n"(SHIFT)
             : "memory");
 }
 
@@ -173,26 +192,27 @@ struct PatchRows {
     __device__ __forceinline__ int step(int row) const { return (row >> 3) * p.ow + (row & 7); }
 };
 
-// OIHW fp32 -> the filter's planes and factors, a block per channel of the (padded) tile columns
+// OIHW fp32 -> the filter's planes and channel words, a block per channel of the (padded) tile columns
 __global__ void __launch_bounds__(256) pack_filter_patch_kernel(
-        const float* __restrict__ src, uint8_t* __restrict__ out, float* __restrict__ factor, int oc, int ic,
+        const float* __restrict__ src, uint8_t* __restrict__ out, uint32_t* __restrict__ word, int oc, int ic,
         int blocks, int bn) {
-    __shared__ float shared[8];
+    __shared__ Magnitudes shared[8];
     const int o = blockIdx.x, column = o / bn, row = o - column * bn;
     const float* w = src + (size_t)o * ic * kTaps;
     const int count = o < oc ? ic * kTaps : 0;
-    float most = 0.f;
+    Magnitudes of = Magnitudes::none();
     for (int i = threadIdx.x; i < count; i += 256)
-        most = fmaxf(most, fabsf(w[i]));
-    const uint32_t field = scale_field(block_largest(most, shared));
+        of.take(w[i]);
+    of = block_magnitudes(of, shared);
+    const uint32_t field = scale_field(of.largest);
     if (threadIdx.x == 0)
-        factor[o] = field_to_float(channel_factor_field(field));
+        word[o] = of.word();
     const size_t plane = (size_t)bn * kBlock * 2;
     for (int i = threadIdx.x; i < blocks * kTaps * kBlock; i += 256) {
         const int segment = i / kBlock, k = i - segment * kBlock;
         const int block = segment / kTaps, tap = segment - block * kTaps, c = block * kBlock + k;
         uint32_t h, l;
-        split_f16(c < ic && o < oc ? w[(size_t)c * kTaps + tap] : 0.f, 0.f, field_to_float(field), h, l);
+        split_f16(c < ic && o < oc ? w[(size_t)c * kTaps + tap] : 0.f, 0.f, SplitScale<false>(field), h, l);
         uint8_t* to = out + ((size_t)column * blocks * kTaps + segment) * 2 * plane + (size_t)row * 128 +
                       (((k >> 3) ^ (row & 7)) << 4) + (k & 7) * 2;
         *reinterpret_cast<uint16_t*>(to) = (uint16_t)h;
@@ -216,8 +236,12 @@ __global__ void __launch_bounds__(Cfg<BN>::kThreads, 1) conv_f32_patch_kernel(
     uint64_t* ready = plane_empty + 2;             // [kBars]
     uint64_t* done = ready + kBars;                // [kBars]
     uint64_t* drain_bar = done + kBars;
-    uint32_t* tmem_slot = (uint32_t*)(drain_bar + 1);
+    uint64_t* exact_bars = drain_bar + 1;          // [2]
+    uint32_t* tmem_slot = (uint32_t*)(exact_bars + 2);
     volatile int* abort_flag = (volatile int*)(tmem_slot + 1);
+    ColumnStates* columns = (ColumnStates*)(tmem_slot + 2);
+    LateTiles* late = reinterpret_cast<LateTiles*>(smem + C::kLateOff);
+    const uint32_t late_a = smem_u32(late);
     float* factors = reinterpret_cast<float*>(smem + C::kFactorOff);  // [kFactorSets][kPixels]
     uint8_t* planes = smem + C::kFrontBytes;       // [2][hi, lo]
     uint8_t* ring_b = planes + C::kPlaneBytes;
@@ -237,9 +261,14 @@ __global__ void __launch_bounds__(Cfg<BN>::kThreads, 1) conv_f32_patch_kernel(
             mbar_init(&done[t], 1);
         }
         mbar_init(drain_bar, 1);
+        mbar_init(&exact_bars[0], 1);
+        mbar_init(&exact_bars[1], 1);
         *abort_flag = 0;
+        columns->reset();
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
+    if (threadIdx.x < sizeof(LateTiles) / 4)
+        late->bits[threadIdx.x] = 0;
     if (warp == 1) {
         asm volatile(
                 "tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(
@@ -342,8 +371,9 @@ __global__ void __launch_bounds__(Cfg<BN>::kThreads, 1) conv_f32_patch_kernel(
                                 umma_f16_ss(leader, d, a_lo + 2 * k, tap_hi + 2 * k, kAHigh, kBHigh, idesc, k != 0);
                                 umma_f16_ss(leader, d, a_hi + 2 * k, tap_lo + 2 * k, kAHigh, kBHigh, idesc, 1);
                             }
+                            umma_f16_ss<kLoShift>(leader, d, a_hi, tap_hi, kAHigh, kBHigh, idesc, 1);
 #pragma unroll
-                            for (int k = 0; k < kSteps; ++k)
+                            for (int k = 1; k < kSteps; ++k)
                                 umma_f16_ss(leader, d, a_hi + 2 * k, tap_hi + 2 * k, kAHigh, kBHigh, idesc, 1);
                         }
                     };
@@ -382,7 +412,7 @@ __global__ void __launch_bounds__(Cfg<BN>::kThreads, 1) conv_f32_patch_kernel(
         const int part = lane & 3, mine = (lane >> 2 & 3) * 2 + (lane >> 4) + cw * 8;
         constexpr int kTurns = (kPixels + 8 * kConverterWarps - 1) / (8 * kConverterWarps);
         const uint32_t plane_full_a = smem_u32(plane_full), plane_empty_a = smem_u32(plane_empty);
-        uint32_t turn = 0;
+        uint32_t turn = 0, ordinal = 0;
         bool ok = true;
         pdl_wait();
         // this lane's channels of its pixel in turn i, zero beyond the image and the channels
@@ -406,7 +436,12 @@ __global__ void __launch_bounds__(Cfg<BN>::kThreads, 1) conv_f32_patch_kernel(
             for (int i = 0; i < kTurns; ++i)
                 load(at, 0, i, v[i]);
         }
-        for (int tile = first_tile; tile < total_tiles && ok; tile += tile_step) {
+        for (int tile = first_tile; tile < total_tiles && ok; tile += tile_step, ++ordinal) {
+            // Operands that the planes do not hold put the tile off
+            const bool strict = __any_sync(0xffffffffu, columns->is_strict(p.n_tiles == 1 ? 0 : tile % p.n_tiles));
+            bool fits = true;
+            LargestValues values;
+            values.reset();
             for (int block = 0; block < p.blocks && ok; ++block, ++turn) {
                 const uint32_t buf = turn & 1;
                 const int left = p.ic - block * kBlock;
@@ -432,7 +467,16 @@ __global__ void __launch_bounds__(Cfg<BN>::kThreads, 1) conv_f32_patch_kernel(
                     most = fmaxf(most, __shfl_xor_sync(0xffffffffu, most, 1));
                     most = fmaxf(most, __shfl_xor_sync(0xffffffffu, most, 2));
                     const uint32_t field = scale_field(most);
-                    const float scale = field_to_float(field);
+                    const SplitScale<false> scale(field);
+                    values.take(most);
+                    if (strict) {
+                        uint32_t least = 0xffffffffu;
+#pragma unroll
+                        for (int u = 0; u < 4; ++u)
+                            least = min(min(least, min(magnitude_0_last(v[i][u].x), magnitude_0_last(v[i][u].y))),
+                                        min(magnitude_0_last(v[i][u].z), magnitude_0_last(v[i][u].w)));
+                        fits = fits && least >= least_magnitude(field);
+                    }
                     if (px < kPixels) {
                         if (part == 0)
                             factor[px] = field_to_float(pixel_factor_field(field));
@@ -453,6 +497,8 @@ __global__ void __launch_bounds__(Cfg<BN>::kThreads, 1) conv_f32_patch_kernel(
                     if (more)
                         load(then, then_block, i, v[i]);
                 }
+                if (block + 1 == p.blocks)
+                    put_tile_off_if(!(fits && values.fit()), late_a, ordinal);
                 asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
                 __syncwarp();
                 if (lane == 0)
@@ -479,6 +525,7 @@ __global__ void __launch_bounds__(Cfg<BN>::kThreads, 1) conv_f32_patch_kernel(
                 mbar_arrive(&ready[t]);
         }
         pdl_wait();  // before the first read of z and the first store
+        find_column_states<32 * kEpilogueWarps, 1>(p.factor, p.oc, BN, (int)threadIdx.x - 64, columns, &late->any);
         for (int tile = first_tile; tile < total_tiles && ok; tile += tile_step) {
             const TilePos at(tile, BN, p);
             const int oy = at.y0 + py, ox = at.x0 + px;
@@ -490,7 +537,8 @@ __global__ void __launch_bounds__(Cfg<BN>::kThreads, 1) conv_f32_patch_kernel(
 #pragma unroll
                 for (int j = lane; j < kCols; j += 32) {
                     const int ch = at.n0 + col0 + j;
-                    channels[set * 2 * BN + j] = ch < p.oc ? __ldg(p.factor + ch) : 0.f;
+                    channels[set * 2 * BN + j] =
+                            ch < p.oc ? channel_factor(__float_as_uint(__ldg(p.factor + ch))) : 0.f;
                     channels[set * 2 * BN + BN + j] = p.ep.bias && ch < p.oc ? __ldg(p.ep.bias + ch) : 0.f;
                 }
             }
@@ -565,9 +613,14 @@ __global__ void __launch_bounds__(Cfg<BN>::kThreads, 1) conv_f32_patch_kernel(
         }
     }
 
-    // ---------------- teardown ----------------
+    // ---------------- the tiles put off, teardown ----------------
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
+    if (*(volatile uint32_t*)&late->any != 0 && !*abort_flag) {
+        exact_tiles<BN>(p, late, columns, planes, tmem_base, exact_bars, abort_flag);
+        asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+        __syncthreads();
+    }
     if (*abort_flag) {
         if (warp == 1 && lane == 0) {
             umma_commit(drain_bar);
@@ -623,7 +676,8 @@ int launch_conv_f32_pack_filter_patch(
     const int bn = tile_columns(a.oc), blocks = (a.ic + kBlock - 1) / kBlock;
     const int channels = (a.oc + bn - 1) / bn * bn;
     pack_filter_patch_kernel<<<channels, 256, 0, st>>>(
-            flt_oihw, (uint8_t*)out, out + (size_t)channels * blocks * kBlock * kTaps, a.oc, a.ic, blocks, bn);
+            flt_oihw, (uint8_t*)out, (uint32_t*)out + (size_t)channels * blocks * kBlock * kTaps, a.oc, a.ic, blocks,
+            bn);
     return check_launch("pack_filter_f32_patch");
 }
 
@@ -646,11 +700,13 @@ bool conv_f32_patch_shape(const ConvF32Args& a) {
 // im2col tiles fewer than the SMs are split over clusters, which gains less than it should: 1.3 times their
 // share (8 x 40 x 40, 128 -> 64: 18.4 in 100 tiles, 14.0 in 120 patches; 1 x 52 x 52, 64 -> 64: 8.5 in 22, 9.8 in 28).
 bool conv_f32_patch_pays(const ConvF32Args& a) {
-    if (tuning().f32_patch != 1)
-        return tuning().f32_patch == 2;
     const int bn = tile_columns(a.oc);
     const long long sms = sm_count(), columns = (a.oc + bn - 1) / bn;
     const long long patches = (long long)a.n * ((a.oh + kTH - 1) / kTH) * ((a.ow + kTW - 1) / kTW) * columns;
+    if (patches > sms * kExactTiles)
+        return false;
+    if (tuning().f32_patch != 1)
+        return tuning().f32_patch == 2;
     const long long tiles = ((long long)a.m + kBM - 1) / kBM * columns;
     const int percent = a.ic > 32 ? (bn == 128 ? 83 : bn == 64 ? 66 : 58)
                         : a.ic > 16 ? (bn == 128 ? 97 : bn == 64 ? 82 : 82)
@@ -660,7 +716,7 @@ bool conv_f32_patch_pays(const ConvF32Args& a) {
 }
 
 int launch_conv_f32_patch(
-        const ConvF32Args& a, const float* src, const float* planes, const float* bias,
+        const ConvF32Args& a, const float* src, const float* planes, const float* weights, const float* bias,
         const float* z, float* dst, cudaStream_t st) {
     const int bn = tile_columns(a.oc);
     PatchF32Params p;
@@ -685,6 +741,7 @@ int launch_conv_f32_patch(
     p.ep.dst_pitch = a.dst_pitch;
     p.filter = reinterpret_cast<const uint8_t*>(planes);
     p.factor = planes + (size_t)p.n_tiles * bn * p.blocks * kBlock * kTaps;
+    p.exact = conv_f32_exact_operands(a, src, weights, false);
     p.status = device_status_word(st);
     if (!p.status)
         return ST_MALLOC;

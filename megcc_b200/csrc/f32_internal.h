@@ -41,14 +41,14 @@ size_t conv_f32_patch_filter_floats(const ConvF32Args& a);
 int launch_conv_f32_pack_filter_patch(
         const ConvF32Args& a, const float* flt_oihw, float* out, cudaStream_t st);
 int launch_conv_f32_patch(
-        const ConvF32Args& a, const float* src, const float* planes, const float* bias,
+        const ConvF32Args& a, const float* src, const float* planes, const float* weights, const float* bias,
         const float* z, float* dst, cudaStream_t st);
 size_t matmul_f32_scratch_floats(const ConvF32Args& a);
 int launch_matmul_f32(
         ConvF32Args a, const float* src, const float* b, float* c, float* scratch, cudaStream_t st);
 int launch_conv_f32_half(
-        const ConvF32Args& a, const CUtensorMap& map_a, bool a_tiled, const float* planes,
-        const float* bias, const float* z, float* dst, cudaStream_t st);
+        const ConvF32Args& a, const CUtensorMap& map_a, bool a_tiled, const float* src, const float* planes,
+        const float* weights, bool weights_raw, const float* bias, const float* z, float* dst, cudaStream_t st);
 bool conv_f32_umma_supported(const ConvF32Args& a, const float* src, const float* dst);
 // the packed filter of a 1x1 ConvBias from [K][N]
 int launch_matmul_f32_pack_b(const ConvF32Args& a, const float* b, float* out, cudaStream_t st);

@@ -495,3 +495,115 @@ def test_packed_filters_serve_every_input(ops, case, packed_as):
             # (2^-22 for the split, 2^-24 for each of at most 36 segment sums, the truncations of a chain)
             assert bool(((got.double().permute(0, 3, 1, 2) - want).abs() <= terms * 2.0 ** -19).all()), (n, h, stride, pad, half, patch)
     assert ops.device_status() == 0
+
+
+# Operands that lie far apart along K, the one axis with no scale of its own: a channel 2^p times the others
+# under weights 2^-p times the others (every term of a sum then has the same size), and the other way round; a
+# huge channel under zero weights, for all results or for all but one; zeros on both sides beside values too
+# small for the planes; one weight too small; all of it at the ends of fp32's range. The kernels on fp16 planes,
+# tiles of one and several steps and columns
+def far_apart(form, src, flt):  # src [n][k]..., flt [oc][k]...
+    k = src.shape[1]
+    if form.startswith("2^"):
+        p = float(form[2:])
+        src[:, k // 2] *= np.float32(2.0 ** p)
+        flt[:, k // 2] *= np.float32(2.0 ** -p)
+    elif form.startswith("sentinel"):
+        src[:, k // 3] = -1e30
+        flt[:, k // 3] = 0
+        if form == "sentinel but one":
+            flt[1, k // 3] = 1e-3
+    elif form == "zeros":
+        np.maximum(src, 0, out=src)
+        src[:, ::3] *= np.float32(2.0 ** -35)
+        flt[:, 1::3] = 0
+        flt[::2, 2::3] = 0
+    elif form == "one weight":
+        src[:, k // 2] *= np.float32(2.0 ** 40)
+        flt[flt.shape[0] // 2, k // 2] *= np.float32(2.0 ** -40)
+    elif form == "large":
+        src *= np.float32(2.0 ** 112)
+        flt *= np.float32(2.0 ** -70)
+    elif form == "small":
+        src *= np.float32(2.0 ** -100)
+        flt *= np.float32(2.0 ** 70)
+
+
+FAR_APART = [f"2^{p}" for p in (14, 18, 24, 28, 29, 31, 33, 40, -18, -28, -30, -40)] + [
+    "sentinel", "sentinel but one", "zeros", "one weight", "large", "small"]
+
+
+@pytest.mark.parametrize("case", [("f32_patch", 16, 16, 8, 16, 8, 3, 1), ("f32_patch", 2, 64, 64, 33, 23, 3, 1),
+                                  ("f32_patch", 1, 196, 257, 20, 20, 3, 1), ("f32_patch", 60, 128, 128, 33, 40, 3, 1),
+                                  ("f32_half", 9, 64, 129, 9, 7, 3, 1), ("f32_half", 2, 96, 200, 17, 19, 3, 2),
+                                  ("f32_half", 160, 128, 128, 13, 13, 1, 1)], ids=lambda c: "x".join(map(str, c)))
+def test_operands_far_apart_along_k(ops, case):
+    option, n, ic, oc, h, w, k, stride = case
+    for form in FAR_APART:
+        r = cases.rng_for(f"f32_along_k_{case}")
+        src = r.standard_normal((n, ic, h, w)).astype(np.float32)
+        flt = (r.standard_normal((oc, ic, k, k)) / np.sqrt(ic * k * k)).astype(np.float32)
+        far_apart(form, src, flt)
+        x, f = dev(src), dev(flt)
+        want = torch.nn.functional.conv2d(x.double(), f.double(), stride=stride, padding=k // 2)
+        terms = torch.nn.functional.conv2d(x.double().abs(), f.double().abs(), stride=stride, padding=k // 2)
+        z = dev(r.standard_normal((n, h // stride + h % stride, w // stride + w % stride, oc)).astype(np.float32))
+        if form in ("large", "small"):
+            z.zero_()
+        p = ops.conv_f32_param(n, ic, h, w, oc, k, k, stride, k // 2)
+        old = ops.set_option(option, 2), ops.set_option("f32_patch", 2 if option == "f32_patch" else 0)
+        try:
+            got = ops.conv_bias_f32_nhwc(p, ops.nchw_to_nhwc_f32(x), ops.pack_filter_f32(p, f), z=z, algo="umma")
+        finally:
+            ops.set_option("f32_patch", old[1]), ops.set_option(option, old[0])
+        z = z.double().permute(0, 3, 1, 2)
+        err = (got.double().permute(0, 3, 1, 2) - (want + z)).abs()
+        # 2^-22 for the split, at most 2^-20 for values too small for the planes, 2^-24 for each of at most 36 segment
+        # sums and for the truncations of a chain; and the rounding of the sum with z
+        bound = terms * 2.0 ** -19 + (want.abs() + z.abs()) * 2.0 ** -24
+        assert bool((err <= bound).all()), (form, float((err / bound).max()))
+    assert ops.device_status() == 0
+
+
+@pytest.mark.parametrize("shape", [(257, 300, 1026), (400, 260, 64), (130, 129, 130)], ids=lambda c: "x".join(map(str, c)))
+def test_products_of_operands_far_apart_along_k(ops, shape):
+    m, n, k = shape
+    for form in FAR_APART:
+        r = cases.rng_for(f"f32_product_along_k_{shape}")
+        a, bt = r.standard_normal((m, k)).astype(np.float32), r.standard_normal((n, k)).astype(np.float32)
+        far_apart(form, a, bt)
+        a, b = dev(a), dev(bt.T)
+        want, terms = a.double() @ b.double(), a.double().abs() @ b.double().abs()
+        for half in (2, 0):
+            old = ops.set_option("f32_half", half)
+            try:
+                got = ops.matmul_f32(a, b)
+            finally:
+                ops.set_option("f32_half", old)
+            err = (got.double() - want).abs()
+            assert bool((err <= terms * 2.0 ** -19).all()), (form, half, float((err / terms).max()) * 2 ** 19)
+    assert ops.device_status() == 0
+
+
+# a residual in the result's own place, which a tile that is stored twice must not see twice
+@pytest.mark.parametrize("case", [(2, 64, 64, 33, 23, 3), (160, 128, 128, 13, 13, 1)], ids=lambda c: "x".join(map(str, c)))
+def test_residual_in_the_results_place(ops, case):
+    n, ic, oc, h, w, k = case
+    r = cases.rng_for(f"f32_in_place_{case}")
+    src = r.standard_normal((n, ic, h, w)).astype(np.float32)
+    flt = (r.standard_normal((oc, ic, k, k)) / np.sqrt(ic * k * k)).astype(np.float32)
+    far_apart("sentinel but one", src, flt)
+    x, f = dev(src), dev(flt)
+    out = dev(r.standard_normal((n, h, w, oc)).astype(np.float32))
+    z = out.double().permute(0, 3, 1, 2)
+    want = torch.nn.functional.conv2d(x.double(), f.double(), padding=k // 2) + z
+    terms = torch.nn.functional.conv2d(x.double().abs(), f.double().abs(), padding=k // 2)
+    old = ops.set_option("f32_half", 2), ops.set_option("f32_patch", 2)
+    try:
+        p = ops.conv_f32_param(n, ic, h, w, oc, k, k, 1, k // 2)
+        ops.conv_bias_f32_nhwc(p, ops.nchw_to_nhwc_f32(x), ops.pack_filter_f32(p, f), z=out, dst=out, algo="umma")
+    finally:
+        ops.set_option("f32_half", old[0]), ops.set_option("f32_patch", old[1])
+    err = (out.double().permute(0, 3, 1, 2) - want).abs()
+    assert bool((err <= terms * 2.0 ** -19 + (want.abs() + z.abs()) * 2.0 ** -24).all())
+    assert ops.device_status() == 0
