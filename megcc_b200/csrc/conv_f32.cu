@@ -1044,10 +1044,16 @@ bool conv_f32_split_planes(const ConvF32Args& a) {
         return false;
     return (a.kh == 1 && a.kw == 1) || a.ic == 16 || a.ic >= 32;
 }
+const float* conv_f32_channel_words(const ConvF32Args& a, const float* flt_packed) {
+    const size_t plane = (size_t)a.oc * a.kh * a.kw * conv_f32_padded_ic(a.ic);
+    if (conv_f32_half_planes(a))
+        return flt_packed + 3 * plane;
+    return conv_f32_patch_planes(a) ? flt_packed + 2 * plane + conv_f32_patch_words_at(a) : nullptr;
+}
 // Filters that 128-channel tiles can be taken for (rows of 128 bytes, more than 64 channels) hold the fp16
 // planes as well: which kernel runs is known only with the batch.
 bool conv_f32_half_planes(const ConvF32Args& a) {
-    return conv_f32_split_planes(a) && a.ic > 16 && a.oc > 64;
+    return (a.forms & F32_HALF_PLANES) && conv_f32_split_planes(a) && a.ic > 16 && a.oc > 64;
 }
 
 // Images of `src` the activation's im2col map describes (see descriptor_images in internal.h)
@@ -1229,18 +1235,28 @@ static int launch_f32_tensor(
                       : launch_f32_kernel<128, 64>(map_a, map_b, p, st);
 }
 
+static bool takes_patches(const ConvF32Args& a) {
+    return conv_f32_patch_shape(a) && !tuning().f32_bn && !tuning().f32_split && conv_f32_patch_pays(a);
+}
+
+int conv_f32_forms(const ConvF32Args& a) {
+    if (!conv_f32_split_planes(a))
+        return 0;
+    return takes_patches(a) ? F32_PATCH_PLANES
+                            : choose_f32_tile(a, conv_f32_half_planes(a)).half ? F32_HALF_PLANES : 0;
+}
+
 int launch_conv_f32_umma(
         const ConvF32Args& a, const float* src, const float* flt_split, const float* bias,
         const float* z, float* dst, cudaStream_t st) {
     // (a residual in the result's own place: the kernels on fp16 planes may store a tile twice)
-    const bool in_place = z == dst;
+    const bool fp16_planes = !a.tf32_only && z != dst;
     const bool has = conv_f32_half_planes(a);
     const float* planes = flt_split + 2 * (size_t)a.oc * a.kh * a.kw * conv_f32_padded_ic(a.ic);
-    if (!in_place && conv_f32_patch_shape(a) && !tuning().f32_bn && !tuning().f32_split && conv_f32_patch_pays(a) &&
-        ((uintptr_t)flt_split & 15) == 0)
+    if (fp16_planes && takes_patches(a) && ((uintptr_t)flt_split & 15) == 0)
         return launch_conv_f32_patch(a, src, planes + (has ? conv_f32_half_filter_floats(a) : 0), flt_split, bias,
                                      z, dst, st);
-    return launch_f32_tensor(a, src, flt_split, planes, nullptr, choose_f32_tile(a, has && !in_place), bias,
+    return launch_f32_tensor(a, src, flt_split, planes, nullptr, choose_f32_tile(a, has && fp16_planes), bias,
                              z, dst, st);
 }
 

@@ -664,26 +664,30 @@ int tile_columns(int oc) {
 
 }  // namespace
 
-// floats of the planes and factors of such a filter
-size_t conv_f32_patch_filter_floats(const ConvF32Args& a) {
+// floats of the planes of such a filter, behind which its channel words lie, and of both
+size_t conv_f32_patch_words_at(const ConvF32Args& a) {
     const int bn = tile_columns(a.oc);
     const size_t channels = (size_t)(a.oc + bn - 1) / bn * bn, blocks = (a.ic + kBlock - 1) / kBlock;
-    return channels * blocks * kBlock * kTaps + channels;
+    return channels * blocks * kBlock * kTaps;
+}
+size_t conv_f32_patch_filter_floats(const ConvF32Args& a) {
+    const int bn = tile_columns(a.oc);
+    return conv_f32_patch_words_at(a) + (size_t)(a.oc + bn - 1) / bn * bn;
 }
 
 int launch_conv_f32_pack_filter_patch(
         const ConvF32Args& a, const float* flt_oihw, float* out, cudaStream_t st) {
     const int bn = tile_columns(a.oc), blocks = (a.ic + kBlock - 1) / kBlock;
     const int channels = (a.oc + bn - 1) / bn * bn;
-    pack_filter_patch_kernel<<<channels, 256, 0, st>>>(
-            flt_oihw, (uint8_t*)out, (uint32_t*)out + (size_t)channels * blocks * kBlock * kTaps, a.oc, a.ic, blocks,
-            bn);
+    pack_filter_patch_kernel<<<channels, 256, 0, st>>>(flt_oihw, (uint8_t*)out,
+                                                       (uint32_t*)out + conv_f32_patch_words_at(a), a.oc, a.ic, blocks, bn);
     return check_launch("pack_filter_f32_patch");
 }
 
-// Does a packed filter hold the planes of this kernel? (By the filter alone, see conv_f32_split_planes.)
+// Does a packed filter hold the planes of this kernel? (By the filter alone, see conv_f32_split_planes, and
+// what it was packed for.)
 bool conv_f32_patch_planes(const ConvF32Args& a) {
-    return conv_f32_split_planes(a) && a.kh == 3 && a.kw == 3;
+    return (a.forms & F32_PATCH_PLANES) && conv_f32_split_planes(a) && a.kh == 3 && a.kw == 3;
 }
 // ... and may the ConvBias take it?
 bool conv_f32_patch_shape(const ConvF32Args& a) {
@@ -740,7 +744,7 @@ int launch_conv_f32_patch(
     p.ep.dst = dst;
     p.ep.dst_pitch = a.dst_pitch;
     p.filter = reinterpret_cast<const uint8_t*>(planes);
-    p.factor = planes + (size_t)p.n_tiles * bn * p.blocks * kBlock * kTaps;
+    p.factor = planes + conv_f32_patch_words_at(a);
     p.exact = conv_f32_exact_operands(a, src, weights, false);
     p.status = device_status_word(st);
     if (!p.status)

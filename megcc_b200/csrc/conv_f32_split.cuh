@@ -21,6 +21,7 @@
 #pragma once
 #include <stdint.h>
 
+#include "f32_internal.h"
 #include "umma_ptx.cuh"
 
 namespace mb200 {
@@ -71,7 +72,8 @@ __device__ __forceinline__ uint32_t least_magnitude(uint32_t scale) { return ((2
 
 // An output channel's word: its factor (a power of two), and in its sign and last bit what its weights are like.
 // `least` over all of them, `least_nonzero` over those that are not 0
-constexpr uint32_t kWideChannel = 0x80000000u, kLooseChannel = 1u;
+// (kWideChannel: f32_internal.h)
+constexpr uint32_t kLooseChannel = 1u;
 __device__ __forceinline__ uint32_t channel_word(float largest, float least, float least_nonzero) {
     const uint32_t scale = scale_field(largest);
     const bool infinite = __float_as_uint(largest) >= 0x7F800000u;

@@ -42,6 +42,8 @@ int make_f32_args(const mb200_conv_f32_param* p, long long dst_pitch, ConvF32Arg
         return set_error(ST_OUT_OF_RANGE, "too many output pixels");
     a->m = (int)m;
     a->act = p->nonline;
+    a->forms = F32_ALL_PLANES;
+    a->tf32_only = false;
     a->src_pitch = p->ic;
     a->dst_pitch = dst_pitch > 0 ? dst_pitch : p->oc;
     a->z_pitch = p->oc;
@@ -62,7 +64,7 @@ namespace mb200 {
 int conv_bias_f32_pitched(
         const mb200_conv_f32_param* p, const float* src, long long src_pitch,
         const float* flt_packed, const float* bias, const float* z, long long z_pitch, float* dst,
-        long long dst_pitch, int algo, cudaStream_t st) {
+        long long dst_pitch, int algo, int forms, bool tf32_only, cudaStream_t st) {
     ConvF32Args a{};
     int rc = make_f32_args(p, dst_pitch, &a);
     if (rc)
@@ -71,6 +73,8 @@ int conv_bias_f32_pitched(
         a.src_pitch = src_pitch;
     if (z_pitch > 0)
         a.z_pitch = z_pitch;
+    a.forms = forms;
+    a.tf32_only = tf32_only;
     if (!src || !flt_packed || !dst)
         return set_error(ST_NULL_PTR, "conv tensor pointer is NULL");
     if (((uintptr_t)src | (uintptr_t)flt_packed | (uintptr_t)dst | (uintptr_t)bias |
@@ -90,31 +94,56 @@ int conv_bias_f32_pitched(
     return launch_conv_f32_direct(a, src, flt_packed, bias, z, dst, st);
 }
 
+int conv_f32_forms(const mb200_conv_f32_param* p) {
+    ConvF32Args a{};
+    return make_f32_args(p, 0, &a) ? 0 : conv_f32_forms(a);
+}
+
+size_t conv_f32_packed_bytes(const mb200_conv_f32_param* p, int forms) {
+    ConvF32Args a{};
+    if (make_f32_args(p, 0, &a))
+        return 0;
+    a.forms = forms;
+    return conv_f32_split_planes(a) ? up256(conv_f32_split_filter_floats(a) * sizeof(float))
+                                    : plain_filter_bytes(a);
+}
+
+int conv_f32_pack(
+        const mb200_conv_f32_param* p, int forms, const float* flt_oihw, float* flt_packed, cudaStream_t st) {
+    ConvF32Args a{};
+    int rc = make_f32_args(p, 0, &a);
+    if (rc)
+        return rc;
+    a.forms = forms;
+    if (!flt_oihw || !flt_packed)
+        return set_error(ST_NULL_PTR, "filter pointer is NULL");
+    if (((uintptr_t)flt_oihw & 3) || ((uintptr_t)flt_packed & 15))
+        return set_error(ST_INVALID_LAYOUT, "filter must be 4-byte, packed filter 16-byte aligned");
+    return conv_f32_split_planes(a) ? launch_conv_f32_pack_filter_split(a, flt_oihw, flt_packed, st)
+                                    : launch_conv_f32_pack_filter_plain(a, flt_oihw, flt_packed, st);
+}
+
+const float* conv_f32_filter_words(
+        const mb200_conv_f32_param* p, int forms, const float* flt_packed, int* count) {
+    ConvF32Args a{};
+    if (make_f32_args(p, 0, &a))
+        return nullptr;
+    a.forms = forms;
+    *count = a.oc;
+    return conv_f32_channel_words(a, flt_packed);
+}
+
 }  // namespace mb200
 
 extern "C" {
 
 size_t mb200_conv_f32_packed_filter_bytes(const mb200_conv_f32_param* p) {
-    ConvF32Args a{};
-    if (make_f32_args(p, 0, &a))
-        return 0;
-    return conv_f32_split_planes(a) ? up256(conv_f32_split_filter_floats(a) * sizeof(float))
-                                      : plain_filter_bytes(a);
+    return conv_f32_packed_bytes(p, F32_ALL_PLANES);
 }
 
 int mb200_conv_f32_pack_filter(
         const mb200_conv_f32_param* p, const float* flt_oihw, float* flt_packed, void* stream) {
-    ConvF32Args a{};
-    int rc = make_f32_args(p, 0, &a);
-    if (rc)
-        return rc;
-    if (!flt_oihw || !flt_packed)
-        return set_error(ST_NULL_PTR, "filter pointer is NULL");
-    if (((uintptr_t)flt_oihw & 3) || ((uintptr_t)flt_packed & 15))
-        return set_error(ST_INVALID_LAYOUT, "filter must be 4-byte, packed filter 16-byte aligned");
-    cudaStream_t st = (cudaStream_t)stream;
-    return conv_f32_split_planes(a) ? launch_conv_f32_pack_filter_split(a, flt_oihw, flt_packed, st)
-                                      : launch_conv_f32_pack_filter_plain(a, flt_oihw, flt_packed, st);
+    return conv_f32_pack(p, F32_ALL_PLANES, flt_oihw, flt_packed, (cudaStream_t)stream);
 }
 
 // (kept, like the workspace arguments, for callers of earlier versions: the operands are split on
@@ -127,8 +156,8 @@ int mb200_conv_bias_f32_nhwc(
         const mb200_conv_f32_param* p, const float* src, const float* flt_packed,
         const float* bias, const float* z, float* dst, long long dst_pitch, void*, size_t, int algo,
         void* stream) {
-    return conv_bias_f32_pitched(p, src, 0, flt_packed, bias, z, 0, dst, dst_pitch, algo,
-                                 (cudaStream_t)stream);
+    return conv_bias_f32_pitched(p, src, 0, flt_packed, bias, z, 0, dst, dst_pitch, algo, F32_ALL_PLANES,
+                                 false, (cudaStream_t)stream);
 }
 
 // ---- fp32 matrix product: a 1x1 ConvBias over M "pixels" with K channels ----

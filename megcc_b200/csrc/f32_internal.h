@@ -21,11 +21,16 @@ struct ConvF32Args {
     long long src_pitch;  // floats between consecutive pixels of src (>= ic)
     long long dst_pitch;  // ... of dst (>= oc): lets a conv write its slice of a concat buffer
     long long z_pitch;    // ... of the optional residual operand
+    int forms;       // fp16 planes that the packed filter may hold (F32Forms)
+    bool tf32_only;  // not the kernels that use them
 };
+// A caller of the C ABI packs a filter for every kernel; a network knows which one will run.
+enum F32Forms : int { F32_HALF_PLANES = 1, F32_PATCH_PLANES = 2, F32_ALL_PLANES = 3 };
 
 int conv_f32_padded_ic(int ic);
 // does the packed filter begin with the two tf32 planes (else: plain K-major)?
 bool conv_f32_split_planes(const ConvF32Args& a);
+int conv_f32_forms(const ConvF32Args& a);
 size_t conv_f32_split_filter_floats(const ConvF32Args& a);
 // fp16 planes for the wide layers (conv_f32_half.cu), behind the tf32 planes of the filters that have them
 bool conv_f32_half_planes(const ConvF32Args& a);
@@ -38,6 +43,7 @@ bool conv_f32_patch_planes(const ConvF32Args& a);
 bool conv_f32_patch_shape(const ConvF32Args& a);
 bool conv_f32_patch_pays(const ConvF32Args& a);
 size_t conv_f32_patch_filter_floats(const ConvF32Args& a);
+size_t conv_f32_patch_words_at(const ConvF32Args& a);
 int launch_conv_f32_pack_filter_patch(
         const ConvF32Args& a, const float* flt_oihw, float* out, cudaStream_t st);
 int launch_conv_f32_patch(
@@ -82,7 +88,17 @@ int launch_pooling_f32(
 int conv_bias_f32_pitched(
         const mb200_conv_f32_param* p, const float* src, long long src_pitch,
         const float* flt_packed, const float* bias, const float* z, long long z_pitch, float* dst,
-        long long dst_pitch, int algo, cudaStream_t st);
+        long long dst_pitch, int algo, int forms, bool tf32_only, cudaStream_t st);
+// the forms that such a ConvBias makes use of, and its filter packed in them
+int conv_f32_forms(const mb200_conv_f32_param* p);
+size_t conv_f32_packed_bytes(const mb200_conv_f32_param* p, int forms);
+int conv_f32_pack(
+        const mb200_conv_f32_param* p, int forms, const float* flt_oihw, float* flt_packed, cudaStream_t st);
+// Has a packed filter weights that its fp16 planes do not hold (conv_f32_split.cuh)? Its channel words tell:
+// where they are (null: it has none), and how many.
+const float* conv_f32_filter_words(const mb200_conv_f32_param* p, int forms, const float* flt_packed, int* count);
+constexpr uint32_t kWideChannel = 0x80000000u;  // in a channel word
+const float* conv_f32_channel_words(const ConvF32Args& a, const float* flt_packed);
 int launch_focus_f32(
         const float* src_nchw, float* dst_nhwc, int n, int c, int h, int w, int c_out,
         cudaStream_t st);

@@ -99,6 +99,8 @@ struct OpPlan {
     int flt44 = 0;         // filter layout: 0 OIHW, 1 / 2 / 3 NCHW44 dense / channel-wise / first layer
     int z_mode = 0;        // fused elemwise step: 0 none, else MB200_QADD + 1 / MB200_QFUSE_ADD_RELU + 1
     bool f32_z = false;    // fp32 ConvBias with a tensor added after the activation
+    int f32_forms = 0;     // ... the planes its filter is packed in beside the tf32 ones
+    bool f32_wide = false; // ... weights that only the tf32 ones hold (known once they are packed)
     int oc = 0, icpg = 0;  // fp32 ConvBias: output channels, input channels per group (symbol)
     // table indices from the model file and the functions they resolved to
     int kernel_id = -1, init_id = -1;
@@ -739,7 +741,7 @@ TinyNNStatus builtin_kernel(
                     &p, (const float*)inputs[0]->ptr, pixel_pitch(inputs[0]),
                     (const float*)inputs[1]->ptr, bias, z,
                     z ? pixel_pitch(inputs[nr_input - 1]) : 0, (float*)dst->ptr, pixel_pitch(dst),
-                    MB200_ALGO_AUTO, (cudaStream_t)st);
+                    MB200_ALGO_AUTO, op.f32_forms, op.f32_wide, (cudaStream_t)st);
         }
         case OP_MATMUL_F32: {
             const Tensor* a = inputs[0];
@@ -872,11 +874,13 @@ TinyNNStatus builtin_init(
             mb200_conv_f32_param p;
             fill_conv_f32_param(op, inputs, &p);
             if (describe) {
-                flat(mb200_conv_f32_packed_filter_bytes(&p) / 4);
+                // (16 floats more for each form's bit: filters packed in other forms have other sizes, which
+                // are multiples of 64 floats, and are not shared)
+                flat(mb200::conv_f32_packed_bytes(&p, op.f32_forms) / 4 + 16 * op.f32_forms);
                 return TinyNN_SUCCESS;
             }
-            return (TinyNNStatus)mb200_conv_f32_pack_filter(
-                    &p, (const float*)w->ptr, (float*)out_weights->ptr, opt->stream);
+            return (TinyNNStatus)mb200::conv_f32_pack(&p, op.f32_forms, (const float*)w->ptr,
+                                                      (float*)out_weights->ptr, (cudaStream_t)opt->stream);
         }
         case OP_MATMUL_F32: {
             if (w->layout.nr_dim != 2)
@@ -1728,6 +1732,11 @@ int upload_weights(Network* net) {
             if (!ins.is_opr || !ins.op.init_fn)
                 continue;
             OpPlan& op = ins.op;
+            if (op.kind == OP_CONV_F32 && op.init_fn == builtin_init) {
+                mb200_conv_f32_param p;
+                fill_conv_f32_param(op, op.inputs.data(), &p);
+                op.f32_forms = mb200::conv_f32_forms(&p);
+            }
             RuntimeOpt opt = net->opt;
             opt.opr = &op;
             int count = 0;
@@ -1810,6 +1819,36 @@ int upload_weights(Network* net) {
         job.op->inputs[job.input] = &net->processed[job.processed];
     if ((e = cudaStreamSynchronize(net->stream)) != cudaSuccess)
         return cuda_fail(e, "weight upload");
+    // fp32 filters that the kernels on fp16 planes would put off tile by tile go to the tf32 one at once
+    std::vector<uint32_t> words;
+    std::vector<std::pair<OpPlan*, size_t>> wordy;  // ... and where the operator's words end
+    for (int fill = 0; fill < 2; ++fill) {
+        size_t at = 0;
+        for (auto& job : jobs) {
+            if (job.op->f32_forms == 0)
+                continue;
+            mb200_conv_f32_param p;
+            fill_conv_f32_param(*job.op, job.op->inputs.data(), &p);
+            int count = 0;
+            const float* from = mb200::conv_f32_filter_words(
+                    &p, job.op->f32_forms, (const float*)job.op->inputs[1]->ptr, &count);
+            if (!from)
+                continue;
+            if (fill && (e = cudaMemcpyAsync(words.data() + at, from, (size_t)count * 4, cudaMemcpyDeviceToHost,
+                                             net->stream)) != cudaSuccess)
+                return cuda_fail(e, "packed filters");
+            at += (size_t)count;
+            if (!fill)
+                wordy.push_back({job.op, at});
+        }
+        words.resize(at);
+    }
+    if (!words.empty() && (e = cudaStreamSynchronize(net->stream)) != cudaSuccess)
+        return cuda_fail(e, "packed filters");
+    size_t at = 0;
+    for (auto& w : wordy)
+        for (; at < w.second; ++at)
+            w.first->f32_wide |= (words[at] & mb200::kWideChannel) != 0;
     if (!mb200::device_status_word(net->stream))
         return fail(TinyNN_ERROR_MEMORY_MALLOC, "%s", mb200_last_error());
     mb200::register_constant_range(net->weight_arena, total);  // nothing writes them from here on

@@ -607,3 +607,35 @@ def test_residual_in_the_results_place(ops, case):
     err = (out.double().permute(0, 3, 1, 2) - want).abs()
     assert bool((err <= terms * 2.0 ** -19 + (want.abs() + z.abs()) * 2.0 ** -24).all())
     assert ops.device_status() == 0
+
+
+# a network whose filters hold a dead input channel (weights that have decayed to 1e-25 beside ordinary ones),
+# with its activations large enough to matter: known as the weights are packed
+def test_networks_with_weights_far_apart(ops, oracle):
+    from megcc_b200 import lite
+    from megcc_b200.compiler import Graph
+    r = cases.rng_for("f32_dead_channel")
+    shapes = {"a": (128, 64, 1, 1), "b": (64, 128, 3, 3), "c": (32, 64, 3, 3)}
+    f = {n: (r.standard_normal(s) / np.sqrt(s[1] * s[2] * s[3])).astype(np.float32) for n, s in shapes.items()}
+    f["a"][:, 3] *= np.float32(1e-25)
+    f["b"][:, 7] *= np.float32(1e-25)
+    src = r.standard_normal((64, 64, 12, 12)).astype(np.float32)
+    src[:, 3] *= np.float32(1e24)
+    g = Graph("dead")
+    x = g.input_f32("data", 64, 12, 12)
+    a = g.conv_f32("a", x, f["a"], None, 1, 0, "RELU")
+    b = g.conv_f32("b", a, f["b"], None, 1, 1, "SILU")
+    g.mark_output(g.conv_f32("c", b, f["c"], None, 1, 1, "IDENTITY"))
+    conv = lambda v, n, pad, act: oracle.conv_bias_f32(v, f[n], None, 1, pad, act)
+    want = conv(conv(conv(src, "a", 0, "RELU"), "b", 1, "SILU"), "c", 1, "IDENTITY")
+    old = ops.set_option("f32_half", 2), ops.set_option("f32_patch", 2)
+    try:
+        net = lite.Network(g.compile([64]))
+        net.set_input("data", src)
+        net.forward()
+        net.wait()
+        close(net.output(net.output_names()[0], dtype=np.float32).reshape(want.shape), want)
+        net.close()
+    finally:
+        ops.set_option("f32_half", old[0]), ops.set_option("f32_patch", old[1])
+    assert ops.device_status() == 0
