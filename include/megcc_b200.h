@@ -390,9 +390,12 @@ MB200_API int mb200_matmul_f32(
         int m, int n, int k, const float* a, const float* b_packed, float* c, void* workspace,
         size_t workspace_bytes, void* stream);
 /* The same with B as it is, [K][N]: preparation and product in one call, with the planes of B that suit the
- * product's sizes, over mb200_matmul_f32_scratch_bytes(m, n, k) bytes of device scratch (16-byte
- * aligned). Tensor cores for every m, n, k where C is 16-byte aligned. */
+ * product's sizes, over mb200_matmul_f32_scratch_bytes_for(m, n, k, a) bytes of device scratch (16-byte
+ * aligned): B's planes, and a copy of A where k % 4 != 0 or A is not 16-byte aligned.
+ * mb200_matmul_f32_scratch_bytes(m, n, k) is enough for every address of A. Tensor cores for every m, n, k
+ * where C is 16-byte aligned. */
 MB200_API size_t mb200_matmul_f32_scratch_bytes(int m, int n, int k);
+MB200_API size_t mb200_matmul_f32_scratch_bytes_for(int m, int n, int k, const float* a);
 MB200_API int mb200_matmul_f32_product(
         int m, int n, int k, const float* a, const float* b, float* c, void* scratch,
         size_t scratch_bytes, void* stream);

@@ -94,6 +94,7 @@ SIGNATURES = {
                                            C.c_longlong, _P, C.c_size_t, C.c_int, _P]),
     "mb200_matmul_f32_packed_b_bytes": (C.c_size_t, [C.c_int, C.c_int]),
     "mb200_matmul_f32_scratch_bytes": (C.c_size_t, [C.c_int] * 3),
+    "mb200_matmul_f32_scratch_bytes_for": (C.c_size_t, [C.c_int] * 3 + [_P]),
     "mb200_matmul_f32_product": (C.c_int, [C.c_int] * 3 + [_P] * 4 + [C.c_size_t, _P]),
     "mb200_matmul_f32_pack_b": (C.c_int, [C.c_int, C.c_int, _P, _P, _P]),
     "mb200_matmul_f32_workspace_bytes": (C.c_size_t, [C.c_int, C.c_int]),
@@ -129,7 +130,7 @@ def lib():
 FAST = ("mb200_conv_bias_qs8_nhwc", "mb200_conv_bias_qs8_nhwc_fused", "mb200_conv_bias_qs8_nchw",
         "mb200_matmul_s8_qs8", "mb200_qelemwise_qs8", "mb200_conv_bias_f32_nhwc",
         "mb200_conv_bias_qs8_nchw_workspace", "mb200_conv_nchw_in_place",
-        "mb200_conv_bias_qs8_nchw_in_place", "mb200_matmul_f32_scratch_bytes",
+        "mb200_conv_bias_qs8_nchw_in_place", "mb200_matmul_f32_scratch_bytes_for",
         "mb200_matmul_f32_product", "mb200_elemwise_f32")
 _fast = None
 

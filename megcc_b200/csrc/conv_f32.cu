@@ -1265,11 +1265,10 @@ static bool product_pads(int k, const float* a) {
     return k % 4 != 0 || ((uintptr_t)a & 15) != 0;
 }
 
-size_t matmul_f32_scratch_floats(const ConvF32Args& a) {
+size_t matmul_f32_scratch_floats(const ConvF32Args& a, const float* src) {
     const int kp = conv_f32_padded_ic(a.ic);
     const size_t b = 2 * (size_t)a.oc * kp + (size_t)(a.oc + 3) / 4 * 4;
-    // (an aligned A of whole vectors needs none: the pointer decides at the call)
-    return b + (size_t)a.m * ((a.ic + 3) / 4 * 4);
+    return b + (product_pads(a.ic, src) ? (size_t)a.m * ((a.ic + 3) / 4 * 4) : 0);
 }
 
 // Which planes of B are made is decided with the sizes of the product. Rows of A that the TMA cannot

@@ -224,9 +224,13 @@ static int product_args(int m, int n, int k, ConvF32Args* a) {
     return rc ? rc : make_f32_args(&p, 0, a);
 }
 
+size_t mb200_matmul_f32_scratch_bytes_for(int m, int n, int k, const float* a) {
+    ConvF32Args args{};
+    return product_args(m, n, k, &args) ? 0 : up256(matmul_f32_scratch_floats(args, a) * sizeof(float));
+}
+
 size_t mb200_matmul_f32_scratch_bytes(int m, int n, int k) {
-    ConvF32Args a{};
-    return product_args(m, n, k, &a) ? 0 : up256(matmul_f32_scratch_floats(a) * sizeof(float));
+    return mb200_matmul_f32_scratch_bytes_for(m, n, k, (const float*)4);  // (an address that needs the copy)
 }
 
 int mb200_matmul_f32_product(
@@ -242,7 +246,7 @@ int mb200_matmul_f32_product(
         return set_error(ST_INVALID_LAYOUT, "fp32 operands must be 4-byte aligned");
     if ((uintptr_t)scratch & 15)
         return set_error(ST_INVALID_LAYOUT, "scratch must be 16-byte aligned");
-    if (scratch_bytes < mb200_matmul_f32_scratch_bytes(m, n, k))
+    if (scratch_bytes < mb200_matmul_f32_scratch_bytes_for(m, n, k, a))
         return set_error(ST_OUT_OF_RANGE, "scratch of %zu bytes is too small", scratch_bytes);
     cudaStream_t st = (cudaStream_t)stream;
     if (((uintptr_t)c & 15) == 0)

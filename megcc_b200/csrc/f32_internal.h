@@ -49,7 +49,7 @@ int launch_conv_f32_pack_filter_patch(
 int launch_conv_f32_patch(
         const ConvF32Args& a, const float* src, const float* planes, const float* weights, const float* bias,
         const float* z, float* dst, cudaStream_t st);
-size_t matmul_f32_scratch_floats(const ConvF32Args& a);
+size_t matmul_f32_scratch_floats(const ConvF32Args& a, const float* src);
 int launch_matmul_f32(
         ConvF32Args a, const float* src, const float* b, float* c, float* scratch, cudaStream_t st);
 int launch_conv_f32_half(

@@ -249,7 +249,7 @@ def matmul_f32(a, b):
     m, k = a.shape
     n = b.shape[1]
     f = fast()
-    nbytes = f.mb200_matmul_f32_scratch_bytes(m, n, k)
+    nbytes = f.mb200_matmul_f32_scratch_bytes_for(m, n, k, _ptr(a))
     scratch = a.new_empty(nbytes // 4, dtype=torch.float32)
     c = a.new_empty((m, n), dtype=torch.float32)
     check(f.mb200_matmul_f32_product(m, n, k, _ptr(a), _ptr(b), _ptr(c), scratch.data_ptr(), nbytes, _stream()))

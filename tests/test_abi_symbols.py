@@ -129,3 +129,18 @@ def test_packed_f32_filter_size_follows_the_filter(ic, oc, k):
     if k == 1:
         sizes.add(_lib.lib().mb200_matmul_f32_packed_b_bytes(ic, oc))
     assert len(sizes) == 1 and sizes.pop() > 0
+
+
+# An fp32 product asks for a copy of A only where the TMA cannot address A's rows.
+@pytest.mark.parametrize("m", [1, 1000, 1 << 20])
+@pytest.mark.parametrize("n,k", [(65, 1000), (128, 64), (1024, 1024)])
+def test_f32_product_scratch_holds_no_copy_of_aligned_operands(m, n, k):
+    from megcc_b200 import _lib
+    L = _lib.lib()
+    planes = L.mb200_matmul_f32_scratch_bytes_for(1, n, k, 4096)
+    assert 8 * n * k <= planes <= 8 * n * (k + 31) + 4 * n + 1024
+    assert L.mb200_matmul_f32_scratch_bytes_for(m, n, k, 4096) == planes
+    whole = L.mb200_matmul_f32_scratch_bytes_for(m, n, k, 4100)
+    assert whole == L.mb200_matmul_f32_scratch_bytes(m, n, k) >= planes + 4 * m * k - 256
+    padded = L.mb200_matmul_f32_scratch_bytes_for(m, n, k - 1, 4096)
+    assert padded == L.mb200_matmul_f32_scratch_bytes(m, n, k - 1) > 4 * m * k
