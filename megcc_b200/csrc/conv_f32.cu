@@ -972,6 +972,8 @@ struct F32Choice {
     int bn, splits;
     bool half;  // 128 columns, from fp16 planes
 };
+int f32_step_clocks(int bn, int rowb) { return (bn == 128 ? 850 : bn == 64 ? 500 : 420) * rowb / 128; }
+int f32_end_clocks(int bn) { return bn == 128 ? 2500 : bn == 64 ? 1500 : 1000; }  // sums, activation, stores
 F32Choice choose_f32_tile(const ConvF32Args& a, bool planes) {
     const int rowb = a.ic <= 16 ? 64 : 128, oc = a.oc;
     const int m_tiles = (a.m + kBM - 1) / kBM;
@@ -982,8 +984,7 @@ F32Choice choose_f32_tile(const ConvF32Args& a, bool planes) {
     for (int b = 128; b >= 32; b /= 2) {
         if (b > 32 && oc <= b / 2)
             continue;
-        const int step = (b == 128 ? 850 : b == 64 ? 500 : 420) * rowb / 128;
-        const int tile_end = b == 128 ? 2500 : b == 64 ? 1500 : 1000;  // sums, activation, stores
+        const int step = f32_step_clocks(b, rowb), tile_end = f32_end_clocks(b);
         const long long tiles = (long long)m_tiles * ((oc + b - 1) / b);
         for (int s = 1; s <= 8; s *= 2) {
             if (s > 1 && (k_iters / s < 2 || tiles > sms / s || tiles > f32_cluster_capacity(b, rowb, s)))
@@ -1024,6 +1025,13 @@ bool plain_matrix(const ConvF32Args& a) {
 // channels the packed (split) filter holds per tap: ic rounded up to a whole TMA row
 int conv_f32_padded_ic(int ic) {
     return ic <= 16 ? 16 : (ic + 31) / 32 * 32;
+}
+
+// the clocks of one tile among others, by the estimates of choose_f32_tile
+long long conv_f32_tile_clocks(const ConvF32Args& a, int bn) {
+    const int rowb = a.ic <= 16 ? 64 : 128;
+    return (long long)a.kh * a.kw * (conv_f32_padded_ic(a.ic) * 4 / rowb) * f32_step_clocks(bn, rowb) +
+           f32_end_clocks(bn);
 }
 
 size_t conv_f32_split_filter_floats(const ConvF32Args& a) {

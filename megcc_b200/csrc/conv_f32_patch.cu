@@ -696,13 +696,18 @@ bool conv_f32_patch_shape(const ConvF32Args& a) {
 
 // ... and is it the faster one then? Both kernels' time goes with the tiles of the busiest SM; a patch that is not
 // full is paid for in full. What a patch takes beside an im2col tile of the same columns and channels, in
-// percent, was measured with full patches and 1600 to 25600 of them (us, im2col -> patches; 32 images of
-// 80 x 80 where nothing else is said):
-//   128 columns: 128 channels 204 -> 170, 32 channels 85 -> 82, 16 channels 63 -> 74
-//    64 columns:  64 channels 102 -> 67,  32 channels 60 -> 49, 16 channels 38 -> 43
-//    32 columns:  36 channels, 64 x 64: 46.8 -> 26.3; 32 channels, 8 of 160 x 160: 41.3 -> 33.9; 16: 30.4 -> 27.6
-// im2col tiles fewer than the SMs are split over clusters, which gains less than it should: 1.3 times their
-// share (8 x 40 x 40, 128 -> 64: 18.4 in 100 tiles, 14.0 in 120 patches; 1 x 52 x 52, 64 -> 64: 8.5 in 22, 9.8 in 28).
+// percent, was measured as what one more on every SM costs, full patches, 200 to 1600 of them (us, im2col -> patches at
+// 400 and 1600; SILU or no activation alike):
+//   128 columns: 128 channels 54.0 -> 43.5, 202 -> 166; 64 channels 31.6 -> 26.3, 110 -> 99; 32 and 16: none better
+//    64 columns:  64 channels 25.9 -> 17.9, 87 -> 63; 32 channels 16.8 -> 14.1, 51.6 -> 41.9; 16: none better
+//    32 columns:  64 channels 21.9 -> 15.5, 71 -> 45; 32 channels 13.1 -> 11.9, 37.6 -> 31.9; 16: 10.3 -> 9.7, 28.9 -> 25.3
+// That is one layer over and over. In a network a patch kernel takes some 3 us more, which im2col kernels, of
+// which the layers around are, do not (kStart, in the clocks of conv_f32_tile_clocks). The detector with every
+// layer that is the faster one by itself, us beside none of them: one image of 256 x 256 +4.0, 416 x 416 +2.8,
+// 480 x 480 +4.1, two of 320 x 320 +5.1, four of 416 x 416 +4.7, of 640 x 640 -40; by this rule +0.3, -0.2, -0.2,
+// -0.2, -5.8 and -39.
+// im2col tiles of at most half the SMs are split over clusters and stay (1 x 80 x 80, 50 of each: 64 -> 64 9.2 and
+// 9.2, 16 -> 32 5.2 and 5.6).
 bool conv_f32_patch_pays(const ConvF32Args& a) {
     const int bn = tile_columns(a.oc);
     const long long sms = sm_count(), columns = (a.oc + bn - 1) / bn;
@@ -712,11 +717,14 @@ bool conv_f32_patch_pays(const ConvF32Args& a) {
     if (tuning().f32_patch != 1)
         return tuning().f32_patch == 2;
     const long long tiles = ((long long)a.m + kBM - 1) / kBM * columns;
-    const int percent = a.ic > 32 ? (bn == 128 ? 83 : bn == 64 ? 66 : 58)
-                        : a.ic > 16 ? (bn == 128 ? 97 : bn == 64 ? 82 : 82)
-                                    : (bn == 128 ? 117 : bn == 64 ? 115 : 90);
-    const long long here = (patches + sms - 1) / sms * percent;
-    return here < (tiles >= sms ? (tiles + sms - 1) / sms * 100 : tiles * 130 / sms);
+    const int percent = a.ic > 32 ? (bn == 128 ? 84 : bn == 64 ? 66 : 60)
+                        : a.ic > 16 ? (bn == 128 ? 100 : bn == 64 ? 80 : 80)
+                                    : (bn == 32 ? 83 : 100);
+    if (percent == 100 || 2 * tiles <= sms)
+        return false;
+    constexpr long long kStart = 4000;
+    const long long tile = conv_f32_tile_clocks(a, bn);
+    return (patches + sms - 1) / sms * percent * tile + 100 * kStart < (tiles + sms - 1) / sms * 100 * tile;
 }
 
 int launch_conv_f32_patch(

@@ -28,6 +28,7 @@ struct ConvF32Args {
 enum F32Forms : int { F32_HALF_PLANES = 1, F32_PATCH_PLANES = 2, F32_ALL_PLANES = 3 };
 
 int conv_f32_padded_ic(int ic);
+long long conv_f32_tile_clocks(const ConvF32Args& a, int bn);
 // does the packed filter begin with the two tf32 planes (else: plain K-major)?
 bool conv_f32_split_planes(const ConvF32Args& a);
 int conv_f32_forms(const ConvF32Args& a);

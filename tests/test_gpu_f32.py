@@ -639,3 +639,20 @@ def test_networks_with_weights_far_apart(ops, oracle):
     finally:
         ops.set_option("f32_half", old[0]), ops.set_option("f32_patch", old[1])
     assert ops.device_status() == 0
+
+
+# Halo patches only where they gain more than a kernel of its own costs among others
+@pytest.mark.parametrize("n,ic,oc,h,patches", [
+    (1, 16, 32, 128, False), (1, 16, 32, 208, False), (1, 32, 32, 120, False), (1, 64, 32, 136, False),
+    (1, 64, 64, 52, False), (4, 16, 64, 320, False), (1, 32, 32, 320, True), (32, 64, 64, 80, True),
+    (8, 16, 32, 320, True), (1, 128, 128, 112, True)])
+def test_layers_that_take_halo_patches(ops, capfd, n, ic, oc, h, patches):
+    src, flt = torch.zeros((n, h, h, ic), device="cuda"), torch.zeros((oc, ic, 3, 3), device="cuda")
+    p = ops.conv_f32_param(n, ic, h, h, oc, 3, 3, 1, 1)
+    packed = ops.pack_filter_f32(p, flt)
+    old = ops.set_option("debug", 1)
+    try:
+        ops.conv_bias_f32_nhwc(p, src, packed)
+    finally:
+        ops.set_option("debug", old)
+    assert ("conv_f32_patch" in capfd.readouterr().err) == patches
