@@ -97,8 +97,9 @@ MB200_API const char* mb200_last_error(void);
  * "f32_half" 0|1|2, "f32_patch" 0|1|2, "debug" 0|1,
  * "pdl" 1|0 (programmatic dependent launch of consecutive kernels). Their initial values come from
  * the environment variables of the same meaning (MB200_CONV_BN, ...), read ONCE per process; no
- * launch consults the environment. Every setting yields bit-identical int8 results; the three of the
- * fp32 kernels change the order of its sums. Process-wide, not thread-safe against concurrent
+ * launch consults the environment. Every setting yields bit-identical int8 results; "f32_bn" and
+ * "f32_split" change the order of fp32 sums, "f32_half" and "f32_patch" also whether operands are split into two
+ * fp16 or two tf32 values. Process-wide, not thread-safe against concurrent
  * launches. */
 MB200_API int mb200_set_option(const char* name, int value);
 MB200_API int mb200_get_option(const char* name, int* value);
@@ -328,7 +329,9 @@ MB200_API int mb200_relayout_nhwc_to_nchw_s8(
  * scalar kernels otherwise. Results agree with the reference's x86 kernels within 1e-4
  * relative / 1e-5 absolute (fp32 sums in a different order), not bit for bit, for finite operands:
  * the tensor-core path multiplies the two halves of a split value, and an infinity, whose second
- * half is a NaN, gives NaN there.
+ * half is a NaN, gives NaN there. However far apart the operands lie, splitting them costs a result at most
+ * 2^-20 of the sum of its terms' magnitudes (two fp16 values hold what lies within 2^29 of the largest of a
+ * pixel's 64 channels, or of an output channel's filter; what does not is multiplied from tf32 values).
  * ====================================================================================== */
 
 /* nonlineMode of an fp32 ConvBias. The reference's fp32 ConvBias kernels take IDENTITY / RELU /

@@ -822,7 +822,7 @@ std::string ConvBiasF32::GetInitBody(TContext* ctx) const {
     Subst s = conv_f32_common(ctx, this, R"(
 TinyNNStatus ${signature} {
     /* three-phase init (runtime/src/data_struct.h:135-142): the OIHW filter becomes the K-major
-     * filter followed by its two tf32 planes, a flat float buffer */
+     * filter or its planes for the tensor-core kernels, a flat float buffer */
     Tensor* in_weights = inputs[1];
     mb200_conv_f32_param p;
     ${symbol}_param(inputs, &p);
@@ -860,10 +860,9 @@ TinyNNStatus ${signature} {
     return s.text;
 }
 
-// must agree with mb200_conv_f32_workspace_bytes (megcc_b200/csrc/f32_abi.cu): the two tf32
-// planes of the activation when the filter is dense and its channels fill whole TMA rows
+// must agree with mb200_conv_f32_workspace_bytes (megcc_b200/csrc/f32_abi.cu)
 size_t ConvBiasF32::WorkspaceBytes(TContext*) const {
-    return 0;  // the activation is split into its tf32 planes in shared memory
+    return 0;  // the activation is split into its planes on chip
 }
 
 // ---- MatrixMul fp32 ----

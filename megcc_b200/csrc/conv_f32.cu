@@ -1002,7 +1002,7 @@ F32Choice choose_f32_tile(const ConvF32Args& a, bool planes) {
         }
     }
     // 128 columns from fp16 planes (conv_f32_half.cu): two rows of A in the time of 1.64 here (32 x 80 x 80
-    // pixels, 128 -> 128 3x3: 251 us and 206; 32 x 20 x 20, 256 -> 256: 100 as 64 columns, 82)
+    // pixels, 128 -> 128 3x3: 282 us and 224; 32 x 20 x 20, 256 -> 256: 100 as 64 columns, 72)
     const long long waves = ((long long)m_tiles * ((oc + 127) / 128) + sms - 1) / sms;
     const bool fits = planes && waves <= kExactTiles;
     c.half = fits && waves * ((long long)((k_iters + 1) / 2) * 1395 + 2500 + (waves > 1 ? 0 : 3000)) < best;

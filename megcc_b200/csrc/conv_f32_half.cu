@@ -23,9 +23,9 @@
 // time; with tf32 it is 224 KB and 1792 against 1536. Measured 1750 to 1950 clocks a segment (tf32:
 // 2300): the converters' chain of a segment (wait, read, largest value, split, write) is 1370, and with
 // the rings three segments deep it and the TMA's round trip overlap only in part. Per call, tf32 and here: 32 x 80 x 80 pixels, 128 -> 128
-// 3x3 251 and 206 us, 128 -> 256 3x3/2 153 and 113, a 2048^3 product without its preparation 77 and 63.
+// 3x3 282 and 224 us, 1x1 59.7 and 47.0, 128 -> 256 3x3/2 137 and 109, a 2048^3 product with its preparation 93 and 80.
 // Against 64 bits the results are no further off (2-norm, N(0,1) operands: K = 1152 2.1e-7 and 1.6e-7,
-// K = 4096 2.2e-7 and 2.0e-7).
+// K = 4096 2.3e-7 and 2.0e-7; K = 1152 with one channel 2^16 to 2^40 up under weights as far down 2.1e-7 and 1.7e-7).
 // Narrower tiles do not gain: their TMA rows (4 clocks each) are the same with either split.
 //
 // Structure: persistent CTAs, warp 0 TMA producer (im2col or plain matrix rows), warp 1 MMA issuer and

@@ -18,8 +18,8 @@
 // is packed as it lies in shared memory and comes in one contiguous copy per group of taps (boxes of a
 // tensor map took 5.7 clocks a row: 32 x 320 x 320, 16 -> 32, 600 us, then 430), stays there where it is the only
 // one, pixels go from global memory to the planes by way of registers, a block ahead, and results leave turned
-// round. 32 images, us, im2col tiles and here: 80 x 80, 64 -> 64: 102, 67; 128 -> 128: 204, 170; 160 x 160, 32 -> 32:
-// 158, 122; 320 x 320, 16 -> 32: 420, 370.
+// round. 32 images, us, im2col tiles and here: 80 x 80, 64 -> 64: 88, 61; 128 -> 128: 224, 184; 160 x 160, 32 -> 32:
+// 164, 123; 320 x 320, 16 -> 32: 419, 388.
 //
 // Structure: persistent CTAs, warp 0 filter producer, warp 1 MMA issuer and TMEM owner, warps 2..9 epilogue,
 // warps 10..17 converters (fp32 patch -> planes), bounded waits.

@@ -220,7 +220,6 @@ bool conv_umma_supported(
 // geom: 0 = WIDE (src NHWC with ic % 16 == 0, filter [OC][KH][KW][IC]). Where the channels are no whole
 //           number of a stage's rows, the load fills the rest of the last row with zeros: a
 //           704 x 5920 x 7328 product takes 27 us that way, 12577 on one CUDA thread per output;
-
 //       1 = TAP16 (src NHWC with exactly 16 channels, stride 1, filter [OC][taps][16] with the
 //           tap count a multiple of 4; `a` then describes that transformed convolution, with
 //           a.ph/a.pw the LOW padding and a.oh/a.ow the output extent)

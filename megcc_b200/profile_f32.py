@@ -1,11 +1,13 @@
-"""Launches the fp32 (split-tf32) tensor-core kernels on small cases: one YOLOX-style ConvBias
+"""Launches the fp32 tensor-core kernels on small cases: one YOLOX-style ConvBias
 (128 -> 128 channels, 3x3, 80 x 80, SiLU; the batch is the first argument) and the fp32
 MatrixMul at 2048^3; once each, then ten times each between two events.
 
 Meant to be run under a profiler, capturing the first launch of the kernel:
 
     ncu --section SpeedOfLight --section MemoryWorkloadAnalysis --clock-control none \
-        -k regex:conv_f32_umma -c 1 python -m megcc_b200.profile_f32 8 conv
+        -k regex:conv_f32_patch -c 1 python -m megcc_b200.profile_f32 8 conv
+
+MB200_F32_PATCH=0 and MB200_F32_HALF=0 leave the case to the kernels on fp16 planes and on tf32 planes.
 """
 import sys
 
